@@ -91,7 +91,6 @@ HDB_API hdb_status hdb_fix_distances(hdb_ctx *h, const float *X, int64_t n, int3
     require_ptr(dist, "dist");
     HDB_REQUIRE(n >= 0 && k >= 1 && d >= 1, HDB_ERR_ARG, "bad n, k or d");
     fix_distances(ctx, X, n, d, ids, k, dist);
-    ctx->sync();
   });
 }
 

@@ -353,7 +353,10 @@ __global__ void __launch_bounds__(32 * kCoreWarps)
     const int64_t row = r0 + lane;
     const bool active = row < n;
     const uint32_t act = __ballot_sync(0xffffffffu, active);
-    const int32_t v = active ? ids[row * k + col] : 0;
+    // the ids of a caller's graph are checked later (k_degrees): one outside
+    // [0, n) stands for the row itself here, so that no gather leaves X
+    int32_t v = active ? ids[row * k + col] : 0;
+    if (active && (v < 0 || v >= n)) v = (int32_t)row;
     float soma = 0.0f;
     for (int c0 = 0; c0 < d; c0 += kCoreCols) {
       const int wd = min(kCoreCols, d - c0);
