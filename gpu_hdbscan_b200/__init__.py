@@ -69,8 +69,10 @@ class Context:
         h = C.c_void_p()
         _lib.check(self.L.hdb_create(C.byref(h), device))
         self.h = h
-        # run on torch's current stream so torch allocations order correctly
-        _lib.check(self.L.hdb_set_stream(self.h, C.c_void_p(torch.cuda.current_stream(self.device).cuda_stream)))
+        # run on torch's current stream so torch allocations order correctly (the default
+        # stream's handle is 0, for which the context keeps its own stream: see _call)
+        self._stream = torch.cuda.current_stream(self.device).cuda_stream
+        _lib.check(self.L.hdb_set_stream(self.h, C.c_void_p(self._stream)))
 
     def set_join_tiles(self, tiles: int):
         """FP32 local join form: 1 or 2 distance tiles of 4 x 4 per lane, or 0
@@ -89,6 +91,15 @@ class Context:
             pass
 
     # -- helpers ----------------------------------------------------------
+    def _call(self, fn, *args):
+        """fn(context, *args) -> its status.  The arguments may still be in the making on
+        torch's current stream (an input's kernels, a conversion by _dev); unless that is the
+        stream the context works on, the call first waits for them."""
+        now = self._torch.cuda.current_stream(self.device)
+        if now.cuda_stream != self._stream or self._stream == 0:
+            now.synchronize()
+        return fn(self.h, *args)
+
     def _dev(self, t, dtype):
         torch = self._torch
         t = torch.as_tensor(t)
@@ -102,7 +113,7 @@ class Context:
         n, d = X.shape
         G = torch.empty((n, k, 2), dtype=torch.int32, device=self.device)
         p = _lib.KnnParams(k, sample_num, iterations, precision)
-        _lib.check(self.L.hdb_nndescent(self.h, _ptr(X), n, d, C.byref(p), _ptr(G)))
+        _lib.check(self._call(self.L.hdb_nndescent, _ptr(X), n, d, C.byref(p), _ptr(G)))
         return G
 
     def KNNMerge(self, X1, G1, X2, G2, sample_num=12, iterations=11):
@@ -123,7 +134,7 @@ class Context:
             raise ValueError("KNNMerge: X1/X2 need the same d and G1/G2 the same k, one row per point")
         G = torch.empty((n1 + n2, k, 2), dtype=torch.int32, device=self.device)
         p = _lib.KnnParams(k, sample_num, iterations, HDB_PREC_FP32)
-        _lib.check(self.L.hdb_knn_merge(self.h, _ptr(X1), n1, _ptr(G1), _ptr(X2), n2, _ptr(G2), d,
+        _lib.check(self._call(self.L.hdb_knn_merge, _ptr(X1), n1, _ptr(G1), _ptr(X2), n2, _ptr(G2), d,
                                         C.byref(p), _ptr(G)))
         return G
 
@@ -133,7 +144,7 @@ class Context:
         n, k, _ = G.shape
         ids = torch.empty((n, k), dtype=torch.int32, device=self.device)
         dist = torch.empty((n, k), dtype=torch.float32, device=self.device)
-        _lib.check(self.L.hdb_knn_split(self.h, _ptr(G), n, k, _ptr(ids), _ptr(dist)))
+        _lib.check(self._call(self.L.hdb_knn_split, _ptr(G), n, k, _ptr(ids), _ptr(dist)))
         return ids, dist
 
     def fix_distances(self, X, ids):
@@ -142,7 +153,7 @@ class Context:
         ids = self._dev(ids, torch.int32)
         n, k = ids.shape
         dist = torch.empty((n, k), dtype=torch.float32, device=self.device)
-        _lib.check(self.L.hdb_fix_distances(self.h, _ptr(X), n, X.shape[1], _ptr(ids), k,
+        _lib.check(self._call(self.L.hdb_fix_distances, _ptr(X), n, X.shape[1], _ptr(ids), k,
                                             _ptr(dist)))
         return dist
 
@@ -156,7 +167,7 @@ class Context:
         counts = self._dev(counts, torch.int32)
         tiles = ids.shape[0]
         out = torch.empty((tiles, 128, 64), dtype=torch.float32, device=self.device)
-        _lib.check(self.L.hdb_bf16_distance_tiles(self.h, _ptr(X), X.shape[0], X.shape[1],
+        _lib.check(self._call(self.L.hdb_bf16_distance_tiles, _ptr(X), X.shape[0], X.shape[1],
                                                   _ptr(ids), _ptr(counts), tiles, _ptr(out)))
         return out
 
@@ -172,7 +183,7 @@ class Context:
         mst = self._dev(mst, torch.int32)
         n, k = ids.shape
         g = _lib.Graph()
-        _lib.check(self.L.hdb_core_sg(self.h, _ptr(ids), _ptr(dist), _ptr(X), n, X.shape[1], k,
+        _lib.check(self._call(self.L.hdb_core_sg, _ptr(ids), _ptr(dist), _ptr(X), n, X.shape[1], k,
                                       _ptr(mst), C.byref(g)))
         empty = torch.empty(0, dtype=torch.int32, device=self.device)
         return EnhancedGraph(g.nodes, g.edges, self._view(g.nindex, g.nodes + 1, torch.int64),
@@ -186,7 +197,7 @@ class Context:
         X = self._dev(X, torch.float32)
         n, k = ids.shape
         g = _lib.Graph()
-        _lib.check(self.L.hdb_enhanced_knng(self.h, _ptr(ids), _ptr(dist), _ptr(X), n,
+        _lib.check(self._call(self.L.hdb_enhanced_knng, _ptr(ids), _ptr(dist), _ptr(X), n,
                                             X.shape[1], k, C.byref(g)))
         return EnhancedGraph(g.nodes, g.edges, self._view(g.nindex, g.nodes + 1, torch.int64),
                              self._view(g.nlist, g.edges, torch.int32),
@@ -231,10 +242,10 @@ class Context:
         inm = torch.empty(graph.edges, dtype=torch.uint8, device=self.device) if with_in_mst else None
         rounds = C.c_int32(0)
         if order is None:
-            _lib.check(self.L.hdb_mst(self.h, C.byref(graph.raw), _ptr(inm), _ptr(mst),
+            _lib.check(self._call(self.L.hdb_mst, C.byref(graph.raw), _ptr(inm), _ptr(mst),
                                       C.byref(rounds)))
         else:
-            _lib.check(self.L.hdb_mst_ordered(self.h, C.byref(graph.raw), order, _ptr(inm),
+            _lib.check(self._call(self.L.hdb_mst_ordered, C.byref(graph.raw), order, _ptr(inm),
                                               _ptr(mst), C.byref(rounds)))
         return mst, inm, rounds.value
 
@@ -249,19 +260,19 @@ class Context:
         mst = torch.empty((n - 1, 3), dtype=torch.int32, device=self.device)
         inm = torch.empty(graph.edges, dtype=torch.uint8, device=self.device) if with_in_mst else None
         rounds, mult = C.c_int32(0), C.c_int32(0)
-        _lib.check(self.L.hdb_mst_quantised(self.h, C.byref(graph.raw), _ptr(dist), dist.shape[1],
+        _lib.check(self._call(self.L.hdb_mst_quantised, C.byref(graph.raw), _ptr(dist), dist.shape[1],
                                             _ptr(inm), _ptr(mst), C.byref(mult), C.byref(rounds)))
         return mst, inm, mult.value, rounds.value
 
     def sort_edges(self, mst):
         """In place: stable ascending sort of MSTedge rows by weight."""
-        _lib.check(self.L.hdb_sort_edges(self.h, _ptr(mst), mst.shape[0]))
+        _lib.check(self._call(self.L.hdb_sort_edges, _ptr(mst), mst.shape[0]))
         return mst
 
     def build_Linkage_tree(self, mst, n):
         torch = self._torch
         hier = torch.empty((n - 1, 4), dtype=torch.int32, device=self.device)
-        _lib.check(self.L.hdb_linkage_tree(self.h, _ptr(mst), n, _ptr(hier)))
+        _lib.check(self._call(self.L.hdb_linkage_tree, _ptr(mst), n, _ptr(hier)))
         return hier
 
     def get_clusters(self, hier, n, mpts, stability=HDB_STAB_FP32, want_tree=False):
@@ -277,7 +288,7 @@ class Context:
             cap = n + 2 * (n // max(mpts, 1)) + 2
             cond = torch.empty((cap, 4), dtype=torch.int32, device=self.device)
             stab = torch.empty((cap, 2), dtype=torch.int32, device=self.device)
-        _lib.check(self.L.hdb_condense_select(self.h, _ptr(hier), n, mpts, stability, _ptr(labels),
+        _lib.check(self._call(self.L.hdb_condense_select, _ptr(hier), n, mpts, stability, _ptr(labels),
                                               C.byref(ncl), _ptr(cond), C.byref(csize), _ptr(stab),
                                               C.byref(nst)))
         if want_tree:
@@ -309,10 +320,10 @@ class Context:
         st = _lib.RunStats()
         if want_graph:
             G = torch.empty((n, k, 2), dtype=torch.int32, device=dev)
-            _lib.check(self.L.hdb_run_with_graph(self.h, _ptr(X), n, d, C.byref(p), _ptr(labels),
+            _lib.check(self._call(self.L.hdb_run_with_graph, _ptr(X), n, d, C.byref(p), _ptr(labels),
                                                  _ptr(G), C.byref(st)))
             return labels, {f: getattr(st, f) for f, _ in _lib.RunStats._fields_}, G
-        _lib.check(self.L.hdb_run(self.h, _ptr(X), n, d, C.byref(p), _ptr(labels), C.byref(st)))
+        _lib.check(self._call(self.L.hdb_run, _ptr(X), n, d, C.byref(p), _ptr(labels), C.byref(st)))
         return labels, {f: getattr(st, f) for f, _ in _lib.RunStats._fields_}
 
     def hdbscan_batched(self, Xs, k=32, mpts=32, sample_num=16, iterations=6,
@@ -372,7 +383,7 @@ class Context:
             rec["G"] = np.fromiter((G_.data_ptr() for G_ in graphs), dtype=np.uint64, count=T)
         insts = (_lib.Instance * T).from_buffer(rec)
         st = _lib.RunStats()
-        rc = fn(self.h, insts, T, C.byref(p), C.byref(st))
+        rc = self._call(fn, insts, T, C.byref(p), C.byref(st))
         if rc != _lib.HDB_OK and (strict or rc != _lib.HDB_ERR_DISCONNECTED):
             _lib.check(rc)
         stats = {f: getattr(st, f) for f, _ in _lib.RunStats._fields_}
@@ -401,7 +412,7 @@ class Context:
         p = _lib.Params(_lib.KnnParams(k, max(1, k // 2), 0, HDB_PREC_FP32), mpts, distance,
                         stability, 1 if host else 0, mst_gpu)
         st = _lib.RunStats()
-        _lib.check(self.L.hdb_run_knn(self.h, _ptr(G), _ptr(X), n, d, C.byref(p), _ptr(labels),
+        _lib.check(self._call(self.L.hdb_run_knn, _ptr(G), _ptr(X), n, d, C.byref(p), _ptr(labels),
                                       C.byref(st)))
         return labels, {f: getattr(st, f) for f, _ in _lib.RunStats._fields_}
 
