@@ -175,10 +175,14 @@ void radix_sort_u32(Context *ctx, uint32_t *keys, uint32_t *values, int64_t n, i
                     int end_bit);
 void radix_sort_u64(Context *ctx, uint64_t *keys, uint32_t *values, int64_t n, int begin_bit,
                     int end_bit);
-// The same with u64 values and digits of up to 9 bits (fewer passes for key
-// ranges just above a multiple of 8 bits, e.g. 25-bit row ids: 3 passes).
-void radix_sort_u32_u64(Context *ctx, uint32_t *keys, uint64_t *values, int64_t n, int begin_bit,
-                        int end_bit);
+// Groups the (key, value) pairs of a list by bits [begin_bit, end_bit) of their
+// keys, in digits of up to 9 bits, stably.  The list's length is on the device
+// (count); cap (< 2^32) bounds it.  The second buffers hold cap entries too;
+// returns whether the result is in them.  base (513 values) receives the last
+// pass's digit starts and total: with a single pass, the groups' starts.
+bool radix_group_u32_u64(Context *ctx, uint32_t *keys, uint64_t *values, uint32_t *keys2,
+                         uint64_t *values2, int64_t cap, const unsigned long long *count,
+                         int begin_bit, int end_bit, uint32_t *base);
 
 void radix_sort_u32_buffers(cudaStream_t st, uint32_t *keys, uint32_t *vals, uint32_t *ktmp,
                             uint32_t *vtmp, uint32_t *counts, uint32_t *offs, uint32_t *scan_sums,

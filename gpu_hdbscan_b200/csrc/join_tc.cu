@@ -108,7 +108,7 @@ struct JoinArgs {
   const int8_t *nf, *of;
   int32_t *nrev, *orev;
   const float *worst;
-  Inbox ib;
+  CandList cl;
   // probe mode
   const int32_t *probe_ids, *probe_counts;
   float *probe_out;
@@ -701,10 +701,10 @@ __device__ void epilogue(const JoinArgs &a, Shared &sh, uint32_t tmem, int64_t n
     const float d1 = __uint_as_float(k1 & ~63u), d2 = __uint_as_float(k2 & ~63u);
     const bool c1 = vrow && id1 >= 0 && d1 < wst;
     const bool c2 = !isnew && lane < nn && id2 >= 0 && d2 < wst2;
-    cands += append_candidates(a.ib, cur, (uint32_t)n, c1, myid, pack(d1, id1), c2, tgt2,
+    cands += append_candidates(a.cl, cur, c1, myid, pack(d1, id1), c2, tgt2,
                                pack(d2, id2));
   }
-  if (!kProbe) list_fill(a.ib, cur.pos, cur.end, (uint32_t)n);  // the rest of the last chunk
+  if (!kProbe) list_fill(a.cl, cur.pos, cur.end);  // the rest of the last chunk
 }
 
 template <bool kProbe>
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   unsigned long long stat = 0;
   if (warp >= kProducerWarp0 && warp < kMmaWarp) {
     producer<kProbe>(warp - kProducerWarp0, &xmap, a, sh, tiles, n, ntiles, kbc, S, stat);
-    if (!kProbe && lane_id() == 0 && stat) atomicAdd(&a.ib.counters[1], stat);
+    if (!kProbe && lane_id() == 0 && stat) atomicAdd(&a.cl.counters[1], stat);
   } else if (warp == kMmaWarp) {
     if (lane_id() == 0) mma_issuer(sh, tiles, tmem, ntiles, kbc, a.idesc, a.err);
     __syncwarp();
@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (!kProbe) {
 #pragma unroll
       for (int o = 16; o; o >>= 1) stat += __shfl_xor_sync(0xffffffffu, stat, o);
-      if (lane_id() == 0 && stat) atomicAdd(&a.ib.counters[2], stat);
+      if (lane_id() == 0 && stat) atomicAdd(&a.cl.counters[2], stat);
     }
   }
   tc_fence_before();
@@ -855,7 +855,7 @@ void tc_join_prepare(Context *ctx, const uint16_t *Xb, int64_t n, int dpad, bool
 
 void tc_join_launch(Context *ctx, const TcJoin &tj, int S, const float *nrm, const int32_t *newS,
                     const int32_t *oldS, const int8_t *nf, const int8_t *of, int32_t *nrev,
-                    int32_t *orev, const float *worst, const Inbox &ib) {
+                    int32_t *orev, const float *worst, const CandList &cl) {
   HDB_REQUIRE(S >= 1 && 2 * S <= 32, HDB_ERR_ARG, "tensor-core join: need 2 * SAMPLE_NUM <= 32");
   k_join_lists<<<grid_for(ctx, tj.n, 8, 8), 256, 0, ctx->stream>>>(
       tj.n, S, const_cast<int32_t *>(newS), const_cast<int32_t *>(oldS),
@@ -863,7 +863,7 @@ void tc_join_launch(Context *ctx, const TcJoin &tj, int S, const float *nrm, con
   ctx->launches++;
   HDB_CHECK_LAUNCH();
   JoinArgs a{nrm,     newS,    oldS,    nf,           of,       nrev,     orev,
-             worst,   ib,      nullptr, nullptr,      nullptr,  ctx->dev_err, tj.idesc,
+             worst,   cl,      nullptr, nullptr,      nullptr,  ctx->dev_err, tj.idesc,
              tj.dscale};
   launch<false>(ctx, tj, (tj.n + 1) / 2, S, a);
 }
@@ -873,7 +873,7 @@ void tc_gram_probe(Context *ctx, const uint16_t *Xb, const float *nrm, int64_t n
   TcJoin tj;
   tc_join_prepare(ctx, Xb, n, dpad, false, -2.0f, &tj);
   JoinArgs a{nrm,     nullptr, nullptr, nullptr, nullptr, nullptr,      nullptr,
-             nullptr, Inbox{}, ids,     counts,  out,     ctx->dev_err, tj.idesc,
+             nullptr, CandList{}, ids,     counts,  out,     ctx->dev_err, tj.idesc,
              tj.dscale};
   launch<true>(ctx, tj, tiles, 1, a);
 }

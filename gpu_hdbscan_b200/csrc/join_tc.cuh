@@ -37,12 +37,11 @@ struct TcJoin {
 void tc_join_prepare(Context *ctx, const uint16_t *Xh, int64_t n, int dpad, bool fp16,
                      float dscale, TcJoin *tj);
 
-// One local-join pass over all rows: the sample lists of k_sample in, the
-// candidates out through the inbox's overflow list only (ib.ovf_cap must hold
-// a pass's candidates; sort_overflow groups them by target for the merge).
+// One local-join pass over all rows: the sample lists in, the candidates
+// appended to the list cl.
 void tc_join_launch(Context *ctx, const TcJoin &tj, int S, const float *nrm, const int32_t *newS,
                     const int32_t *oldS, const int8_t *nf, const int8_t *of, int32_t *nrev,
-                    int32_t *orev, const float *worst, const knn::Inbox &ib);
+                    int32_t *orev, const float *worst, const knn::CandList &cl);
 
 // Distance tiles for explicit slot lists (testing the gather / MMA / TMEM
 // path): ids [tiles * 128], counts [tiles * 4] = (new0, old0, new1, old1),

@@ -6,11 +6,11 @@
 // its closest old neighbour and every old neighbour its closest new one --
 // laid out for one B200:
 //  * no per-row spin locks (InsertToGlobalGraph, nndescent.cu:969-1028): the
-//    join appends candidates to a fixed per-row inbox (one atomicAdd each,
-//    pre-filtered against the row's current k-th distance), and the next
-//    pass merges each row's inbox in one warp (sort, de-duplicate, merge);
+//    joins append their candidates (pre-filtered against the target row's
+//    current k-th distance) to one list, which is grouped by target row, and
+//    the next pass merges each row's part, one warp per row;
 //  * the three sampling kernels, MarkAllToOld and the merge are one kernel
-//    (k_sample), so an iteration is two launches;
+//    (k_sample);
 //  * distances are the reference's sequential FP32 difference sum
 //    (nndescent.cu:1086-1093, fmaf per element), so every pair has one exact
 //    value wherever it is computed.
@@ -490,36 +490,73 @@ __device__ __forceinline__ void merge_batch(int k, uint64_t &rkey, int32_t &lab,
   }
 }
 
-// Merge of everything offered to a row (inbox, best dropped, the row's
-// segment of the sorted candidate list) into its sorted list (one warp), in
-// batches of 64.  On return, lane j (< k) holds the j-th entry of the merged
-// row.  The list forms keep no inboxes (ib.inboxes = 0).
-__device__ __forceinline__ void merge_row(int64_t row, int k, int32_t &lab, float &dist,
-                                          const Inbox &ib, MergeSmem &ms) {
+// Sample (PrepareGraph :44-98 and reverse samples PrepareReverseGraph :293-346)
+// and MarkAllToOld (:1398) of one row held one entry per lane.  split > 0 is
+// the merge of two point sets [0, split) and [split, n) (PrepareGraphForMerge
+// :100-166): old entries are sampled only from the row's own set; new entries
+// and reverse samples are not filtered.
+struct SampleOut {
+  int32_t *newS, *oldS;  // [n][2S]: forward slots 0..S-1, reverse slots S..2S-1
+  int8_t *nf, *of;       // [n] forward samples
+  int32_t *nrev, *orev;  // [n] reverse samples offered
+};
+// The candidate list grouped by row.
+struct RowList {
+  const uint32_t *start;     // [n + 1]
+  const uint64_t *key;
+  unsigned long long *best;  // [n] the best candidate of each row that found no room in the list
+};
+
+__device__ __forceinline__ void sample_row(int64_t row, int k, int S, int64_t split, int32_t lab,
+                                           float dist, int32_t *__restrict__ gid,
+                                           float *__restrict__ gdist, float *__restrict__ worst,
+                                           const SampleOut &so) {
   const int lane = lane_id();
-  int cnt = ib.inboxes ? ib.cnt[row] : 0;
-  const uint64_t ov = ib.best[row];  // the best candidate that found no room (normally none)
-  const uint32_t o0 = ib.ostart[row], o1 = ib.oend[row];
-  if (cnt == 0 && ov == ~0ull && o0 == o1) return;
-  __syncwarp();
-  if (lane == 0) {
-    if (cnt != 0) ib.cnt[row] = 0;
-    if (ov != ~0ull) ib.best[row] = ~0ull;
-    if (o0 != o1) { ib.ostart[row] = 0; ib.oend[row] = 0; }
+  const bool have = lane < k;
+  const int32_t id = decode(lab);
+  const bool isnew = have && lab >= 0;
+  const bool isold = have && lab < 0 && (split <= 0 || ((row < split) == (id < split)));
+  const uint32_t nm = __ballot_sync(0xffffffffu, isnew), om = __ballot_sync(0xffffffffu, isold);
+  const int rn = __popc(nm & lanemask_lt()), ro = __popc(om & lanemask_lt());
+  const int64_t sb = row * (2 * S);
+  if (isnew && rn < S) {
+    so.newS[sb + rn] = id;
+    const int p = atomicAdd(&so.nrev[id], 1);
+    if (p < S) so.newS[(int64_t)id * (2 * S) + S + p] = (int32_t)row;
   }
-  if (cnt > kInboxCap) cnt = kInboxCap;
+  if (isold && ro < S) {
+    so.oldS[sb + ro] = id;
+    const int p = atomicAdd(&so.orev[id], 1);
+    if (p < S) so.oldS[(int64_t)id * (2 * S) + S + p] = (int32_t)row;
+  }
+  if (lane == 0) {
+    so.nf[row] = (int8_t)min(__popc(nm), S);
+    so.of[row] = (int8_t)min(__popc(om), S);
+  }
+  if (have) {
+    gid[row * k + lane] = isnew ? -id - 1 : lab;  // MarkAllToOld
+    gdist[row * k + lane] = dist;
+  }
+  const float w = __shfl_sync(0xffffffffu, dist, k - 1);
+  if (lane == 0) worst[row] = w;
+}
+
+// Merge of a row's part of the candidate list, and of the best candidate that
+// found no room in it (normally none), into its sorted list (one warp), in
+// batches of 64.  On return, lane j (< k) holds the j-th entry of the merged row.
+__device__ __forceinline__ void merge_row(int64_t row, int k, int32_t &lab, float &dist,
+                                          const RowList &rl, MergeSmem &ms) {
+  const int lane = lane_id();
+  const uint64_t ov = rl.best[row];
+  const uint32_t o0 = rl.start[row], o1 = rl.start[row + 1];
+  if (ov == ~0ull && o0 == o1) return;
+  __syncwarp();
+  if (lane == 0 && ov != ~0ull) rl.best[row] = ~0ull;
   const bool have = lane < k;
   uint64_t rkey = have ? pack(dist, decode(lab)) : ~0ull;
-  // candidate i of the row: inbox slots, then the best dropped, then the
-  // segment of the sorted list
-  const uint64_t *inbox = ib.slots + row * kInboxCap;
   const int64_t nov = ov != ~0ull ? 1 : 0;
-  const int64_t m = (int64_t)cnt + nov + (int64_t)(o1 - o0);
-  auto at = [&](int64_t i) -> uint64_t {
-    if (i < cnt) return inbox[i];
-    if (i < cnt + nov) return ov;
-    return ib.ovf_key[o0 + (i - cnt - nov)];
-  };
+  const int64_t m = nov + (int64_t)(o1 - o0);
+  auto at = [&](int64_t i) -> uint64_t { return i < nov ? ov : rl.key[o0 + (i - nov)]; };
   for (int64_t base = 0; base < m; base += 64) {
     const uint64_t c0 = base + lane < m ? at(base + lane) : ~0ull;
     const uint64_t c1 = base + 32 + lane < m ? at(base + 32 + lane) : ~0ull;
@@ -528,58 +565,35 @@ __device__ __forceinline__ void merge_row(int64_t row, int k, int32_t &lab, floa
   if (have) dist = pk_dist(rkey);
 }
 
-// Merge (iterations >= 1), sample (PrepareGraph :44-98 and reverse samples
-// PrepareReverseGraph :293-346) and MarkAllToOld (:1398), one warp per row.
-// split > 0 is the merge of two point sets [0, split) and [split, n)
-// (PrepareGraphForMerge :100-166): old entries are sampled only from the
-// row's own set; new entries and reverse samples are not filtered.
+// Merge (iterations >= 1), sample and MarkAllToOld, one warp per row.  The order
+// in which rows arrive decides whose reverse samples are taken (a row keeps the
+// first S).  It follows the blocks that are resident together -- the grid's
+// first five per SM walk through all their rows before the others start -- so
+// unused shared memory (kSampleRoom) keeps it at five blocks whatever the
+// compiler makes of the registers: another order gives graphs as good, but
+// other ones.
+constexpr size_t kSampleRoom = 28 * 1024;
 __global__ void k_sample(int64_t n, int k, int S, int do_merge, int32_t *__restrict__ gid,
-                         float *__restrict__ gdist, float *__restrict__ worst, Inbox ib,
-                         int32_t *__restrict__ newS,
-                         int32_t *__restrict__ oldS, int8_t *__restrict__ nf, int8_t *__restrict__ of,
-                         int32_t *__restrict__ nrev, int32_t *__restrict__ orev, int64_t split) {
+                         float *__restrict__ gdist, float *__restrict__ worst, RowList rl,
+                         unsigned long long *counters, SampleOut so, int64_t split) {
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
   __shared__ MergeSmem merge_smem[8];  // per-warp merge scratch (8 warps per block)
   MergeSmem &ms = merge_smem[threadIdx.x >> 5];
+  if (blockIdx.x == 0 && threadIdx.x == 0) counters[3] = 0;  // the next join's list is empty
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
     const bool have = lane < k;
     int32_t lab = have ? gid[row * k + lane] : 0;
     float dist = have ? gdist[row * k + lane] : 0.0f;
-    if (do_merge) merge_row(row, k, lab, dist, ib, ms);
-    const int32_t id = decode(lab);
-    const bool isnew = have && lab >= 0;
-    const bool isold = have && lab < 0 && (split <= 0 || ((row < split) == (id < split)));
-    uint32_t nm = __ballot_sync(0xffffffffu, isnew), om = __ballot_sync(0xffffffffu, isold);
-    int rn = __popc(nm & lanemask_lt()), ro = __popc(om & lanemask_lt());
-    const int64_t sb = row * (2 * S);
-    if (isnew && rn < S) {
-      newS[sb + rn] = id;
-      int p = atomicAdd(&nrev[id], 1);
-      if (p < S) newS[(int64_t)id * (2 * S) + S + p] = (int32_t)row;
-    }
-    if (isold && ro < S) {
-      oldS[sb + ro] = id;
-      int p = atomicAdd(&orev[id], 1);
-      if (p < S) oldS[(int64_t)id * (2 * S) + S + p] = (int32_t)row;
-    }
-    if (lane == 0) {
-      nf[row] = (int8_t)min(__popc(nm), S);
-      of[row] = (int8_t)min(__popc(om), S);
-    }
-    if (have) {
-      gid[row * k + lane] = isnew ? -id - 1 : lab;  // MarkAllToOld
-      gdist[row * k + lane] = dist;
-    }
-    float w = __shfl_sync(0xffffffffu, dist, k - 1);
-    if (lane == 0) worst[row] = w;
+    if (do_merge) merge_row(row, k, lab, dist, rl, ms);
+    sample_row(row, k, S, split, lab, dist, gid, gdist, worst, so);
   }
 }
 
 // Final merge after the last join; writes NNDElement rows with their flags.
 __global__ void k_finalize(int64_t n, int k, const int32_t *__restrict__ gid,
-                           const float *__restrict__ gdist, Inbox ib,
+                           const float *__restrict__ gdist, RowList rl,
                            hdb_nnd_element *__restrict__ out) {
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
@@ -587,15 +601,82 @@ __global__ void k_finalize(int64_t n, int k, const int32_t *__restrict__ gid,
   MergeSmem &ms = merge_smem[threadIdx.x >> 5];
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
-    const bool have = lane < k;
-    int32_t lab = have ? gid[row * k + lane] : 0;
-    float dist = have ? gdist[row * k + lane] : 0.0f;
-    merge_row(row, k, lab, dist, ib, ms);
-    if (have) {
-      hdb_nnd_element e;
-      e.distance_ = dist;
-      e.label_ = lab;
-      out[row * k + lane] = e;
+    int32_t lab = lane < k ? gid[row * k + lane] : 0;
+    float dist = lane < k ? gdist[row * k + lane] : 0.0f;
+    merge_row(row, k, lab, dist, rl, ms);
+    if (lane < k) out[row * k + lane] = hdb_nnd_element{dist, lab};
+  }
+}
+
+// The candidate list grouped by bucket of 2^shift consecutive rows (bstart)
+// -> grouped by row: one block per bucket counts its rows' candidates in shared
+// memory, scans the counts (the rows' starts) and moves the keys to their
+// rows.  A bucket's part is some 50 KB, so its scattered 8-byte stores meet in
+// L2.  In place of a further pass of the radix sort and of the search for the
+// rows' bounds in the sorted targets.
+constexpr int kBucketRows = 256;    // most rows of a bucket
+constexpr int kGroupThreads = 512;
+__global__ void __launch_bounds__(kGroupThreads)
+    k_group_rows(int64_t n, int shift, const uint32_t *__restrict__ tgt,
+                 const uint64_t *__restrict__ key, const uint32_t *__restrict__ bstart,
+                 uint32_t *__restrict__ start, uint64_t *__restrict__ out) {
+  __shared__ uint32_t cnt[kBucketRows];
+  __shared__ uint32_t wsum[kBucketRows / 32];
+  const int lane = lane_id(), w = threadIdx.x >> 5, tid = threadIdx.x;
+  const uint32_t row0 = (uint32_t)((int64_t)blockIdx.x << shift);
+  const int rows = (int)min((int64_t)1 << shift, n - (int64_t)row0);
+  const uint32_t b0 = bstart[blockIdx.x], b1 = bstart[blockIdx.x + 1];  // the unused slots lie behind
+  if (tid < kBucketRows) cnt[tid] = 0;
+  __syncthreads();
+#pragma unroll 4
+  for (uint32_t i = b0 + tid; i < b1; i += kGroupThreads) atomicAdd(&cnt[tgt[i] - row0], 1u);
+  __syncthreads();
+  const uint32_t c = tid < kBucketRows ? cnt[tid] : 0;
+  uint32_t x = c;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31 && w < kBucketRows / 32) wsum[w] = x;
+  __syncthreads();
+  uint32_t at = b0 + x - c;
+  if (tid < kBucketRows) {
+    for (int v = 0; v < w; v++) at += wsum[v];
+    cnt[tid] = at;
+  }
+  if (tid < rows) start[row0 + tid] = at;
+  if (tid == rows - 1 && (int64_t)row0 + rows == n) start[n] = at + c;
+  __syncthreads();
+#pragma unroll 4
+  for (uint32_t i = b0 + tid; i < b1; i += kGroupThreads)
+    out[atomicAdd(&cnt[tgt[i] - row0], 1u)] = key[i];
+}
+
+// Start of every bucket in the list grouped by bucket (tgt >> shift), and the
+// end of the last one: bstart[0..buckets].  Four targets per thread.
+__global__ void k_bucket_bounds(const uint32_t *__restrict__ tgt,
+                                const unsigned long long *__restrict__ count, int64_t cap, int shift,
+                                int64_t buckets, uint32_t *__restrict__ bstart) {
+  const int64_t c = min((int64_t)*count, cap);
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  if (c == 0) {
+    for (int64_t b = t0; b <= buckets; b += stride) bstart[b] = 0;
+    return;
+  }
+  for (int64_t i = 4 * t0; i < c; i += 4 * stride) {
+    const uint4 v = *reinterpret_cast<const uint4 *>(tgt + i);  // the buffer has room past its end
+    int64_t prev = i == 0 ? -1 : (int64_t)(tgt[i - 1] >> shift);
+    const uint32_t t[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      if (i + j >= c) break;
+      const int64_t b = min((int64_t)(t[j] >> shift), buckets);
+      for (int64_t q = prev + 1; q <= b; q++) bstart[q] = (uint32_t)(i + j);
+      prev = b > prev ? b : prev;
+      if (i + j == c - 1)
+        for (int64_t q = b + 1; q <= buckets; q++) bstart[q] = (uint32_t)c;
     }
   }
 }
@@ -703,7 +784,7 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
     k_join(const float *__restrict__ X, int64_t n, int d, int S, const int32_t *__restrict__ newS,
            const int32_t *__restrict__ oldS, const int8_t *__restrict__ nf,
            const int8_t *__restrict__ of, int32_t *__restrict__ nrev, int32_t *__restrict__ orev,
-           const float *__restrict__ worst, Inbox ib, int cross_only) {
+           const float *__restrict__ worst, CandList cl, int cross_only) {
   extern __shared__ __align__(16) unsigned char smem_join[];
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
@@ -855,8 +936,7 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
     }  // passes
     __syncwarp();
     // the candidates that can enter their target's list go to the candidate
-    // list, which is sorted by target before the merge (space reserved 1024
-    // slots at a time per warp; no returning atomic per candidate)
+    // list (space reserved a chunk at a time; no returning atomic per candidate)
     const int32_t x = lane < nn ? ids[lane] : 0;
     const uint64_t b1 = lane < nn ? best1[lane] : ~0ull, b2 = lane < nn ? best2[lane] : ~0ull;
     const float wx = lane < nn ? worst[x] : 0.0f;
@@ -865,18 +945,18 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
     const float wx3 = lane < no ? worst[x3] : 0.0f;
     const bool v1 = b1 != ~0ull && pk_dist(b1) < wx, v2 = b2 != ~0ull && pk_dist(b2) < wx;
     const bool v3 = b3 != ~0ull && pk_dist(b3) < wx3;
-    w_cands += append_candidates(ib, cur, (uint32_t)n, v1, x, b1, v2, x, b2);
-    w_cands += append_candidates(ib, cur, (uint32_t)n, v3, x3, b3, false, 0, 0ull);
+    w_cands += append_candidates(cl, cur, v1, x, b1, v2, x, b2);
+    w_cands += append_candidates(cl, cur, v3, x3, b3, false, 0, 0ull);
     __syncwarp();
   }
-  list_fill(ib, cur.pos, cur.end, (uint32_t)n);  // the rest of the last chunk
+  list_fill(cl, cur.pos, cur.end);  // the rest of the last chunk
   // per-warp totals, one atomic each (no block-wide barrier)
 #pragma unroll
   for (int o = 16; o; o >>= 1) w_cands += __shfl_xor_sync(0xffffffffu, w_cands, o);
   if (lane == 0) {
-    if (w_rows) atomicAdd(&ib.counters[1], w_rows);
-    if (w_cands) atomicAdd(&ib.counters[2], w_cands);
-    if (w_pairs) atomicAdd(&ib.counters[4], w_pairs);
+    if (w_rows) atomicAdd(&cl.counters[1], w_rows);
+    if (w_cands) atomicAdd(&cl.counters[2], w_cands);
+    if (w_pairs) atomicAdd(&cl.counters[4], w_pairs);
   }
 }
 // ---------------------------------------------------------------------------
@@ -1006,7 +1086,7 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
                                                    const int8_t *__restrict__ of,
                                                    int32_t *__restrict__ nrev,
                                                    int32_t *__restrict__ orev,
-                                                   const float *__restrict__ worst, Inbox ib) {
+                                                   const float *__restrict__ worst, CandList cl) {
   extern __shared__ __align__(16) unsigned char smem_bf[];
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
@@ -1019,6 +1099,7 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
   const int ld = dpad + 8;  // row stride in elements (16-byte aligned, ldmatrix conflict free)
   const int chunks = dpad >> 3;  // 16-byte chunks per row
   unsigned long long w_rows = 0, w_cands = 0;
+  ListCursor cur;
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
     const int cnf = nf[row], cof = of[row];
@@ -1157,25 +1238,22 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
         if (lane < 4 && c < no) best3[c] = m;
       }
     __syncwarp();
-    int pushed = 0;
-    if (lane < nn) {
-      const int32_t x = ids[lane];
-      const uint64_t b1 = best1[lane], b2 = best2[lane];
-      if (b1 != ~0ull) pushed += push_candidate(x, pk_id(b1), pk_dist(b1), worst, ib);
-      if (b2 != ~0ull) pushed += push_candidate(x, pk_id(b2), pk_dist(b2), worst, ib);
-    }
-    if (lane < no) {
-      const uint64_t b3 = best3[lane];
-      if (b3 != ~0ull) pushed += push_candidate(ids[32 + lane], pk_id(b3), pk_dist(b3), worst, ib);
-    }
-    w_cands += pushed;
+    const int32_t x = lane < nn ? ids[lane] : 0, x3 = lane < no ? ids[32 + lane] : 0;
+    const uint64_t b1 = lane < nn ? best1[lane] : ~0ull, b2 = lane < nn ? best2[lane] : ~0ull;
+    const uint64_t b3 = lane < no ? best3[lane] : ~0ull;
+    const float wx = lane < nn ? worst[x] : 0.0f, wx3 = lane < no ? worst[x3] : 0.0f;
+    const bool v1 = b1 != ~0ull && pk_dist(b1) < wx, v2 = b2 != ~0ull && pk_dist(b2) < wx;
+    const bool v3 = b3 != ~0ull && pk_dist(b3) < wx3;
+    w_cands += append_candidates(cl, cur, v1, x, b1, v2, x, b2);
+    w_cands += append_candidates(cl, cur, v3, x3, b3, false, 0, 0ull);
     __syncwarp();
   }
+  list_fill(cl, cur.pos, cur.end);
 #pragma unroll
   for (int o = 16; o; o >>= 1) w_cands += __shfl_xor_sync(0xffffffffu, w_cands, o);
   if (lane == 0) {
-    if (w_rows) atomicAdd(&ib.counters[1], w_rows);
-    if (w_cands) atomicAdd(&ib.counters[2], w_cands);
+    if (w_rows) atomicAdd(&cl.counters[1], w_rows);
+    if (w_cands) atomicAdd(&cl.counters[2], w_cands);
   }
 }
 
@@ -1240,20 +1318,6 @@ __global__ void k_fix_distances(const float *__restrict__ X, int64_t n, int d,
       continue;
     }
     dist[i] = euclid_ref(X + row * d, X + (int64_t)v * d, d);
-  }
-}
-
-// Segment [ostart, oend) of every target row in the target-sorted overflow
-// list; sentinel entries (target n, the unused tail of a chunk) sort last and
-// are skipped.
-__global__ void k_ovf_bounds(const uint32_t *__restrict__ tgt, int64_t cnt, int64_t n,
-                             uint32_t *__restrict__ ostart, uint32_t *__restrict__ oend) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t t = tgt[i];
-    if (t >= n) continue;
-    if (i == 0 || tgt[i - 1] != t) ostart[t] = (uint32_t)i;
-    if (i == cnt - 1 || tgt[i + 1] != t) oend[t] = (uint32_t)(i + 1);
   }
 }
 
@@ -1402,25 +1466,6 @@ int bits_for_rows(int64_t n) {
 
 }  // namespace
 
-// Sorts the join's overflow list by target row and records each row's
-// segment for the next merge; resets the list.
-static void sort_overflow(Context *ctx, const Inbox &ib, int64_t n) {
-  cudaStream_t st = ctx->stream;
-  unsigned long long *h = reinterpret_cast<unsigned long long *>(ctx->pinned);
-  HDB_CUDA(cudaMemcpyAsync(h, ib.counters + 3, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-  ctx->sync();
-  int64_t c = (int64_t)h[0];
-  if (c == 0) return;
-  if (c > ib.ovf_cap) c = ib.ovf_cap;
-  // the packed candidates move with their targets, so the merge reads each
-  // row's segment contiguously
-  // n + 1 values: the rows and the sentinel n of unused chunk slots
-  radix_sort_u32_u64(ctx, ib.ovf_tgt, ib.ovf_key, c, 0, bits_for_rows(n + 1));
-  k_ovf_bounds<<<grid_for(ctx, c, 256), 256, 0, st>>>(ib.ovf_tgt, c, n, ib.ostart, ib.oend); ctx->launches++;
-  HDB_CHECK_LAUNCH();
-  HDB_CUDA(cudaMemsetAsync(ib.counters + 3, 0, sizeof(unsigned long long), st));
-}
-
 namespace {
 
 // Dynamic shared memory of the kernels that stage rows for difference sums
@@ -1431,20 +1476,35 @@ void stage_smem_attrs(size_t bytes) {
   HDB_CUDA(cudaFuncSetAttribute(k_rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
+// Rows per bucket of the candidate list's grouping, 2^shift: the fewest (from
+// 8) whose buckets, and the one of the unused slots behind them, fit one digit
+// of the radix passes (9 bits), so that one pass and k_group_rows group the list,
+// as long as that is at most kBucketRows; beyond, 128 rows, and two passes up to
+// 2^25 rows.  (Sorting the list by row took two and three passes.)
+int bucket_shift(int64_t n) {
+  int shift = 3;
+  while (ceil_div(n, int64_t(1) << shift) >= 512) shift++;
+  return (1 << shift) <= kBucketRows ? shift : 7;
+}
+
 // Device state of one NN-Descent run over n rows: the graph lists, the
-// samples of an iteration and the join's inboxes and candidate list.
-// list_only: the tensor-core join, which keeps no inboxes and appends a whole
-// iteration's candidates to the list.
+// samples of an iteration and the join's candidate list (with the second
+// buffer of its grouping).  warps: the most warps that append to the list.
 struct NndState {
-  Buf<int32_t> gid, newS, oldS, nrev, orev, inbox_cnt;
+  int64_t n;
+  int k, S, shift;
+  int64_t buckets;
+  Buf<int32_t> gid, newS, oldS, nrev, orev;
   Buf<float> gdist, worst;
   Buf<int8_t> nf, of;
-  Buf<uint64_t> inbox, ovf_key;
-  Buf<unsigned long long> ovf, dropped;
-  Buf<uint32_t> ovf_tgt, ostart, oend;
-  Inbox ib;
+  Buf<uint64_t> list_key, list_key2;
+  Buf<unsigned long long> best, counters;
+  Buf<uint32_t> list_tgt, list_tgt2, bstart, rstart;
+  CandList cl;
+  RowList rl;
 
-  NndState(Context *ctx, int64_t n, int k, int S, bool list_only) {
+  NndState(Context *ctx, int64_t n, int k, int S, int64_t warps)
+      : n(n), k(k), S(S), shift(bucket_shift(n)), buckets(ceil_div(n, int64_t(1) << shift)) {
     cudaStream_t st = ctx->stream;
     gid = Buf<int32_t>(ctx, n * k);
     gdist = Buf<float>(ctx, n * k);
@@ -1453,38 +1513,76 @@ struct NndState {
     oldS = Buf<int32_t>(ctx, n * 2 * S);
     nrev = Buf<int32_t>(ctx, n);
     orev = Buf<int32_t>(ctx, n);
-    inbox_cnt = Buf<int32_t>(ctx, n);
     nf = Buf<int8_t>(ctx, n);
     of = Buf<int8_t>(ctx, n);
-    inbox = Buf<uint64_t>(ctx, list_only ? 1 : (size_t)n * kInboxCap);
-    ovf = Buf<unsigned long long>(ctx, n);
-    dropped = Buf<unsigned long long>(ctx, 5);
-    // room for a pass's candidates; the joins' warps also leave the unused
-    // tail of their last list chunk (at most one chunk per warp: 8 epilogue
-    // warps per SM in the tensor-core join, up to 24 in the FP32 join)
-    const int64_t rows = list_only ? 64 : 16;
-    const int64_t cap = (n * rows > (1 << 22) ? n * rows : (1 << 22)) +
-                        (list_only ? (int64_t)24 * ctx->num_sms * kListChunk : 0);
-    ovf_tgt = Buf<uint32_t>(ctx, cap);
-    ovf_key = Buf<uint64_t>(ctx, cap);
-    ostart = Buf<uint32_t>(ctx, n);
-    oend = Buf<uint32_t>(ctx, n);
-    HDB_CUDA(cudaMemsetAsync(ostart, 0, n * 4, st));
-    HDB_CUDA(cudaMemsetAsync(oend, 0, n * 4, st));
-    ib = Inbox{inbox_cnt, inbox, ovf, ovf_tgt, ovf_key, ostart, oend, dropped, cap, list_only ? 0 : 1};
+    best = Buf<unsigned long long>(ctx, n);
+    counters = Buf<unsigned long long>(ctx, 5);
+    // room for an iteration's candidates (about 42 per row where it was
+    // counted; a row's join offers at most 96, so a small list cannot fill up)
+    // and for the tails of the warps' last chunks
+    const uint32_t chunk = list_chunk(40 * n / warps);
+    const int64_t cap =
+        std::min<int64_t>(std::max<int64_t>(64 * n, std::min<int64_t>(96 * n, int64_t(64) << 20)) +
+                              warps * chunk,
+                          (int64_t(1) << 32) - 1);
+    list_tgt = Buf<uint32_t>(ctx, cap);
+    list_key = Buf<uint64_t>(ctx, cap);
+    list_tgt2 = Buf<uint32_t>(ctx, cap);
+    list_key2 = Buf<uint64_t>(ctx, cap);
+    bstart = Buf<uint32_t>(ctx, std::max<int64_t>(513, buckets + 1));
+    rstart = Buf<uint32_t>(ctx, n + 1);
+    cl = CandList{best, list_tgt, list_key, counters, cap, chunk, (uint32_t)(buckets << shift)};
     HDB_CUDA(cudaMemsetAsync(nrev, 0, n * 4, st));
     HDB_CUDA(cudaMemsetAsync(orev, 0, n * 4, st));
-    clear_inboxes(ctx, n);
+    HDB_CUDA(cudaMemsetAsync(best, 0xff, n * 8, st));
+    clear_list(ctx);
   }
-  // the inbox state a join starts an iteration from: empty inboxes, no
-  // candidates in the list, nothing dropped
-  void clear_inboxes(Context *ctx, int64_t n) {
-    cudaStream_t st = ctx->stream;
-    HDB_CUDA(cudaMemsetAsync(inbox_cnt, 0, n * 4, st));
-    HDB_CUDA(cudaMemsetAsync(ovf, 0xff, n * 8, st));
-    HDB_CUDA(cudaMemsetAsync(dropped, 0, 5 * sizeof(unsigned long long), st));
+  void clear_list(Context *ctx) {
+    HDB_CUDA(cudaMemsetAsync(counters, 0, 5 * sizeof(unsigned long long), ctx->stream));
+  }
+  SampleOut samples() const { return SampleOut{newS, oldS, nf, of, nrev, orev}; }
+
+  // the samples of an iteration; after the first, of the rows merged with the
+  // candidates of the join before
+  void sample(Context *ctx, bool merge, int64_t split) {
+    k_sample<<<grid_for(ctx, n, 8, 16), 256, kSampleRoom, ctx->stream>>>(
+        n, k, S, merge, gid, gdist, worst, rl, counters, samples(), split);
+    ctx->launches++;
+    HDB_CHECK_LAUNCH();
+  }
+  void finalize(Context *ctx, hdb_nnd_element *out) {
+    k_finalize<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(n, k, gid, gdist, rl, out);
+    ctx->launches++;
+    HDB_CHECK_LAUNCH();
+  }
+  // groups a join's candidates by row
+  void group(Context *ctx) {
+    const int bits = bits_for_rows((int64_t)cl.none + 1);
+    const bool second = radix_group_u32_u64(ctx, list_tgt, list_key, list_tgt2, list_key2, cl.cap,
+                                            counters.get() + 3, shift, bits, bstart);
+    uint32_t *tgt = second ? list_tgt2 : list_tgt;
+    uint64_t *key = second ? list_key2 : list_key, *out = second ? list_key : list_key2;
+    if (bits - shift > 9) {  // several passes: the digit starts of the last one are not the buckets'
+      k_bucket_bounds<<<grid_for(ctx, ceil_div(cl.cap, 4), 256), 256, 0, ctx->stream>>>(
+          tgt, counters.get() + 3, cl.cap, shift, buckets, bstart);
+      ctx->launches++;
+      HDB_CHECK_LAUNCH();
+    }
+    k_group_rows<<<(unsigned)buckets, kGroupThreads, 0, ctx->stream>>>(n, shift, tgt, key, bstart, rstart,
+                                                                    out);
+    ctx->launches++;
+    HDB_CHECK_LAUNCH();
+    rl = RowList{rstart, out, best};
   }
 };
+
+// Warps of the joins that append to the list.
+int64_t fp32_join_warps(const Context *ctx, int64_t n) {
+  return (int64_t)kJoinWarps * grid_for(ctx, n, kJoinWarps, 3);
+}
+int64_t tc_join_warps(const Context *ctx, int64_t n) {
+  return 4 * std::min<int64_t>((n + 1) / 2, 2 * (int64_t)ctx->num_sms);
+}
 
 // One FP32 local join over s's samples with `tiles` 4 x 4 tiles per lane.
 void fp32_join(Context *ctx, int tiles, const float *X, int64_t n, int d, int S, const NndState &s,
@@ -1499,11 +1597,11 @@ void fp32_join(Context *ctx, int tiles, const float *X, int64_t n, int d, int S,
   if (tiles == 1) {
     HDB_CUDA(cudaFuncSetAttribute(k_join<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_join<1><<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev,
-                                           s.worst, s.ib, cross_only);
+                                           s.worst, s.cl, cross_only);
   } else {
     HDB_CUDA(cudaFuncSetAttribute(k_join<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_join<2><<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev,
-                                           s.worst, s.ib, cross_only);
+                                           s.worst, s.cl, cross_only);
   }
   ctx->launches++;
 }
@@ -1533,8 +1631,8 @@ std::map<std::array<int, 5>, int> g_join_tiles;
 // (sample, join, merge) so that the rows hold old and new entries as in the
 // later iterations, the second sample, then both forms -- k_join<1> (80
 // registers, three blocks per SM) and k_join<2> (122 registers, two blocks
-// per SM) -- three times each, alternating, from the same sample and inbox
-// state, the first round untimed.  The faster form is kept for the process.
+// per SM) -- three times each, alternating, from the same samples and an
+// empty list, the first round untimed.  The faster form is kept for the process.
 // Without Xw (the merge) an untuned shape takes two.  The trial's launches
 // count in ctx->launches.
 int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const float *Xw, int64_t n) {
@@ -1550,7 +1648,7 @@ int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const floa
   const int64_t want = (int64_t(256) << 20) / (4 * (int64_t)d);
   const int64_t m = std::min<int64_t>(
       n, std::max<int64_t>(65536, std::min<int64_t>(int64_t(1) << 20, want)));
-  NndState t(ctx, m, k, S, true);
+  NndState t(ctx, m, k, S, fp32_join_warps(ctx, m));
   Buf<int32_t> nrev0(ctx, m), orev0(ctx, m);
   const int wpb = 8;
   const int grid_rows = grid_for(ctx, m, wpb, 16);
@@ -1560,17 +1658,11 @@ int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const floa
                                                   t.gdist, t.worst);
   ctx->launches++;
   HDB_CHECK_LAUNCH();
-  for (int it = 0; it < 2; it++) {
-    if (it == 1) {
-      fp32_join(ctx, 2, Xw, m, d, S, t, 0);
-      HDB_CHECK_LAUNCH();
-      sort_overflow(ctx, t.ib, m);
-    }
-    k_sample<<<grid_rows, 32 * wpb, 0, st>>>(m, k, S, it, t.gid, t.gdist, t.worst, t.ib, t.newS,
-                                             t.oldS, t.nf, t.of, t.nrev, t.orev, 0);
-    ctx->launches++;
-    HDB_CHECK_LAUNCH();
-  }
+  t.sample(ctx, false, 0);
+  fp32_join(ctx, 2, Xw, m, d, S, t, 0);
+  HDB_CHECK_LAUNCH();
+  t.group(ctx);
+  t.sample(ctx, true, 0);
   // the join clears the reverse-sample counts it reads: each trial starts
   // from a copy
   HDB_CUDA(cudaMemcpyAsync(nrev0, t.nrev, m * 4, cudaMemcpyDeviceToDevice, st));
@@ -1581,7 +1673,7 @@ int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const floa
     for (int tiles = 1; tiles <= 2; tiles++) {
       HDB_CUDA(cudaMemcpyAsync(t.nrev, nrev0, m * 4, cudaMemcpyDeviceToDevice, st));
       HDB_CUDA(cudaMemcpyAsync(t.orev, orev0, m * 4, cudaMemcpyDeviceToDevice, st));
-      t.clear_inboxes(ctx, m);
+      t.clear_list(ctx);
       HDB_CUDA(cudaEventRecord(ev.a, st));
       fp32_join(ctx, tiles, Xw, m, d, S, t, 0);
       HDB_CUDA(cudaEventRecord(ev.b, st));
@@ -1602,13 +1694,11 @@ int64_t nndescent_bytes_per_point(int32_t d, const hdb_knn_params &p) {
   const int64_t k = p.k, S = p.sample_num;
   const bool half = p.precision == HDB_PREC_BF16 || p.precision == HDB_PREC_FP16;
   const bool tc = half && tc_dpad(d) <= kTcMaxDpad;
-  const bool list = tc || !half;                 // the tensor-core and FP32 joins
   const int64_t dpad = tc ? tc_dpad(d) : (d + 15) & ~15;
   int64_t b = 4 * (int64_t)d;                    // X in locality order
   if (half) b += 2 * dpad + 4;                   // 16-bit rows + norms
   b += 8 * k + 4 + 16 * S + 30;                  // lists, worst, samples, counters
-  if (!list) b += 8 * kInboxCap;                 // per-row inboxes
-  b += 2 * 12 * (list ? 64 : 16);                // candidate list + sort buffers
+  b += 2 * 12 * 64;                              // candidate list, both buffers
   b += 8 * k;                                    // graph in locality order
   return b;
 }
@@ -1626,20 +1716,31 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
                   p.precision == HDB_PREC_FP16,
               HDB_ERR_ARG, "NN-Descent: unknown precision");
   cudaStream_t st = ctx->stream;
-  // The tensor-core join and the FP32 join append every candidate to the
-  // list that sort_overflow groups by target for the merge (a returning inbox
-  // atomic per candidate cost them more than the sort), so they need no
-  // inboxes and a list for a whole iteration's candidates.  The mma.sync join
-  // (16-bit forms past 256 dimensions) keeps the per-row inboxes.
-  const bool tc_form = (p.precision == HDB_PREC_BF16 || p.precision == HDB_PREC_FP16) &&
-                       tc_dpad(d) <= kTcMaxDpad;
-  const bool list_form = tc_form || p.precision == HDB_PREC_FP32;
-  NndState s(ctx, n, k, S, list_form);
+  // 16-bit forms: BF16, or FP16 of the rows scaled by one power of two; the
+  // tensor-core tile pipeline (tcgen05) up to 256 padded dimensions, the
+  // mma.sync join beyond
+  const bool fp16 = p.precision == HDB_PREC_FP16;
+  const bool bf16 = p.precision == HDB_PREC_BF16 || fp16;
+  const bool use_tc = bf16 && tc_dpad(d) <= kTcMaxDpad;
+  const int dpad = use_tc ? tc_dpad(d) : (d + 15) & ~15;
+  const int jw16 = 4;  // warps per block of the mma.sync join
+  size_t smem_bf = 0;
+  int grid_bf = 0;
+  if (bf16 && !use_tc) {
+    smem_bf = JoinSmemBf16::bytes(dpad) * jw16;
+    HDB_REQUIRE(smem_bf <= 227 * 1024, HDB_ERR_ARG, "NN-Descent 16-bit form: d too large for the join tile");
+    const auto fn = fp16 ? k_join_bf16<true> : k_join_bf16<false>;
+    HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bf));
+    int resident = 0;  // a persistent grid, as of the other joins
+    HDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fn, 32 * jw16, smem_bf));
+    grid_bf = grid_for(ctx, n, jw16, std::max(1, resident));
+  }
+  NndState s(ctx, n, k, S,
+             use_tc ? tc_join_warps(ctx, n) : bf16 ? (int64_t)grid_bf * jw16 : fp32_join_warps(ctx, n));
   int32_t *gid = s.gid, *newS = s.newS, *oldS = s.oldS, *nrev = s.nrev, *orev = s.orev;
   float *gdist = s.gdist, *worst = s.worst;
   int8_t *nf = s.nf, *of = s.of;
-  const Inbox &ib = s.ib;
-  unsigned long long *dropped = s.dropped;
+  const CandList &cl = s.cl;
   std::vector<cudaEvent_t> jev;
   if (js) {
     jev.resize(2 * (size_t)p.iterations);
@@ -1677,18 +1778,8 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
   }
   const float *Xw = Xp;
   Buf<hdb_nnd_element> Gp(ctx, (size_t)n * k);
-  // 16-bit forms: BF16, or FP16 of the rows scaled by one power of two; the
-  // tensor-core tile pipeline (tcgen05) up to 256 padded dimensions, the
-  // mma.sync join beyond
-  const bool fp16 = p.precision == HDB_PREC_FP16;
-  const bool bf16 = p.precision == HDB_PREC_BF16 || fp16;
-  const bool use_tc = bf16 && tc_dpad(d) <= kTcMaxDpad;
-  const int dpad = use_tc ? tc_dpad(d) : (d + 15) & ~15;
   Buf<uint16_t> Xb;
   Buf<float> nrm;
-  int jw16 = 4;
-  size_t smem_bf = 0;
-  int grid_bf = 0;
   float dscale = -2.0f;
   TcJoin tj;
   if (bf16) {
@@ -1723,52 +1814,41 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
     }
     ctx->launches++;
     HDB_CHECK_LAUNCH();
-    if (use_tc) {
-      tc_join_prepare(ctx, Xb, n, dpad, fp16, dscale, &tj);
-    } else {
-      smem_bf = JoinSmemBf16::bytes(dpad) * jw16;
-      HDB_REQUIRE(smem_bf <= 227 * 1024, HDB_ERR_ARG, "NN-Descent 16-bit form: d too large for the join tile");
-      HDB_CUDA(cudaFuncSetAttribute(fp16 ? k_join_bf16<true> : k_join_bf16<false>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bf));
-      grid_bf = grid_for(ctx, n, jw16, 64);
-    }
+    if (use_tc) tc_join_prepare(ctx, Xb, n, dpad, fp16, dscale, &tj);
   }
   // FP32 form: the join's tile slots per lane, tuned per shape
   const int tiles =
       bf16 ? 0 : fp32_join_tiles(ctx, d, k, S, n * d * 4 <= ctx->l2_bytes, Xw, n);
   if (js) js->config = tiles;
   for (int it = 0; it < p.iterations; it++) {
-    k_sample<<<grid_rows, 32 * wpb, 0, st>>>(n, k, S, it > 0, gid, gdist, worst, ib,
-                                                       newS, oldS, nf, of, nrev, orev, 0); ctx->launches++;
-    HDB_CHECK_LAUNCH();
+    s.sample(ctx, it > 0, 0);
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it], st));
     if (use_tc) {
-      tc_join_launch(ctx, tj, S, nrm, newS, oldS, nf, of, nrev, orev, worst, ib);
+      tc_join_launch(ctx, tj, S, nrm, newS, oldS, nf, of, nrev, orev, worst, cl);
     } else {
       if (fp16)
         k_join_bf16<true><<<grid_bf, 32 * jw16, smem_bf, st>>>(Xb, nrm, n, dpad, S, dscale, newS,
-                                                               oldS, nf, of, nrev, orev, worst, ib);
+                                                               oldS, nf, of, nrev, orev, worst, cl);
       else if (bf16)
         k_join_bf16<false><<<grid_bf, 32 * jw16, smem_bf, st>>>(Xb, nrm, n, dpad, S, dscale, newS,
-                                                                oldS, nf, of, nrev, orev, worst, ib);
+                                                                oldS, nf, of, nrev, orev, worst, cl);
       else
         fp32_join(ctx, tiles, Xw, n, d, S, s, 0);
       if (bf16) ctx->launches++;
     }
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it + 1], st));
     HDB_CHECK_LAUNCH();
-    sort_overflow(ctx, ib, n);
-    HDB_CHECK_LAUNCH();
+    s.group(ctx);
   }
-  k_finalize<<<grid_rows, 32 * wpb, 0, st>>>(n, k, gid, gdist, ib, Gp); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  if (p.iterations == 0) s.group(ctx);  // an empty list
+  s.finalize(ctx, Gp);
   if (bf16) {
     k_rerank<<<grid_rows, 32 * wpb, smem_stage, st>>>(Xw, n, d, k, Gp); ctx->launches++;
     HDB_CHECK_LAUNCH();
   }
   k_loc_restore<<<grid_rows, 32 * wpb, 0, st>>>(Gp, order, n, k, G); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, dropped, 5 * sizeof(unsigned long long),
+  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.counters, 5 * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
   ctx->sync();
   if (use_tc)
@@ -1812,18 +1892,14 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
   HDB_CUDA(cudaMemcpyAsync(X.get(), X1, (size_t)n1 * d * sizeof(float), cudaMemcpyDeviceToDevice, st));
   HDB_CUDA(cudaMemcpyAsync(X.get() + (size_t)n1 * d, X2, (size_t)n2 * d * sizeof(float),
                            cudaMemcpyDeviceToDevice, st));
-  NndState s(ctx, n, k, S, true);
-  int32_t *gid = s.gid;
-  float *gdist = s.gdist, *worst = s.worst;
-  const Inbox &ib = s.ib;
-  unsigned long long *dropped = s.dropped;
+  NndState s(ctx, n, k, S, fp32_join_warps(ctx, n));
 
   const int wpb = 8;
   const int grid_rows = grid_for(ctx, n, wpb, 16);
   const size_t smem_stage = (size_t)wpb * kStageFloats * sizeof(float);
   stage_smem_attrs(smem_stage);
-  k_merge_init<<<grid_rows, 32 * wpb, smem_stage, st>>>(X, n, d, k, n1, G1, G2, gid, gdist, worst,
-                                                        ctx->dev_err);
+  k_merge_init<<<grid_rows, 32 * wpb, smem_stage, st>>>(X, n, d, k, n1, G1, G2, s.gid,
+                                                        s.gdist, s.worst, ctx->dev_err);
   ctx->launches++;
   HDB_CHECK_LAUNCH();
   ctx->sync();
@@ -1838,18 +1914,14 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
   // NNDescentForMerge (nndescent.cu:1999-2087): PrepareForUpdateForMerge +
   // UpdateGraphForMerge per iteration
   for (int it = 0; it < p.iterations; it++) {
-    k_sample<<<grid_rows, 32 * wpb, 0, st>>>(n, k, S, it > 0, gid, gdist, worst, ib, s.newS,
-                                             s.oldS, s.nf, s.of, s.nrev, s.orev, n1);
-    ctx->launches++;
-    HDB_CHECK_LAUNCH();
+    s.sample(ctx, it > 0, n1);
     fp32_join(ctx, tiles, X, n, d, S, s, 1);
     HDB_CHECK_LAUNCH();
-    sort_overflow(ctx, ib, n);
-    HDB_CHECK_LAUNCH();
+    s.group(ctx);
   }
-  k_finalize<<<grid_rows, 32 * wpb, 0, st>>>(n, k, gid, gdist, ib, G); ctx->launches++;
-  HDB_CHECK_LAUNCH();
-  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, dropped, sizeof(unsigned long long),
+  if (p.iterations == 0) s.group(ctx);  // an empty list
+  s.finalize(ctx, G);
+  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.counters, sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
   ctx->sync();
   if (dropped_out) *dropped_out = *static_cast<const int64_t *>(ctx->pinned);

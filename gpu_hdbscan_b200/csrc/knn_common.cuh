@@ -1,6 +1,5 @@
 // Shared pieces of the NN-Descent kernels (knn.cu, join_tc.cu): packed
-// (distance, id) keys, the per-row candidate inbox and the push of one
-// candidate into it.
+// (distance, id) keys and the candidate list that the joins append to.
 #pragma once
 #include "hdb_internal.cuh"
 
@@ -8,7 +7,6 @@ namespace hdb {
 namespace knn {
 
 constexpr int kMaxK = 32;
-constexpr int kInboxCap = 127;  // + 1 overflow slot = 128 sorted candidates per merge
 
 // Key of a candidate: distance bits (non-negative floats order as unsigned)
 // above the id, so an unsigned compare orders by (distance, id).
@@ -21,39 +19,46 @@ __device__ __forceinline__ int32_t pk_id(uint64_t k) { return (int32_t)(uint32_t
 // NNDElement::label(): "old" entries are stored as -id-1.
 __device__ __forceinline__ int32_t decode(int32_t label) { return label >= 0 ? label : -label - 1; }
 
-// Where the join leaves its candidates: a fixed inbox per row, then a global
-// overflow list (radix-sorted by target row between the join and the merge).
-// Only when the overflow list is full is a candidate dropped; the best
-// dropped one per row is still kept in `best`.
-struct Inbox {
-  int32_t *cnt;                  // [n] candidates offered this iteration
-  uint64_t *slots;               // [n * kInboxCap] packed (distance, id)
+// Where the joins leave their candidates: one list of (target row, packed
+// candidate), grouped by blocks of target rows between the join and the merge.
+// Only when the list is full is a candidate dropped; the best dropped one per
+// row is still kept in `best`.
+struct CandList {
   unsigned long long *best;      // [n]
-  uint32_t *ovf_tgt;             // [ovf_cap] overflow: target row (sorted in place)
-  uint64_t *ovf_key;             // [ovf_cap] overflow: packed candidate (sorted along)
-  uint32_t *ostart, *oend;       // [n] segment of each row in the sorted overflow list
-  unsigned long long *counters;  // [0] dropped [1] rows gathered [2] candidates [3] overflow
+  uint32_t *tgt;                 // [cap] target row
+  uint64_t *key;                 // [cap] packed candidate
+  unsigned long long *counters;  // [0] dropped [1] rows gathered [2] candidates [3] list length
                                  // [4] distance pairs computed (FP32 join)
-  int64_t ovf_cap;
-  int32_t inboxes;               // 0: no per-row inboxes (the tensor-core join's list only)
+  int64_t cap;
+  uint32_t chunk;                // slots that a warp takes at a time
+  uint32_t none;                 // target of an unused slot: past every bucket of rows
 };
 
 // Space of the candidate list a warp writes into: [pos, end), taken from the
-// list in chunks of kListChunk slots with one atomic on the list's counter,
-// so that the warps of a join do not all queue on that one counter.
-constexpr uint32_t kListChunk = 1024;
+// list `chunk` slots at a time with one atomic on the list's counter, so that
+// the warps of a join do not all queue on that one counter.  The tail that a
+// warp leaves unused in its last chunk is sorted along as sentinels, so the
+// chunk follows the work: about a quarter of what a warp will append, between
+// kListChunkMin (one append's most) and 1,024 slots.  (With 1,024 always, the
+// list of 1,500 rows held 1.5 M slots for some 50 k candidates.)
+constexpr uint32_t kListChunkMin = 64, kListChunkMax = 1024;
+inline uint32_t list_chunk(int64_t candidates_per_warp) {
+  uint32_t c = kListChunkMin;
+  while (c < kListChunkMax && 8 * (int64_t)c <= candidates_per_warp) c *= 2;
+  return c;
+}
 struct ListCursor {
   unsigned long long pos = 0, end = 0;
 };
 
-// Writes the sentinel entry (target row `n`, sorted after every row and
-// skipped by the segment bounds; key ~0) at list positions [from, to).
-__device__ __forceinline__ void list_fill(const Inbox &ib, unsigned long long from,
-                                          unsigned long long to, uint32_t n) {
+// Writes the sentinel entry (target `none`, sorted after every row's; key ~0)
+// at list positions [from, to).
+__device__ __forceinline__ void list_fill(const CandList &cl, unsigned long long from,
+                                          unsigned long long to) {
   for (unsigned long long p = from + (threadIdx.x & 31); p < to; p += 32)
-    if ((int64_t)p < ib.ovf_cap) {
-      ib.ovf_tgt[p] = n;
-      ib.ovf_key[p] = ~0ull;
+    if ((int64_t)p < cl.cap) {
+      cl.tgt[p] = cl.none;
+      cl.key[p] = ~0ull;
     }
 }
 
@@ -63,9 +68,9 @@ __device__ __forceinline__ void list_fill(const Inbox &ib, unsigned long long fr
 // cursor; when they do not fit in the cursor's chunk, the rest of that chunk
 // becomes sentinel entries and one lane takes a new chunk.  Past the list's
 // capacity only the best dropped candidate of each target is kept.  Returns
-// the lane's count.  Called by all 32 lanes of a warp; n is the row count.
-__device__ __forceinline__ int append_candidates(const Inbox &ib, ListCursor &cur, uint32_t n,
-                                                 bool v0, int32_t t0, uint64_t k0, bool v1,
+// the lane's count.  Called by all 32 lanes of a warp.
+__device__ __forceinline__ int append_candidates(const CandList &cl, ListCursor &cur, bool v0,
+                                                 int32_t t0, uint64_t k0, bool v1,
                                                  int32_t t1, uint64_t k1) {
   const int lane = threadIdx.x & 31;
   uint32_t lt;
@@ -74,12 +79,12 @@ __device__ __forceinline__ int append_candidates(const Inbox &ib, ListCursor &cu
   const uint32_t tot = __popc(b0) + __popc(b1);
   if (tot == 0) return 0;
   if (cur.pos + tot > cur.end) {
-    list_fill(ib, cur.pos, cur.end, n);
+    list_fill(cl, cur.pos, cur.end);
     unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&ib.counters[3], (unsigned long long)kListChunk);
+    if (lane == 0) base = atomicAdd(&cl.counters[3], (unsigned long long)cl.chunk);
     base = __shfl_sync(0xffffffffu, base, 0);
     cur.pos = base;
-    cur.end = base + kListChunk;
+    cur.end = base + cl.chunk;
   }
   const unsigned long long p0 = cur.pos + __popc(b0 & lt);
   const unsigned long long p1 = cur.pos + __popc(b0) + __popc(b1 & lt);
@@ -91,35 +96,15 @@ __device__ __forceinline__ int append_candidates(const Inbox &ib, ListCursor &cu
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     if (!vv[q]) continue;
-    if ((int64_t)pp[q] < ib.ovf_cap) {
-      ib.ovf_tgt[pp[q]] = (uint32_t)tt[q];
-      ib.ovf_key[pp[q]] = kk[q];
+    if ((int64_t)pp[q] < cl.cap) {
+      cl.tgt[pp[q]] = (uint32_t)tt[q];
+      cl.key[pp[q]] = kk[q];
     } else {
-      atomicMin(&ib.best[tt[q]], (unsigned long long)kk[q]);
-      atomicAdd(&ib.counters[0], 1ull);
+      atomicMin(&cl.best[tt[q]], (unsigned long long)kk[q]);
+      atomicAdd(&cl.counters[0], 1ull);
     }
   }
   return (v0 ? 1 : 0) + (v1 ? 1 : 0);
-}
-
-__device__ __forceinline__ int push_candidate(int32_t target, int32_t id, float d,
-                                              const float *__restrict__ worst, const Inbox &ib) {
-  if (!(d < worst[target])) return 0;  // cannot enter the target's list
-  int slot = atomicAdd(&ib.cnt[target], 1);
-  uint64_t key = pack(d, id);
-  if (slot < kInboxCap) {
-    ib.slots[(int64_t)target * kInboxCap + slot] = key;
-  } else {
-    unsigned long long pos = atomicAdd(&ib.counters[3], 1ull);
-    if ((int64_t)pos < ib.ovf_cap) {
-      ib.ovf_tgt[pos] = (uint32_t)target;
-      ib.ovf_key[pos] = key;
-    } else {
-      atomicMin(&ib.best[target], (unsigned long long)key);
-      atomicAdd(&ib.counters[0], 1ull);
-    }
-  }
-  return 1;
 }
 
 }  // namespace knn

@@ -1,6 +1,11 @@
 // Device-wide primitives used by every stage: exclusive scans and a stable
 // LSD radix sort.  Both are plain HBM-streaming kernels (tiles of 2048
 // elements per 256-thread block); no library code.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <utility>
+
 #include "hdb_internal.cuh"
 
 namespace hdb {
@@ -134,7 +139,15 @@ constexpr int kSortThreads = 256;
 constexpr int kSortWarps = kSortThreads / 32;
 constexpr int kSortItems = 16;          // tile-major sorts: 4096-key tiles
 constexpr int kSortItemsFlat = 8;       // digit-major (caller-buffer) sort: 2048-key tiles
-constexpr int kColRows = 512;           // tiles per chunk of the column scan
+constexpr uint32_t kColOneTiles = 2048; // up to here one cluster does the whole column scan
+
+// How many keys there are: n, or what the device holds where the host only
+// knows a bound (a list that kernels append to).
+__device__ __forceinline__ int64_t key_count(int64_t n, const unsigned long long *__restrict__ dev) {
+  if (!dev) return n;
+  const int64_t c = (int64_t)*dev;
+  return c < n ? c : n;
+}
 
 // Dynamic shared memory of one scatter block: the tile's keys and values in
 // digit order, the per-warp digit counts, each digit's first tile position
@@ -159,9 +172,12 @@ template <typename K, int kBins, int kItems, bool kTileMajor>
 __global__ void __launch_bounds__(kSortThreads) radix_hist(const K *__restrict__ keys,
                                                             uint32_t *__restrict__ counts,
                                                             int64_t n, int shift, uint32_t mask,
-                                                            uint32_t nblocks) {
+                                                            uint32_t nblocks,
+                                                            const unsigned long long *dev_n) {
   constexpr int kTile = kSortThreads * kItems;
   __shared__ uint32_t hist[kBins];
+  n = key_count(n, dev_n);
+  if ((int64_t)blockIdx.x * kTile >= n) return;
   for (int i = threadIdx.x; i < kBins; i += kSortThreads) hist[i] = 0;
   __syncthreads();
   const int64_t base = (int64_t)blockIdx.x * kTile;
@@ -190,9 +206,11 @@ template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileM
 __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
     const K *__restrict__ keys_in, const V *__restrict__ vals_in, K *__restrict__ keys_out,
     V *__restrict__ vals_out, const uint32_t *__restrict__ offsets, int64_t n, int shift,
-    uint32_t mask, uint32_t nblocks) {
+    uint32_t mask, uint32_t nblocks, const unsigned long long *dev_n) {
   using L = SortSmem<K, V, kVals, kBins, kItems>;
   constexpr int kTile = L::kTile;
+  n = key_count(n, dev_n);
+  if ((int64_t)blockIdx.x * kTile >= n) return;
   constexpr int kPer = kBins / kSortThreads;  // digits owned by each thread in the scan
   extern __shared__ __align__(16) unsigned char sort_smem[];
   K *tk = reinterpret_cast<K *>(sort_smem);
@@ -292,15 +310,90 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
   }
 }
 
-// Column scan of tile-major counts [nblocks][kBins], one thread per digit.
-// (1) per chunk of kColRows tiles, each digit's count in the chunk;
+// Column scan of tile-major counts [tiles][kBins]: every tile's output position
+// of its first key of each digit, and each digit's first position (base, with
+// the total behind it).
+//
+// Up to kColOneTiles tiles, one cluster does it in one launch: CTA c owns 64
+// digits, 16 threads each, a thread a run of consecutive tiles; the digits'
+// totals are scanned over the cluster through distributed shared memory.  At
+// 60 tiles of 512 bins it takes 4.7 us, where three launches with 512 tiles to a
+// block took 33 us; at 1,300 tiles 16.4 us, as the three launches below with
+// their gaps.
+constexpr int kColDigits = 64, kColLanes = 16;
+template <int kBins>
+__global__ void __cluster_dims__(kBins / kColDigits, 1, 1) __launch_bounds__(kColDigits *kColLanes)
+    radix_col_one(const uint32_t *__restrict__ counts, uint32_t *__restrict__ base,
+                  uint32_t *__restrict__ offs, int64_t n, const unsigned long long *dev_n) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  constexpr int kTile = kSortThreads * kSortItems;
+  __shared__ uint32_t part[kColLanes][kColDigits];
+  __shared__ uint32_t first[kColDigits];
+  __shared__ uint32_t cta_total, half_total;
+  n = key_count(n, dev_n);
+  const uint32_t tiles = (uint32_t)((n + kTile - 1) / kTile);
+  const int dl = threadIdx.x % kColDigits, l = threadIdx.x / kColDigits;
+  const int rank = (int)cluster.block_rank(), lane = threadIdx.x & 31;
+  const int d = rank * kColDigits + dl;
+  const uint32_t per = (tiles + kColLanes - 1) / kColLanes;
+  const uint32_t r0 = min((uint32_t)l * per, tiles), r1 = min(r0 + per, tiles);
+  uint32_t s = 0;
+#pragma unroll 8
+  for (uint32_t r = r0; r < r1; r++) s += counts[(int64_t)r * kBins + d];
+  part[l][dl] = s;
+  __syncthreads();
+  uint32_t total = 0, incl = 0;
+  if (l == 0) {  // two warps: the digit's total, then an inclusive scan over the CTA's digits
+#pragma unroll
+    for (int j = 0; j < kColLanes; j++) {
+      const uint32_t c = part[j][dl];
+      part[j][dl] = total;
+      total += c;
+    }
+    incl = total;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (threadIdx.x == 31) half_total = incl;
+  }
+  __syncthreads();
+  if (l == 0) {
+    if (threadIdx.x >= 32) incl += half_total;
+    if (threadIdx.x == kColDigits - 1) cta_total = incl;
+  }
+  cluster.sync();
+  if (l == 0) {
+    uint32_t before = 0;
+    for (int c = 0; c < rank; c++) before += *cluster.map_shared_rank(&cta_total, c);
+    first[dl] = before + incl - total;
+    base[d] = before + incl - total;
+    if (d == kBins - 1) base[kBins] = before + incl;
+  }
+  cluster.sync();  // the other CTAs have read cta_total; `first` is written
+  uint32_t run = first[dl] + part[l][dl];
+#pragma unroll 8
+  for (uint32_t r = r0; r < r1; r++) {
+    const int64_t at = (int64_t)r * kBins + d;
+    const uint32_t c = counts[at];
+    offs[at] = run;
+    run += c;
+  }
+}
+
+// More tiles: one thread per digit and chunk of `rows` tiles, in three
+// launches.  (1) per chunk, each digit's count in it;
 template <int kBins>
 __global__ void __launch_bounds__(kBins) radix_col_sums(const uint32_t *__restrict__ counts,
-                                                        uint32_t *__restrict__ csum,
-                                                        uint32_t nblocks) {
+                                                        uint32_t *__restrict__ csum, uint32_t rows,
+                                                        int64_t n, const unsigned long long *dev_n) {
+  constexpr int kTile = kSortThreads * kSortItems;
+  const int64_t nblocks = (key_count(n, dev_n) + kTile - 1) / kTile;
   const int d = threadIdx.x;
-  const int64_t r0 = (int64_t)blockIdx.x * kColRows;
-  const int64_t r1 = r0 + kColRows < (int64_t)nblocks ? r0 + kColRows : (int64_t)nblocks;
+  const int64_t r0 = (int64_t)blockIdx.x * rows;
+  const int64_t r1 = r0 + rows < nblocks ? r0 + rows : nblocks;
   uint32_t s = 0;
 #pragma unroll 8
   for (int64_t r = r0; r < r1; r++) s += counts[r * kBins + d];
@@ -329,6 +422,7 @@ __global__ void __launch_bounds__(kBins) radix_col_scan(uint32_t *__restrict__ c
   }
   uint32_t total;
   base[d] = block_exclusive_scan<uint32_t>(run, &total, warp_sums);
+  if (d == 0) base[kBins] = total;
 }
 
 // (3) every tile's output position of its first key of each digit.
@@ -336,11 +430,13 @@ template <int kBins>
 __global__ void __launch_bounds__(kBins) radix_col_apply(const uint32_t *__restrict__ counts,
                                                          const uint32_t *__restrict__ csum,
                                                          const uint32_t *__restrict__ base,
-                                                         uint32_t *__restrict__ offs,
-                                                         uint32_t nblocks) {
+                                                         uint32_t *__restrict__ offs, uint32_t rows,
+                                                         int64_t n, const unsigned long long *dev_n) {
+  constexpr int kTile = kSortThreads * kSortItems;
+  const int64_t nblocks = (key_count(n, dev_n) + kTile - 1) / kTile;
   const int d = threadIdx.x;
-  const int64_t r0 = (int64_t)blockIdx.x * kColRows;
-  const int64_t r1 = r0 + kColRows < (int64_t)nblocks ? r0 + kColRows : (int64_t)nblocks;
+  const int64_t r0 = (int64_t)blockIdx.x * rows;
+  const int64_t r1 = r0 + rows < nblocks ? r0 + rows : nblocks;
   uint32_t run = base[d] + csum[(int64_t)blockIdx.x * kBins + d];
 #pragma unroll 8
   for (int64_t r = r0; r < r1; r++) {
@@ -352,66 +448,91 @@ __global__ void __launch_bounds__(kBins) radix_col_apply(const uint32_t *__restr
 
 template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor>
 void launch_scatter(cudaStream_t st, const K *kin, const V *vin, K *kout, V *vout,
-                    const uint32_t *offs, int64_t n, int shift, uint32_t mask, uint32_t nb) {
+                    const uint32_t *offs, int64_t n, int shift, uint32_t mask, uint32_t nb,
+                    const unsigned long long *dev_n = nullptr) {
   using L = SortSmem<K, V, kVals, kBins, kItems>;
   auto *fn = radix_scatter<K, V, kVals, kBins, kItems, kTileMajor>;
   if (L::kBytes > 48 * 1024)
     HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kBytes));
-  fn<<<nb, kSortThreads, L::kBytes, st>>>(kin, vin, kout, vout, offs, n, shift, mask, nb);
+  fn<<<nb, kSortThreads, L::kBytes, st>>>(kin, vin, kout, vout, offs, n, shift, mask, nb, dev_n);
   HDB_CHECK_LAUNCH();
 }
 
-// Digit widths: the fewest passes of at most log2(kBins) bits over
-// [begin_bit, end_bit), the bits spread evenly over them (25 bits with 512
-// bins: 9 + 8 + 8).
+// Stable LSD sort of the pairs in (keys, vals) with (ktmp, vtmp) as the second
+// buffer; returns whether the result is in the second one.  Digit widths: the
+// fewest passes of at most log2(kBins) bits over [begin_bit, end_bit), the bits
+// spread evenly over them (25 bits with 512 bins: 9 + 8 + 8).  dev_n: the count
+// on the device, n then being a bound.  base_out (optional): the last pass's
+// base, kBins + 1 values.
 template <typename K, typename V, int kBins>
-void radix_sort_impl(Context *ctx, K *keys, V *vals, int64_t n, int begin_bit, int end_bit) {
-  if (n <= 1 || end_bit <= begin_bit) return;
+bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64_t n, int begin_bit,
+                         int end_bit, const unsigned long long *dev_n, uint32_t *base_out) {
   HDB_REQUIRE(n < (int64_t(1) << 32), HDB_ERR_ARG, "radix sort: more than 2^32 elements");
   constexpr int kMaxBits = kBins == 512 ? 9 : 8;
   static_assert(kBins == 256 || kBins == 512, "radix sort: 256 or 512 bins");
   constexpr int kTile = kSortThreads * kSortItems;
   const cudaStream_t st = ctx->stream;
   const uint32_t nb = (uint32_t)ceil_div(n, kTile);
-  const uint32_t nchunks = (uint32_t)ceil_div(nb, kColRows);
-  Buf<K> ktmp(ctx, n);
-  Buf<V> vtmp;
-  if (vals) vtmp = Buf<V>(ctx, n);
+  // chunks of the column scan: a few per SM, at most 512 tiles each
+  const uint32_t rows = (uint32_t)std::min<int64_t>(
+      512, std::max<int64_t>(32, ceil_div(nb, 4 * (int64_t)ctx->num_sms)));
+  const bool one = nb <= kColOneTiles;
+  const uint32_t nchunks = one ? 1 : (uint32_t)ceil_div(nb, rows);
   Buf<uint32_t> counts(ctx, (size_t)nb * kBins), offs(ctx, (size_t)nb * kBins),
-      csum(ctx, (size_t)nchunks * kBins), base(ctx, kBins);
+      csum(ctx, (size_t)nchunks * kBins), base_buf;
+  uint32_t *base = base_out;
+  if (!base) {
+    base_buf = Buf<uint32_t>(ctx, kBins + 1);
+    base = base_buf;
+  }
   K *kin = keys, *kout = ktmp;
-  V *vin = vals, *vout = vals ? vtmp.get() : nullptr;
+  V *vin = vals, *vout = vtmp;
   int passes = 0;
   int left = end_bit - begin_bit;
   int npass = (left + kMaxBits - 1) / kMaxBits;
   for (int shift = begin_bit; left > 0; passes++, npass--) {
     const int bits = (left + npass - 1) / npass;
     const uint32_t mask = (1u << bits) - 1u;
-    radix_hist<K, kBins, kSortItems, true><<<nb, kSortThreads, 0, st>>>(kin, counts, n, shift,
-                                                                       mask, nb);
+    radix_hist<K, kBins, kSortItems, true><<<nb, kSortThreads, 0, st>>>(kin, counts, n, shift, mask,
+                                                                       nb, dev_n);
     HDB_CHECK_LAUNCH();
-    radix_col_sums<kBins><<<nchunks, kBins, 0, st>>>(counts, csum, nb);
-    HDB_CHECK_LAUNCH();
-    radix_col_scan<kBins><<<1, kBins, 0, st>>>(csum, base, nchunks);
-    HDB_CHECK_LAUNCH();
-    radix_col_apply<kBins><<<nchunks, kBins, 0, st>>>(counts, csum, base, offs, nb);
+    if (one) {
+      radix_col_one<kBins><<<kBins / kColDigits, kColDigits * kColLanes, 0, st>>>(counts, base, offs,
+                                                                                 n, dev_n);
+      ctx->launches++;
+    } else {
+      radix_col_sums<kBins><<<nchunks, kBins, 0, st>>>(counts, csum, rows, n, dev_n);
+      radix_col_scan<kBins><<<1, kBins, 0, st>>>(csum, base, nchunks);
+      radix_col_apply<kBins><<<nchunks, kBins, 0, st>>>(counts, csum, base, offs, rows, n, dev_n);
+      ctx->launches += 3;
+    }
     HDB_CHECK_LAUNCH();
     if (vals)
       launch_scatter<K, V, true, kBins, kSortItems, true>(st, kin, vin, kout, vout, offs, n, shift,
-                                                          mask, nb);
+                                                          mask, nb, dev_n);
     else
       launch_scatter<K, V, false, kBins, kSortItems, true>(st, kin, nullptr, kout, nullptr, offs,
-                                                           n, shift, mask, nb);
-    ctx->launches += 5;
-    K *t = kin; kin = kout; kout = t;
-    V *tv = vin; vin = vout; vout = tv;
+                                                           n, shift, mask, nb, dev_n);
+    ctx->launches += 2;
+    std::swap(kin, kout);
+    std::swap(vin, vout);
     shift += bits;
     left -= bits;
   }
-  if (passes & 1) {
-    HDB_CUDA(cudaMemcpyAsync(keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, st));
+  return (passes & 1) != 0;
+}
+
+template <typename K, typename V, int kBins>
+void radix_sort_impl(Context *ctx, K *keys, V *vals, int64_t n, int begin_bit, int end_bit) {
+  if (n <= 1 || end_bit <= begin_bit) return;
+  Buf<K> ktmp(ctx, n);
+  Buf<V> vtmp;
+  if (vals) vtmp = Buf<V>(ctx, n);
+  if (radix_sort_pingpong<K, V, kBins>(ctx, keys, vals, ktmp, vals ? vtmp.get() : nullptr, n,
+                                       begin_bit, end_bit, nullptr, nullptr)) {
+    HDB_CUDA(cudaMemcpyAsync(keys, ktmp, n * sizeof(K), cudaMemcpyDeviceToDevice, ctx->stream));
     if (vals)
-      HDB_CUDA(cudaMemcpyAsync(vals, vin, n * sizeof(V), cudaMemcpyDeviceToDevice, st));
+      HDB_CUDA(cudaMemcpyAsync(vals, vtmp, n * sizeof(V), cudaMemcpyDeviceToDevice, ctx->stream));
   }
 }
 
@@ -446,9 +567,11 @@ void radix_sort_u64(Context *ctx, uint64_t *keys, uint32_t *values, int64_t n, i
   else
     radix_sort_impl<uint64_t, uint32_t, 256>(ctx, keys, values, n, begin_bit, end_bit);
 }
-void radix_sort_u32_u64(Context *ctx, uint32_t *keys, uint64_t *values, int64_t n, int begin_bit,
-                        int end_bit) {
-  radix_sort_impl<uint32_t, uint64_t, 512>(ctx, keys, values, n, begin_bit, end_bit);
+bool radix_group_u32_u64(Context *ctx, uint32_t *keys, uint64_t *values, uint32_t *keys2,
+                         uint64_t *values2, int64_t cap, const unsigned long long *count,
+                         int begin_bit, int end_bit, uint32_t *base) {
+  return radix_sort_pingpong<uint32_t, uint64_t, 512>(ctx, keys, values, keys2, values2, cap,
+                                                      begin_bit, end_bit, count, base);
 }
 
 // Stable LSD radix sort of u32 keys with u32 values in caller-provided
@@ -467,8 +590,8 @@ void radix_sort_u32_buffers(cudaStream_t st, uint32_t *keys, uint32_t *vals, uin
   uint32_t *kin = keys, *kout = ktmp, *vin = vals, *vout = vtmp;
   int passes = 0;
   for (int shift = begin_bit; shift < end_bit; shift += 8, passes++) {
-    radix_hist<uint32_t, 256, kSortItemsFlat, false><<<nb, kSortThreads, 0, st>>>(kin, counts, n,
-                                                                                 shift, 0xffu, nb);
+    radix_hist<uint32_t, 256, kSortItemsFlat, false><<<nb, kSortThreads, 0, st>>>(
+        kin, counts, n, shift, 0xffu, nb, nullptr);
     HDB_CHECK_LAUNCH();
     if (ns == 1) {
       scan_tile_apply<uint32_t, uint32_t><<<1, kScanThreads, 0, st>>>(counts, offs, nullptr, nc,
