@@ -23,6 +23,8 @@
 // Stability is summed per cluster in the reference's row order (chain nodes
 // top-down, identical terms for the points of each small side), in FP32 with
 // separate multiply/add roundings, or in FP64 when asked.
+#include <algorithm>
+
 #include "hdb_internal.cuh"
 #include "trees.cuh"
 
@@ -534,75 +536,236 @@ __device__ T add_repeated(T s, T v, int64_t cnt) {
   return s;
 }
 
-// One warp per cluster: stability in the reference's row order.  The warp
-// loads 32 chain items at a time (coalesced) and every lane replays the same
-// sequential sum from registers, so the serial chain walk never waits on a
-// dependent global load; lane 0 stores the result.
-// Stability of each cluster: its chain items summed in FP32 in the
-// reference's row order (and in FP64 alongside when kBoth).  One warp per
-// cluster, 32 items per load; each lane forms its item's addends first, so the
-// serial part is just the chain of adds, unrolled over the 32 items.  Items
-// that stand for many rows with one addend go through add_repeated.
+// A chain item's addends in the reference's row order: a points with lambda
+// each, or for the split that ends the chain (lambda - birth) * child_size of
+// its left and then its right child.
+template <typename T>
+struct Addends {
+  T y0, y1;
+  int32_t m0;  // rows that add y0
+  __device__ __forceinline__ Addends(const ChainItem &it, float birth) {
+    using B = FpBits<T>;
+    const T v = B::sub((T)it.lam, (T)birth);
+    const bool split = it.a < 0;
+    y0 = split ? B::mul(v, (T)(-it.a)) : v;
+    y1 = split ? B::mul(v, (T)it.b) : T(0);
+    m0 = split ? 1 : it.a;
+  }
+};
+
+// The running sum s = q * u, u its ulp.  While s stays in one binade, adding
+// y >= 0 with round-to-nearest moves q by y / u rounded to an integer, whatever
+// q is, unless y / u lies halfway between two integers (the even one of the
+// two neighbours of q + y / u is taken then).  So a run of additions that
+// neither meets such a tie nor leaves the binade is a sum of integers, in any
+// order: every thread rounds its own addends.  A long chain leaves a binade some
+// twenty times and, once s is large, meets hardly any ties; those stretches
+// are added one by one.
+template <typename T>
+struct Binade {
+  double u, inv_u;  // powers of two
+  int64_t q, top;   // s / u, and where the binade ends
+  double item_top;  // an addend of this many steps leaves it for certain
+  bool ok;
+  __device__ __forceinline__ explicit Binade(T s) {
+    using B = FpBits<T>;
+    const int e = B::exp_field(s) - B::kBias;
+    // normal, and far enough from the ends of the double range for u and 1 / u
+    ok = s > T(0) && e > (B::kMant == 52 ? -900 : -126) && e < (B::kMant == 52 ? 900 : 128);
+    u = ok ? FpBits<double>::pow2(e - B::kMant) : 1.0;
+    inv_u = ok ? FpBits<double>::pow2(B::kMant - e) : 1.0;
+    q = ok ? (int64_t)((double)s * inv_u) : 0;
+    top = int64_t(1) << (B::kMant + 1);
+    item_top = (double)(int64_t(1) << B::kMant);
+  }
+  // m additions of y: their steps into `steps`, and about as many into `about`
+  // (which cannot overflow); false if they have to be taken one by one
+  __device__ __forceinline__ bool take(T y, int32_t m, uint64_t &steps, double &about) const {
+    const double x = (double)y * inv_u;  // exact
+    const double r = rint(x);
+    if (!(y >= T(0)) || !(x * (double)m < item_top) || fabs(x - r) == 0.5) return false;
+    steps += (uint64_t)m * (uint64_t)r;
+    about += (double)m * r;
+    return true;
+  }
+  __device__ __forceinline__ bool stays(uint64_t steps, double about) const {
+    return about < (double)top && q + (int64_t)steps < top;
+  }
+  __device__ __forceinline__ T after(uint64_t steps) const { return (T)((double)(q + (int64_t)steps) * u); }
+};
+
+// s after the m items that the warp's first m lanes hold, one by one.
+template <typename T>
+__device__ T add_serially(T s, const ChainItem &mine, float birth, int m) {
+  using B = FpBits<T>;
+  const Addends<T> ad(mine, birth);
+  const int lane = lane_id();
+  const uint32_t split_mask = __ballot_sync(0xffffffffu, lane < m && mine.a < 0);
+  const uint32_t rep_mask = __ballot_sync(0xffffffffu, lane < m && mine.a > 1);
+  for (int t = 0; t < m; t++) {
+    const T y0 = __shfl_sync(0xffffffffu, ad.y0, t), y1 = __shfl_sync(0xffffffffu, ad.y1, t);
+    const int32_t m0 = __shfl_sync(0xffffffffu, ad.m0, t);
+    if ((rep_mask >> t) & 1u) s = add_repeated<T>(s, y0, m0);
+    else s = B::add(s, y0);
+    if ((split_mask >> t) & 1u) s = B::add(s, y1);
+  }
+  return s;
+}
+
+// s after the m <= 32 items of a warp.
+template <typename T>
+__device__ __forceinline__ T add_warp(T s, const ChainItem &mine, float birth, int m) {
+  const Binade<T> bin(s);
+  const Addends<T> ad(mine, birth);
+  uint64_t steps = 0;
+  double about = 0.0;
+  const bool fine = lane_id() >= m || (bin.ok && bin.take(ad.y0, ad.m0, steps, about) &&
+                                       bin.take(ad.y1, 1, steps, about));
+  if (__all_sync(0xffffffffu, fine)) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      steps += __shfl_xor_sync(0xffffffffu, steps, o);
+      about += __shfl_xor_sync(0xffffffffu, about, o);
+    }
+    if (bin.stays(steps, about)) return bin.after(steps);
+  }
+  return add_serially<T>(s, mine, birth, m);
+}
+
+// Stability of each cluster: its chain items summed in FP32 in the reference's
+// row order (and in FP64 alongside when kBoth).  One warp per cluster, 32 items
+// per load, the next ones in flight; chains of more than kLongChain items are
+// left to k_stability_long (their clusters listed in long_list).
+// Both kernels stream 16 bytes an item and are bound by the latency of a step
+// (load, round, reduce); the sum one by one had a chain of 32 additions and 64
+// shuffles per 32 items instead.  10M x 12, 200 blobs, one chain holding most
+// of the points: 238 -> 6.1 ms; 20M x 128, 200 blobs: 52 ms before.
+constexpr int kLongChain = 4096;
 template <bool kBoth>
 __global__ void k_stability(int64_t C, const int64_t *__restrict__ seg_start,
                             const int64_t *__restrict__ seg_end, const ChainItem *__restrict__ items,
                             const float *__restrict__ birth, float *__restrict__ stab,
-                            double *__restrict__ stab64) {
+                            double *__restrict__ stab64, int32_t *__restrict__ long_list,
+                            int32_t *__restrict__ long_count) {
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
   for (int64_t c = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); c < C;
        c += (int64_t)gridDim.x * wpb) {
+    const int64_t s0 = seg_start[c], e = seg_end[c];
+    if (e - s0 > kLongChain) {
+      if (lane == 0) long_list[atomicAdd(long_count, 1)] = (int32_t)c;
+      continue;
+    }
     const float b = birth[c];
     float s = 0.0f;
     double s64 = 0.0;
-    const int64_t e = seg_end[c];
-    for (int64_t base = seg_start[c]; base < e; base += 32) {
-      ChainItem mine = {0.0f, 1, 0, 0};
-      const bool valid = base + lane < e;
-      if (valid) mine = items[base + lane];
+    ChainItem next = {0.0f, 0, 0, 0};
+    if (s0 + lane < e) next = items[s0 + lane];
+    for (int64_t base = s0; base < e; base += 32) {
+      const ChainItem mine = next;
+      if (base + 32 + lane < e) next = items[base + 32 + lane];
       const int m = (int)min((int64_t)32, e - base);
-      const float v = __fsub_rn(mine.lam, b);
-      // split rows: (lambda - birth) * child_size, left then right; one row: v
-      const bool split = mine.a < 0;
-      const float x0 = split ? __fmul_rn(v, (float)(-mine.a)) : v;
-      const float x1 = split ? __fmul_rn(v, (float)mine.b) : 0.0f;
-      const uint32_t split_mask = __ballot_sync(0xffffffffu, valid && split);
-      const uint32_t rep_mask = __ballot_sync(0xffffffffu, valid && mine.a > 1);
-      if (!kBoth && rep_mask == 0) {
-#pragma unroll
-        for (int t = 0; t < 32; t++) {
-          const float y0 = __shfl_sync(0xffffffffu, x0, t);
-          const float y1 = __shfl_sync(0xffffffffu, x1, t);
-          if (t < m) {
-            s = __fadd_rn(s, y0);
-            if ((split_mask >> t) & 1u) s = __fadd_rn(s, y1);
-          }
-        }
-        continue;
-      }
-      for (int t = 0; t < m; t++) {
-        const float lam = __shfl_sync(0xffffffffu, mine.lam, t);
-        const int32_t ia = __shfl_sync(0xffffffffu, mine.a, t);
-        const int32_t ib = __shfl_sync(0xffffffffu, mine.b, t);
-        const float vt = __fsub_rn(lam, b);
-        const double v64 = __dsub_rn((double)lam, (double)b);
-        if (ia < 0) {
-          s = __fadd_rn(s, __fmul_rn(vt, (float)(-ia)));
-          s = __fadd_rn(s, __fmul_rn(vt, (float)ib));
-          if (kBoth) {
-            s64 = __dadd_rn(s64, __dmul_rn(v64, (double)(-ia)));
-            s64 = __dadd_rn(s64, __dmul_rn(v64, (double)ib));
-          }
-        } else if (ia == 1) {  // one row
-          s = __fadd_rn(s, vt);
-          if (kBoth) s64 = __dadd_rn(s64, v64);
-        } else {  // one row per point falling out here
-          s = add_repeated<float>(s, vt, ia);
-          if (kBoth) s64 = add_repeated<double>(s64, v64, ia);
-        }
-      }
+      s = add_warp<float>(s, mine, b, m);
+      if (kBoth) s64 = add_warp<double>(s64, mine, b, m);
     }
     if (lane == 0) {
+      stab[c] = s;
+      stab64[c] = kBoth ? s64 : (double)s;
+    }
+  }
+}
+
+// One block per long chain, 4,096 items a step; a step with a tie or the end
+// of a binade in it is taken again by one warp, 32 items at a time.
+constexpr int kLongThreads = 1024, kLongItems = 4;
+template <typename T>
+struct LongStep {
+  uint64_t steps;
+  double about;
+};
+template <typename T>
+__device__ T add_block(T s, const ChainItem (&mine)[kLongItems], float birth, int64_t base, int64_t e,
+                       const ChainItem *__restrict__ items, LongStep<T> *sh, T *sh_s) {
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  const Binade<T> bin(s);
+  uint64_t steps = 0;
+  double about = 0.0;
+  bool fine = bin.ok;
+#pragma unroll
+  for (int j = 0; j < kLongItems; j++) {
+    if (base + j * kLongThreads + threadIdx.x >= e) continue;
+    const Addends<T> ad(mine[j], birth);
+    fine = fine && bin.take(ad.y0, ad.m0, steps, about) && bin.take(ad.y1, 1, steps, about);
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    steps += __shfl_xor_sync(0xffffffffu, steps, o);
+    about += __shfl_xor_sync(0xffffffffu, about, o);
+  }
+  if (lane == 0) sh[w] = LongStep<T>{steps, about};
+  const bool all = __syncthreads_and(fine);
+  if (all) {
+    steps = sh[lane].steps;
+    about = sh[lane].about;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      steps += __shfl_xor_sync(0xffffffffu, steps, o);
+      about += __shfl_xor_sync(0xffffffffu, about, o);
+    }
+    if (bin.stays(steps, about)) {  // the same in every thread
+      __syncthreads();  // sh is free again
+      return bin.after(steps);
+    }
+  }
+  if (w == 0) {
+    const int64_t end = min(e, base + kLongThreads * kLongItems);
+    for (int64_t i = base; i < end; i += 32) {
+      const ChainItem it = i + lane < end ? items[i + lane] : ChainItem{0.0f, 0, 0, 0};
+      s = add_warp<T>(s, it, birth, (int)min((int64_t)32, end - i));
+    }
+    if (lane == 0) *sh_s = s;
+  }
+  __syncthreads();
+  s = *sh_s;
+  __syncthreads();
+  return s;
+}
+
+template <bool kBoth>
+__global__ void __launch_bounds__(kLongThreads)
+    k_stability_long(const int32_t *__restrict__ long_list, const int32_t *__restrict__ long_count,
+                     const int64_t *__restrict__ seg_start, const int64_t *__restrict__ seg_end,
+                     const ChainItem *__restrict__ items, const float *__restrict__ birth,
+                     float *__restrict__ stab, double *__restrict__ stab64) {
+  static_assert(kLongThreads == 32 * 32, "one partial sum per lane");
+  __shared__ LongStep<double> sh[32];
+  __shared__ double sh_s;
+  const int32_t count = *long_count;
+  for (int32_t l = blockIdx.x; l < count; l += gridDim.x) {
+    const int32_t c = long_list[l];
+    const int64_t s0 = seg_start[c], e = seg_end[c];
+    const float b = birth[c];
+    float s = 0.0f;
+    double s64 = 0.0;
+    ChainItem next[kLongItems];
+    auto load = [&](int64_t base) {
+#pragma unroll
+      for (int j = 0; j < kLongItems; j++) {
+        const int64_t i = base + j * kLongThreads + threadIdx.x;
+        if (i < e) next[j] = items[i];
+      }
+    };
+    load(s0);
+    for (int64_t base = s0; base < e; base += kLongThreads * kLongItems) {
+      ChainItem mine[kLongItems];
+#pragma unroll
+      for (int j = 0; j < kLongItems; j++) mine[j] = next[j];
+      load(base + kLongThreads * kLongItems);
+      s = add_block<float>(s, mine, b, base, e, items, reinterpret_cast<LongStep<float> *>(sh),
+                           reinterpret_cast<float *>(&sh_s));
+      if (kBoth) s64 = add_block<double>(s64, mine, b, base, e, items, sh, &sh_s);
+    }
+    if (threadIdx.x == 0) {
       stab[c] = s;
       stab64[c] = kBoth ? s64 : (double)s;
     }
@@ -1001,10 +1164,17 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
     Buf<ChainItem> items(ctx, nv_total);
     k_chain_items<<<grid_for(ctx, nv_total, 256), 256, 0, st>>>(t, chain, nv_total, kind, lam,
                                                                 items); ctx->launches++;
-    if (stab_mode == HDB_STAB_FP64)
-      k_stability<true><<<grid_for(ctx, C, 4), 128, 0, st>>>(C, s0, s1, items, birth, stab, stab64);
-    else
-      k_stability<false><<<grid_for(ctx, C, 4), 128, 0, st>>>(C, s0, s1, items, birth, stab, stab64);
+    // at most m / kLongChain clusters have a long chain
+    Buf<int32_t> long_list(ctx, m / kLongChain + 1), long_count(ctx, 1);
+    HDB_CUDA(cudaMemsetAsync(long_count, 0, sizeof(int32_t), st));
+    const int gs = grid_for(ctx, C, 4), gl = (int)std::min<int64_t>(m / kLongChain, 2 * ctx->num_sms);
+    auto warps = stab_mode == HDB_STAB_FP64 ? k_stability<true> : k_stability<false>;
+    auto blocks = stab_mode == HDB_STAB_FP64 ? k_stability_long<true> : k_stability_long<false>;
+    warps<<<gs, 128, 0, st>>>(C, s0, s1, items, birth, stab, stab64, long_list, long_count);
+    if (gl > 0) {
+      blocks<<<gl, kLongThreads, 0, st>>>(long_list, long_count, s0, s1, items, birth, stab, stab64);
+      ctx->launches++;
+    }
     ctx->launches++;
     HDB_CHECK_LAUNCH();
   }
