@@ -569,10 +569,10 @@ __device__ __forceinline__ void merge_row(int64_t row, int k, int32_t &lab, floa
 // in which rows arrive decides whose reverse samples are taken (a row keeps the
 // first S).  It follows the blocks that are resident together -- the grid's
 // first five per SM walk through all their rows before the others start -- so
-// unused shared memory (kSampleRoom) keeps it at five blocks whatever the
-// compiler makes of the registers: another order gives graphs as good, but
-// other ones.
-constexpr size_t kSampleRoom = 28 * 1024;
+// the shared memory's share of L1 (kSampleShare, 64 KB for 12 KB a block) keeps
+// it at five blocks whatever the compiler makes of the registers: another order
+// gives graphs as good, but other ones.
+constexpr int kSampleShare = 28;  // per cent
 __global__ void k_sample(int64_t n, int k, int S, int do_merge, int32_t *__restrict__ gid,
                          float *__restrict__ gdist, float *__restrict__ worst, RowList rl,
                          unsigned long long *counters, SampleOut so, int64_t split) {
@@ -1545,7 +1545,8 @@ struct NndState {
   // the samples of an iteration; after the first, of the rows merged with the
   // candidates of the join before
   void sample(Context *ctx, bool merge, int64_t split) {
-    k_sample<<<grid_for(ctx, n, 8, 16), 256, kSampleRoom, ctx->stream>>>(
+    HDB_CUDA(cudaFuncSetAttribute(k_sample, cudaFuncAttributePreferredSharedMemoryCarveout, kSampleShare));
+    k_sample<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(
         n, k, S, merge, gid, gdist, worst, rl, counters, samples(), split);
     ctx->launches++;
     HDB_CHECK_LAUNCH();
