@@ -76,7 +76,8 @@ class Context:
 
     def set_join_tiles(self, tiles: int):
         """FP32 local join form: 1 or 2 distance tiles of 4 x 4 per lane, or 0
-        to time both per shape and keep the faster (the default)."""
+        (the default): by rows up to 28 dimensions, beyond both tile forms are
+        timed per shape and the faster is kept."""
         _lib.check(self.L.hdb_set_join_tiles(self.h, int(tiles)))
 
     def close(self):

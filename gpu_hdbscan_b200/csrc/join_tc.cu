@@ -701,8 +701,10 @@ __device__ void epilogue(const JoinArgs &a, Shared &sh, uint32_t tmem, int64_t n
     const float d1 = __uint_as_float(k1 & ~63u), d2 = __uint_as_float(k2 & ~63u);
     const bool c1 = vrow && id1 >= 0 && d1 < wst;
     const bool c2 = !isnew && lane < nn && id2 >= 0 && d2 < wst2;
-    cands += append_candidates(a.cl, cur, c1, myid, pack(d1, id1), c2, tgt2,
-                               pack(d2, id2));
+    const bool av[2] = {c1, c2};
+    const int32_t at[2] = {myid, tgt2};
+    const uint64_t ak[2] = {pack(d1, id1), pack(d2, id2)};
+    cands += append_candidates(a.cl, cur, av, at, ak);
   }
   if (!kProbe) list_fill(a.cl, cur.pos, cur.end);  // the rest of the last chunk
 }

@@ -682,17 +682,70 @@ __global__ void k_bucket_bounds(const uint32_t *__restrict__ tgt,
 }
 
 // ---- FP32 local join -----------------------------------------------------
-// Shared memory of one warp: best candidates (u64: best other-new and best old
-// per new row; best new per old row) | slot ids | one chunk of kJc dimensions
+// Shared memory of one warp: best candidates (distance bits, then ids: best
+// other-new and best old per new row; best new per old row) | slot ids | one chunk of kJc dimensions
 // of every staged row.  Rows are staged a chunk at a time, so a warp needs
 // ~9 KB whatever d is and an SM keeps 16 warps of joins in flight.
 constexpr int kJc = 32;              // dimensions per staged chunk
 constexpr int kJoinWarps = 8;
 struct JoinSmem {
-  static constexpr int kBest = 96;   // u64 entries
+  static constexpr int kBest = 96;   // distances and ids
   static constexpr int kIds = 64;
   static constexpr size_t kBytes = kBest * 8 + kIds * 4 + (size_t)64 * kJc * 4;
 };
+
+// A row's counts and both sample lists in one memory round trip, loaded one row
+// ahead so that they are in flight while the previous row is joined.
+struct SlotLists {
+  int32_t nraw = 0, oraw = 0;
+  int cnf = 0, cof = 0, cnr = 0, cor = 0;
+  __device__ __forceinline__ void load(int64_t r, int64_t n, int S, const int32_t *__restrict__ newS,
+                                       const int32_t *__restrict__ oldS, const int8_t *__restrict__ nf,
+                                       const int8_t *__restrict__ of, const int32_t *nrev,
+                                       const int32_t *orev) {
+    if (r >= n) return;
+    const int lane = lane_id();
+    const int64_t sb = r * (2 * S);
+    nraw = lane < 2 * S ? newS[sb + lane] : 0;
+    oraw = lane < 2 * S ? oldS[sb + lane] : 0;
+    cnf = nf[r];
+    cof = of[r];
+    cnr = nrev[r];
+    cor = orev[r];
+  }
+  // The slots in use: new rows into ids[0..nn), old ones into ids[32..32+no).
+  __device__ __forceinline__ void compact(int S, int32_t *ids, int &nn, int &no) const {
+    const int lane = lane_id();
+    const int nr = min(cnr, S), orv = min(cor, S);
+    // slot t < S: forward sample t; slot S + t: reverse sample t
+    bool vn = (lane < S) ? (lane < cnf) : (lane < 2 * S && lane - S < nr);
+    bool vo = (lane < S) ? (lane < cof) : (lane < 2 * S && lane - S < orv);
+    const int32_t nid = vn ? nraw : -1 - lane;
+    const int32_t oid = vo ? oraw : -100 - lane;
+    // de-duplicate (ShrinkGraph RemoveDuplicates, :285-291)
+    const uint32_t pn = __match_any_sync(0xffffffffu, nid);
+    vn = vn && (__ffs(pn) - 1 == lane);
+    const uint32_t po = __match_any_sync(0xffffffffu, oid);
+    vo = vo && (__ffs(po) - 1 == lane);
+    const uint32_t bo = __ballot_sync(0xffffffffu, vo);
+    no = __popc(bo);
+    if (vo) ids[32 + __popc(bo & lanemask_lt())] = oid;
+    __syncwarp();
+    // new \ old (:468-486)
+    bool in_old = false;  // independent reads, not a chain
+#pragma unroll 8
+    for (int t = 0; t < no; t++) in_old |= ids[32 + t] == nid;
+    vn = vn && !in_old;
+    const uint32_t bn = __ballot_sync(0xffffffffu, vn);
+    nn = __popc(bn);
+    if (vn) ids[__popc(bn & lanemask_lt())] = nid;
+    __syncwarp();
+  }
+};
+
+// floor(x / m) for 1 <= m <= 8 and 0 <= x < 1024: x * ceil(2^16 / m) >> 16.
+__constant__ uint32_t kRecip[9] = {0, 65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192};
+__device__ __forceinline__ int div_small(int x, int m) { return (int)(((uint32_t)x * kRecip[m]) >> 16); }
 
 // Float offset of 16-byte piece q of staged row r: the pieces of a row are
 // permuted by the row's group of four, so the rows one warp-wide 16-byte load
@@ -719,7 +772,7 @@ __device__ __forceinline__ void stage_chunk(const float *__restrict__ X, int d, 
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   } else if (vec) {
     for (int it = lane; it < items; it += 32) {
-      const int r = it / nq, q = it - r * nq;
+      const int r = div_small(it, nq), q = it - r * nq;
       const int slot = r < nn ? r : 32 + (r - nn);
       const float *src = X + (int64_t)ids[slot] * d + c0 + 4 * q;
       const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + stage_off(slot, q));
@@ -728,7 +781,7 @@ __device__ __forceinline__ void stage_chunk(const float *__restrict__ X, int d, 
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
   } else {
     for (int it = lane; it < items; it += 32) {
-      const int r = it / nq, q = it - r * nq;
+      const int r = div_small(it, nq), q = it - r * nq;
       const int slot = r < nn ? r : 32 + (r - nn);
       const float *src = X + (int64_t)ids[slot] * d;
       float4 v;
@@ -751,14 +804,18 @@ __device__ __forceinline__ void stage_chunk(const float *__restrict__ X, int d, 
 __device__ __forceinline__ int tile_of(int t, int rg, int cgn, int cgo, int &r0, int &c0) {
   const int tri = cgn > 0 ? rg * (rg + 1) / 2 : 0;
   if (t < tri) {
-    int i = 0;
-    while (t >= rg - i) { t -= rg - i; i++; }
+    int i = 0, first = 0;  // row group i holds tiles first .. first + rg - i - 1
+#pragma unroll
+    for (int r = 1; r < 8; r++) {
+      const int f = r * rg - r * (r - 1) / 2;
+      if (r < rg && t >= f) { i = r; first = f; }
+    }
     r0 = 4 * i;
-    c0 = 4 * (i + t);
-    return t == 0 ? 1 : 2;
+    c0 = 4 * (i + t - first);
+    return t == first ? 1 : 2;
   }
   t -= tri;
-  const int i = t / cgo;
+  const int i = div_small(t, cgo);
   r0 = 4 * i;
   c0 = 32 + 4 * (t - i * cgo);
   return 3;
@@ -769,10 +826,13 @@ __device__ __forceinline__ int tile_of(int t, int rg, int cgn, int cgo, int &r0,
 // kJoinTiles per lane; a lane keeps its tiles' sums in registers while the
 // rows pass through shared memory a chunk of kJc dimensions at a time, so
 // every pair is the reference's sequential FP32 difference sum over
-// j = 0..d-1.  Tile row/column minima go to the per-row best candidates with
-// one 64-bit shared-memory atomicMin each: every new neighbour gets its closest
+// j = 0..d-1.  The tiles' row and column minima meet in shared memory: first
+// the least distance of every slot (its bits, a 32-bit atomicMin), then, among the
+// pairs at that distance, the least id.  Every new neighbour gets its closest
 // other new one and its closest old one, every old neighbour its closest new
-// one.  cross_only (the merge join, TiledNewOldNeighborsCompareKernelForMerge
+// one.  (One 64-bit atomicMin of distance and id per tile row and column, which
+// is a compare-and-swap loop in shared memory, took about 1,000 of the 2,500
+// instructions of a row-join at d = 12.)  cross_only (the merge join, TiledNewOldNeighborsCompareKernelForMerge
 // :1328-1383 launched without the new x new kernel, UpdateGraphForMerge
 // :1582-1640) leaves out the new x new tiles: new neighbours get their closest
 // old one only.
@@ -789,64 +849,28 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
   unsigned char *base = smem_join + (threadIdx.x >> 5) * JoinSmem::kBytes;
-  unsigned long long *best = reinterpret_cast<unsigned long long *>(base);
-  unsigned long long *best1 = best, *best2 = best + 32, *best3 = best + 64;
+  uint32_t *bdist = reinterpret_cast<uint32_t *>(base);
+  uint32_t *bid = bdist + JoinSmem::kBest;
   int32_t *ids = reinterpret_cast<int32_t *>(base + JoinSmem::kBest * 8);
   float *Xs = reinterpret_cast<float *>(base + JoinSmem::kBest * 8 + JoinSmem::kIds * 4);
   const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
   unsigned long long w_rows = 0, w_cands = 0, w_pairs = 0;
   ListCursor cur;  // this warp's space in the candidate list
   const int64_t stride = (int64_t)gridDim.x * wpb;
-  // a row's counts and both sample lists in one memory round trip, loaded one
-  // row ahead so that they are in flight while the previous row is joined
-  int32_t q_nraw = 0, q_oraw = 0;
-  int q_cnf = 0, q_cof = 0, q_cnr = 0, q_cor = 0;
-  auto load_lists = [&](int64_t r) {
-    if (r >= n) return;
-    const int64_t sb = r * (2 * S);
-    q_nraw = lane < 2 * S ? newS[sb + lane] : 0;
-    q_oraw = lane < 2 * S ? oldS[sb + lane] : 0;
-    q_cnf = nf[r];
-    q_cof = of[r];
-    q_cnr = nrev[r];
-    q_cor = orev[r];
-  };
+  SlotLists lists;
   int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5);
-  load_lists(row);
+  lists.load(row, n, S, newS, oldS, nf, of, nrev, orev);
   for (; row < n; row += stride) {
-    const int32_t nraw = q_nraw, oraw = q_oraw;
-    const int cnf = q_cnf, cof = q_cof;
-    const int cnr = min(q_cnr, S), cor = min(q_cor, S);
-    load_lists(row + stride);
-    __syncwarp();
-    if (lane == 0) { nrev[row] = 0; orev[row] = 0; }
-    // slot t < S: forward sample t; slot S + t: reverse sample t
-    bool vn = (lane < S) ? (lane < cnf) : (lane < 2 * S && lane - S < cnr);
-    bool vo = (lane < S) ? (lane < cof) : (lane < 2 * S && lane - S < cor);
-    const int32_t nid = vn ? nraw : -1 - lane;
-    const int32_t oid = vo ? oraw : -100 - lane;
-    // de-duplicate (ShrinkGraph RemoveDuplicates, :285-291)
-    const uint32_t pn = __match_any_sync(0xffffffffu, nid);
-    vn = vn && (__ffs(pn) - 1 == lane);
-    const uint32_t po = __match_any_sync(0xffffffffu, oid);
-    vo = vo && (__ffs(po) - 1 == lane);
-    const uint32_t bo = __ballot_sync(0xffffffffu, vo);
-    const int no = __popc(bo);
-    if (vo) ids[32 + __popc(bo & lanemask_lt())] = oid;
-    __syncwarp();
-    // new \ old (:468-486)
+    int nn, no;
     {
-      bool in_old = false;  // independent reads, not a chain
-#pragma unroll 8
-      for (int t = 0; t < no; t++) in_old |= ids[32 + t] == nid;
-      vn = vn && !in_old;
+      const SlotLists mine = lists;
+      lists.load(row + stride, n, S, newS, oldS, nf, of, nrev, orev);
+      __syncwarp();
+      if (lane == 0) { nrev[row] = 0; orev[row] = 0; }
+      mine.compact(S, ids, nn, no);
     }
-    const uint32_t bn = __ballot_sync(0xffffffffu, vn);
-    const int nn = __popc(bn);
-    if (vn) ids[__popc(bn & lanemask_lt())] = nid;
-    best1[lane] = ~0ull;
-    best2[lane] = ~0ull;
-    best3[lane] = ~0ull;
+#pragma unroll
+    for (int g = 0; g < JoinSmem::kBest; g += 32) bdist[g + lane] = bid[g + lane] = 0xffffffffu;
     __syncwarp();
     if (nn == 0 || nn + no < 2 || (cross_only && no == 0)) continue;
     w_rows += nn + no;
@@ -854,6 +878,7 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
     const int rg = (nn + 3) >> 2;                              // row groups (new rows)
     const int cgn = cross_only ? 0 : rg, cgo = (no + 3) >> 2;  // column groups: new, old
     const int tiles = (cgn > 0 ? rg * (rg + 1) / 2 : 0) + rg * cgo;
+    uint32_t before[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
     // up to 32 * kTiles tiles per pass through the rows (rows with more
     // samples take further passes; at most 100 tiles)
     for (int t0 = 0; t0 < tiles; t0 += 32 * kTiles) {
@@ -861,6 +886,8 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
       float acc[kTiles][4][4];
 #pragma unroll
       for (int u = 0; u < kTiles; u++) {
+        kind[u] = r0[u] = c0[u] = 0;
+        if (t0 + 32 * u >= tiles) continue;  // for the whole warp
         const int t = t0 + lane + 32 * u;
         kind[u] = t < tiles ? tile_of(t, rg, cgn, cgo, r0[u], c0[u]) : 0;
         if (kind[u] == 0) { r0[u] = 0; c0[u] = 0; }
@@ -875,7 +902,7 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
         stage_chunk(X, d, cd, nq, ids, nn, no, Xs, vec);
 #pragma unroll
         for (int u = 0; u < kTiles; u++) {
-          if (kind[u] == 0) continue;
+          if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
           // the four rows of a tile side share one piece permutation
           const int ka = (r0[u] >> 2) & 7, kc = (c0[u] >> 2) & 7;
           for (int q = 0; q < nq; q++) {
@@ -900,53 +927,82 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
           }
         }
       }
-      // tile minima -> per-row best candidates
+      // the least distances; what is no pair of the join gets all ones
 #pragma unroll
       for (int u = 0; u < kTiles; u++) {
-        if (kind[u] == 0) continue;
+        if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
         const bool oldcols = kind[u] == 3;
-        const int ncol = oldcols ? no : nn;
         const int cb = oldcols ? c0[u] - 32 : c0[u];  // first column within its block
-        uint64_t colmin[4] = {~0ull, ~0ull, ~0ull, ~0ull};
+        const int nr = nn - r0[u], nc = (oldcols ? no : nn) - cb;
+        uint32_t cmin[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+        uint32_t *rows = bdist + (oldcols ? 32 : 0) + r0[u];
+        uint32_t *cols = bdist + (oldcols ? 64 : 0) + cb;
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          const int a = r0[u] + i;
-          if (a >= nn) continue;
-          uint64_t rmin = ~0ull;
+          uint32_t rmin = 0xffffffffu;
 #pragma unroll
           for (int j = 0; j < 4; j++) {
-            const int c = cb + j;
-            if (c >= ncol || (kind[u] == 1 && c == a)) continue;
-            const uint64_t kr = pack(acc[u][i][j], ids[c0[u] + j]);
-            rmin = kr < rmin ? kr : rmin;
-            if (kind[u] != 1) {
-              const uint64_t kc = pack(acc[u][i][j], ids[a]);
-              colmin[j] = kc < colmin[j] ? kc : colmin[j];
-            }
+            uint32_t v = __float_as_uint(acc[u][i][j]);
+            if (i >= nr || j >= nc || (i == j && kind[u] == 1)) v = 0xffffffffu;
+            acc[u][i][j] = __uint_as_float(v);
+            rmin = min(rmin, v);
+            cmin[j] = min(cmin[j], v);
           }
-          if (rmin != ~0ull) atomicMin(oldcols ? &best2[a] : &best1[a], (unsigned long long)rmin);
+          if (i < nr) atomicMin(&rows[i], rmin);
         }
         if (kind[u] != 1) {
 #pragma unroll
           for (int j = 0; j < 4; j++)
-            if (colmin[j] != ~0ull)
-              atomicMin(oldcols ? &best3[cb + j] : &best1[cb + j], (unsigned long long)colmin[j]);
+            if (j < nc) atomicMin(&cols[j], cmin[j]);
+        }
+      }
+      __syncwarp();
+      if (t0 > 0) {  // a slot whose least distance this pass has lowered starts over
+#pragma unroll
+        for (int g = 0; g < 3; g++) {
+          const uint32_t now = bdist[32 * g + lane];
+          if (now != before[g]) bid[32 * g + lane] = 0xffffffffu;
+        }
+        __syncwarp();
+      }
+#pragma unroll
+      for (int g = 0; g < 3; g++) before[g] = bdist[32 * g + lane];
+      // the least ids at those distances
+#pragma unroll
+      for (int u = 0; u < kTiles; u++) {
+        if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
+        const bool oldcols = kind[u] == 3;
+        const int cb = oldcols ? c0[u] - 32 : c0[u];
+        const int rat = (oldcols ? 32 : 0) + r0[u], cat = (oldcols ? 64 : 0) + cb;
+        const uint4 rm = *reinterpret_cast<const uint4 *>(bdist + rat);
+        const uint4 cm = *reinterpret_cast<const uint4 *>(bdist + cat);
+        const uint32_t rms[4] = {rm.x, rm.y, rm.z, rm.w}, cms[4] = {cm.x, cm.y, cm.z, cm.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const uint32_t v = __float_as_uint(acc[u][i][j]);
+            if (v == 0xffffffffu) continue;
+            if (v == rms[i]) atomicMin(&bid[rat + i], (uint32_t)ids[c0[u] + j]);
+            if (v == cms[j] && kind[u] != 1) atomicMin(&bid[cat + j], (uint32_t)ids[r0[u] + i]);
+          }
         }
       }
     }  // passes
     __syncwarp();
     // the candidates that can enter their target's list go to the candidate
     // list (space reserved a chunk at a time; no returning atomic per candidate)
-    const int32_t x = lane < nn ? ids[lane] : 0;
-    const uint64_t b1 = lane < nn ? best1[lane] : ~0ull, b2 = lane < nn ? best2[lane] : ~0ull;
-    const float wx = lane < nn ? worst[x] : 0.0f;
-    const int32_t x3 = lane < no ? ids[32 + lane] : 0;
-    const uint64_t b3 = lane < no ? best3[lane] : ~0ull;
-    const float wx3 = lane < no ? worst[x3] : 0.0f;
-    const bool v1 = b1 != ~0ull && pk_dist(b1) < wx, v2 = b2 != ~0ull && pk_dist(b2) < wx;
-    const bool v3 = b3 != ~0ull && pk_dist(b3) < wx3;
-    w_cands += append_candidates(cl, cur, v1, x, b1, v2, x, b2);
-    w_cands += append_candidates(cl, cur, v3, x3, b3, false, 0, 0ull);
+    const int32_t x = lane < nn ? ids[lane] : 0, x3 = lane < no ? ids[32 + lane] : 0;
+    const uint32_t d1 = bdist[lane], d2 = bdist[32 + lane], d3 = bdist[64 + lane];
+    const float wx = lane < nn ? worst[x] : 0.0f, wx3 = lane < no ? worst[x3] : 0.0f;
+    auto key = [&](uint32_t dist, int at) { return ((uint64_t)dist << 32) | bid[at]; };
+    const bool v1 = lane < nn && d1 != 0xffffffffu && __uint_as_float(d1) < wx;
+    const bool v2 = lane < nn && d2 != 0xffffffffu && __uint_as_float(d2) < wx;
+    const bool v3 = lane < no && d3 != 0xffffffffu && __uint_as_float(d3) < wx3;
+    const bool av[3] = {v1, v2, v3};
+    const int32_t at[3] = {x, x, x3};
+    const uint64_t ak[3] = {key(d1, lane), key(d2, 32 + lane), key(d3, 64 + lane)};
+    w_cands += append_candidates(cl, cur, av, at, ak);
     __syncwarp();
   }
   list_fill(cl, cur.pos, cur.end);  // the rest of the last chunk
@@ -959,6 +1015,196 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
     if (w_pairs) atomicAdd(&cl.counters[4], w_pairs);
   }
 }
+
+// ---- FP32 local join of short rows ------------------------------------------
+// The same join for d <= 28 (kQ = ceil(d / 4) 16-byte pieces a row): with so
+// few dimensions the sums are a small part of the work, and what the tiles need
+// around them (the tiles' places, their minima meeting in shared memory) is
+// more than they save.  Here a lane holds one new row in registers and takes the
+// other staged rows one after the other, each read by all lanes at once; the
+// row's closest new and old rows are running minima of the lane, an old row's
+// closest new row is a minimum over the warp.  With at most 16 (8) new rows the
+// warp's halves (quarters) take every second (fourth) staged row.  Bound by
+// instruction issue (76 % of the slots at 1M x 12, 1,670 warp instructions a
+// row-join, against 2,040 at 56 % in tiles).
+//
+// Where the line lies, by the join time of six iterations, rows against the
+// better of the tile forms: 1M points, k = 32: d = 8 9.7 / 14.9 ms, 12 12.2 /
+// 17.4, 16 15.6 / 18.9, 24 19.2 / 22.2, 28 21.4 / 24.1, 32 27.4 / 24.9; 300k,
+// k = 16: d = 31 4.74 / 4.74 ms; 50k x 8, k = 16: 0.40 / 0.58; 1,500 x 8: 0.077 /
+// 0.083.
+constexpr int kRowJoinMaxDim = 28;
+
+template <int kQ>
+__device__ __forceinline__ float row_dist(const float4 *__restrict__ b, const float4 (&own)[kQ]) {
+  float s = 0.0f;
+#pragma unroll
+  for (int q = 0; q < kQ; q++) {
+    const float4 x = b[q];
+    const float2 d01 = neg_diff2(make_float2(x.x, x.y), make_float2(own[q].x, own[q].y));
+    const float2 d23 = neg_diff2(make_float2(x.z, x.w), make_float2(own[q].z, own[q].w));
+    s = __fmaf_rn(d01.x, d01.x, s);
+    s = __fmaf_rn(d01.y, d01.y, s);
+    s = __fmaf_rn(d23.x, d23.x, s);
+    s = __fmaf_rn(d23.y, d23.y, s);
+  }
+  return s;
+}
+
+template <int kQ>
+__global__ void __launch_bounds__(32 * kJoinWarps, kQ <= 4 ? 4 : 3)
+    k_join_rows(const float *__restrict__ X, int64_t n, int d, int S, const int32_t *__restrict__ newS,
+                const int32_t *__restrict__ oldS, const int8_t *__restrict__ nf,
+                const int8_t *__restrict__ of, int32_t *__restrict__ nrev, int32_t *__restrict__ orev,
+                const float *__restrict__ worst, CandList cl, int cross_only) {
+  extern __shared__ __align__(16) unsigned char smem_join[];
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  constexpr size_t kWarpBytes = (size_t)64 * kQ * 16 + 64 * 4;
+  float4 *Xs = reinterpret_cast<float4 *>(smem_join + w * kWarpBytes);  // new rows, then old ones
+  int32_t *ids = reinterpret_cast<int32_t *>(smem_join + w * kWarpBytes + (size_t)64 * kQ * 16);
+  const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+  unsigned long long w_rows = 0, w_cands = 0, w_pairs = 0;
+  ListCursor cur;
+  const int64_t stride = (int64_t)gridDim.x * kJoinWarps;
+  SlotLists lists;
+  int64_t row = (int64_t)blockIdx.x * kJoinWarps + w;
+  lists.load(row, n, S, newS, oldS, nf, of, nrev, orev);
+  for (; row < n; row += stride) {
+    int nn, no;
+    {
+      const SlotLists mine = lists;
+      lists.load(row + stride, n, S, newS, oldS, nf, of, nrev, orev);
+      __syncwarp();
+      if (lane == 0) { nrev[row] = 0; orev[row] = 0; }
+      mine.compact(S, ids, nn, no);
+    }
+    if (nn == 0 || nn + no < 2 || (cross_only && no == 0)) continue;
+    w_rows += nn + no;
+    w_pairs += (cross_only ? 0 : nn * (nn - 1) / 2) + nn * no;  // the reference's pairs
+    const int T = nn + no;
+    if (vec) {
+      for (int it = lane; it < T * kQ; it += 32) {
+        const int r = it / kQ, q = it - r * kQ;
+        const float *src = X + (int64_t)ids[r < nn ? r : 32 + r - nn] * d + 4 * q;
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + it);
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
+      }
+      asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    } else {
+      for (int it = lane; it < T * kQ; it += 32) {
+        const int r = it / kQ, c = 4 * (it - r * kQ);
+        const float *src = X + (int64_t)ids[r < nn ? r : 32 + r - nn] * d;
+        float4 v;  // zero padded: fmaf(0, 0, s) = s
+        v.x = c < d ? __ldg(src + c) : 0.0f;
+        v.y = c + 1 < d ? __ldg(src + c + 1) : 0.0f;
+        v.z = c + 2 < d ? __ldg(src + c + 2) : 0.0f;
+        v.w = c + 3 < d ? __ldg(src + c + 3) : 0.0f;
+        Xs[it] = v;
+      }
+    }
+    __syncwarp();
+    // lane -> new row a, and the part g of the staged rows that it takes
+    const int lgp = nn <= 8 ? 3 : nn <= 16 ? 4 : 5;
+    const int P = 1 << lgp, h = 32 >> lgp, a = lane & (P - 1), g = lane >> lgp;
+    float4 own[kQ];
+#pragma unroll
+    for (int q = 0; q < kQ; q++) own[q] = Xs[(a < nn ? a : 0) * kQ + q];
+    // running minima: distance bits and the slot; equal distances are settled
+    // below by the ids, in a second walk that compares both
+    uint32_t m1 = 0xffffffffu, m2 = 0xffffffffu, m3 = 0xffffffffu;
+    int i1 = 0, i2 = 0;
+    bool tie = false;
+    const bool isrow = a < nn;
+    if (!cross_only) {
+#pragma unroll 4
+      for (int c = g; c < nn; c += h) {
+        uint32_t v = __float_as_uint(row_dist<kQ>(Xs + c * kQ, own));
+        if (c == a) v = 0xffffffffu;
+        tie = tie || (v == m1 && c != a);  // the own column is not one
+        if (v < m1) { m1 = v; i1 = c; }
+      }
+    }
+    uint32_t at3 = 0;  // the new rows at the held old row's least distance
+    if (h == 1) {
+#pragma unroll 4
+      for (int c = 0; c < no; c++) {
+        uint32_t v = __float_as_uint(row_dist<kQ>(Xs + (nn + c) * kQ, own));
+        if (!isrow) v = 0xffffffffu;
+        tie = tie || v == m2;
+        if (v < m2) { m2 = v; i2 = c; }
+        const uint32_t least = __reduce_min_sync(0xffffffffu, v);
+        const uint32_t at = __ballot_sync(0xffffffffu, v == least);
+        if (lane == c) { m3 = least; at3 = at; }
+      }
+    } else {
+      const uint32_t part = ((1u << P) - 1u) << (g << lgp);
+      for (int c0 = 0; c0 < no; c0 += h) {  // every part the same number of steps
+        const int c = c0 + g;
+        uint32_t v = 0xffffffffu;
+        if (c < no && isrow) v = __float_as_uint(row_dist<kQ>(Xs + (nn + c) * kQ, own));
+        tie = tie || v == m2;
+        if (v < m2) { m2 = v; i2 = c; }
+        uint32_t least = v;
+        for (int o = P >> 1; o; o >>= 1) least = min(least, __shfl_xor_sync(0xffffffffu, least, o));
+        const uint32_t at = __ballot_sync(0xffffffffu, v == least) & part;
+        if (a == c0 >> (5 - lgp)) { m3 = least; at3 = at; }  // lane c / h of the part keeps it
+      }
+    }
+    tie = tie && isrow;
+    const int i3 = (__ffs(at3) - 1) & (P - 1);
+    tie = tie || ((at3 & (at3 - 1)) != 0 && m3 != 0xffffffffu);
+    for (int o = P; o < 32; o <<= 1) {  // the parts of one new row
+      const uint32_t o1 = __shfl_xor_sync(0xffffffffu, m1, o), o2 = __shfl_xor_sync(0xffffffffu, m2, o);
+      const int p1 = __shfl_xor_sync(0xffffffffu, i1, o), p2 = __shfl_xor_sync(0xffffffffu, i2, o);
+      tie = tie || (isrow && ((o1 == m1 && m1 != 0xffffffffu) || (o2 == m2 && m2 != 0xffffffffu)));
+      if (o1 < m1) { m1 = o1; i1 = p1; }
+      if (o2 < m2) { m2 = o2; i2 = p2; }
+    }
+    int32_t id1 = ids[i1], id2 = ids[32 + (i2 & 31)], id3 = ids[i3];
+    const int c3 = (a << (5 - lgp)) + g;  // the held old row
+    if (__any_sync(0xffffffffu, tie)) {
+      // the least id at each least distance
+      uint32_t b1 = 0xffffffffu, b2 = 0xffffffffu, b3 = 0xffffffffu;
+      if (!cross_only)
+        for (int c = 0; c < nn; c++) {
+          const uint32_t v = __float_as_uint(row_dist<kQ>(Xs + c * kQ, own));
+          if (c != a && v == m1) b1 = min(b1, (uint32_t)ids[c]);
+        }
+      for (int c = 0; c < no; c++) {
+        const uint32_t v = __float_as_uint(row_dist<kQ>(Xs + (nn + c) * kQ, own));
+        if (v == m2) b2 = min(b2, (uint32_t)ids[32 + c]);
+        // lane l of the first part speaks for new row l
+        const int holder = ((c & (h - 1)) << lgp) + (c >> (5 - lgp));
+        const uint32_t least = __shfl_sync(0xffffffffu, m3, holder);
+        const uint32_t id = __reduce_min_sync(0xffffffffu, isrow && v == least ? (uint32_t)ids[a] : 0xffffffffu);
+        if (lane == holder) b3 = id;
+      }
+      id1 = (int32_t)b1;
+      id2 = (int32_t)b2;
+      id3 = (int32_t)b3;
+    }
+    const bool first = g == 0 && isrow, holds = c3 < no;
+    const int32_t x = first ? ids[a] : 0, x3 = holds ? ids[32 + c3] : 0;
+    const float wx = first ? worst[x] : 0.0f, wx3 = holds ? worst[x3] : 0.0f;
+    const bool av[3] = {first && m1 != 0xffffffffu && __uint_as_float(m1) < wx,
+                        first && m2 != 0xffffffffu && __uint_as_float(m2) < wx,
+                        holds && m3 != 0xffffffffu && __uint_as_float(m3) < wx3};
+    const int32_t at[3] = {x, x, x3};
+    const uint64_t ak[3] = {pack(__uint_as_float(m1), id1), pack(__uint_as_float(m2), id2),
+                            pack(__uint_as_float(m3), id3)};
+    w_cands += append_candidates(cl, cur, av, at, ak);
+    __syncwarp();
+  }
+  list_fill(cl, cur.pos, cur.end);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) w_cands += __shfl_xor_sync(0xffffffffu, w_cands, o);
+  if (lane == 0) {
+    if (w_rows) atomicAdd(&cl.counters[1], w_rows);
+    if (w_cands) atomicAdd(&cl.counters[2], w_cands);
+    if (w_pairs) atomicAdd(&cl.counters[4], w_pairs);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // BF16 tensor-core form of the local join.
 //
@@ -1244,8 +1490,10 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
     const float wx = lane < nn ? worst[x] : 0.0f, wx3 = lane < no ? worst[x3] : 0.0f;
     const bool v1 = b1 != ~0ull && pk_dist(b1) < wx, v2 = b2 != ~0ull && pk_dist(b2) < wx;
     const bool v3 = b3 != ~0ull && pk_dist(b3) < wx3;
-    w_cands += append_candidates(cl, cur, v1, x, b1, v2, x, b2);
-    w_cands += append_candidates(cl, cur, v3, x3, b3, false, 0, 0ull);
+    const bool av[3] = {v1, v2, v3};
+    const int32_t at[3] = {x, x, x3};
+    const uint64_t ak[3] = {b1, b2, b3};
+    w_cands += append_candidates(cl, cur, av, at, ak);
     __syncwarp();
   }
   list_fill(cl, cur.pos, cur.end);
@@ -1579,15 +1827,33 @@ struct NndState {
 
 // Warps of the joins that append to the list.
 int64_t fp32_join_warps(const Context *ctx, int64_t n) {
-  return (int64_t)kJoinWarps * grid_for(ctx, n, kJoinWarps, 3);
+  return (int64_t)kJoinWarps * grid_for(ctx, n, kJoinWarps, 4);
 }
 int64_t tc_join_warps(const Context *ctx, int64_t n) {
   return 4 * std::min<int64_t>((n + 1) / 2, 2 * (int64_t)ctx->num_sms);
 }
 
-// One FP32 local join over s's samples with `tiles` 4 x 4 tiles per lane.
+template <int kQ>
+void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
+  const size_t smem = (size_t)kJoinWarps * (64 * kQ * 16 + 64 * 4);
+  HDB_CUDA(cudaFuncSetAttribute(k_join_rows<kQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int grid = grid_for(ctx, n, kJoinWarps, kQ <= 4 ? 4 : 3);
+  k_join_rows<kQ><<<grid, 32 * kJoinWarps, smem, ctx->stream>>>(
+      X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev, s.worst, s.cl, cross_only);
+  ctx->launches++;
+}
+
+// One FP32 local join over s's samples: by rows (tiles = 0, d <= kRowJoinMaxDim)
+// or with `tiles` 4 x 4 tiles per lane.
 void fp32_join(Context *ctx, int tiles, const float *X, int64_t n, int d, int S, const NndState &s,
                int cross_only) {
+  if (tiles == 0) {
+    using Join = void (*)(Context *, const float *, int64_t, int, int, const NndState &, int);
+    static const Join by_pieces[7] = {join_rows<1>, join_rows<2>, join_rows<3>, join_rows<4>,
+                                      join_rows<5>, join_rows<6>, join_rows<7>};
+    by_pieces[(d + 3) / 4 - 1](ctx, X, n, d, S, s, cross_only);
+    return;
+  }
   const int jw = kJoinWarps;
   const size_t smem = JoinSmem::kBytes * jw;
   // the blocks that fit on the GPU at once (a grid-stride loop over the rows):
@@ -1595,15 +1861,10 @@ void fp32_join(Context *ctx, int tiles, const float *X, int64_t n, int d, int S,
   // list loses to unused chunk tails
   const int grid = grid_for(ctx, n, jw, tiles == 1 ? 3 : 2);
   cudaStream_t st = ctx->stream;
-  if (tiles == 1) {
-    HDB_CUDA(cudaFuncSetAttribute(k_join<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_join<1><<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev,
-                                           s.worst, s.cl, cross_only);
-  } else {
-    HDB_CUDA(cudaFuncSetAttribute(k_join<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_join<2><<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev,
-                                           s.worst, s.cl, cross_only);
-  }
+  const auto fn = tiles == 1 ? k_join<1> : k_join<2>;
+  HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fn<<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev, s.worst, s.cl,
+                                  cross_only);
   ctx->launches++;
 }
 
@@ -1626,7 +1887,8 @@ std::map<std::array<int, 5>, int> g_join_tiles;
 }  // namespace
 
 // Tile slots per lane of the FP32 local join: the one forced on the context,
-// else the one tuned for this shape.  An untuned shape is timed on the first
+// else none (0: by rows) up to kRowJoinMaxDim dimensions, else the one tuned for
+// this shape.  An untuned shape is timed on the first
 // m rows of Xw (the caller's rows in locality order; m = 64K..1M, enough to
 // leave L2 at d >= 64): the initial graph of those rows, one iteration
 // (sample, join, merge) so that the rows hold old and new entries as in the
@@ -1638,6 +1900,7 @@ std::map<std::array<int, 5>, int> g_join_tiles;
 // count in ctx->launches.
 int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const float *Xw, int64_t n) {
   if (ctx->join_tiles) return ctx->join_tiles;
+  if (d <= kRowJoinMaxDim) return 0;
   const std::array<int, 5> key{ctx->device, d, k, S, resident ? 1 : 0};
   {
     std::lock_guard<std::mutex> g(g_tune_mutex);
@@ -1820,7 +2083,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
   // FP32 form: the join's tile slots per lane, tuned per shape
   const int tiles =
       bf16 ? 0 : fp32_join_tiles(ctx, d, k, S, n * d * 4 <= ctx->l2_bytes, Xw, n);
-  if (js) js->config = tiles;
+  if (js) js->config = bf16 ? 0 : std::max(1, tiles);
   for (int it = 0; it < p.iterations; it++) {
     s.sample(ctx, it > 0, 0);
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it], st));

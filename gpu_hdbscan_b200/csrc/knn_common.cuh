@@ -39,9 +39,9 @@ struct CandList {
 // the warps of a join do not all queue on that one counter.  The tail that a
 // warp leaves unused in its last chunk is sorted along as sentinels, so the
 // chunk follows the work: about a quarter of what a warp will append, between
-// kListChunkMin (one append's most) and 1,024 slots.  (With 1,024 always, the
+// kListChunkMin (one append's most) and 768 slots.  (With 1,024 always, the
 // list of 1,500 rows held 1.5 M slots for some 50 k candidates.)
-constexpr uint32_t kListChunkMin = 64, kListChunkMax = 1024;
+constexpr uint32_t kListChunkMin = 96, kListChunkMax = 768;
 inline uint32_t list_chunk(int64_t candidates_per_warp) {
   uint32_t c = kListChunkMin;
   while (c < kListChunkMax && 8 * (int64_t)c <= candidates_per_warp) c *= 2;
@@ -62,21 +62,28 @@ __device__ __forceinline__ void list_fill(const CandList &cl, unsigned long long
     }
 }
 
-// Appends this lane's candidates (up to two: target row, packed key; the
+// Appends this lane's candidates (up to kMax: target row, packed key; the
 // caller has checked each against its target's worst[]) to the list that is
-// sorted by target before the next merge.  The warp writes them at its
+// grouped by target before the next merge.  The warp writes them at its
 // cursor; when they do not fit in the cursor's chunk, the rest of that chunk
 // becomes sentinel entries and one lane takes a new chunk.  Past the list's
 // capacity only the best dropped candidate of each target is kept.  Returns
 // the lane's count.  Called by all 32 lanes of a warp.
-__device__ __forceinline__ int append_candidates(const CandList &cl, ListCursor &cur, bool v0,
-                                                 int32_t t0, uint64_t k0, bool v1,
-                                                 int32_t t1, uint64_t k1) {
+template <int kMax>
+__device__ __forceinline__ int append_candidates(const CandList &cl, ListCursor &cur,
+                                                 const bool (&v)[kMax], const int32_t (&t)[kMax],
+                                                 const uint64_t (&k)[kMax]) {
+  static_assert(32 * kMax <= (int)kListChunkMin, "a chunk holds one append");
   const int lane = threadIdx.x & 31;
   uint32_t lt;
   asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
-  const uint32_t b0 = __ballot_sync(0xffffffffu, v0), b1 = __ballot_sync(0xffffffffu, v1);
-  const uint32_t tot = __popc(b0) + __popc(b1);
+  uint32_t b[kMax], at[kMax], tot = 0;
+#pragma unroll
+  for (int q = 0; q < kMax; q++) {
+    b[q] = __ballot_sync(0xffffffffu, v[q]);
+    at[q] = tot + __popc(b[q] & lt);
+    tot += __popc(b[q]);
+  }
   if (tot == 0) return 0;
   if (cur.pos + tot > cur.end) {
     list_fill(cl, cur.pos, cur.end);
@@ -86,25 +93,23 @@ __device__ __forceinline__ int append_candidates(const CandList &cl, ListCursor 
     cur.pos = base;
     cur.end = base + cl.chunk;
   }
-  const unsigned long long p0 = cur.pos + __popc(b0 & lt);
-  const unsigned long long p1 = cur.pos + __popc(b0) + __popc(b1 & lt);
+  const unsigned long long first = cur.pos;
   cur.pos += tot;
-  const int32_t tt[2] = {t0, t1};
-  const uint64_t kk[2] = {k0, k1};
-  const unsigned long long pp[2] = {p0, p1};
-  const bool vv[2] = {v0, v1};
+  int mine = 0;
 #pragma unroll
-  for (int q = 0; q < 2; q++) {
-    if (!vv[q]) continue;
-    if ((int64_t)pp[q] < cl.cap) {
-      cl.tgt[pp[q]] = (uint32_t)tt[q];
-      cl.key[pp[q]] = kk[q];
+  for (int q = 0; q < kMax; q++) {
+    if (!v[q]) continue;
+    mine++;
+    const unsigned long long p = first + at[q];
+    if ((int64_t)p < cl.cap) {
+      cl.tgt[p] = (uint32_t)t[q];
+      cl.key[p] = k[q];
     } else {
-      atomicMin(&cl.best[tt[q]], (unsigned long long)kk[q]);
+      atomicMin(&cl.best[t[q]], (unsigned long long)k[q]);
       atomicAdd(&cl.counters[0], 1ull);
     }
   }
-  return (v0 ? 1 : 0) + (v1 ? 1 : 0);
+  return mine;
 }
 
 }  // namespace knn

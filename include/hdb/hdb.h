@@ -119,7 +119,8 @@ typedef struct {
   int64_t gpu_launches;         /* kernel launches issued by the call */
   int32_t mst_multiplier;       /* mst_gpu = 1: the weight scale exponent m (single runs) */
   int32_t join_config;          /* FP32 local join: 4 x 4 distance tiles per lane (1 or 2),
-                                   forced (hdb_set_join_tiles) or tuned; 0 for a 16-bit join */
+                                   forced (hdb_set_join_tiles) or tuned, 1 also for the form
+                                   without tiles; 0 for a 16-bit join */
   int64_t join_pairs;           /* FP32 local join: distance pairs computed, all launches
                                    (the reference's new x new and new x old pairs); 0 for a
                                    16-bit join */
@@ -139,9 +140,10 @@ HDB_API hdb_status hdb_set_stream(hdb_ctx *ctx, void *stream);
  * nndescent.cu:1487-1580, has one form).  tiles = 1 or 2 distance tiles of
  * 4 x 4 per lane forces that form (1: fewer registers, three blocks per SM;
  * 2: two blocks per SM, fewer passes over the staged rows); 0 (the default)
- * times both once per (device, d, k, SAMPLE_NUM, rows fit in L2) on the
- * first FP32 NN-Descent of that shape and keeps the faster for the process.
- * Both forms give the same graph. */
+ * leaves the choice to the library: up to 28 dimensions a form without tiles
+ * (reported as 1), beyond the faster of the two, timed once per (device, d, k,
+ * SAMPLE_NUM, rows fit in L2) on the first FP32 NN-Descent of that shape and
+ * kept for the process.  All forms give the same graph. */
 HDB_API hdb_status hdb_set_join_tiles(hdb_ctx *ctx, int32_t tiles);
 
 /* gpuknn::NNDescent, gpuknn/nndescent.cuh:40-42 (nndescent.cu:2088-2199):
