@@ -12,8 +12,10 @@
 // block of ranks [s, s+S) unions its lower half with a lock-free union-find,
 // tags each component with its largest rank, and relabels the endpoints of its
 // upper half by those tags.  Endpoint labels seen by different blocks of one
-// level are disjoint, so all blocks share one union-find array.  After log2(N)
-// levels every edge's endpoint labels are exactly its two children.
+// level are disjoint, so all blocks share one union-find array.  Once the blocks
+// are small enough for a thread block (k_link_blocks), the remaining levels run
+// in its shared memory.  After log2(N) levels every edge's endpoint labels are
+// exactly its two children.
 //
 // Condensed tree.  A node is visited by the reference's BFS iff it is the root
 // or holds >= mpts points.  Chains of "one big child" nodes share a cluster; a
@@ -119,7 +121,13 @@ __global__ void k_validate_mst(const hdb_mst_edge *__restrict__ mst, int64_t m, 
 // upper levels most active edges of a block share one root, so the lanes that
 // share the first active lane's root combine their rank maximum and point
 // count with redux.sync and one of them updates the root; the other lanes
-// update their own roots.
+// update their own roots.  The same components' labels stand on most of those
+// edges, so a label's mark is read before it is taken: as an exchange each, the
+// marks of one label queued up (20M points: 51 ms over 16 levels, 33 with the read).
+__device__ __forceinline__ bool first_seen(UfNode *u, int32_t x) {
+  if (*reinterpret_cast<volatile int32_t *>(&u[x].seen) != 0) return false;
+  return atomicExch(&u[x].seen, 1) == 0;
+}
 __global__ void k_level_tag(const int32_t *__restrict__ la, const int32_t *__restrict__ lb,
                             int64_t m, int64_t S, int64_t n, UfNode *u,
                             const int32_t *__restrict__ size) {
@@ -131,8 +139,8 @@ __global__ void k_level_tag(const int32_t *__restrict__ la, const int32_t *__res
     if (act) {
       const int32_t a = la[r], b = lb[r];
       root = uf_find(u, a);
-      if (atomicExch(&u[a].seen, 1) == 0) add += a < n ? 1 : size[a];
-      if (atomicExch(&u[b].seen, 1) == 0) add += b < n ? 1 : size[b];
+      if (first_seen(u, a)) add += a < n ? 1 : size[a];
+      if (first_seen(u, b)) add += b < n ? 1 : size[b];
     }
     const uint32_t am = __ballot_sync(0xffffffffu, act);
     if (!act) continue;
@@ -152,21 +160,18 @@ __global__ void k_level_tag(const int32_t *__restrict__ la, const int32_t *__res
   }
 }
 
-__global__ void k_level_produce(const int32_t *__restrict__ la, int64_t m, int64_t S, int64_t n,
-                                UfNode *u, int32_t *__restrict__ size) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    if (!active_lower(r, S, m)) continue;
-    const int32_t root = uf_find(u, la[r]);
-    if (u[root].maxr == (int32_t)r) size[n + r] = u[root].acc;
-  }
-}
-
+// The size of every component's new node (lower halves), and the new labels of
+// the upper halves.
 __global__ void k_level_relabel(int32_t *__restrict__ la, int32_t *__restrict__ lb, int64_t m,
-                                int64_t S, int64_t n, UfNode *u) {
+                                int64_t S, int64_t n, UfNode *u, int32_t *__restrict__ size) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
        r += (int64_t)gridDim.x * blockDim.x) {
-    if ((r & (S - 1)) < (S >> 1)) continue;
+    if ((r & (S - 1)) < (S >> 1)) {
+      if (!active_lower(r, S, m)) continue;
+      const int32_t root = uf_find(u, la[r]);
+      if (u[root].maxr == (int32_t)r) size[n + r] = u[root].acc;
+      continue;
+    }
     int32_t a = la[r], b = lb[r];
     int32_t ra = uf_find(u, a), rb = uf_find(u, b);
     int32_t ma = u[ra].maxr, mb = u[rb].maxr;
@@ -186,19 +191,167 @@ __global__ void k_level_reset(const int32_t *__restrict__ la, const int32_t *__r
   }
 }
 
-__global__ void k_link_out(const hdb_mst_edge *__restrict__ mst, const int32_t *__restrict__ la,
-                           const int32_t *__restrict__ lb, const int32_t *__restrict__ size,
-                           int64_t m, int64_t n, hdb_linkage_node *__restrict__ out) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    int32_t a = la[r], b = lb[r];
-    hdb_linkage_node o;
-    o.left_node = a;
-    o.right_node = b;
-    o.weight = mst[r].weight;
-    o.node_size = (a < n ? 1 : size[a]) + (b < n ? 1 : size[b]);
-    out[r] = o;
+// The levels of S ranks and fewer, one thread block per S consecutive ranks, in
+// shared memory, and the tree's nodes.  The labels that the block's edges come
+// with take the slots of a hash table (their local names); the node of the
+// block's rank i is local name kSlots + i.  Every level runs the same steps as
+// the kernels above, its labels' state in shared memory and the edges' labels in
+// registers, with four block barriers; a level of the kernels above is a pass
+// over all edges per step.  S = 512 fills an SM with four blocks; up to
+// one block of 2,048 per SM (303 k edges) larger blocks leave two levels fewer
+// outside.
+template <int S>
+struct LinkSmem {
+  static constexpr int kSlotBits = S == 512 ? 11 : 13, kSlots = 1 << kSlotBits, kNames = kSlots + S;
+  static_assert(kSlots == 4 * S, "S = 512 or 2048");
+  int32_t label[kSlots];  // -1: empty
+  int32_t p[kNames], maxr[kNames], acc[kNames], size[kNames];
+  uint32_t seen[(kNames + 31) / 32];
+};
+
+__device__ __forceinline__ int32_t sm_find(int32_t *p, int32_t x, int bound) {
+  volatile int32_t *vp = p;
+  for (int s = 0; s < bound; s++) {
+    const int32_t px = vp[x];
+    if (px == x) return x;
+    const int32_t ppx = vp[px];
+    if (ppx != px) vp[x] = ppx;
+    x = px;
   }
+  return x;
+}
+
+template <int S, int kThreads>
+__global__ void __launch_bounds__(kThreads)
+    k_link_blocks(const hdb_mst_edge *__restrict__ mst, const int32_t *__restrict__ la,
+                  const int32_t *__restrict__ lb, const int32_t *__restrict__ size, int64_t m,
+                  int64_t n, hdb_linkage_node *__restrict__ out, uint32_t *err) {
+  using L = LinkSmem<S>;
+  constexpr int kPer = S / kThreads;
+  extern __shared__ __align__(16) unsigned char smem_link[];
+  L &sh = *reinterpret_cast<L *>(smem_link);
+  const int64_t first = (int64_t)blockIdx.x * S;
+  const int cnt = (int)min((int64_t)S, m - first);
+  for (int i = threadIdx.x; i < L::kNames; i += kThreads) {
+    if (i < L::kSlots) sh.label[i] = -1;
+    sh.p[i] = i;
+    sh.maxr[i] = -1;
+    sh.acc[i] = 0;
+  }
+  for (int i = threadIdx.x; i < (int)(sizeof(sh.seen) / 4); i += kThreads) sh.seen[i] = 0;
+  __syncthreads();
+  int32_t a[kPer], b[kPer];  // local names of the edge's endpoint labels
+  auto name = [&](int32_t label) -> int32_t {
+    uint32_t h = ((uint32_t)label * 0x9E3779B1u) >> (32 - L::kSlotBits);
+    for (int probe = 0; probe < L::kSlots; probe++) {  // at most 2 S labels in 4 S slots
+      const int32_t prev = atomicCAS(&sh.label[h], -1, label);
+      if (prev == -1) sh.size[h] = label < n ? 1 : size[label];
+      if (prev == -1 || prev == label) break;
+      h = h + 1 == (uint32_t)L::kSlots ? 0 : h + 1;
+    }
+    return (int32_t)h;
+  };
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    const int i = j * kThreads + threadIdx.x;
+    a[j] = b[j] = 0;
+    if (i < cnt) {
+      a[j] = name(la[first + i]);
+      b[j] = name(lb[first + i]);
+    }
+  }
+  __syncthreads();
+  for (int s = S; s >= 2; s >>= 1) {
+    const int half = s >> 1;
+    if (half >= cnt) continue;  // no upper half: for the whole block
+    auto lower = [&](int i) { return i < cnt && (i & (s - 1)) < half && (i & ~(s - 1)) + half < cnt; };
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      if (!lower(j * kThreads + threadIdx.x)) continue;
+      int32_t x = a[j], y = b[j];
+      int step = 0;
+      for (; step < L::kNames; step++) {
+        x = sm_find(sh.p, x, L::kNames);
+        y = sm_find(sh.p, y, L::kNames);
+        if (x == y) break;
+        if (x < y) { const int32_t t = x; x = y; y = t; }
+        if (atomicCAS(&sh.p[y], y, x) == y) break;
+      }
+      if (step == L::kNames) atomicOr(err, DEVERR_TIMEOUT);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const int i = j * kThreads + threadIdx.x;
+      if (!lower(i)) continue;
+      const int32_t root = sm_find(sh.p, a[j], L::kNames);
+      int32_t add = 0;
+      for (int32_t x : {a[j], b[j]}) {
+        const uint32_t bit = 1u << (x & 31);
+        volatile uint32_t *mark = &sh.seen[x >> 5];
+        if (!(*mark & bit) && !(atomicOr(&sh.seen[x >> 5], bit) & bit)) add += sh.size[x];
+      }
+      if (*reinterpret_cast<volatile int32_t *>(&sh.maxr[root]) < i) atomicMax(&sh.maxr[root], i);
+      if (add) atomicAdd(&sh.acc[root], add);
+    }
+    __syncthreads();
+    int32_t na[kPer], nb[kPer];
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      const int i = j * kThreads + threadIdx.x;
+      na[j] = a[j];
+      nb[j] = b[j];
+      if (lower(i)) {
+        const int32_t root = sm_find(sh.p, a[j], L::kNames);
+        if (sh.maxr[root] == i) sh.size[L::kSlots + i] = sh.acc[root];
+      } else if (i < cnt && (i & (s - 1)) >= half) {
+        const int32_t ma = sh.maxr[sm_find(sh.p, a[j], L::kNames)];
+        const int32_t mb = sh.maxr[sm_find(sh.p, b[j], L::kNames)];
+        if (ma >= 0) na[j] = L::kSlots + ma;
+        if (mb >= 0) nb[j] = L::kSlots + mb;
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kPer; j++) {
+      if (lower(j * kThreads + threadIdx.x)) {
+        for (int32_t x : {a[j], b[j]}) {
+          sh.p[x] = x;
+          sh.maxr[x] = -1;
+          sh.acc[x] = 0;
+          atomicAnd(&sh.seen[x >> 5], ~(1u << (x & 31)));
+        }
+      }
+      a[j] = na[j];
+      b[j] = nb[j];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < kPer; j++) {
+    const int i = j * kThreads + threadIdx.x;
+    if (i >= cnt) continue;
+    auto global = [&](int32_t x) {
+      return x < L::kSlots ? sh.label[x] : (int32_t)(n + first) + (x - L::kSlots);
+    };
+    hdb_linkage_node o;
+    o.left_node = global(a[j]);
+    o.right_node = global(b[j]);
+    o.weight = mst[first + i].weight;
+    o.node_size = sh.size[a[j]] + sh.size[b[j]];
+    out[first + i] = o;
+  }
+}
+
+template <int S, int kThreads>
+void link_blocks(Context *ctx, const hdb_mst_edge *mst, const int32_t *la, const int32_t *lb,
+                 const int32_t *size, int64_t m, int64_t n, hdb_linkage_node *out) {
+  const int smem = (int)sizeof(LinkSmem<S>);
+  HDB_CUDA(cudaFuncSetAttribute(k_link_blocks<S, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  k_link_blocks<S, kThreads><<<(unsigned)ceil_div(m, S), kThreads, smem, ctx->stream>>>(
+      mst, la, lb, size, m, n, out, ctx->dev_err);
+  ctx->launches++;
+  HDB_CHECK_LAUNCH();
 }
 
 // ---------------------------------------------------------------------------
@@ -999,18 +1152,21 @@ void linkage_tree(Context *ctx, const hdb_mst_edge *mst, int64_t n, hdb_linkage_
   k_link_init<<<gm, 256, 0, st>>>(mst, m, la, lb); ctx->launches++;
   k_uf_init<<<gt, 256, 0, st>>>(total, n, u, size); ctx->launches++;
   HDB_CHECK_LAUNCH();
+  const bool few = m <= (int64_t)ctx->num_sms * 2048;
+  const int64_t inner = few ? 2048 : 512;
   int64_t S = 1;
   while (S < m) S <<= 1;
-  for (; S >= 2; S >>= 1) {
+  for (; S > inner; S >>= 1) {
     k_level_union<<<gm, 256, 0, st>>>(la, lb, m, S, u, ctx->dev_err); ctx->launches++;
     k_level_tag<<<gm, 256, 0, st>>>(la, lb, m, S, n, u, size); ctx->launches++;
-    k_level_produce<<<gm, 256, 0, st>>>(la, m, S, n, u, size); ctx->launches++;
-    k_level_relabel<<<gm, 256, 0, st>>>(la, lb, m, S, n, u); ctx->launches++;
-    k_level_reset<<<gm, 256, 0, st>>>(la, lb, m, S, u); ctx->launches++;
+    k_level_relabel<<<gm, 256, 0, st>>>(la, lb, m, S, n, u, size); ctx->launches++;
+    if (S > 2 * inner) {
+      k_level_reset<<<gm, 256, 0, st>>>(la, lb, m, S, u); ctx->launches++;
+    }
     HDB_CHECK_LAUNCH();
   }
-  k_link_out<<<gm, 256, 0, st>>>(mst, la, lb, size, m, n, out); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  if (few) link_blocks<2048, 1024>(ctx, mst, la, lb, size, m, n, out);
+  else link_blocks<512, 512>(ctx, mst, la, lb, size, m, n, out);
   HDB_REQUIRE(!(ctx->take_dev_err() & DEVERR_TIMEOUT), HDB_ERR_INTERNAL,
               "linkage tree: union-find exceeded its step bound");
 }
