@@ -19,9 +19,14 @@
 //
 // Condensed tree.  A node is visited by the reference's BFS iff it is the root
 // or holds >= mpts points.  Chains of "one big child" nodes share a cluster; a
-// node whose children are both big starts two clusters, numbered in BFS order
-// (depth, then left-to-right = preorder).  Depth, preorder and chain heads come
-// from pointer jumping; each point falls out at the lowest visited ancestor.
+// node whose children are both big (a split) starts two clusters, numbered in
+// BFS order (depth, then left to right).  Chain heads come from pointer jumping
+// over the nodes.  Everything else about the order follows from two facts: down a
+// chain the ranks descend, so the nodes in descending rank, grouped by cluster,
+// are the chains top-down; and two nodes of one depth part at a split, so a
+// split's depth and the number of points to its left, which place it in BFS
+// order, are sums over the few splits above it of their chains' lengths and their
+// left children's sizes.  Each point falls out at the lowest visited ancestor.
 // Stability is summed per cluster in the reference's row order (chain nodes
 // top-down, identical terms for the points of each small side), in FP32 with
 // separate multiply/add roundings, or in FP64 when asked.
@@ -418,115 +423,170 @@ __global__ void k_nodes(TreeView t, int32_t *__restrict__ par, int8_t *__restric
   }
 }
 
-// Doubling state for visited nodes: jump pointer, depth and preorder sums,
-// and the chain-head pointer.
-__global__ void k_path_init(TreeView t, const int32_t *__restrict__ par, const int8_t *__restrict__ side,
+// Chain-head pointers: a node that continues its parent's chain points to the
+// parent, a head to itself.
+__global__ void k_head_init(TreeView t, const int32_t *__restrict__ par, const int8_t *__restrict__ side,
                             const int8_t *__restrict__ kind, const int8_t *__restrict__ visited,
-                            int32_t *__restrict__ jmp, int64_t *__restrict__ dep,
-                            int64_t *__restrict__ pre, int32_t *__restrict__ head) {
+                            int32_t *__restrict__ head, int32_t *__restrict__ split,
+                            int32_t *__restrict__ vis) {
   const int64_t m = t.m;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
        r += (int64_t)gridDim.x * blockDim.x) {
-    if (!visited[r]) { jmp[r] = -1; head[r] = -1; continue; }
-    int64_t x = t.n + r;
-    if (t.is_root(r)) {
-      jmp[r] = -1; dep[r] = 0; pre[r] = 0; head[r] = (int32_t)r;
-      continue;
+    const bool v = visited[r];
+    vis[r] = v;
+    split[r] = v && kind[r] == KIND_SPLIT;
+    if (!v) { head[r] = -1; continue; }
+    int32_t h = (int32_t)r;
+    if (!t.is_root(r)) {
+      const int64_t x = t.n + r;
+      const int32_t pr = par[x] - (int32_t)t.n;
+      const int8_t pk = kind[pr];
+      if ((pk == KIND_LEFTBIG && side[x] == 0) || (pk == KIND_RIGHTBIG && side[x] == 1)) h = pr;
     }
-    int32_t p = par[x];
-    int64_t pr = p - t.n;
-    jmp[r] = (int32_t)pr;
-    dep[r] = 1;
-    int64_t d = 1;
-    if (side[x] == 1) {
-      int32_t sib = t.h[pr].left_node;
-      d += 2 * (int64_t)t.sz(sib) - 1;
-    }
-    pre[r] = d;
-    int8_t pk = kind[pr];
-    bool inherit = (pk == KIND_LEFTBIG && side[x] == 0) || (pk == KIND_RIGHTBIG && side[x] == 1);
-    head[r] = inherit ? (int32_t)pr : (int32_t)r;
+    head[r] = h;
   }
 }
 
-__global__ void k_path_jump(int64_t m, const int32_t *__restrict__ jmp, const int64_t *__restrict__ dep,
-                            const int64_t *__restrict__ pre, int32_t *__restrict__ jmp2,
-                            int64_t *__restrict__ dep2, int64_t *__restrict__ pre2,
-                            int32_t *changed) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    int32_t j = jmp[r];
-    if (j < 0) { jmp2[r] = j; dep2[r] = dep[r]; pre2[r] = pre[r]; continue; }
-    dep2[r] = dep[r] + dep[j];
-    pre2[r] = pre[r] + pre[j];
-    jmp2[r] = jmp[j];
-    *changed = 1;
-  }
-}
-
-__global__ void k_head_jump(int64_t m, int32_t *head, int32_t *changed) {
+// Round `it` of the jumping, in place (a pointer read late has jumped further
+// already); once a round changed nothing the later ones return at once, so the
+// host queues as many as the longest chain could take and waits for none.
+__global__ void k_head_jump(int64_t m, int32_t *head, int32_t *changed, int it) {
+  if (it > 0 && changed[it - 1] == 0) return;
   volatile int32_t *vh = head;
+  bool any = false;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
        r += (int64_t)gridDim.x * blockDim.x) {
-    int32_t h = vh[r];
+    const int32_t h = vh[r];
     if (h < 0) continue;
-    int32_t hh = vh[h];
+    const int32_t hh = vh[h];
     if (hh != h) {
       vh[r] = hh;
-      *changed = 1;
+      any = true;
     }
   }
+  if (__any_sync(0xffffffffu, any) && lane_id() == 0) changed[it] = 1;
 }
 
-__global__ void k_split_keys(int64_t m, const int8_t *__restrict__ kind,
-                             const int8_t *__restrict__ visited, const int64_t *__restrict__ dep,
-                             const int64_t *__restrict__ pre, int32_t *__restrict__ flag) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x)
-    flag[r] = visited[r] && kind[r] == KIND_SPLIT;
+// Provisional clusters: 0 .. trees - 1 the roots', trees + 2 q + side those of
+// the q-th split's children (splits in ascending rank).  cid is indexed by the
+// clusters' head nodes.
+__global__ void k_split_nodes(TreeView t, const int32_t *__restrict__ split,
+                              const int64_t *__restrict__ pos, int64_t trees,
+                              int32_t *__restrict__ node, int32_t *__restrict__ cid) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < t.m;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    if (t.is_root(r)) cid[r] = t.seg.count > 0 ? t.seg.of_rank(r) : 0;
+    if (!split[r]) continue;
+    const int64_t q = pos[r];
+    node[q] = (int32_t)r;
+    const hdb_linkage_node h = t.h[r];
+    cid[h.left_node - t.n] = (int32_t)(trees + 2 * q);
+    cid[h.right_node - t.n] = (int32_t)(trees + 2 * q + 1);
+  }
 }
 
-__global__ void k_split_emit(int64_t m, const int32_t *__restrict__ flag, const int64_t *__restrict__ pos,
-                             const int64_t *__restrict__ dep, const int64_t *__restrict__ pre,
-                             uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+// Cluster of every visited node, and the visited nodes in descending rank with
+// their cluster as the sort key.
+__global__ void k_node_cluster(int64_t m, const int32_t *__restrict__ vis,
+                               const int64_t *__restrict__ vpos, int64_t nv,
+                               const int32_t *__restrict__ head, const int32_t *__restrict__ cid,
+                               int32_t *__restrict__ ncl, uint32_t *__restrict__ keys,
+                               uint32_t *__restrict__ vals) {
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
        r += (int64_t)gridDim.x * blockDim.x) {
-    if (!flag[r]) continue;
-    keys[pos[r]] = ((uint64_t)dep[r] << 32) | (uint64_t)pre[r];
-    vals[pos[r]] = (uint32_t)r;
+    const int32_t c = vis[r] ? cid[head[r]] : -1;
+    ncl[r] = c;
+    if (c < 0) continue;
+    const int64_t at = nv - 1 - vpos[r];
+    keys[at] = (uint32_t)c;
+    vals[at] = (uint32_t)r;
   }
 }
 
-// Cluster ids: root = n; the t-th split node in BFS order gives n+1+2t (left)
-// and n+2+2t (right).  cid is indexed by internal-node rank r (-1 otherwise).
-// A forest numbers its clusters tree after tree: the splits are sorted by
-// (instance, BFS order), split q of instance s gives indices s+1+2q and
-// s+2+2q, and instance s's root the index just before its first split's.
-__global__ void k_assign_cids(TreeView t, const uint32_t *__restrict__ split_nodes, int64_t ns,
-                              const uint32_t *__restrict__ split_inst, int32_t *__restrict__ cid,
-                              int32_t *__restrict__ split_rank) {
+__global__ void k_seg_bounds(const uint32_t *__restrict__ keys, int64_t cnt, int64_t *__restrict__ s0,
+                             int64_t *__restrict__ s1) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t c = keys[i];
+    if (i == 0 || keys[i - 1] != c) s0[c] = i;
+    if (i == cnt - 1 || keys[i + 1] != c) s1[c] = i + 1;
+  }
+}
+
+// A split's place, relative to the split above it: its chain's length, and the
+// points to the left of the child that starts the chain.
+struct SplitUp {
+  int32_t up, depth, left, pad;
+};
+__global__ void k_split_up(TreeView t, int64_t ns, int64_t trees, const int32_t *__restrict__ node,
+                           const int32_t *__restrict__ ncl, const int64_t *__restrict__ s0,
+                           const int64_t *__restrict__ s1, SplitUp *__restrict__ out) {
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < ns;
        q += (int64_t)gridDim.x * blockDim.x) {
-    int64_t r = split_nodes[q];
-    const int64_t base = split_inst ? split_inst[q] : 0;
-    hdb_linkage_node h = t.h[r];
-    cid[h.left_node - t.n] = (int32_t)(t.n + base + 1 + 2 * q);
-    cid[h.right_node - t.n] = (int32_t)(t.n + base + 2 + 2 * q);
-    split_rank[r] = (int32_t)q;
+    const int32_t c = ncl[node[q]];
+    SplitUp u{-1, (int32_t)(s1[c] - s0[c]), 0, 0};
+    if (c >= trees) {
+      u.up = (int32_t)((c - trees) >> 1);
+      if ((c - trees) & 1) u.left = (int32_t)t.sz(t.h[node[u.up]].left_node);
+    }
+    out[q] = u;
   }
 }
 
-__global__ void k_split_inst(const uint32_t *__restrict__ split_nodes, int64_t ns, Segments seg,
-                             uint32_t *__restrict__ inst) {
+__device__ __forceinline__ SplitUp split_jump(const SplitUp *in, int64_t q) {
+  SplitUp u = in[q];
+  if (u.up >= 0) {
+    const SplitUp v = in[u.up];
+    u = SplitUp{v.up, u.depth + v.depth, u.left + v.left, 0};
+  }
+  return u;
+}
+
+__global__ void k_split_jump(int64_t ns, const SplitUp *__restrict__ in, SplitUp *__restrict__ out) {
   for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < ns;
        q += (int64_t)gridDim.x * blockDim.x)
-    inst[q] = (uint32_t)seg.of_rank(split_nodes[q]);
+    out[q] = split_jump(in, q);
+}
+
+// BFS order as a sort key: depth, then points to the left (bits wide).
+__global__ void k_split_keys(int64_t ns, const SplitUp *__restrict__ up, int bits,
+                             uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < ns;
+       q += (int64_t)gridDim.x * blockDim.x) {
+    keys[q] = ((uint64_t)up[q].depth << bits) | (uint64_t)up[q].left;
+    vals[q] = (uint32_t)q;
+  }
+}
+
+__global__ void k_split_inst(const uint32_t *__restrict__ order, const int32_t *__restrict__ node,
+                             int64_t ns, Segments seg, uint32_t *__restrict__ inst) {
+  for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < ns;
+       q += (int64_t)gridDim.x * blockDim.x)
+    inst[q] = (uint32_t)seg.of_rank(node[order[q]]);
+}
+
+// Final cluster indices: the root 0, the t-th split in BFS order gives 1 + 2 t
+// (left) and 2 + 2 t (right).  A forest numbers its clusters tree after tree:
+// the splits are sorted by (instance, BFS order), split t of instance s gives
+// s + 1 + 2 t and s + 2 + 2 t, and instance s's root the index just before its
+// first split's.  fin maps the provisional clusters; split_nodes the order.
+__global__ void k_final_ids(int64_t ns, int64_t trees, const uint32_t *__restrict__ order,
+                            const int32_t *__restrict__ node, const uint32_t *__restrict__ split_inst,
+                            int32_t *__restrict__ fin, uint32_t *__restrict__ split_nodes) {
+  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t0 == 0 && !split_inst) fin[0] = 0;
+  for (int64_t t = t0; t < ns; t += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = order[t], base = split_inst ? split_inst[t] : 0;
+    split_nodes[t] = (uint32_t)node[q];
+    fin[trees + 2 * q] = (int32_t)(base + 1 + 2 * t);
+    fin[trees + 2 * q + 1] = (int32_t)(base + 2 + 2 * t);
+  }
 }
 
 // One thread per instance s: its root's cluster index croot[s] = s + 2 *
-// (splits of earlier instances), the root node's cid, and cseg of the root.
+// (splits of earlier instances), and cseg of the root.
 __global__ void k_forest_roots(TreeView t, const uint32_t *__restrict__ split_inst, int64_t ns,
-                               int32_t *__restrict__ cid, int32_t *__restrict__ croot,
+                               int32_t *__restrict__ fin, int32_t *__restrict__ croot,
                                int32_t *__restrict__ cseg, int64_t C) {
   const int32_t T = t.seg.count;
   for (int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; s <= T;
@@ -540,17 +600,24 @@ __global__ void k_forest_roots(TreeView t, const uint32_t *__restrict__ split_in
     const int64_t c = s + 2 * lo;
     croot[s] = (int32_t)c;
     cseg[c] = (int32_t)s;
-    cid[t.seg.off[s + 1] - s - 2] = (int32_t)(t.n + c);
+    fin[s] = (int32_t)c;
   }
 }
 
-// Cluster of every visited node; per-cluster info (index c - n).
-__global__ void k_node_cluster(int64_t m, int64_t n, const int8_t *__restrict__ visited,
-                               const int32_t *__restrict__ head, const int32_t *__restrict__ cid,
-                               int32_t *__restrict__ ncl) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x)
-    ncl[r] = visited[r] ? cid[head[r]] : -1;
+// The nodes' clusters as ids n + index, and the chains' segments, in the final
+// numbering.
+__global__ void k_final_clusters(int64_t m, int64_t n, int64_t C, const int32_t *__restrict__ fin,
+                                 int32_t *__restrict__ ncl, const int64_t *__restrict__ t0,
+                                 const int64_t *__restrict__ t1, int64_t *__restrict__ s0,
+                                 int64_t *__restrict__ s1) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m || r < C;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    if (r < m && ncl[r] >= 0) ncl[r] = (int32_t)n + fin[ncl[r]];
+    if (r < C) {
+      s0[fin[r]] = t0[r];
+      s1[fin[r]] = t1[r];
+    }
+  }
 }
 
 __global__ void k_cluster_info(TreeView t, const uint32_t *__restrict__ split_nodes, int64_t ns,
@@ -570,18 +637,6 @@ __global__ void k_cluster_info(TreeView t, const uint32_t *__restrict__ split_no
     cparent[c0] = pc - (int32_t)t.n;
     cparent[c1] = pc - (int32_t)t.n;
     ckid0[pc - t.n] = c0;
-  }
-}
-
-// Chain nodes grouped by cluster, top-down: key (cluster index << 32) | depth.
-__global__ void k_chain_keys(int64_t m, int64_t n, const int32_t *__restrict__ ncl,
-                             const int64_t *__restrict__ dep, const int64_t *__restrict__ pos,
-                             uint64_t *__restrict__ keys, uint32_t *__restrict__ vals) {
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    if (ncl[r] < 0) continue;
-    keys[pos[r]] = ((uint64_t)(ncl[r] - n) << 32) | (uint64_t)dep[r];
-    vals[pos[r]] = (uint32_t)r;
   }
 }
 
@@ -967,58 +1022,61 @@ __global__ void k_eom(int64_t C, const int32_t *__restrict__ ckid0, const int32_
   }
 }
 
-// Nearest self-selected proper ancestor (roots excluded) by doubling.
-__global__ void k_sel_init(int64_t C, const int32_t *__restrict__ cparent, const int8_t *__restrict__ self_sel,
-                           int32_t *__restrict__ jmp, int8_t *__restrict__ anc) {
+// The cluster that covers each one: the highest cluster that selects itself on
+// its way up (itself included, roots not), by doubling.  A cluster that covers
+// itself is selected (get_clusters drops what lies below a selected cluster).
+struct Cover {
+  int32_t up, top;
+};
+__global__ void k_cover_init(int64_t C, const int32_t *__restrict__ cparent,
+                             const int8_t *__restrict__ self_sel, Cover *__restrict__ out) {
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
-    int32_t p = cparent[c];
-    if (p < 0 || cparent[p] < 0) { jmp[c] = -1; anc[c] = 0; }
-    else { jmp[c] = p; anc[c] = self_sel[p]; }
+    const int32_t p = cparent[c];
+    out[c] = Cover{p >= 0 && cparent[p] >= 0 ? p : -1, p >= 0 && self_sel[c] ? (int32_t)c : -1};
   }
 }
 
-__global__ void k_sel_jump(int64_t C, const int32_t *__restrict__ jmp, const int8_t *__restrict__ anc,
-                           int32_t *__restrict__ jmp2, int8_t *__restrict__ anc2, int32_t *changed) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    int32_t j = jmp[c];
-    if (j < 0) { jmp2[c] = -1; anc2[c] = anc[c]; continue; }
-    anc2[c] = anc[c] | anc[j];
-    jmp2[c] = jmp[j];
-    *changed = 1;
+__device__ __forceinline__ Cover cover_jump(const Cover *in, int64_t c) {
+  Cover x = in[c];
+  if (x.up >= 0) {
+    const Cover y = in[x.up];
+    x = Cover{y.up, y.top >= 0 ? y.top : x.top};
   }
+  return x;
 }
 
-__global__ void k_selected(int64_t C, const int32_t *__restrict__ cparent,
-                           const int8_t *__restrict__ self_sel, const int8_t *__restrict__ anc,
-                           int32_t *__restrict__ sel) {
+__global__ void k_cover_jump(int64_t C, const Cover *__restrict__ in, Cover *__restrict__ out) {
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x)
-    sel[c] = (cparent[c] >= 0 && self_sel[c] && !anc[c]) ? 1 : 0;
+    out[c] = cover_jump(in, c);
 }
 
-// Selected cluster covering each cluster (itself or nearest selected ancestor).
-__global__ void k_cover_init(int64_t C, const int32_t *__restrict__ cparent, const int32_t *__restrict__ sel,
-                             int32_t *__restrict__ jmp, int32_t *__restrict__ cover) {
-  for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C;
-       c += (int64_t)gridDim.x * blockDim.x) {
-    if (sel[c]) { cover[c] = (int32_t)c; jmp[c] = -1; continue; }
-    cover[c] = -1;
-    int32_t p = cparent[c];
-    jmp[c] = (p >= 0 && cparent[p] >= 0) ? p : -1;
+// All rounds of a doubling over few items in one block (one launch instead of
+// one a round): a and b are the two buffers, read and written in turn, so
+// neither is read through the read-only cache.
+constexpr int64_t kOneBlockItems = 8192;
+template <typename T, T (*kJump)(const T *, int64_t)>
+__device__ __forceinline__ void jump_all(int64_t count, T *a, T *b, int rounds) {
+  for (int i = 0; i < rounds; i++) {
+    for (int64_t q = threadIdx.x; q < count; q += blockDim.x) b[q] = kJump(a, q);
+    __syncthreads();
+    T *t = a; a = b; b = t;
   }
 }
+__global__ void __launch_bounds__(1024) k_split_jump_all(int64_t ns, SplitUp *a, SplitUp *b, int rounds) {
+  jump_all<SplitUp, split_jump>(ns, a, b, rounds);
+}
+__global__ void __launch_bounds__(1024) k_cover_jump_all(int64_t C, Cover *a, Cover *b, int rounds) {
+  jump_all<Cover, cover_jump>(C, a, b, rounds);
+}
 
-__global__ void k_cover_jump(int64_t C, const int32_t *__restrict__ jmp, const int32_t *__restrict__ cover,
-                             int32_t *__restrict__ jmp2, int32_t *__restrict__ cover2, int32_t *changed) {
+__global__ void k_selected(int64_t C, const Cover *__restrict__ cov, int32_t *__restrict__ sel,
+                           int32_t *__restrict__ cover) {
   for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < C;
        c += (int64_t)gridDim.x * blockDim.x) {
-    int32_t j = jmp[c];
-    if (cover[c] >= 0 || j < 0) { cover2[c] = cover[c]; jmp2[c] = -1; continue; }
-    cover2[c] = cover[j];
-    jmp2[c] = cover[j] >= 0 ? -1 : jmp[j];
-    *changed = 1;
+    cover[c] = cov[c].top;
+    sel[c] = cov[c].top == (int32_t)c ? 1 : 0;
   }
 }
 
@@ -1113,22 +1171,6 @@ __global__ void k_stab_out(int64_t C, int64_t n, const float *__restrict__ stab,
   }
 }
 
-__global__ void k_seg_bounds(const uint64_t *__restrict__ keys, int64_t cnt, int64_t *__restrict__ s0,
-                             int64_t *__restrict__ s1) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt;
-       i += (int64_t)gridDim.x * blockDim.x) {
-    uint32_t c = (uint32_t)(keys[i] >> 32);
-    if (i == 0 || (uint32_t)(keys[i - 1] >> 32) != c) s0[c] = i;
-    if (i == cnt - 1 || (uint32_t)(keys[i + 1] >> 32) != c) s1[c] = i + 1;
-  }
-}
-
-__global__ void k_flag_nonneg(const int32_t *__restrict__ v, int64_t m, int32_t *__restrict__ flag) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
-       i += (int64_t)gridDim.x * blockDim.x)
-    flag[i] = v[i] >= 0;
-}
-
 int bits_for(int64_t v) {
   int b = 0;
   while (b < 63 && (int64_t(1) << b) <= v) b++;
@@ -1200,82 +1242,80 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
   k_nodes<<<gm, 256, 0, st>>>(t, par, side, kind, visited, lam); ctx->launches++;
   HDB_CHECK_LAUNCH();
 
-  // depth / preorder / chain heads by pointer jumping
-  Buf<int32_t> jmp(ctx, m), jmp2(ctx, m), head(ctx, m);
-  Buf<int64_t> dep(ctx, m), dep2(ctx, m), pre(ctx, m), pre2(ctx, m);
-  Buf<int32_t> changed(ctx, 2);
-  k_path_init<<<gm, 256, 0, st>>>(t, par, side, kind, visited, jmp, dep, pre, head); ctx->launches++;
+  // chain heads by pointer jumping; the splits and the visited nodes counted
+  Buf<int32_t> head(ctx, m), split(ctx, m), vis(ctx, m), changed(ctx, 64);
+  Buf<int64_t> spos(ctx, m + 1), vpos(ctx, m + 1);
+  HDB_CUDA(cudaMemsetAsync(changed, 0, 64 * sizeof(int32_t), st));
+  k_head_init<<<gm, 256, 0, st>>>(t, par, side, kind, visited, head, split, vis); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  int32_t *j0 = jmp, *j1 = jmp2;
-  int64_t *d0 = dep, *d1 = dep2, *p0 = pre, *p1 = pre2;
-  for (int it = 0; it < 64; it++) {
-    HDB_CUDA(cudaMemsetAsync(changed, 0, 2 * sizeof(int32_t), st));
-    k_path_jump<<<gm, 256, 0, st>>>(m, j0, d0, p0, j1, d1, p1, changed); ctx->launches++;
-    k_head_jump<<<gm, 256, 0, st>>>(m, head, changed.get() + 1); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-    HDB_CUDA(cudaMemcpyAsync(hflag, changed, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    ctx->sync();
-    std::swap(j0, j1);
-    std::swap(d0, d1);
-    std::swap(p0, p1);
-    if (!hflag[0] && !hflag[1]) break;
-    HDB_REQUIRE(it < 63, HDB_ERR_INTERNAL, "condensed tree: pointer jumping did not converge");
+  scan_exclusive_i32_i64(ctx, split, spos, m, spos.get() + m);
+  scan_exclusive_i32_i64(ctx, vis, vpos, m, vpos.get() + m);
+  HDB_CUDA(cudaMemcpyAsync(hp, spos.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  HDB_CUDA(cudaMemcpyAsync(hp + 1, vpos.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+  for (int it = 0; it < bits_for(m); it++) {  // 2^rounds > m: the longest chain
+    k_head_jump<<<gm, 256, 0, st>>>(m, head, changed, it); ctx->launches++;
   }
-  // head pointers may need extra rounds beyond the path sums
-  for (int it = 0; it < 64; it++) {
-    HDB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int32_t), st));
-    k_head_jump<<<gm, 256, 0, st>>>(m, head, changed); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-    HDB_CUDA(cudaMemcpyAsync(hflag, changed, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    ctx->sync();
-    if (!hflag[0]) break;
-  }
-
-  // split nodes in BFS order -> cluster ids
-  Buf<int32_t> flag(ctx, m);
-  Buf<int64_t> pos(ctx, m + 1);
-  k_split_keys<<<gm, 256, 0, st>>>(m, kind, visited, d0, p0, flag); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  scan_exclusive_i32_i64(ctx, flag, pos, m, pos.get() + m);
-  HDB_CUDA(cudaMemcpyAsync(hp, pos.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
   ctx->sync();
-  const int64_t ns = hp[0];
+  const int64_t ns = hp[0], nv = hp[1];
   const int64_t C = trees + 2 * ns;
-  Buf<uint64_t> skeys(ctx, ns > 0 ? ns : 1);
+
+  // provisional clusters; the chains, top-down, grouped by cluster
+  Buf<int32_t> node(ctx, ns > 0 ? ns : 1), cid(ctx, m), ncl(ctx, m);
+  k_split_nodes<<<gm, 256, 0, st>>>(t, split, spos, trees, node, cid); ctx->launches++;
+  Buf<uint32_t> ckeys(ctx, nv), chain(ctx, nv);
+  k_node_cluster<<<gm, 256, 0, st>>>(m, vis, vpos, nv, head, cid, ncl, ckeys, chain); ctx->launches++;
+  HDB_CHECK_LAUNCH();
+  radix_sort_u32(ctx, ckeys, chain, nv, 0, bits_for(C));
+  Buf<int64_t> t0(ctx, C), t1(ctx, C), s0(ctx, C), s1(ctx, C);
+  k_seg_bounds<<<grid_for(ctx, nv, 256), 256, 0, st>>>(ckeys, nv, t0, t1); ctx->launches++;
+  HDB_CHECK_LAUNCH();
+
+  // splits in BFS order -> final cluster numbers
   Buf<uint32_t> snodes(ctx, ns > 0 ? ns : 1), sinst;
-  Buf<int32_t> cid(ctx, m), split_rank(ctx, m), cseg, croot;
-  HDB_CUDA(cudaMemsetAsync(cid, 0xff, m * sizeof(int32_t), st));
+  Buf<int32_t> fin(ctx, C), cseg, croot;
   if (forest) {
     sinst = Buf<uint32_t>(ctx, ns > 0 ? ns : 1);
     cseg = Buf<int32_t>(ctx, C);
     croot = Buf<int32_t>(ctx, trees + 1);
   }
-  if (ns > 0) {
-    k_split_emit<<<gm, 256, 0, st>>>(m, flag, pos, d0, p0, skeys, snodes); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-    radix_sort_u64(ctx, skeys, snodes, ns, 0, 64);
-    if (forest) {  // (instance, BFS order)
-      k_split_inst<<<grid_for(ctx, ns, 256), 256, 0, st>>>(snodes, ns, seg, sinst); ctx->launches++;
+  {
+    const int gs = grid_for(ctx, ns, 256);
+    Buf<uint32_t> order(ctx, ns > 0 ? ns : 1);
+    if (ns > 0) {
+      Buf<SplitUp> up(ctx, ns), up2(ctx, ns);
+      Buf<uint64_t> skeys(ctx, ns);
+      k_split_up<<<gs, 256, 0, st>>>(t, ns, trees, node, ncl, t0, t1, up); ctx->launches++;
+      SplitUp *ua = up, *ub = up2;
+      const int rounds = bits_for(ns);
+      if (ns <= kOneBlockItems) {
+        k_split_jump_all<<<1, 1024, 0, st>>>(ns, ua, ub, rounds); ctx->launches++;
+        if (rounds & 1) std::swap(ua, ub);
+      } else {
+        for (int it = 0; it < rounds; it++) {
+          k_split_jump<<<gs, 256, 0, st>>>(ns, ua, ub); ctx->launches++;
+          std::swap(ua, ub);
+        }
+      }
+      const int bits = bits_for(n);  // depth and points to the left are below n
+      k_split_keys<<<gs, 256, 0, st>>>(ns, ua, bits, skeys, order); ctx->launches++;
       HDB_CHECK_LAUNCH();
-      radix_sort_u32(ctx, sinst, snodes, ns, 0, bits_for(seg.count));
+      radix_sort_u64(ctx, skeys, order, ns, 0, 2 * bits);
+      if (forest) {  // (instance, BFS order)
+        k_split_inst<<<gs, 256, 0, st>>>(order, node, ns, seg, sinst); ctx->launches++;
+        HDB_CHECK_LAUNCH();
+        radix_sort_u32(ctx, sinst, order, ns, 0, bits_for(seg.count));
+      }
     }
-    k_assign_cids<<<grid_for(ctx, ns, 256), 256, 0, st>>>(t, snodes, ns, sinst.get(), cid,
-                                                           split_rank); ctx->launches++;
+    k_final_ids<<<gs, 256, 0, st>>>(ns, trees, order, node, sinst.get(), fin, snodes); ctx->launches++;
     HDB_CHECK_LAUNCH();
   }
-  // root cluster ids
   if (forest) {
-    k_forest_roots<<<grid_for(ctx, trees + 1, 256), 256, 0, st>>>(t, sinst, ns, cid, croot, cseg,
+    k_forest_roots<<<grid_for(ctx, trees + 1, 256), 256, 0, st>>>(t, sinst, ns, fin, croot, cseg,
                                                                    C); ctx->launches++;
     HDB_CHECK_LAUNCH();
-  } else {
-    int32_t root_cid = (int32_t)n;
-    HDB_CUDA(cudaMemcpyAsync(cid.get() + (m - 1), &root_cid, sizeof(int32_t),
-                             cudaMemcpyHostToDevice, st));
-    ctx->sync();
   }
-  Buf<int32_t> ncl(ctx, m);
-  k_node_cluster<<<gm, 256, 0, st>>>(m, n, visited, head, cid, ncl); ctx->launches++;
+  k_final_clusters<<<gm, 256, 0, st>>>(m, n, C, fin, ncl, t0, t1, s0, s1); ctx->launches++;
   HDB_CHECK_LAUNCH();
 
   // per-cluster info
@@ -1293,33 +1333,10 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
                                                             birth, cparent, ckid0, cseg.get()); ctx->launches++;
     HDB_CHECK_LAUNCH();
   }
-
-  // chain segments (cluster, depth), then stability per cluster
-  Buf<int64_t> s0(ctx, C), s1(ctx, C);
-  HDB_CUDA(cudaMemsetAsync(s0, 0, C * sizeof(int64_t), st));
-  HDB_CUDA(cudaMemsetAsync(s1, 0, C * sizeof(int64_t), st));
-  Buf<uint32_t> chain(ctx, m);
-  int64_t nv_total = 0;
-  {
-    k_flag_nonneg<<<gm, 256, 0, st>>>(ncl, m, flag); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-    scan_exclusive_i32_i64(ctx, flag, pos, m, pos.get() + m);
-    HDB_CUDA(cudaMemcpyAsync(hp, pos.get() + m, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    ctx->sync();
-    const int64_t nv = hp[0];
-    nv_total = nv;
-    Buf<uint64_t> ckeys(ctx, nv);
-    k_chain_keys<<<gm, 256, 0, st>>>(m, n, ncl, d0, pos, ckeys, chain); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-    radix_sort_u64(ctx, ckeys, chain, nv, 0, 32 + bits_for(C));
-    k_seg_bounds<<<grid_for(ctx, nv, 256), 256, 0, st>>>(ckeys, nv, s0, s1); ctx->launches++;
-    HDB_CHECK_LAUNCH();
-  }
   const int gc = grid_for(ctx, C, 128);
   {
-    Buf<ChainItem> items(ctx, nv_total);
-    k_chain_items<<<grid_for(ctx, nv_total, 256), 256, 0, st>>>(t, chain, nv_total, kind, lam,
-                                                                items); ctx->launches++;
+    Buf<ChainItem> items(ctx, nv);
+    k_chain_items<<<grid_for(ctx, nv, 256), 256, 0, st>>>(t, chain, nv, kind, lam, items); ctx->launches++;
     // at most m / kLongChain clusters have a long chain
     Buf<int32_t> long_list(ctx, m / kLongChain + 1), long_count(ctx, 1);
     HDB_CUDA(cudaMemsetAsync(long_count, 0, sizeof(int32_t), st));
@@ -1339,46 +1356,28 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
   const int fp64 = stab_mode == HDB_STAB_FP64;
   k_eom<<<gc, 128, 0, st>>>(C, ckid0, cparent, stab, stab64, fp64, sub, sub64, self_sel, arrive); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  Buf<int32_t> cj(ctx, C), cj2(ctx, C), sel(ctx, C), cover(ctx, C), cover2(ctx, C);
-  Buf<int8_t> anc(ctx, C), anc2(ctx, C);
-  k_sel_init<<<gc, 128, 0, st>>>(C, cparent, self_sel, cj, anc); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  Buf<int32_t> sel(ctx, C), cover(ctx, C);
   {
-    int32_t *ja = cj, *jb = cj2;
-    int8_t *aa = anc, *ab = anc2;
-    for (int it = 0; it < 64; it++) {
-      HDB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int32_t), st));
-      k_sel_jump<<<gc, 128, 0, st>>>(C, ja, aa, jb, ab, changed); ctx->launches++;
-      HDB_CHECK_LAUNCH();
-      HDB_CUDA(cudaMemcpyAsync(hflag, changed, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-      ctx->sync();
-      std::swap(ja, jb);
-      std::swap(aa, ab);
-      if (!hflag[0]) break;
+    Buf<Cover> cov(ctx, C), cov2(ctx, C);
+    Cover *ca = cov, *cb = cov2;
+    k_cover_init<<<gc, 128, 0, st>>>(C, cparent, self_sel, ca); ctx->launches++;
+    const int rounds = bits_for(C);
+    if (C <= kOneBlockItems) {
+      k_cover_jump_all<<<1, 1024, 0, st>>>(C, ca, cb, rounds); ctx->launches++;
+      if (rounds & 1) std::swap(ca, cb);
+    } else {
+      for (int it = 0; it < rounds; it++) {
+        k_cover_jump<<<gc, 128, 0, st>>>(C, ca, cb); ctx->launches++;
+        std::swap(ca, cb);
+      }
     }
-    k_selected<<<gc, 128, 0, st>>>(C, cparent, self_sel, aa, sel); ctx->launches++;
+    k_selected<<<gc, 128, 0, st>>>(C, ca, sel, cover); ctx->launches++;
     HDB_CHECK_LAUNCH();
   }
   Buf<int32_t> selpos(ctx, C + 1), label_of(ctx, C);
   scan_exclusive_i32_i32(ctx, sel, selpos, C, selpos.get() + C);
   k_label_map<<<gc, 128, 0, st>>>(C, sel, selpos, cseg.get(), croot.get(), label_of); ctx->launches++;
-  k_cover_init<<<gc, 128, 0, st>>>(C, cparent, sel, cj, cover); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  int32_t *cov_final = cover;
-  {
-    int32_t *ja = cj, *jb = cj2, *ca = cover, *cb = cover2;
-    for (int it = 0; it < 64; it++) {
-      HDB_CUDA(cudaMemsetAsync(changed, 0, sizeof(int32_t), st));
-      k_cover_jump<<<gc, 128, 0, st>>>(C, ja, ca, jb, cb, changed); ctx->launches++;
-      HDB_CHECK_LAUNCH();
-      HDB_CUDA(cudaMemcpyAsync(hflag, changed, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-      ctx->sync();
-      std::swap(ja, jb);
-      std::swap(ca, cb);
-      if (!hflag[0]) break;
-    }
-    cov_final = ca;
-  }
 
   // labels (and the per-point condensed rows when asked)
   Buf<int32_t> pcl;
@@ -1387,7 +1386,7 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
     pcl = Buf<int32_t>(ctx, n);
     plam = Buf<float>(ctx, n);
   }
-  k_points<<<gn, 256, 0, st>>>(t, par, ncl, lam, cov_final, birth, label_of, labels,
+  k_points<<<gn, 256, 0, st>>>(t, par, ncl, lam, cover, birth, label_of, labels,
                                condensed ? pcl.get() : nullptr, condensed ? plam.get() : nullptr); ctx->launches++;
   HDB_CHECK_LAUNCH();
   HDB_CUDA(cudaMemcpyAsync(hflag, selpos.get() + C, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
