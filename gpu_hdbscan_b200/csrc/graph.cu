@@ -62,49 +62,59 @@ __global__ void k_degrees(const int32_t *__restrict__ ids, int64_t n, int k, Seg
   }
 }
 
-// Histogram of degrees (clamped to the last bin), warp-aggregated.
-__global__ void k_degree_hist(const int32_t *__restrict__ deg, int64_t n,
-                              uint32_t *__restrict__ hist) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  for (; i - threadIdx.x < n; i += stride) {
-    bool ok = i < n;
-    int v = ok ? min(deg[i], kDegHistBins - 1) : -1;
-    uint32_t peers = __match_any_sync(0xffffffffu, v);
-    if (ok && (threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&hist[v], __popc(peers));
+// Histogram of degrees (clamped to the last bin): the first kDegNear bins,
+// where nearly all are, are counted in shared memory first.
+constexpr int kDegNear = 2048;
+__global__ void __launch_bounds__(256) k_degree_hist(const int32_t *__restrict__ deg, int64_t n,
+                                                     uint32_t *__restrict__ hist) {
+  __shared__ uint32_t near[kDegNear];
+  for (int i = threadIdx.x; i < kDegNear; i += blockDim.x) near[i] = 0;
+  __syncthreads();
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const int v = min(deg[i], kDegHistBins - 1);
+    if (v < kDegNear) atomicAdd(&near[v], 1u);
+    else atomicAdd(&hist[v], 1u);
   }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kDegNear; i += blockDim.x)
+    if (near[i]) atomicAdd(&hist[i], near[i]);
 }
 
 // Finds the threshold degree T = the P-th smallest degree.  out[0] = T,
-// out[1] = #{deg < T}, out[2] = #{deg == T}.  One block of 1024 threads, each
-// owning a chunk of 64 bins.
-__global__ void k_find_threshold(const uint32_t *__restrict__ hist, int64_t P, int64_t *out) {
-  __shared__ int64_t chunk_sum[1024];
-  const int per = kDegHistBins / 1024;
-  int64_t s = 0;
-  for (int b = 0; b < per; b++) s += hist[threadIdx.x * per + b];
-  chunk_sum[threadIdx.x] = s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int64_t cum = 0;
-    int c = 0;
-    while (c < 1024 && cum + chunk_sum[c] < P) cum += chunk_sum[c++];
-    int64_t T = -1, below = 0, at = 0;
-    if (c < 1024) {
-      for (int b = c * per; b < (c + 1) * per; b++) {
-        if (cum + (int64_t)hist[b] >= P) {
-          T = b;
-          below = cum;
-          at = hist[b];
-          break;
-        }
-        cum += hist[b];
-      }
+// out[1] = #{deg < T}, out[2] = #{deg == T}; T = -1 if there are fewer than P.
+// One block walks the bins 1,024 at a time up to T.
+__global__ void __launch_bounds__(1024) k_find_threshold(const uint32_t *__restrict__ hist, int64_t P,
+                                                         int64_t *out) {
+  __shared__ int64_t warp_sums[32];
+  const int lane = lane_id(), w = threadIdx.x >> 5;
+  int64_t cum = 0;  // points below the bins of this step
+  for (int b0 = 0; b0 < kDegHistBins; b0 += 1024) {
+    const int64_t c = hist[b0 + threadIdx.x];
+    int64_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
-    out[0] = T;
-    out[1] = below;
-    out[2] = at;
+    if (lane == 31) warp_sums[w] = x;
+    __syncthreads();
+    int64_t before = cum, total = 0;
+    for (int q = 0; q < 32; q++) {
+      if (q < w) before += warp_sums[q];
+      total += warp_sums[q];
+    }
+    before += x - c;
+    if (before < P && before + c >= P) {
+      out[0] = b0 + threadIdx.x;
+      out[1] = before;
+      out[2] = c;
+    }
+    cum += total;
+    if (cum >= P) return;  // the same in every thread
+    __syncthreads();
   }
+  if (threadIdx.x == 0) out[0] = -1;
 }
 
 __global__ void k_flag_eq(const int32_t *__restrict__ deg, int64_t n, int32_t T,

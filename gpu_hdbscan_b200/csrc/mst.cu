@@ -31,6 +31,13 @@ namespace {
 
 constexpr int kWarps = 8;
 
+// What a Boruvka round starts with.  Each round's kernels read its counts from
+// the device and leave the next round's there, so the host can queue several
+// rounds before it looks; a round without edges returns at once.
+struct RoundCounts {
+  unsigned long long edges, reps;
+};
+
 struct alignas(16) CEdge {
   int32_t a, b;  // current component representatives of the endpoints
   uint64_t key;  // float_key(weight) << 32 | CSR edge index
@@ -193,9 +200,10 @@ __global__ void k_iota(int32_t *__restrict__ v, int64_t n) {
 // the least high half) and one lane of the run updates minkey.  The `b`
 // endpoints of a run are distinct targets; each updates its own entry behind
 // a read of the current minimum.
-__global__ void k_min_edge(const CEdge *__restrict__ el, int64_t m,
+__global__ void k_min_edge(const CEdge *__restrict__ el, const RoundCounts *__restrict__ rc,
                            unsigned long long *__restrict__ minkey) {
   const int lane = lane_id();
+  const int64_t m = (int64_t)rc->edges;
   for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x; i0 < m; i0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = i0 + threadIdx.x;
     const bool valid = i < m;
@@ -226,8 +234,9 @@ __global__ void k_min_edge(const CEdge *__restrict__ el, int64_t m,
   }
 }
 
-__global__ void k_winner(const CEdge *__restrict__ el, int64_t m,
+__global__ void k_winner(const CEdge *__restrict__ el, const RoundCounts *__restrict__ rc,
                          const unsigned long long *__restrict__ minkey, int32_t *__restrict__ other) {
+  const int64_t m = (int64_t)rc->edges;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m;
        i += (int64_t)gridDim.x * blockDim.x) {
     CEdge c = el[i];
@@ -236,13 +245,15 @@ __global__ void k_winner(const CEdge *__restrict__ el, int64_t m,
   }
 }
 
-// Hook every representative to the component across its minimum edge.  The
-// chosen keys are appended with one atomicAdd per warp.
-__global__ void k_hook(const int32_t *__restrict__ reps, int64_t nr,
+// Hook every representative to the component across its minimum edge, and clear
+// the minimum for the next round.  The chosen keys are appended with one
+// atomicAdd per warp.
+__global__ void k_hook(const int32_t *__restrict__ reps, const RoundCounts *__restrict__ rc,
                        unsigned long long *__restrict__ minkey, const int32_t *__restrict__ other,
                        int32_t *__restrict__ parent, uint64_t *__restrict__ mst_keys,
                        unsigned long long *__restrict__ mst_count, int64_t cap) {
   const int lane = lane_id();
+  const int64_t nr = rc->edges ? (int64_t)rc->reps : 0;
   for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < nr; t0 += (int64_t)gridDim.x * blockDim.x) {
     const int64_t t = t0 + threadIdx.x;
     bool emit = false;
@@ -251,6 +262,7 @@ __global__ void k_hook(const int32_t *__restrict__ reps, int64_t nr,
       const int32_t v = reps[t];
       mk = minkey[v];
       if (mk != ~0ull) {
+        minkey[v] = ~0ull;
         const int32_t o = other[v];
         const bool mutual = other[o] == v;
         parent[v] = (mutual && v < o) ? v : o;
@@ -268,17 +280,11 @@ __global__ void k_hook(const int32_t *__restrict__ reps, int64_t nr,
   }
 }
 
-__global__ void k_reset_minkey(const int32_t *__restrict__ reps, int64_t nr,
-                               unsigned long long *__restrict__ minkey) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nr;
-       t += (int64_t)gridDim.x * blockDim.x)
-    minkey[reps[t]] = ~0ull;
-}
-
 // Pointer jumping to the roots (concurrent halving: every write moves a
 // pointer up its own tree, so each thread's walk ends at its root).
-__global__ void k_jump(const int32_t *__restrict__ reps, int64_t nr, int32_t *parent,
-                       uint32_t *err) {
+__global__ void k_jump(const int32_t *__restrict__ reps, const RoundCounts *__restrict__ rc,
+                       int32_t *parent, uint32_t *err) {
+  const int64_t nr = rc->edges ? (int64_t)rc->reps : 0;
   volatile int32_t *vp = parent;
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nr;
        t += (int64_t)gridDim.x * blockDim.x) {
@@ -306,8 +312,10 @@ __global__ void k_jump(const int32_t *__restrict__ reps, int64_t nr, int32_t *pa
 // counts.
 constexpr int kRfItems = 4, kRfThreads = 256;
 __global__ void __launch_bounds__(kRfThreads)
-    k_relabel_filter(const CEdge *__restrict__ el, int64_t m, const int32_t *__restrict__ parent,
-                     CEdge *__restrict__ out, unsigned long long *__restrict__ out_count) {
+    k_relabel_filter(const CEdge *__restrict__ el, const RoundCounts *__restrict__ rc,
+                     const int32_t *__restrict__ parent, CEdge *__restrict__ out,
+                     unsigned long long *__restrict__ out_count) {
+  const int64_t m = (int64_t)rc->edges;
   __shared__ uint32_t wofs[kRfThreads / 32];
   __shared__ unsigned long long bbase;
   const int lane = lane_id(), w = threadIdx.x >> 5;
@@ -358,10 +366,11 @@ __global__ void __launch_bounds__(kRfThreads)
   }
 }
 
-__global__ void k_roots(const int32_t *__restrict__ reps, int64_t nr,
+__global__ void k_roots(const int32_t *__restrict__ reps, const RoundCounts *__restrict__ rc,
                         const int32_t *__restrict__ parent, int32_t *__restrict__ out,
                         unsigned long long *__restrict__ count) {
   const int lane = lane_id();
+  const int64_t nr = rc->edges ? (int64_t)rc->reps : 0;
   for (int64_t t0 = (int64_t)blockIdx.x * blockDim.x; t0 < nr; t0 += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = t0 + threadIdx.x;
     int32_t v = 0;
@@ -535,46 +544,54 @@ int64_t boruvka_mst(Context *ctx, const hdb_graph *g, uint8_t *in_mst, hdb_mst_e
   Buf<unsigned long long> minkey(ctx, n);
   Buf<int32_t> other(ctx, n), parent(ctx, n), reps(ctx, n), reps2(ctx, n);
   Buf<uint64_t> keys(ctx, n);
-  Buf<unsigned long long> counters(ctx, 4);  // [0] mst edges, [1] live edges, [2] reps
+  // [0] MST edges, [1] the device error word's copy, then every round's counts
+  constexpr int kMaxRounds = 64, kQueued = 3;
+  static_assert(sizeof(unsigned long long) * (2 + 2 * (kMaxRounds + 1)) <= kPinnedErrOffset, "staging");
+  Buf<unsigned long long> counters(ctx, 2 + 2 * (kMaxRounds + 1));
+  RoundCounts *rc = reinterpret_cast<RoundCounts *>(counters.get() + 2);
+  unsigned long long *hc = static_cast<unsigned long long *>(ctx->pinned);
+  const size_t counter_bytes = sizeof(unsigned long long) * (2 + 2 * (kMaxRounds + 1));
   HDB_CUDA(cudaMemsetAsync(minkey, 0xff, n * sizeof(unsigned long long), st));
-  HDB_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned long long), st));
+  HDB_CUDA(cudaMemsetAsync(counters, 0, counter_bytes, st));
+  const RoundCounts first{(unsigned long long)m, (unsigned long long)n};
+  HDB_CUDA(cudaMemcpyAsync(rc, &first, sizeof(first), cudaMemcpyHostToDevice, st));
   const int gn = grid_for(ctx, n, 256);
   k_iota<<<gn, 256, 0, st>>>(parent, n); ctx->launches++;
   k_iota<<<gn, 256, 0, st>>>(reps, n); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  int64_t nr = n;
+  int64_t nr = n, chosen = 0;
   int rounds = 0;
   int32_t *rp = reps, *rp2 = reps2;
   CEdge *ep = el, *ep2 = el2;
   while (m > 0) {
-    HDB_REQUIRE(rounds < 64, HDB_ERR_INTERNAL, "MST: Boruvka did not converge");
-    rounds++;
-    const int ge = grid_for(ctx, m, 256);
-    const int gr = grid_for(ctx, nr, 256);
-    k_min_edge<<<ge, 256, 0, st>>>(ep, m, minkey); ctx->launches++;
-    k_winner<<<ge, 256, 0, st>>>(ep, m, minkey, other); ctx->launches++;
-    k_hook<<<gr, 256, 0, st>>>(rp, nr, minkey, other, parent, keys, counters, me); ctx->launches++;
-    k_reset_minkey<<<gr, 256, 0, st>>>(rp, nr, minkey); ctx->launches++;
-    k_jump<<<gr, 256, 0, st>>>(rp, nr, parent, ctx->dev_err); ctx->launches++;
-    HDB_CUDA(cudaMemsetAsync(counters.get() + 1, 0, 2 * sizeof(unsigned long long), st));
-    k_relabel_filter<<<grid_for(ctx, (m + kRfItems - 1) / kRfItems, kRfThreads), kRfThreads, 0, st>>>(
-        ep, m, parent, ep2, counters.get() + 1); ctx->launches++;
-    k_roots<<<gr, 256, 0, st>>>(rp, nr, parent, rp2, counters.get() + 2); ctx->launches++;
+    // a few rounds at a time: a round leaves at most half of the components, so
+    // the counts the host knows bound those of the queued rounds
+    const int ge = grid_for(ctx, m, 256), gr = grid_for(ctx, nr, 256);
+    const int gf = grid_for(ctx, (m + kRfItems - 1) / kRfItems, kRfThreads);
+    const int from = rounds;
+    HDB_REQUIRE(from + kQueued <= kMaxRounds, HDB_ERR_INTERNAL, "MST: Boruvka did not converge");
+    for (int i = from; i < from + kQueued; i++) {
+      k_min_edge<<<ge, 256, 0, st>>>(ep, rc + i, minkey); ctx->launches++;
+      k_winner<<<ge, 256, 0, st>>>(ep, rc + i, minkey, other); ctx->launches++;
+      k_hook<<<gr, 256, 0, st>>>(rp, rc + i, minkey, other, parent, keys, counters, me); ctx->launches++;
+      k_jump<<<gr, 256, 0, st>>>(rp, rc + i, parent, ctx->dev_err); ctx->launches++;
+      k_relabel_filter<<<gf, kRfThreads, 0, st>>>(ep, rc + i, parent, ep2, &rc[i + 1].edges); ctx->launches++;
+      k_roots<<<gr, 256, 0, st>>>(rp, rc + i, parent, rp2, &rc[i + 1].reps); ctx->launches++;
+      std::swap(ep, ep2);
+      std::swap(rp, rp2);
+    }
     HDB_CHECK_LAUNCH();
-    HDB_CUDA(cudaMemcpyAsync(h, counters, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    HDB_CUDA(cudaMemcpyAsync(counters.get() + 1, ctx->dev_err, sizeof(uint32_t),
+                             cudaMemcpyDeviceToDevice, st));
+    HDB_CUDA(cudaMemcpyAsync(hc, counters, counter_bytes, cudaMemcpyDeviceToHost, st));
     ctx->sync();
-    m = h[1];
-    nr = h[2];
-    HDB_REQUIRE(!(ctx->take_dev_err() & DEVERR_TIMEOUT), HDB_ERR_INTERNAL,
-                "MST: pointer jumping exceeded its bound");
-    std::swap(ep, ep2);
-    std::swap(rp, rp2);
+    HDB_REQUIRE(!((uint32_t)hc[1] & DEVERR_TIMEOUT) || !(ctx->take_dev_err() & DEVERR_TIMEOUT),
+                HDB_ERR_INTERNAL, "MST: pointer jumping exceeded its bound");
+    while (rounds < from + kQueued && hc[2 + 2 * rounds] > 0) rounds++;
+    m = (int64_t)hc[2 + 2 * (from + kQueued)];
+    nr = (int64_t)hc[3 + 2 * (from + kQueued)];
+    chosen = (int64_t)hc[0];
   }
-  if (rounds == 0) {
-    HDB_CUDA(cudaMemcpyAsync(h, counters, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    ctx->sync();
-  }
-  const int64_t chosen = h[0];
   if (id_order && chosen > 0 && chosen <= me) {
     // sorted by (weight, rank) now; the low halves become edge indices after
     radix_sort_u64(ctx, keys, nullptr, chosen, 0, 64);

