@@ -39,11 +39,12 @@
 // .sync.aligned: the warp is reconverged with __syncwarp() right before each,
 // because the code ahead of them branches per lane.
 //
-// Row minima: each distance is clamped at 0 and its float bits (order-preserving
-// for non-negative floats) have their low 6 bits replaced by the column, so one
-// unsigned min picks the closest column; the pushed distance is that value with
-// the column bits cleared.  The candidate therefore carries its distance to
-// within 2^-17 relative, and every (row, column) pair maps to one value.
+// Row minima: each distance's float bits have their low 6 bits replaced by the
+// column, so a signed min picks the closest column (a distance that rounding left
+// below zero comes out first, and counts as zero); the pushed distance is that
+// value with the column bits cleared.  The candidate therefore carries its
+// distance to within 2^-17 relative, and every (row, column) pair maps to one
+// value.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>
@@ -70,7 +71,7 @@ constexpr int kMmaWarp = kProducerWarp0 + kProducers;
 constexpr int kThreads = 32 * (kMmaWarp + 1);
 constexpr uint32_t kMetaArrivals = 1 + 32;          // producer + one cp.async arrival per lane
 constexpr uint64_t kWaitNs = 2000000000ull;         // 2 s
-constexpr uint32_t kNoKey = 0x7F800000u;            // keys at or above: no candidate
+constexpr int32_t kNoKey = 0x7F800000;              // keys at or above: no candidate
 // Shared memory is padded to at least this size so that no more than two
 // CTAs (2 x 256 tensor-memory columns = all 512) are resident on one SM.
 constexpr size_t kMinSmem = 80 * 1024;
@@ -567,26 +568,38 @@ __device__ void mma_issuer(Shared &sh, unsigned char *tiles, uint32_t tmem, int6
     atomicOr(err, DEVERR_TIMEOUT);
 }
 
-// Row minimum over 32 columns: key = clamped distance bits with the column in
-// the low 6 bits (skip_col: the row's own column, or -1).
-template <bool kSkip>
-__device__ __forceinline__ uint32_t row_min32(const uint32_t (&v)[32], const float *cn, float na,
-                                              float dscale, int skip_col) {
-  uint32_t best[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};  // four chains
+// The distances' keys of columns c and c + 1 as signed integers: the float bits
+// with the column in the low 6 bits.  (Two distances per packed instruction, each
+// the one rounding of na + nc and the one of the multiply-add.)
+__device__ __forceinline__ void two_keys(uint32_t a0, uint32_t a1, float n0, float n1, float na,
+                                         float dscale, uint32_t &d0, uint32_t &d1) {
+  const float2 s = __fadd2_rn(make_float2(na, na), make_float2(n0, n1));
+  const float2 dd = __ffma2_rn(make_float2(dscale, dscale),
+                               make_float2(__uint_as_float(a0), __uint_as_float(a1)), s);
+  d0 = __float_as_uint(dd.x);
+  d1 = __float_as_uint(dd.y);
+}
+
+// Row minimum over 32 columns other than the row's own (skip_col).
+__device__ __forceinline__ int32_t row_min32(const uint32_t (&v)[32], const float *cn, float na,
+                                             float dscale, int skip_col) {
+  int32_t best[2] = {0x7fffffff, 0x7fffffff};
 #pragma unroll
   for (int c4 = 0; c4 < 8; c4++) {
     const float4 nc = reinterpret_cast<const float4 *>(cn)[c4];
-    const float ncs[4] = {nc.x, nc.y, nc.z, nc.w};
+    uint32_t d[4];
+    two_keys(v[4 * c4], v[4 * c4 + 1], nc.x, nc.y, na, dscale, d[0], d[1]);
+    two_keys(v[4 * c4 + 2], v[4 * c4 + 3], nc.z, nc.w, na, dscale, d[2], d[3]);
+    int32_t key[4];
 #pragma unroll
     for (int e = 0; e < 4; e++) {
       const int c = 4 * c4 + e;
-      const float dd = fmaxf(__fmaf_rn(dscale, __uint_as_float(v[c]), __fadd_rn(na, ncs[e])), 0.0f);
-      uint32_t key = (__float_as_uint(dd) & ~63u) | (uint32_t)c;
-      if (kSkip) key = c == skip_col ? 0xffffffffu : key;
-      best[e] = min(best[e], key);
+      key[e] = c == skip_col ? 0x7fffffff : (int32_t)((d[e] & ~63u) | (uint32_t)c);
     }
+    best[0] = __vimin3_s32(best[0], key[0], key[1]);
+    best[1] = __vimin3_s32(best[1], key[2], key[3]);
   }
-  return min(min(best[0], best[1]), min(best[2], best[3]));
+  return min(best[0], best[1]);
 }
 
 // row_min32 of this lane's row (keys carry the column) and, from the same
@@ -594,21 +607,23 @@ __device__ __forceinline__ uint32_t row_min32(const uint32_t (&v)[32], const flo
 // lane l holds column l's minimum, keyed by the row's lane.  The column minima
 // take 31 shuffles: at each step a lane keeps half of its live columns and
 // takes the other lane's values for them (recursive halving).
-__device__ __forceinline__ uint32_t row_col_min32(uint32_t (&v)[32], const float *cn, float na,
-                                                  float dscale, int lane, uint32_t &colmin) {
-  uint32_t best[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
+__device__ __forceinline__ int32_t row_col_min32(uint32_t (&v)[32], const float *cn, float na,
+                                                 float dscale, int lane, int32_t &colmin) {
+  int32_t best[2] = {0x7fffffff, 0x7fffffff};
 #pragma unroll
   for (int c4 = 0; c4 < 8; c4++) {
     const float4 nc = reinterpret_cast<const float4 *>(cn)[c4];
-    const float ncs[4] = {nc.x, nc.y, nc.z, nc.w};
+    uint32_t d[4];
+    two_keys(v[4 * c4], v[4 * c4 + 1], nc.x, nc.y, na, dscale, d[0], d[1]);
+    two_keys(v[4 * c4 + 2], v[4 * c4 + 3], nc.z, nc.w, na, dscale, d[2], d[3]);
 #pragma unroll
-    for (int e = 0; e < 4; e++) {
+    for (int e = 0; e < 4; e += 2) {
       const int c = 4 * c4 + e;
-      const float dd = fmaxf(__fmaf_rn(dscale, __uint_as_float(v[c]), __fadd_rn(na, ncs[e])), 0.0f);
-      const uint32_t db = __float_as_uint(dd) & ~63u;
-      best[e] = min(best[e], db | (uint32_t)c);
-      v[c] = db | (uint32_t)lane;
+      best[e >> 1] = __vimin3_s32(best[e >> 1], (int32_t)((d[e] & ~63u) | (uint32_t)c),
+                                  (int32_t)((d[e + 1] & ~63u) | (uint32_t)(c + 1)));
     }
+#pragma unroll
+    for (int e = 0; e < 4; e++) v[4 * c4 + e] = (d[e] & ~63u) | (uint32_t)lane;
   }
 #pragma unroll
   for (int s = 16; s >= 1; s >>= 1) {
@@ -617,12 +632,15 @@ __device__ __forceinline__ uint32_t row_col_min32(uint32_t (&v)[32], const float
     for (int i = 0; i < s; i++) {
       const uint32_t send = up ? v[i] : v[i + s];
       const uint32_t keep = up ? v[i + s] : v[i];
-      v[i] = min(keep, __shfl_xor_sync(0xffffffffu, send, s));
+      v[i] = (uint32_t)min((int32_t)keep, (int32_t)__shfl_xor_sync(0xffffffffu, send, s));
     }
   }
-  colmin = v[0];
-  return min(min(best[0], best[1]), min(best[2], best[3]));
+  colmin = (int32_t)v[0];
+  return min(best[0], best[1]);
 }
+
+// The distance of a minimum's key; one that rounding left below zero counts as zero.
+__device__ __forceinline__ float key_dist(int32_t k) { return fmaxf(__int_as_float(k & ~63), 0.0f); }
 
 template <bool kProbe>
 __device__ void epilogue(const JoinArgs &a, Shared &sh, uint32_t tmem, int64_t n, int64_t ntiles,
@@ -681,24 +699,24 @@ __device__ void epilogue(const JoinArgs &a, Shared &sh, uint32_t tmem, int64_t n
     // row, and -- the new x old block being the transpose of the old x new
     // one -- the closest old row of every new row, as column minima over the
     // old rows; lane l then speaks for new row l.
-    uint32_t k1, k2 = 0xffffffffu;
+    int32_t k1, k2 = 0x7fffffff;
     int32_t id1 = -1, id2 = -1, tgt2 = -1;
     float wst2 = 0.0f;
     if (isnew) {
-      k1 = row_min32<true>(v0, cn, na, a.dscale, lane);
+      k1 = row_min32(v0, cn, na, a.dscale, lane);
     } else {
       k1 = row_col_min32(v0, cn, na, a.dscale, lane, k2);
-      if (k2 < kNoKey) id2 = M.ids[64 * j + 32 + (k2 & 63u)];
+      if (k2 < kNoKey) id2 = M.ids[64 * j + 32 + (k2 & 63)];
       tgt2 = M.ids[64 * j + lane];
       wst2 = M.wst[64 * j + lane];
     }
-    if (k1 < kNoKey) id1 = M.ids[64 * j + (k1 & 63u)];
+    if (k1 < kNoKey) id1 = M.ids[64 * j + (k1 & 63)];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.mempty[m]);
     // candidates that can enter their target's list, appended to the list
     // that is sorted by target before the next merge: one reservation per
     // warp instead of a returning inbox atomic per candidate
-    const float d1 = __uint_as_float(k1 & ~63u), d2 = __uint_as_float(k2 & ~63u);
+    const float d1 = key_dist(k1), d2 = key_dist(k2);
     const bool c1 = vrow && id1 >= 0 && d1 < wst;
     const bool c2 = !isnew && lane < nn && id2 >= 0 && d2 < wst2;
     const bool av[2] = {c1, c2};
