@@ -75,9 +75,9 @@ class Context:
         _lib.check(self.L.hdb_set_stream(self.h, C.c_void_p(self._stream)))
 
     def set_join_tiles(self, tiles: int):
-        """FP32 local join form: 1 or 2 distance tiles of 4 x 4 per lane, or 0
-        (the default): by rows up to 28 dimensions, beyond both tile forms are
-        timed per shape and the faster is kept."""
+        """FP32 local join form: 1 or 2 for distance tiles at any number of
+        dimensions (both the same form), or 0 (the default): by rows up to 28
+        dimensions, in tiles beyond."""
         _lib.check(self.L.hdb_set_join_tiles(self.h, int(tiles)))
 
     def close(self):

@@ -153,7 +153,6 @@ HDB_API hdb_status hdb_create(hdb_ctx **out, int32_t device) {
     Context &c = h->c;
     c.device = device;
     c.num_sms = prop.multiProcessorCount;
-    c.l2_bytes = prop.l2CacheSize;
     try {
       HDB_CUDA(cudaStreamCreateWithFlags(&c.own_stream, cudaStreamNonBlocking));
       c.stream = c.own_stream;

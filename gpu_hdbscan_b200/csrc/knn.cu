@@ -18,11 +18,8 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
-#include <array>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <vector>
 
 #include "hdb_internal.cuh"
@@ -682,17 +679,7 @@ __global__ void k_bucket_bounds(const uint32_t *__restrict__ tgt,
 }
 
 // ---- FP32 local join -----------------------------------------------------
-// Shared memory of one warp: best candidates (distance bits, then ids: best
-// other-new and best old per new row; best new per old row) | slot ids | one chunk of kJc dimensions
-// of every staged row.  Rows are staged a chunk at a time, so a warp needs
-// ~9 KB whatever d is and an SM keeps 16 warps of joins in flight.
-constexpr int kJc = 32;              // dimensions per staged chunk
 constexpr int kJoinWarps = 8;
-struct JoinSmem {
-  static constexpr int kBest = 96;   // distances and ids
-  static constexpr int kIds = 64;
-  static constexpr size_t kBytes = kBest * 8 + kIds * 4 + (size_t)64 * kJc * 4;
-};
 
 // A row's counts and both sample lists in one memory round trip, loaded one row
 // ahead so that they are in flight while the previous row is joined.
@@ -747,118 +734,124 @@ struct SlotLists {
 __constant__ uint32_t kRecip[9] = {0, 65536, 32768, 21846, 16384, 13108, 10923, 9363, 8192};
 __device__ __forceinline__ int div_small(int x, int m) { return (int)(((uint32_t)x * kRecip[m]) >> 16); }
 
-// Float offset of 16-byte piece q of staged row r: the pieces of a row are
-// permuted by the row's group of four, so the rows one warp-wide 16-byte load
-// reads (one per tile group) fall into different bank groups.
-__device__ __forceinline__ int stage_off(int r, int q) { return r * kJc + ((q ^ ((r >> 2) & 7)) << 2); }
+// Shared memory of one warp: best candidates (distance bits, then ids: best
+// other-new and best old per new row; best new per old row) | slot ids | a chunk
+// of kJc dimensions of every staged row (new rows, then old ones).  A staged row
+// takes nine 16-byte pieces of which eight hold data: rows that follow one another
+// then start in different bank groups.
+constexpr int kJc = 32;         // dimensions per staged chunk
+constexpr int kJPitch = kJc / 4 + 1;
+constexpr int kJCols = 8;       // most columns of a tile
+struct JoinSmem {
+  static constexpr int kBest = 96;   // distances and ids
+  static constexpr int kIds = 64;
+  static constexpr int kChunk = 64 * kJPitch;  // 16-byte pieces
+  static constexpr size_t kBytes = kBest * 8 + kIds * 4 + (size_t)kChunk * 16;
+};
 
-// Stages dimensions [c0, c0 + 4 * nq) of the nn new rows (slots 0..) and the
-// no old rows (slots 32..): 16-byte cp.async copies when every row piece is
-// 16-byte aligned (d % 4 == 0), else scalar loads, zero padded to a multiple
-// of four (adding fmaf(0, 0, s) = s leaves every sum unchanged).
+// Copies dimensions [c0, c0 + 4 * nq) of the nn new and no old rows: 16-byte
+// cp.async copies when every row piece is 16-byte aligned (d % 4 == 0; one
+// group is committed), else scalar loads, zero padded to a multiple of four
+// (adding fmaf(0, 0, s) = s leaves every sum unchanged).
 __device__ __forceinline__ void stage_chunk(const float *__restrict__ X, int d, int c0, int nq,
-                                            const int32_t *ids, int nn, int no, float *Xs,
-                                            bool vec) {
+                                            const int32_t *ids, int nn, int T, float4 *Xs, bool vec) {
   const int lane = lane_id();
-  const int items = (nn + no) * nq;
-  if (vec && nq == kJc / 4) {  // full chunk: eight pieces per row, no division
-    for (int it = lane; it < items; it += 32) {
-      const int r = it >> 3, q = it & 7;
-      const int slot = r < nn ? r : 32 + (r - nn);
-      const float *src = X + (int64_t)ids[slot] * d + c0 + 4 * q;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + stage_off(slot, q));
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  } else if (vec) {
-    for (int it = lane; it < items; it += 32) {
-      const int r = div_small(it, nq), q = it - r * nq;
-      const int slot = r < nn ? r : 32 + (r - nn);
-      const float *src = X + (int64_t)ids[slot] * d + c0 + 4 * q;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + stage_off(slot, q));
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src) : "memory");
-    }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
-  } else {
-    for (int it = lane; it < items; it += 32) {
-      const int r = div_small(it, nq), q = it - r * nq;
-      const int slot = r < nn ? r : 32 + (r - nn);
-      const float *src = X + (int64_t)ids[slot] * d;
+  const int items = T * nq;
+  for (int it = lane; it < items; it += 32) {
+    const int r = nq == kJc / 4 ? it / (kJc / 4) : div_small(it, nq), q = it - r * nq;
+    const float *src = X + (int64_t)ids[r < nn ? r : 32 + r - nn] * d + c0 + 4 * q;
+    float4 *dst = Xs + r * kJPitch + q;
+    if (vec) {
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(
+                       (uint32_t)__cvta_generic_to_shared(dst)),
+                   "l"(src)
+                   : "memory");
+    } else {
+      const int left = d - c0 - 4 * q;
       float4 v;
-      const int c = c0 + 4 * q;
-      v.x = c < d ? __ldg(src + c) : 0.0f;
-      v.y = c + 1 < d ? __ldg(src + c + 1) : 0.0f;
-      v.z = c + 2 < d ? __ldg(src + c + 2) : 0.0f;
-      v.w = c + 3 < d ? __ldg(src + c + 3) : 0.0f;
-      *reinterpret_cast<float4 *>(Xs + stage_off(slot, q)) = v;
+      v.x = left > 0 ? __ldg(src) : 0.0f;
+      v.y = left > 1 ? __ldg(src + 1) : 0.0f;
+      v.z = left > 2 ? __ldg(src + 2) : 0.0f;
+      v.w = left > 3 ? __ldg(src + 3) : 0.0f;
+      *dst = v;
     }
   }
-  __syncwarp();
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
 }
 
-// Tile t of a row-join with rg row groups (new rows), cgn new and cgo old
-// column groups: the new x new tiles are the upper triangle i <= j (a pair of
-// different groups is computed once and offered to both rows), then the new x
-// old tiles.  Returns the first slot of its rows (r0) and of its columns (c0)
-// and its kind: 1 diagonal, 2 above the diagonal, 3 old columns.
-__device__ __forceinline__ int tile_of(int t, int rg, int cgn, int cgo, int &r0, int &c0) {
-  const int tri = cgn > 0 ? rg * (rg + 1) / 2 : 0;
-  if (t < tri) {
-    int i = 0, first = 0;  // row group i holds tiles first .. first + rg - i - 1
+// Adds a staged chunk's nq pieces to the sums of four rows (from piece `ra`)
+// and cw columns (from piece `cb`, `step` pieces apart, none past `last`).  One
+// loop with a way out after each column: a loop for every width runs 1.5x slower,
+// as the warps of an SM, each at another width, then miss the instruction cache.
+__device__ __forceinline__ void tile_sums(float (&acc)[4][kJCols], const float4 *Xs, int ra, int cb,
+                                          int step, int last, int nq, int cw) {
+#pragma unroll 2
+  for (int q = 0; q < nq; q++) {
+    float4 xa[4], xc = Xs[cb + q];
 #pragma unroll
-    for (int r = 1; r < 8; r++) {
-      const int f = r * rg - r * (r - 1) / 2;
-      if (r < rg && t >= f) { i = r; first = f; }
+    for (int i = 0; i < 4; i++) xa[i] = Xs[ra + i * kJPitch + q];
+#pragma unroll
+    for (int j = 0; j < kJCols; j++) {
+      const float4 next = Xs[min(cb + (j + 1) * step, last) + q];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const float2 d01 = neg_diff2(make_float2(xc.x, xc.y), make_float2(xa[i].x, xa[i].y));
+        const float2 d23 = neg_diff2(make_float2(xc.z, xc.w), make_float2(xa[i].z, xa[i].w));
+        float s_ = __fmaf_rn(d01.x, d01.x, acc[i][j]);
+        s_ = __fmaf_rn(d01.y, d01.y, s_);
+        s_ = __fmaf_rn(d23.x, d23.x, s_);
+        acc[i][j] = __fmaf_rn(d23.y, d23.y, s_);
+      }
+      if (j + 1 >= cw) break;
+      xc = next;
     }
-    r0 = 4 * i;
-    c0 = 4 * (i + t - first);
-    return t == first ? 1 : 2;
   }
-  t -= tri;
-  const int i = div_small(t, cgo);
-  r0 = 4 * i;
-  c0 = 32 + 4 * (t - i * cgo);
-  return 3;
 }
 
-// Local join, one warp per row (UpdateGraph, nndescent.cu:1487-1580).  The
-// distance matrix new x (new U old) is cut into 4 x 4 tiles, up to
-// kJoinTiles per lane; a lane keeps its tiles' sums in registers while the
-// rows pass through shared memory a chunk of kJc dimensions at a time, so
-// every pair is the reference's sequential FP32 difference sum over
-// j = 0..d-1.  The tiles' row and column minima meet in shared memory: first
-// the least distance of every slot (its bits, a 32-bit atomicMin), then, among the
-// pairs at that distance, the least id.  Every new neighbour gets its closest
-// other new one and its closest old one, every old neighbour its closest new
-// one.  (One 64-bit atomicMin of distance and id per tile row and column, which
-// is a compare-and-swap loop in shared memory, took about 1,000 of the 2,500
-// instructions of a row-join at d = 12.)  cross_only (the merge join, TiledNewOldNeighborsCompareKernelForMerge
-// :1328-1383 launched without the new x new kernel, UpdateGraphForMerge
-// :1582-1640) leaves out the new x new tiles: new neighbours get their closest
-// old one only.
-// kTiles: 4 x 4 register tiles per lane and pass (32 * kTiles per pass over
-// the staged rows); one tile needs 80 registers and fits three blocks per SM,
-// two need 122 and fit two -- the FP32 join tuner picks per (d, k, S).
-template <int kTiles>
-__global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
+// Local join, one warp per row (UpdateGraph, nndescent.cu:1487-1580).  With the
+// new rows first and the old ones behind them (T in all), the pairs are (a, c)
+// with a new row a < c.  Four rows at a time (group i: rows 4i .. 4i + 3, columns
+// from 4i) they are cut into tiles of cw columns, a group's tile l taking every
+// n_i-th column from the l-th on; cw is the least that gives every tile of the
+// row-join a lane of its own, up to kJCols (row-joins that need more take further
+// passes over the rows).  A lane keeps its tile's sums in registers while the rows
+// pass through shared memory a chunk of kJc dimensions at a time, so every pair is
+// the reference's sequential FP32 difference sum over j = 0..d-1.  The tiles' row
+// and column minima meet in shared memory: first the least distance of every slot
+// (its bits, a 32-bit atomicMin), then, among the pairs at that distance, the
+// least id.  Every new neighbour gets its closest other new one and its closest
+// old one, every old neighbour its closest new one.  cross_only (the merge join,
+// TiledNewOldNeighborsCompareKernelForMerge :1328-1383 launched without the new x
+// new kernel, UpdateGraphForMerge :1582-1640) leaves out the new x new pairs: new
+// neighbours get their closest old one only.
+//
+// Bound by the FMA pipe and the shared-memory pipe together (about 65 % and 70 %
+// busy at 200k x 128, k = 32): a row-join's pairs give a lane some 30 sums, so 11
+// operand loads feed 28 pairs and no more.  Against tiles of 4 x 4, one or two per lane
+// (the last slot of them mostly empty), six iterations: 200k x 128, k = 16 8.4 ->
+// 6.0 ms, k = 32 12.9 -> 12.3; 1M x 64, k = 32 37.9 -> 37.3; 100k x 784 35.2 ->
+// 33.2.  Chunks of 16 dimensions with the next on its way are 4 % slower than
+// chunks of 32 without, five columns at three blocks per SM 10-20 %.
+__global__ void __launch_bounds__(32 * kJoinWarps, 2)
     k_join(const float *__restrict__ X, int64_t n, int d, int S, const int32_t *__restrict__ newS,
            const int32_t *__restrict__ oldS, const int8_t *__restrict__ nf,
            const int8_t *__restrict__ of, int32_t *__restrict__ nrev, int32_t *__restrict__ orev,
            const float *__restrict__ worst, CandList cl, int cross_only) {
   extern __shared__ __align__(16) unsigned char smem_join[];
+  using Smem = JoinSmem;
   const int lane = lane_id();
-  const int wpb = blockDim.x >> 5;
-  unsigned char *base = smem_join + (threadIdx.x >> 5) * JoinSmem::kBytes;
+  unsigned char *base = smem_join + (threadIdx.x >> 5) * Smem::kBytes;
   uint32_t *bdist = reinterpret_cast<uint32_t *>(base);
-  uint32_t *bid = bdist + JoinSmem::kBest;
-  int32_t *ids = reinterpret_cast<int32_t *>(base + JoinSmem::kBest * 8);
-  float *Xs = reinterpret_cast<float *>(base + JoinSmem::kBest * 8 + JoinSmem::kIds * 4);
+  uint32_t *bid = bdist + Smem::kBest;
+  int32_t *ids = reinterpret_cast<int32_t *>(base + Smem::kBest * 8);
+  float4 *Xs = reinterpret_cast<float4 *>(base + Smem::kBest * 8 + Smem::kIds * 4);
   const bool vec = (d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
   unsigned long long w_rows = 0, w_cands = 0, w_pairs = 0;
   ListCursor cur;  // this warp's space in the candidate list
-  const int64_t stride = (int64_t)gridDim.x * wpb;
+  const int64_t stride = (int64_t)gridDim.x * kJoinWarps;
+  const int chunks = (d + kJc - 1) / kJc;
   SlotLists lists;
-  int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5);
+  int64_t row = (int64_t)blockIdx.x * kJoinWarps + (threadIdx.x >> 5);
   lists.load(row, n, S, newS, oldS, nf, of, nrev, orev);
   for (; row < n; row += stride) {
     int nn, no;
@@ -869,91 +862,90 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
       if (lane == 0) { nrev[row] = 0; orev[row] = 0; }
       mine.compact(S, ids, nn, no);
     }
-#pragma unroll
-    for (int g = 0; g < JoinSmem::kBest; g += 32) bdist[g + lane] = bid[g + lane] = 0xffffffffu;
-    __syncwarp();
     if (nn == 0 || nn + no < 2 || (cross_only && no == 0)) continue;
-    w_rows += nn + no;
+    const int T = nn + no;
+    w_rows += T;
     w_pairs += (cross_only ? 0 : nn * (nn - 1) / 2) + nn * no;  // the reference's pairs
-    const int rg = (nn + 3) >> 2;                              // row groups (new rows)
-    const int cgn = cross_only ? 0 : rg, cgo = (no + 3) >> 2;  // column groups: new, old
-    const int tiles = (cgn > 0 ? rg * (rg + 1) / 2 : 0) + rg * cgo;
+#pragma unroll
+    for (int g = 0; g < Smem::kBest; g += 32) bdist[g + lane] = bid[g + lane] = 0xffffffffu;
+    // lane i < rg: the columns of row group i
+    const int rg = (nn + 3) >> 2;
+    const int first_col = cross_only ? nn : 4 * lane;
+    const int len = lane < rg ? T - first_col : 0;
+    int cw = kJCols;
+    int tiles_i = div_small(len + cw - 1, cw);  // of group `lane`
+    int tiles = __reduce_add_sync(0xffffffffu, tiles_i);
+    while (cw > 1 && tiles <= 32) {  // narrower, as long as a slot holds them
+      const int t_i = div_small(len + cw - 2, cw - 1);
+      const int t = __reduce_add_sync(0xffffffffu, t_i);
+      if (t > 32) break;
+      cw--;
+      tiles_i = t_i;
+      tiles = t;
+    }
+    int upto = tiles_i;  // tiles of the groups up to and with `lane`'s
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
     uint32_t before[3] = {0xffffffffu, 0xffffffffu, 0xffffffffu};
-    // up to 32 * kTiles tiles per pass through the rows (rows with more
-    // samples take further passes; at most 100 tiles)
-    for (int t0 = 0; t0 < tiles; t0 += 32 * kTiles) {
-      int r0[kTiles], c0[kTiles], kind[kTiles];
-      float acc[kTiles][4][4];
+    for (int t0 = 0; t0 < tiles; t0 += 32) {
+      // tile t0 + lane: its row group, columns c0, c0 + step, ...
+      const int t = t0 + lane;
+      int grp = 0;
 #pragma unroll
-      for (int u = 0; u < kTiles; u++) {
-        kind[u] = r0[u] = c0[u] = 0;
-        if (t0 + 32 * u >= tiles) continue;  // for the whole warp
-        const int t = t0 + lane + 32 * u;
-        kind[u] = t < tiles ? tile_of(t, rg, cgn, cgo, r0[u], c0[u]) : 0;
-        if (kind[u] == 0) { r0[u] = 0; c0[u] = 0; }
+      for (int r = 0; r < 7; r++) grp += t >= __shfl_sync(0xffffffffu, upto, r) ? 1 : 0;
+      grp = min(grp, rg - 1);
+      const int step = __shfl_sync(0xffffffffu, tiles_i, grp);
+      const int start = __shfl_sync(0xffffffffu, upto, grp) - step;
+      const int r0 = 4 * grp, c0 = (cross_only ? nn : r0) + t - start;
+      const bool mine = t < tiles;
+      float acc[4][kJCols];
 #pragma unroll
-        for (int i = 0; i < 4; i++)
+      for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[u][i][j] = 0.0f;
-      }
-      for (int cd = 0; cd < d; cd += kJc) {
-        const int nq = (min(kJc, d - cd) + 3) >> 2;
-        __syncwarp();  // the previous chunk is no longer read
-        stage_chunk(X, d, cd, nq, ids, nn, no, Xs, vec);
-#pragma unroll
-        for (int u = 0; u < kTiles; u++) {
-          if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
-          // the four rows of a tile side share one piece permutation
-          const int ka = (r0[u] >> 2) & 7, kc = (c0[u] >> 2) & 7;
-          for (int q = 0; q < nq; q++) {
-            const float *pa = Xs + r0[u] * kJc + ((q ^ ka) << 2);
-            const float *pc = Xs + c0[u] * kJc + ((q ^ kc) << 2);
-            float4 xc[4];
-#pragma unroll
-            for (int j = 0; j < 4; j++) xc[j] = *reinterpret_cast<const float4 *>(pc + j * kJc);
-#pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const float4 xa = *reinterpret_cast<const float4 *>(pa + i * kJc);
-#pragma unroll
-              for (int j = 0; j < 4; j++) {
-                const float2 d01 = neg_diff2(make_float2(xc[j].x, xc[j].y), make_float2(xa.x, xa.y));
-                const float2 d23 = neg_diff2(make_float2(xc[j].z, xc[j].w), make_float2(xa.z, xa.w));
-                float s_ = __fmaf_rn(d01.x, d01.x, acc[u][i][j]);
-                s_ = __fmaf_rn(d01.y, d01.y, s_);
-                s_ = __fmaf_rn(d23.x, d23.x, s_);
-                acc[u][i][j] = __fmaf_rn(d23.y, d23.y, s_);
-              }
-            }
-          }
-        }
+        for (int j = 0; j < kJCols; j++) acc[i][j] = 0.0f;
+      const int last = (T - 1) * kJPitch;
+      const int ra = r0 * kJPitch, cb = min(mine ? c0 : 0, T - 1) * kJPitch;
+      __syncwarp();  // the staged rows of the pass before are no longer read; ids are written
+      stage_chunk(X, d, 0, min(kJc / 4, (d + 3) >> 2), ids, nn, T, Xs, vec);
+      for (int ch = 0; ch < chunks; ch++) {
+        const int nq = min(kJc / 4, (d - ch * kJc + 3) >> 2);
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncwarp();
+        tile_sums(acc, Xs, ra, cb, step * kJPitch, last, nq, cw);
+        __syncwarp();  // this chunk is no longer read
+        if (ch + 1 < chunks)
+          stage_chunk(X, d, (ch + 1) * kJc, min(kJc / 4, (d - (ch + 1) * kJc + 3) >> 2), ids, nn, T, Xs,
+                      vec);
       }
       // the least distances; what is no pair of the join gets all ones
+      {
+        uint32_t rnew[4], rold[4];
 #pragma unroll
-      for (int u = 0; u < kTiles; u++) {
-        if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
-        const bool oldcols = kind[u] == 3;
-        const int cb = oldcols ? c0[u] - 32 : c0[u];  // first column within its block
-        const int nr = nn - r0[u], nc = (oldcols ? no : nn) - cb;
-        uint32_t cmin[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
-        uint32_t *rows = bdist + (oldcols ? 32 : 0) + r0[u];
-        uint32_t *cols = bdist + (oldcols ? 64 : 0) + cb;
+        for (int i = 0; i < 4; i++) rnew[i] = rold[i] = 0xffffffffu;
+#pragma unroll
+        for (int j = 0; j < kJCols; j++) {
+          if (j >= cw) break;  // for the whole warp
+          const int c = c0 + j * step;
+          const bool there = mine && c < T, old = c >= nn;
+          uint32_t cmin = 0xffffffffu;
+#pragma unroll
+          for (int i = 0; i < 4; i++) {
+            uint32_t v = __float_as_uint(acc[i][j]);
+            if (!there || r0 + i >= nn || r0 + i >= c) v = 0xffffffffu;
+            acc[i][j] = __uint_as_float(v);
+            cmin = min(cmin, v);
+            rnew[i] = min(rnew[i], old ? 0xffffffffu : v);
+            rold[i] = min(rold[i], old ? v : 0xffffffffu);
+          }
+          if (cmin != 0xffffffffu) atomicMin(&bdist[old ? 64 + c - nn : c], cmin);
+        }
 #pragma unroll
         for (int i = 0; i < 4; i++) {
-          uint32_t rmin = 0xffffffffu;
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            uint32_t v = __float_as_uint(acc[u][i][j]);
-            if (i >= nr || j >= nc || (i == j && kind[u] == 1)) v = 0xffffffffu;
-            acc[u][i][j] = __uint_as_float(v);
-            rmin = min(rmin, v);
-            cmin[j] = min(cmin[j], v);
-          }
-          if (i < nr) atomicMin(&rows[i], rmin);
-        }
-        if (kind[u] != 1) {
-#pragma unroll
-          for (int j = 0; j < 4; j++)
-            if (j < nc) atomicMin(&cols[j], cmin[j]);
+          if (rnew[i] != 0xffffffffu) atomicMin(&bdist[r0 + i], rnew[i]);
+          if (rold[i] != 0xffffffffu) atomicMin(&bdist[32 + r0 + i], rold[i]);
         }
       }
       __syncwarp();
@@ -967,26 +959,35 @@ __global__ void __launch_bounds__(32 * kJoinWarps, kTiles == 1 ? 3 : 2)
       }
 #pragma unroll
       for (int g = 0; g < 3; g++) before[g] = bdist[32 * g + lane];
-      // the least ids at those distances
+      // the least ids at those distances: first which pairs are at a minimum (bit
+      // 4 j + i; unrolled, as the sums are in registers), then a loop over those few
+      uint32_t at_row = 0, at_col = 0;
+      {
+        // no pair of the join: a value that no sum takes
+        auto held = [](uint32_t v) { return v == 0xffffffffu ? 0xfffffffeu : v; };
+        const uint4 mn = *reinterpret_cast<const uint4 *>(bdist + r0);
+        const uint4 mo = *reinterpret_cast<const uint4 *>(bdist + 32 + r0);
+        const uint32_t mns[4] = {held(mn.x), held(mn.y), held(mn.z), held(mn.w)};
+        const uint32_t mos[4] = {held(mo.x), held(mo.y), held(mo.z), held(mo.w)};
 #pragma unroll
-      for (int u = 0; u < kTiles; u++) {
-        if (t0 + 32 * u >= tiles || kind[u] == 0) continue;
-        const bool oldcols = kind[u] == 3;
-        const int cb = oldcols ? c0[u] - 32 : c0[u];
-        const int rat = (oldcols ? 32 : 0) + r0[u], cat = (oldcols ? 64 : 0) + cb;
-        const uint4 rm = *reinterpret_cast<const uint4 *>(bdist + rat);
-        const uint4 cm = *reinterpret_cast<const uint4 *>(bdist + cat);
-        const uint32_t rms[4] = {rm.x, rm.y, rm.z, rm.w}, cms[4] = {cm.x, cm.y, cm.z, cm.w};
+        for (int j = 0; j < kJCols; j++) {
+          if (j >= cw) break;  // for the whole warp
+          const int c = min(c0 + j * step, T - 1);
+          const bool old = c >= nn;
+          const uint32_t cm = held(bdist[old ? 64 + c - nn : c]);
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-#pragma unroll
-          for (int j = 0; j < 4; j++) {
-            const uint32_t v = __float_as_uint(acc[u][i][j]);
-            if (v == 0xffffffffu) continue;
-            if (v == rms[i]) atomicMin(&bid[rat + i], (uint32_t)ids[c0[u] + j]);
-            if (v == cms[j] && kind[u] != 1) atomicMin(&bid[cat + j], (uint32_t)ids[r0[u] + i]);
+          for (int i = 0; i < 4; i++) {
+            const uint32_t v = __float_as_uint(acc[i][j]);
+            at_row |= v == (old ? mos[i] : mns[i]) ? 1u << (4 * j + i) : 0u;
+            at_col |= v == cm ? 1u << (4 * j + i) : 0u;
           }
         }
+      }
+      for (uint32_t m = at_row | at_col; m; m &= m - 1) {
+        const int b = __ffs(m) - 1, i = b & 3, c = c0 + (b >> 2) * step;
+        const bool old = c >= nn;
+        if ((at_row >> b) & 1) atomicMin(&bid[(old ? 32 : 0) + r0 + i], (uint32_t)ids[old ? 32 + c - nn : c]);
+        if ((at_col >> b) & 1) atomicMin(&bid[old ? 64 + c - nn : c], (uint32_t)ids[r0 + i]);
       }
     }  // passes
     __syncwarp();
@@ -1843,28 +1844,24 @@ void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndS
   ctx->launches++;
 }
 
-// One FP32 local join over s's samples: by rows (tiles = 0, d <= kRowJoinMaxDim)
-// or with `tiles` 4 x 4 tiles per lane.
-void fp32_join(Context *ctx, int tiles, const float *X, int64_t n, int d, int S, const NndState &s,
-               int cross_only) {
-  if (tiles == 0) {
+// One FP32 local join over s's samples: by rows up to kRowJoinMaxDim dimensions
+// (unless the context forces tiles), else in tiles.
+void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
+  if (d <= kRowJoinMaxDim && !ctx->join_tiles) {
     using Join = void (*)(Context *, const float *, int64_t, int, int, const NndState &, int);
     static const Join by_pieces[7] = {join_rows<1>, join_rows<2>, join_rows<3>, join_rows<4>,
                                       join_rows<5>, join_rows<6>, join_rows<7>};
     by_pieces[(d + 3) / 4 - 1](ctx, X, n, d, S, s, cross_only);
     return;
   }
-  const int jw = kJoinWarps;
-  const size_t smem = JoinSmem::kBytes * jw;
   // the blocks that fit on the GPU at once (a grid-stride loop over the rows):
   // each warp holds one chunk of list space, so their number bounds what the
   // list loses to unused chunk tails
-  const int grid = grid_for(ctx, n, jw, tiles == 1 ? 3 : 2);
-  cudaStream_t st = ctx->stream;
-  const auto fn = tiles == 1 ? k_join<1> : k_join<2>;
-  HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  fn<<<grid, 32 * jw, smem, st>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev, s.worst, s.cl,
-                                  cross_only);
+  const int grid = grid_for(ctx, n, kJoinWarps, 2);
+  const size_t smem = kJoinWarps * JoinSmem::kBytes;
+  HDB_CUDA(cudaFuncSetAttribute(k_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k_join<<<grid, 32 * kJoinWarps, smem, ctx->stream>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev,
+                                                       s.orev, s.worst, s.cl, cross_only);
   ctx->launches++;
 }
 
@@ -1880,79 +1877,7 @@ struct EventPair {
   }
 };
 
-std::mutex g_tune_mutex;
-// (device, d, k, S, whether the rows fit in L2) -> tile slots
-std::map<std::array<int, 5>, int> g_join_tiles;
-
 }  // namespace
-
-// Tile slots per lane of the FP32 local join: the one forced on the context,
-// else none (0: by rows) up to kRowJoinMaxDim dimensions, else the one tuned for
-// this shape.  An untuned shape is timed on the first
-// m rows of Xw (the caller's rows in locality order; m = 64K..1M, enough to
-// leave L2 at d >= 64): the initial graph of those rows, one iteration
-// (sample, join, merge) so that the rows hold old and new entries as in the
-// later iterations, the second sample, then both forms -- k_join<1> (80
-// registers, three blocks per SM) and k_join<2> (122 registers, two blocks
-// per SM) -- three times each, alternating, from the same samples and an
-// empty list, the first round untimed.  The faster form is kept for the process.
-// Without Xw (the merge) an untuned shape takes two.  The trial's launches
-// count in ctx->launches.
-int fp32_join_tiles(Context *ctx, int d, int k, int S, bool resident, const float *Xw, int64_t n) {
-  if (ctx->join_tiles) return ctx->join_tiles;
-  if (d <= kRowJoinMaxDim) return 0;
-  const std::array<int, 5> key{ctx->device, d, k, S, resident ? 1 : 0};
-  {
-    std::lock_guard<std::mutex> g(g_tune_mutex);
-    auto it = g_join_tiles.find(key);
-    if (it != g_join_tiles.end()) return it->second;
-  }
-  if (!Xw) return 2;
-  cudaStream_t st = ctx->stream;
-  const int64_t want = (int64_t(256) << 20) / (4 * (int64_t)d);
-  const int64_t m = std::min<int64_t>(
-      n, std::max<int64_t>(65536, std::min<int64_t>(int64_t(1) << 20, want)));
-  NndState t(ctx, m, k, S, fp32_join_warps(ctx, m));
-  Buf<int32_t> nrev0(ctx, m), orev0(ctx, m);
-  const int wpb = 8;
-  const int grid_rows = grid_for(ctx, m, wpb, 16);
-  const size_t smem_stage = (size_t)wpb * kStageFloats * sizeof(float);
-  stage_smem_attrs(smem_stage);
-  k_init<<<grid_rows, 32 * wpb, smem_stage, st>>>(Xw, m, d, k, Segments{}, nullptr, nullptr, t.gid,
-                                                  t.gdist, t.worst);
-  ctx->launches++;
-  HDB_CHECK_LAUNCH();
-  t.sample(ctx, false, 0);
-  fp32_join(ctx, 2, Xw, m, d, S, t, 0);
-  HDB_CHECK_LAUNCH();
-  t.group(ctx);
-  t.sample(ctx, true, 0);
-  // the join clears the reverse-sample counts it reads: each trial starts
-  // from a copy
-  HDB_CUDA(cudaMemcpyAsync(nrev0, t.nrev, m * 4, cudaMemcpyDeviceToDevice, st));
-  HDB_CUDA(cudaMemcpyAsync(orev0, t.orev, m * 4, cudaMemcpyDeviceToDevice, st));
-  EventPair ev;
-  double ms[3] = {0.0, 0.0, 0.0};
-  for (int rep = 0; rep < 3; rep++) {
-    for (int tiles = 1; tiles <= 2; tiles++) {
-      HDB_CUDA(cudaMemcpyAsync(t.nrev, nrev0, m * 4, cudaMemcpyDeviceToDevice, st));
-      HDB_CUDA(cudaMemcpyAsync(t.orev, orev0, m * 4, cudaMemcpyDeviceToDevice, st));
-      t.clear_list(ctx);
-      HDB_CUDA(cudaEventRecord(ev.a, st));
-      fp32_join(ctx, tiles, Xw, m, d, S, t, 0);
-      HDB_CUDA(cudaEventRecord(ev.b, st));
-      HDB_CHECK_LAUNCH();
-      HDB_CUDA(cudaEventSynchronize(ev.b));
-      float e = 0.0f;
-      HDB_CUDA(cudaEventElapsedTime(&e, ev.a, ev.b));
-      if (rep > 0) ms[tiles] += e;
-    }
-  }
-  const int pick = ms[1] < ms[2] ? 1 : 2;
-  std::lock_guard<std::mutex> g(g_tune_mutex);
-  g_join_tiles[key] = pick;
-  return pick;
-}
 
 int64_t nndescent_bytes_per_point(int32_t d, const hdb_knn_params &p) {
   const int64_t k = p.k, S = p.sample_num;
@@ -2080,10 +2005,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
     HDB_CHECK_LAUNCH();
     if (use_tc) tc_join_prepare(ctx, Xb, n, dpad, fp16, dscale, &tj);
   }
-  // FP32 form: the join's tile slots per lane, tuned per shape
-  const int tiles =
-      bf16 ? 0 : fp32_join_tiles(ctx, d, k, S, n * d * 4 <= ctx->l2_bytes, Xw, n);
-  if (js) js->config = bf16 ? 0 : std::max(1, tiles);
+  if (js) js->config = bf16 ? 0 : std::max(1, ctx->join_tiles);
   for (int it = 0; it < p.iterations; it++) {
     s.sample(ctx, it > 0, 0);
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it], st));
@@ -2097,7 +2019,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
         k_join_bf16<false><<<grid_bf, 32 * jw16, smem_bf, st>>>(Xb, nrm, n, dpad, S, dscale, newS,
                                                                 oldS, nf, of, nrev, orev, worst, cl);
       else
-        fp32_join(ctx, tiles, Xw, n, d, S, s, 0);
+        fp32_join(ctx, Xw, n, d, S, s, 0);
       if (bf16) ctx->launches++;
     }
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it + 1], st));
@@ -2172,14 +2094,11 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
   HDB_REQUIRE(!(e & DEVERR_SELF_ID), HDB_ERR_ARG, "KNNMerge: a subgraph row lists itself");
   HDB_REQUIRE(!(e & DEVERR_DUP_ID), HDB_ERR_ARG, "KNNMerge: a subgraph row repeats an id");
 
-  // the merge takes the forced tile slots, else the ones tuned for this
-  // shape by an earlier nndescent call, else two
-  const int tiles = fp32_join_tiles(ctx, d, k, S, n * d * 4 <= ctx->l2_bytes, nullptr, 0);
   // NNDescentForMerge (nndescent.cu:1999-2087): PrepareForUpdateForMerge +
   // UpdateGraphForMerge per iteration
   for (int it = 0; it < p.iterations; it++) {
     s.sample(ctx, it > 0, n1);
-    fp32_join(ctx, tiles, X, n, d, S, s, 1);
+    fp32_join(ctx, X, n, d, S, s, 1);
     HDB_CHECK_LAUNCH();
     s.group(ctx);
   }

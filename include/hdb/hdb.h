@@ -118,9 +118,8 @@ typedef struct {
   int64_t join_candidates;      /* candidates that passed the k-th distance filter */
   int64_t gpu_launches;         /* kernel launches issued by the call */
   int32_t mst_multiplier;       /* mst_gpu = 1: the weight scale exponent m (single runs) */
-  int32_t join_config;          /* FP32 local join: 4 x 4 distance tiles per lane (1 or 2),
-                                   forced (hdb_set_join_tiles) or tuned, 1 also for the form
-                                   without tiles; 0 for a 16-bit join */
+  int32_t join_config;          /* FP32 local join: the form set by hdb_set_join_tiles (1 or
+                                   2), 1 where none is set; 0 for a 16-bit join */
   int64_t join_pairs;           /* FP32 local join: distance pairs computed, all launches
                                    (the reference's new x new and new x old pairs); 0 for a
                                    16-bit join */
@@ -137,13 +136,11 @@ HDB_API hdb_status hdb_destroy(hdb_ctx *ctx);
  * context's own stream. */
 HDB_API hdb_status hdb_set_stream(hdb_ctx *ctx, void *stream);
 /* FP32 local join form (no reference counterpart: the reference's join,
- * nndescent.cu:1487-1580, has one form).  tiles = 1 or 2 distance tiles of
- * 4 x 4 per lane forces that form (1: fewer registers, three blocks per SM;
- * 2: two blocks per SM, fewer passes over the staged rows); 0 (the default)
- * leaves the choice to the library: up to 28 dimensions a form without tiles
- * (reported as 1), beyond the faster of the two, timed once per (device, d, k,
- * SAMPLE_NUM, rows fit in L2) on the first FP32 NN-Descent of that shape and
- * kept for the process.  All forms give the same graph. */
+ * nndescent.cu:1487-1580, has one form).  0 (the default): up to 28 dimensions
+ * a form without tiles, beyond tiles of 4 rows x 1 to 8 columns per lane, as many
+ * columns as the row's samples need.  1 or 2: the tiles at any number of
+ * dimensions (two numbers from when there were two sizes of tile: the same form).
+ * Both forms give the same graph. */
 HDB_API hdb_status hdb_set_join_tiles(hdb_ctx *ctx, int32_t tiles);
 
 /* gpuknn::NNDescent, gpuknn/nndescent.cuh:40-42 (nndescent.cu:2088-2199):
