@@ -81,12 +81,6 @@ __device__ __forceinline__ void warp_sort32_with(uint64_t &v, int32_t &pl) {
 }
 
 // ---------------------------------------------------------------------------
-// Exact sequential difference sums of one row against up to 32 other rows,
-// one per lane.  The 32 rows are staged through shared memory 32 dimensions
-// at a time, read as coalesced row segments (lanes on consecutive columns),
-// and each lane then walks its own row's staged segment in dimension order:
-// the reference's sequential FP32 difference sum (nndescent.cu:1086-1093),
-// sum = fmaf(a_j - b_j, a_j - b_j, sum) for j = 0..d-1.
 // Two FP32 differences b - a with one packed instruction: b + (-a), per
 // component the same rounding as __fsub_rn(b, a) = -__fsub_rn(a, b), so its
 // square is the square of the reference's a - b, bit for bit.
@@ -94,129 +88,98 @@ __device__ __forceinline__ float2 neg_diff2(float2 b, float2 a) {
   return __fadd2_rn(b, make_float2(-a.x, -a.y));
 }
 
-constexpr int kStageCols = 32;
-constexpr int kStageLd = kStageCols + 1;                    // conflict-free column walk
-constexpr int kRingSlot = kStageCols + 32 * kStageCols;     // 16-byte form: own + 32 rows
-constexpr int kStageFloats = 2 * kRingSlot;                 // >= kStageCols + 32 * kStageLd
+// Exact sequential difference sums of one row against m <= 32 other rows, one per
+// lane (its id): sum = fmaf(a_j - b_j, a_j - b_j, sum) for j = 0..d-1, the reference's
+// FP32 difference sum (nndescent.cu:1086-1093).  The 33 rows are copied to shared
+// memory whole (up to kStageCols dimensions at a time), all copies of a chunk in
+// flight together, and each lane then walks its own row.  kV floats a copy: 4
+// where every row is 16-byte aligned (d % 4 == 0), 2 where it is 8-byte aligned,
+// else 1.  Rows take an odd number
+// of copies, so the lanes' walks read distinct bank groups.
+//
+// Bound by the gather: at 20M x 128, k = 32, k_init takes 66 ms and k_rerank 47 (99
+// and 74 with chunks of 32 dimensions in a ring of two), of 50 ms for 328 GB at the
+// measured copy rate; at 10M x 12 k_init takes 10.4 ms (21), as the shared memory
+// for a short row lets 32 warps run on an SM instead of 24.  64 dimensions, k_init
+// and k_rerank at 20M x 128 and at 200k x 128 in L2: 65.5 + 46.8 ms, 0.44 + 0.38;
+// 128: 67.3 + 48.1, 0.53 + 0.44 (half the warps); 32: 76.4 + 64.8, 0.46 + 0.40 (a row
+// comes from memory in four visits).
+constexpr int kStageCols = 64;
+constexpr int kStageWarps = 4;  // per block
 
-// 16-byte form for d % 4 == 0 (rows 16-byte aligned): a two-slot ring of
-// chunks filled by cp.async, so the next chunk of the 33 rows is in flight
-// while this one is summed.  Per chunk, lane i copies piece q = i & 7 of rows
-// i >> 3, + 4, ... (eight 16-byte copies per lane) into rows of 32 floats
-// whose pieces are permuted by the row (piece q of row r at q ^ (r & 7)), so
-// the lanes' walks of their own rows read distinct bank groups.  Same sums as
-// below, element by element.
-__device__ __forceinline__ float diffsum_staged_v4(const float *__restrict__ X, int d, int64_t row,
-                                                   int32_t id, bool active, float *__restrict__ sm) {
+inline int stage_floats(const float *X, int d) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(X) | 4 * (uintptr_t)d;
+  return (a & 15) == 0 ? 4 : (a & 7) == 0 ? 2 : 1;
+}
+__host__ __device__ constexpr int stage_pitch(int d, int kV) {
+  return ((d < kStageCols ? d : kStageCols) / kV) | 1;
+}
+inline size_t stage_bytes(int d, int kV) { return (size_t)33 * stage_pitch(d, kV) * kV * 4; }
+
+template <int kV>
+__device__ __forceinline__ float diffsum_staged(const float *__restrict__ X, int d, int64_t row,
+                                                int32_t id, int m, float *__restrict__ sm) {
   const int lane = lane_id();
-  const uint32_t act = __ballot_sync(0xffffffffu, active);
-  const int q = lane & 7, rb = lane >> 3;
-  int32_t rid[8];
-#pragma unroll
-  for (int t = 0; t < 8; t++) rid[t] = __shfl_sync(0xffffffffu, id, rb + 4 * t);
-  const int nchunks = (d + kStageCols - 1) / kStageCols;
-  // chunk c into ring slot c & 1: the own row's segment and the rows' pieces
-  auto issue = [&](int c) {
-    const int c0 = c * kStageCols;
-    const int nq = min(kStageCols, d - c0) >> 2;
-    float *own = sm + (c & 1) * kRingSlot;
-    float *nb = own + kStageCols;
-    if (lane < nq) {
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(own + 4 * lane);
-      asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst),
-                   "l"(X + row * d + c0 + 4 * lane)
-                   : "memory");
-    }
-    if (q < nq) {
-#pragma unroll
-      for (int t = 0; t < 8; t++) {
-        const int r = rb + 4 * t;
-        if ((act >> r) & 1u) {
-          const uint32_t dst =
-              (uint32_t)__cvta_generic_to_shared(nb + r * kStageCols + 4 * (q ^ (r & 7)));
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(dst),
-                       "l"(X + (int64_t)rid[t] * d + c0 + 4 * q)
-                       : "memory");
-        }
+  const int pitch = stage_pitch(d, kV);
+  auto copy = [&](float *dst, const float *src) {
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst);
+    if (kV == 4)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to), "l"(src) : "memory");
+    else if (kV == 2)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(to), "l"(src) : "memory");
+    else
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(to), "l"(src) : "memory");
+  };
+  float *own = sm + 32 * pitch * kV;
+  float s = 0.0f;
+  for (int c0 = 0; c0 < d; c0 += kStageCols) {
+    const int w = min(d - c0, kStageCols) / kV;
+    __syncwarp();  // the rows before are no longer read
+    for (int q = lane; q < w; q += 32) copy(own + q * kV, X + row * d + c0 + q * kV);
+    // the m rows' w copies each, numbered through: lane l takes l, l + 32, ...
+    const int dr = 32 / w, dq = 32 - dr * w;
+    int r = lane / w, q = lane - r * w;
+#pragma unroll 4
+    for (int i = 0; i < m * w; i += 32) {
+      const int32_t rid = __shfl_sync(0xffffffffu, id, r & 31);
+      if (r < m) copy(sm + (r * pitch + q) * kV, X + (int64_t)rid * d + c0 + q * kV);
+      r += dr;
+      q += dq;
+      if (q >= w) {
+        q -= w;
+        r++;
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-  };
-  __syncwarp();  // the ring's previous contents are no longer read
-  issue(0);
-  float s = 0.0f;
-  for (int c = 0; c < nchunks; c++) {
-    if (c + 1 < nchunks) {
-      __syncwarp();  // slot (c + 1) & 1 held chunk c - 1, summed by every lane
-      issue(c + 1);
-      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-    } else {
-      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-    __syncwarp();  // every lane's copies of chunk c have landed
-    if (active) {
-      const int nq = min(kStageCols, d - c * kStageCols) >> 2;
-      const float *own = sm + (c & 1) * kRingSlot;
-      const float *mine = own + kStageCols + lane * kStageCols;
-      for (int p = 0; p < nq; p++) {
-        const float4 b = *reinterpret_cast<const float4 *>(mine + 4 * (p ^ (lane & 7)));
-        const float4 a = *reinterpret_cast<const float4 *>(own + 4 * p);
-        const float2 d01 = neg_diff2(make_float2(b.x, b.y), make_float2(a.x, a.y));
-        const float2 d23 = neg_diff2(make_float2(b.z, b.w), make_float2(a.z, a.w));
-        s = __fmaf_rn(d01.x, d01.x, s);
-        s = __fmaf_rn(d01.y, d01.y, s);
-        s = __fmaf_rn(d23.x, d23.x, s);
-        s = __fmaf_rn(d23.y, d23.y, s);
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+    __syncwarp();  // every lane's copies have landed
+    if (lane < m) {
+      const float *mine = sm + lane * pitch * kV;
+      if (kV == 4) {
+#pragma unroll 4
+        for (int p = 0; p < w; p++) {
+          const float4 b = reinterpret_cast<const float4 *>(mine)[p];
+          const float4 a = reinterpret_cast<const float4 *>(own)[p];
+          const float2 d01 = neg_diff2(make_float2(b.x, b.y), make_float2(a.x, a.y));
+          const float2 d23 = neg_diff2(make_float2(b.z, b.w), make_float2(a.z, a.w));
+          s = __fmaf_rn(d01.x, d01.x, s);
+          s = __fmaf_rn(d01.y, d01.y, s);
+          s = __fmaf_rn(d23.x, d23.x, s);
+          s = __fmaf_rn(d23.y, d23.y, s);
+        }
+      } else {
+#pragma unroll 4
+        for (int p = 0; p < w; p++) {
+          const float df = __fsub_rn(own[p * kV], mine[p * kV]);
+          s = __fmaf_rn(df, df, s);
+          if (kV == 2) {
+            const float dg = __fsub_rn(own[p * kV + 1], mine[p * kV + 1]);
+            s = __fmaf_rn(dg, dg, s);
+          }
+        }
       }
     }
   }
   __syncwarp();
-  return s;
-}
-
-__device__ __forceinline__ float diffsum_staged(const float *__restrict__ X, int d, int64_t row,
-                                                int32_t id, bool active, float *__restrict__ sm) {
-  const int lane = lane_id();
-  if ((d & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0)
-    return diffsum_staged_v4(X, d, row, id, active, sm);
-  float *own = sm;
-  float *nb = sm + kStageCols;
-  const uint32_t act = __ballot_sync(0xffffffffu, active);
-  float s = 0.0f;
-  for (int c0 = 0; c0 < d; c0 += kStageCols) {
-    const int w = min(kStageCols, d - c0);
-    __syncwarp();
-    if (lane < w) own[lane] = X[row * d + c0 + lane];
-    if (w == kStageCols) {
-      // full chunk: row i's segment is one coalesced load (lane = column), and
-      // all 32 are issued before any is stored, so they are in flight together
-      float t[kStageCols];
-#pragma unroll
-      for (int i = 0; i < kStageCols; i++) {
-        const int32_t rid = __shfl_sync(0xffffffffu, id, i);
-        t[i] = ((act >> i) & 1u) ? __ldg(X + (int64_t)rid * d + c0 + lane) : 0.0f;
-      }
-#pragma unroll
-      for (int i = 0; i < kStageCols; i++) nb[i * kStageLd + lane] = t[i];
-    } else {
-      // ragged chunk: 32 rows x w columns, flattened: element e -> row e / w, column e % w
-#pragma unroll 8
-      for (int i = 0; i < w; i++) {
-        const int e = i * 32 + lane;
-        const int r = e / w, c = e - r * w;
-        const int32_t rid = __shfl_sync(0xffffffffu, id, r);
-        if ((act >> r) & 1u) nb[r * kStageLd + c] = __ldg(X + (int64_t)rid * d + c0 + c);
-      }
-    }
-    __syncwarp();
-    if (active) {
-      const float *mine = nb + lane * kStageLd;
-      for (int j = 0; j < w; j++) {
-        float df = __fsub_rn(own[j], mine[j]);
-        s = __fmaf_rn(df, df, s);
-      }
-    }
-  }
   return s;
 }
 
@@ -227,14 +190,15 @@ __device__ __forceinline__ float diffsum_staged(const float *__restrict__ X, int
 // the ids are drawn for the caller's row from the caller's numbering and then
 // mapped, so the lists are exactly the caller-numbered initial graph
 // renumbered (instances keep their ranges under the renumbering).
-__global__ void __launch_bounds__(256, 3) k_init(const float *__restrict__ X, int64_t n, int d, int k, Segments seg,
+template <int kV>
+__global__ void __launch_bounds__(32 * kStageWarps, 8) k_init(const float *__restrict__ X, int64_t n, int d, int k, Segments seg,
                        const uint32_t *__restrict__ order, const int32_t *__restrict__ inv,
                        int32_t *__restrict__ gid, float *__restrict__ gdist,
                        float *__restrict__ worst) {
   extern __shared__ float smem_stage[];
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
-  float *sm = smem_stage + (threadIdx.x >> 5) * kStageFloats;
+  float *sm = smem_stage + (threadIdx.x >> 5) * 33 * stage_pitch(d, kV) * kV;
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
     int64_t base = 0, cnt = n;
@@ -265,7 +229,7 @@ __global__ void __launch_bounds__(256, 3) k_init(const float *__restrict__ X, in
     }
     int64_t lab64 = (int64_t)label + base;
     if (order && lane < k) lab64 = inv[lab64];
-    const float ds = diffsum_staged(X, d, row, (int32_t)lab64, lane < k, sm);
+    const float ds = diffsum_staged<kV>(X, d, row, (int32_t)lab64, k, sm);
     uint64_t key = ~0ull;
     if (lane < k) key = pack(ds, (int32_t)lab64);
     key = warp_sort32(key);
@@ -292,7 +256,8 @@ __global__ void __launch_bounds__(256, 3) k_init(const float *__restrict__ X, in
 // the other set are the new ones.  Own-subgraph ids outside their set, self
 // ids and repeats set DEVERR_ID_RANGE / SELF / DUP and are replaced by a
 // valid id of the set so that no gather leaves X.
-__global__ void __launch_bounds__(256, 3) k_merge_init(const float *__restrict__ X, int64_t n, int d, int k, int64_t n1,
+template <int kV>
+__global__ void __launch_bounds__(32 * kStageWarps, 8) k_merge_init(const float *__restrict__ X, int64_t n, int d, int k, int64_t n1,
                              const hdb_nnd_element *__restrict__ G1,
                              const hdb_nnd_element *__restrict__ G2, int32_t *__restrict__ gid,
                              float *__restrict__ gdist, float *__restrict__ worst,
@@ -300,7 +265,7 @@ __global__ void __launch_bounds__(256, 3) k_merge_init(const float *__restrict__
   extern __shared__ float smem_stage[];
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
-  float *sm = smem_stage + (threadIdx.x >> 5) * kStageFloats;
+  float *sm = smem_stage + (threadIdx.x >> 5) * 33 * stage_pitch(d, kV) * kV;
   const int h = k - k / 2, r = k / 2;
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
@@ -341,7 +306,7 @@ __global__ void __launch_bounds__(256, 3) k_merge_init(const float *__restrict__
       if (lane < h) label = (local + 1 + lane) % own_n;
     }
     label += lane < h ? own_off : oth_off;
-    const float ds = diffsum_staged(X, d, row, (int32_t)label, lane < k, sm);
+    const float ds = diffsum_staged<kV>(X, d, row, (int32_t)label, k, sm);
     uint64_t key = ~0ull;
     if (lane < k) key = pack(ds, (int32_t)label);
     key = warp_sort32(key);
@@ -1509,18 +1474,19 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
 // FP32 re-rank of every kept neighbour (one warp per row): the reference's
 // difference sum for each (row, neighbour) pair, rows re-sorted by (distance,
 // id); old/new flags travel with their ids.
-__global__ void __launch_bounds__(256, 3) k_rerank(const float *__restrict__ X, int64_t n, int d, int k,
+template <int kV>
+__global__ void __launch_bounds__(32 * kStageWarps, 8) k_rerank(const float *__restrict__ X, int64_t n, int d, int k,
                          hdb_nnd_element *__restrict__ G) {
   extern __shared__ float smem_stage[];
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
-  float *sm = smem_stage + (threadIdx.x >> 5) * kStageFloats;
+  float *sm = smem_stage + (threadIdx.x >> 5) * 33 * stage_pitch(d, kV) * kV;
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
     int32_t lab = 0;
     if (lane < k) lab = G[row * k + lane].label_;
     const int32_t id = decode(lab);
-    const float ds = diffsum_staged(X, d, row, id, lane < k, sm);
+    const float ds = diffsum_staged<kV>(X, d, row, id, k, sm);
     uint64_t key = lane < k ? pack(ds, id) : ~0ull;
     int32_t slab = lab;  // the entry (with its old/new flag) moves with its key
     warp_sort32_with(key, slab);
@@ -1717,12 +1683,18 @@ int bits_for_rows(int64_t n) {
 
 namespace {
 
-// Dynamic shared memory of the kernels that stage rows for difference sums
-// (two ring slots of 33 rows x 32 dimensions per warp: 66 KB for 8 warps).
-void stage_smem_attrs(size_t bytes) {
-  HDB_CUDA(cudaFuncSetAttribute(k_init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  HDB_CUDA(cudaFuncSetAttribute(k_merge_init, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-  HDB_CUDA(cudaFuncSetAttribute(k_rerank, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+// Launches one of the kernels that stage rows for difference sums over the rows
+// of X: shared memory for the rows' width, four turns of resident blocks.
+template <class Kernel, class... Args>
+void launch_staged(Context *ctx, Kernel by4, Kernel by2, Kernel by1, const float *X, int64_t n, int d,
+                   Args... args) {
+  const int kV = stage_floats(X, d);
+  const Kernel fn = kV == 4 ? by4 : kV == 2 ? by2 : by1;
+  const size_t smem = kStageWarps * stage_bytes(d, kV);
+  const int resident = (int)std::min<size_t>(8, (size_t(220) << 10) / (smem + 1024));
+  HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  fn<<<grid_for(ctx, n, kStageWarps, 4 * resident), 32 * kStageWarps, smem, ctx->stream>>>(X, n, d, args...);
+  ctx->launches++;
 }
 
 // Rows per bucket of the candidate list's grouping, 2^shift: the fewest (from
@@ -1938,8 +1910,6 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
 
   const int wpb = 8;
   const int grid_rows = grid_for(ctx, n, wpb, 16);
-  const size_t smem_stage = (size_t)wpb * kStageFloats * sizeof(float);
-  stage_smem_attrs(smem_stage);
   // renumber the points in locality order (k_loc_project); X stays the
   // caller's, the iterations work on Xw and the renumbered lists, and the
   // initial graph is drawn straight into the new numbering
@@ -1961,8 +1931,8 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
     k_loc_inverse<<<grid_for(ctx, n, 256), 256, 0, st>>>(order, n, inv); ctx->launches++;
     k_loc_rows<<<grid_rows, 32 * wpb, 0, st>>>(X, order, n, d, Xp); ctx->launches++;
     HDB_CHECK_LAUNCH();
-    k_init<<<grid_rows, 32 * wpb, smem_stage, st>>>(Xp, n, d, k, seg, order, inv, gid, gdist, worst);
-    ctx->launches++;
+    launch_staged(ctx, k_init<4>, k_init<2>, k_init<1>, Xp, n, d, k, seg, order.get(), inv.get(), gid, gdist,
+                  worst);
     HDB_CHECK_LAUNCH();
   }
   const float *Xw = Xp;
@@ -2029,7 +1999,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
   if (p.iterations == 0) s.group(ctx);  // an empty list
   s.finalize(ctx, Gp);
   if (bf16) {
-    k_rerank<<<grid_rows, 32 * wpb, smem_stage, st>>>(Xw, n, d, k, Gp); ctx->launches++;
+    launch_staged(ctx, k_rerank<4>, k_rerank<2>, k_rerank<1>, Xw, n, d, k, Gp.get());
     HDB_CHECK_LAUNCH();
   }
   k_loc_restore<<<grid_rows, 32 * wpb, 0, st>>>(Gp, order, n, k, G); ctx->launches++;
@@ -2080,13 +2050,8 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
                            cudaMemcpyDeviceToDevice, st));
   NndState s(ctx, n, k, S, fp32_join_warps(ctx, n));
 
-  const int wpb = 8;
-  const int grid_rows = grid_for(ctx, n, wpb, 16);
-  const size_t smem_stage = (size_t)wpb * kStageFloats * sizeof(float);
-  stage_smem_attrs(smem_stage);
-  k_merge_init<<<grid_rows, 32 * wpb, smem_stage, st>>>(X, n, d, k, n1, G1, G2, s.gid,
-                                                        s.gdist, s.worst, ctx->dev_err);
-  ctx->launches++;
+  launch_staged(ctx, k_merge_init<4>, k_merge_init<2>, k_merge_init<1>, X, n, d, k, n1, G1, G2, s.gid.get(), s.gdist.get(),
+                s.worst.get(), ctx->dev_err);
   HDB_CHECK_LAUNCH();
   ctx->sync();
   const uint32_t e = ctx->take_dev_err();
