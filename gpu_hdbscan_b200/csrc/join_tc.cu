@@ -301,46 +301,24 @@ __device__ __forceinline__ void tmem_wait_ld(uint32_t (&v)[32]) {
 __global__ void k_join_lists(int64_t n, int S, int32_t *__restrict__ newS, int32_t *__restrict__ oldS,
                              int8_t *__restrict__ nf, int8_t *__restrict__ of,
                              int32_t *__restrict__ nrev, int32_t *__restrict__ orev) {
-  __shared__ int32_t news_smem[8][32], olds_smem[8][32];  // launched with 8 warps
+  __shared__ __align__(16) int32_t ids_smem[8][64];  // launched with 8 warps
   const int lane = lane_id();
   const int wpb = blockDim.x >> 5;
-  int32_t *news = news_smem[threadIdx.x >> 5];
-  int32_t *olds = olds_smem[threadIdx.x >> 5];
-  for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
-       row += (int64_t)gridDim.x * wpb) {
-    // the row's counts and both lists are loaded together (the lists do not
-    // wait for the counts: one memory round trip per row)
+  int32_t *ids = ids_smem[threadIdx.x >> 5];
+  const int64_t stride = (int64_t)gridDim.x * wpb;
+  int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5);
+  SampleLists next;  // loaded one row ahead
+  next.load(row, n, S, newS, oldS, nf, of, nrev, orev);
+  for (; row < n; row += stride) {
+    const SampleLists lists = next;
+    next.load(row + stride, n, S, newS, oldS, nf, of, nrev, orev);
     const int64_t sb = row * (2 * S);
-    const int32_t nraw = lane < 2 * S ? newS[sb + lane] : 0;
-    const int32_t oraw = lane < 2 * S ? oldS[sb + lane] : 0;
-    const int cnf = nf[row], cof = of[row];
-    const int cnr = min(nrev[row], S), cor = min(orev[row], S);
-    bool vn = (lane < S) ? (lane < cnf) : (lane < 2 * S && lane - S < cnr);
-    bool vo = (lane < S) ? (lane < cof) : (lane < 2 * S && lane - S < cor);
-    const int32_t nid = vn ? nraw : -1 - lane;
-    const int32_t oid = vo ? oraw : -100 - lane;
-    const uint32_t pn = __match_any_sync(0xffffffffu, nid);
-    vn = vn && (__ffs(pn) - 1 == lane);
-    const uint32_t po = __match_any_sync(0xffffffffu, oid);
-    vo = vo && (__ffs(po) - 1 == lane);
-    const uint32_t bo = __ballot_sync(0xffffffffu, vo);
-    int no = __popc(bo);
-    if (vo) olds[__popc(bo & lanemask_lt())] = oid;
-    __syncwarp();
-    {
-      bool in_old = false;  // independent reads, not a chain
-#pragma unroll 8
-      for (int t = 0; t < no; t++) in_old |= olds[t] == nid;
-      vn = vn && !in_old;
-    }
-    const uint32_t bn = __ballot_sync(0xffffffffu, vn);
-    int nn = __popc(bn);
-    if (vn) news[__popc(bn & lanemask_lt())] = nid;
+    int nn, no;
+    lists.compact(S, ids, nn, no);
     if (nn == 0 || nn + no < 2) nn = no = 0;  // nothing to compare
-    __syncwarp();
     // compact lists; the last group of four padded with its first id
-    int32_t outn = lane < nn ? news[lane] : 0;
-    int32_t outo = lane < no ? olds[lane] : 0;
+    int32_t outn = lane < nn ? ids[lane] : 0;
+    int32_t outo = lane < no ? ids[32 + lane] : 0;
     const int32_t firstn = __shfl_sync(0xffffffffu, outn, lane & ~3);
     const int32_t firsto = __shfl_sync(0xffffffffu, outo, lane & ~3);
     if (lane >= nn) outn = firstn;

@@ -1314,32 +1314,12 @@ __global__ void __launch_bounds__(128) k_join_bf16(const uint16_t *__restrict__ 
   ListCursor cur;
   for (int64_t row = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); row < n;
        row += (int64_t)gridDim.x * wpb) {
-    const int cnf = nf[row], cof = of[row];
-    const int cnr = min(nrev[row], S), cor = min(orev[row], S);
+    SampleLists lists;
+    lists.load(row, n, S, newS, oldS, nf, of, nrev, orev);
     __syncwarp();
     if (lane == 0) { nrev[row] = 0; orev[row] = 0; }
-    const int64_t sb = row * (2 * S);
-    bool vn = (lane < S) ? (lane < cnf) : (lane < 2 * S && lane - S < cnr);
-    bool vo = (lane < S) ? (lane < cof) : (lane < 2 * S && lane - S < cor);
-    int32_t nid = vn ? newS[sb + lane] : -1 - lane;
-    int32_t oid = vo ? oldS[sb + lane] : -100 - lane;
-    uint32_t pn = __match_any_sync(0xffffffffu, nid);
-    vn = vn && (__ffs(pn) - 1 == lane);
-    uint32_t po = __match_any_sync(0xffffffffu, oid);
-    vo = vo && (__ffs(po) - 1 == lane);
-    uint32_t bo = __ballot_sync(0xffffffffu, vo);
-    const int no = __popc(bo);
-    if (vo) ids[32 + __popc(bo & lanemask_lt())] = oid;
-    __syncwarp();
-    {
-      bool in_old = false;  // independent reads, not a chain
-#pragma unroll 8
-      for (int t = 0; t < no; t++) in_old |= ids[32 + t] == nid;
-      vn = vn && !in_old;
-    }
-    uint32_t bn = __ballot_sync(0xffffffffu, vn);
-    const int nn = __popc(bn);
-    if (vn) ids[__popc(bn & lanemask_lt())] = nid;
+    int nn, no;
+    lists.compact(S, ids, nn, no);
     best1[lane] = ~0ull;
     best2[lane] = ~0ull;
     best3[lane] = ~0ull;
