@@ -175,7 +175,7 @@ void radix_sort_u32(Context *ctx, uint32_t *keys, uint32_t *values, int64_t n, i
 void radix_sort_u64(Context *ctx, uint64_t *keys, uint32_t *values, int64_t n, int begin_bit,
                     int end_bit);
 // Groups the (key, value) pairs of a list by bits [begin_bit, end_bit) of their
-// keys, in digits of up to 9 bits, stably.  The list's length is on the device
+// keys, in digits of up to 9 bits, a group in any order.  The list's length is on the device
 // (count); cap (< 2^32) bounds it.  The second buffers hold cap entries too;
 // returns whether the result is in them.  base (513 values) receives the last
 // pass's digit starts and total: with a single pass, the groups' starts.

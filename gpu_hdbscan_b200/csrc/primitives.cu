@@ -152,12 +152,13 @@ __device__ __forceinline__ int64_t key_count(int64_t n, const unsigned long long
 // Dynamic shared memory of one scatter block: the tile's keys and values in
 // digit order, the per-warp digit counts, each digit's first tile position
 // and first output position, and the warp totals of the digit scan.
-template <typename K, typename V, bool kVals, int kBins, int kItems>
+template <typename K, typename V, bool kVals, int kBins, int kItems, bool kStable>
 struct SortSmem {
+  static constexpr int kHists = kStable ? kSortWarps : 1;  // ranks per warp, or over the block
   static constexpr int kTile = kSortThreads * kItems;
   static constexpr size_t kValsAt = sizeof(K) * kTile;
   static constexpr size_t kHistAt = kValsAt + (kVals ? sizeof(V) * kTile : 0);
-  static constexpr size_t kStartAt = kHistAt + sizeof(uint32_t) * kSortWarps * kBins;
+  static constexpr size_t kStartAt = kHistAt + sizeof(uint32_t) * kHists * kBins;
   static constexpr size_t kGofsAt = kStartAt + sizeof(uint32_t) * kBins;
   static constexpr size_t kWsumAt = kGofsAt + sizeof(uint32_t) * kBins;
   static constexpr size_t kBytes = kWsumAt + sizeof(uint32_t) * kSortWarps;
@@ -197,17 +198,23 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist(const K *__restrict__
     counts[count_at<kTileMajor>(i, blockIdx.x, nblocks, kBins)] = hist[i];
 }
 
-// Scatter of one tile for one digit.  Keys are ranked per warp (match_any),
-// the tile is laid out in digit order in shared memory (stable: input order
-// within a digit), and each digit's run is then written by consecutive
-// threads to consecutive addresses.  Values of type V (u32 or u64) move with
-// their keys when kVals.
-template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor>
-__global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
+// Scatter of one tile for one digit.  Keys are ranked, the tile is laid out in
+// digit order in shared memory, and each digit's run is then written by
+// consecutive threads to consecutive addresses.  Values of type V (u32 or u64)
+// move with their keys when kVals.  kStable keeps the input order within a digit:
+// the lanes of a digit find one another with match_any, which takes a turn per
+// distinct digit of the warp and bounds the kernel (63 % of that unit's rate over
+// the whole of it).  Without it the ranks are the arrivals at the digit's count,
+// and one count per digit does for the block, which leaves room for four blocks on
+// an SM: six lists of 100k x 12 in one pass of 9 bits 348 -> 245 us, the first pass
+// of six lists of 1M x 12 2.70 -> 2.36 ms.  (Masks in shared memory instead of
+// match_any are no faster: 2.7 -> 2.9 ms at 6 bits.)
+template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor, bool kStable>
+__global__ void __launch_bounds__(kSortThreads, kStable ? 3 : 4) radix_scatter(
     const K *__restrict__ keys_in, const V *__restrict__ vals_in, K *__restrict__ keys_out,
     V *__restrict__ vals_out, const uint32_t *__restrict__ offsets, int64_t n, int shift,
     uint32_t mask, uint32_t nblocks, const unsigned long long *dev_n) {
-  using L = SortSmem<K, V, kVals, kBins, kItems>;
+  using L = SortSmem<K, V, kVals, kBins, kItems, kStable>;
   constexpr int kTile = L::kTile;
   n = key_count(n, dev_n);
   if ((int64_t)blockIdx.x * kTile >= n) return;
@@ -220,7 +227,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
   uint32_t *gofs = reinterpret_cast<uint32_t *>(sort_smem + L::kGofsAt);
   uint32_t *wsum = reinterpret_cast<uint32_t *>(sort_smem + L::kWsumAt);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < kSortWarps * kBins; i += kSortThreads) (&whist[0][0])[i] = 0;
+  for (int i = threadIdx.x; i < L::kHists * kBins; i += kSortThreads) (&whist[0][0])[i] = 0;
   __syncthreads();
   const int64_t tile0 = (int64_t)blockIdx.x * kTile;
   const int64_t base = tile0 + (int64_t)warp * (32 * kItems);
@@ -236,17 +243,21 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
 #pragma unroll
   for (int j = 0; j < kItems; j++) {
     const bool ok = base + j * 32 + lane < n;
-    // past the end: a digit of its own per lane, outside [0, kBins)
-    const uint32_t d = ok ? ((uint32_t)(k[j] >> shift) & mask) : ((uint32_t)kBins + lane);
-    const uint32_t peers = __match_any_sync(0xffffffffu, d);
-    const uint32_t rank = __popc(peers & lanemask_lt());
-    const int leader = __ffs(peers) - 1;
-    uint32_t b = 0;
-    if (ok) b = whist[warp][d];
-    __syncwarp();
-    if (ok && lane == leader) whist[warp][d] = b + __popc(peers);
-    __syncwarp();
-    dl[j] = d | ((b + rank) << 16);
+    const uint32_t d = ok ? ((uint32_t)(k[j] >> shift) & mask) : (uint32_t)kBins;  // past the end: no digit
+    uint32_t rank = 0;
+    if (!kStable) {
+      if (ok) rank = atomicAdd(&whist[0][d], 1u);
+    } else {
+      // past the end: a digit of its own per lane, outside [0, kBins)
+      const uint32_t peers = __match_any_sync(0xffffffffu, ok ? d : d + lane);
+      const int leader = __ffs(peers) - 1;
+      if (ok) rank = whist[warp][d];
+      __syncwarp();
+      if (ok && lane == leader) whist[warp][d] = rank + __popc(peers);
+      __syncwarp();
+      rank += __popc(peers & lanemask_lt());
+    }
+    dl[j] = d | (rank << 16);
   }
   __syncthreads();
   {
@@ -259,7 +270,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
       const int d = threadIdx.x * kPer + r;
       uint32_t acc = 0;
 #pragma unroll
-      for (int w = 0; w < kSortWarps; w++) {
+      for (int w = 0; w < L::kHists; w++) {
         const uint32_t c = whist[w][d];
         whist[w][d] = acc;
         acc += c;
@@ -290,7 +301,7 @@ __global__ void __launch_bounds__(kSortThreads, 3) radix_scatter(
   for (int j = 0; j < kItems; j++) {
     const uint32_t d = dl[j] & 0xffffu;
     if (d < (uint32_t)kBins) {
-      const uint32_t pos = dstart[d] + whist[warp][d] + (dl[j] >> 16);
+      const uint32_t pos = dstart[d] + (kStable ? whist[warp][d] : 0u) + (dl[j] >> 16);
       tk[pos] = k[j];
       if (kVals) tv[pos] = v[j];
     }
@@ -446,25 +457,29 @@ __global__ void __launch_bounds__(kBins) radix_col_apply(const uint32_t *__restr
   }
 }
 
-template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor>
+template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor, bool kStable = true>
 void launch_scatter(cudaStream_t st, const K *kin, const V *vin, K *kout, V *vout,
                     const uint32_t *offs, int64_t n, int shift, uint32_t mask, uint32_t nb,
                     const unsigned long long *dev_n = nullptr) {
-  using L = SortSmem<K, V, kVals, kBins, kItems>;
-  auto *fn = radix_scatter<K, V, kVals, kBins, kItems, kTileMajor>;
+  using L = SortSmem<K, V, kVals, kBins, kItems, kStable>;
+  auto *fn = radix_scatter<K, V, kVals, kBins, kItems, kTileMajor, kStable>;
   if (L::kBytes > 48 * 1024)
     HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::kBytes));
   fn<<<nb, kSortThreads, L::kBytes, st>>>(kin, vin, kout, vout, offs, n, shift, mask, nb, dev_n);
   HDB_CHECK_LAUNCH();
 }
 
-// Stable LSD sort of the pairs in (keys, vals) with (ktmp, vtmp) as the second
+// LSD sort of the pairs in (keys, vals) with (ktmp, vtmp) as the second
 // buffer; returns whether the result is in the second one.  Digit widths: the
 // fewest passes of at most log2(kBins) bits over [begin_bit, end_bit), the bits
-// spread evenly over them (25 bits with 512 bins: 9 + 8 + 8).  dev_n: the count
+// spread evenly over them (25 bits with 512 bins: 9 + 8 + 8).  Stable with kStable.
+// Without it the first pass leaves a digit's keys in any order and takes as many
+// bits as it can, the later ones, whose match_any is the cheaper the fewer digits
+// there are, the rest (1M x 12, 12 bits: 9 + 3 2.2 ms for the second passes, 6 + 6
+// 2.7).  dev_n: the count
 // on the device, n then being a bound.  base_out (optional): the last pass's
 // base, kBins + 1 values.
-template <typename K, typename V, int kBins>
+template <typename K, typename V, int kBins, bool kStable = true>
 bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64_t n, int begin_bit,
                          int end_bit, const unsigned long long *dev_n, uint32_t *base_out) {
   HDB_REQUIRE(n < (int64_t(1) << 32), HDB_ERR_ARG, "radix sort: more than 2^32 elements");
@@ -491,7 +506,7 @@ bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64
   int left = end_bit - begin_bit;
   int npass = (left + kMaxBits - 1) / kMaxBits;
   for (int shift = begin_bit; left > 0; passes++, npass--) {
-    const int bits = (left + npass - 1) / npass;
+    const int bits = kStable ? (left + npass - 1) / npass : std::min(left, kMaxBits);
     const uint32_t mask = (1u << bits) - 1u;
     radix_hist<K, kBins, kSortItems, true><<<nb, kSortThreads, 0, st>>>(kin, counts, n, shift, mask,
                                                                        nb, dev_n);
@@ -507,7 +522,10 @@ bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64
       ctx->launches += 3;
     }
     HDB_CHECK_LAUNCH();
-    if (vals)
+    if (!kStable && passes == 0)
+      launch_scatter<K, V, true, kBins, kSortItems, true, kStable>(st, kin, vin, kout, vout, offs, n,
+                                                                   shift, mask, nb, dev_n);
+    else if (vals)
       launch_scatter<K, V, true, kBins, kSortItems, true>(st, kin, vin, kout, vout, offs, n, shift,
                                                           mask, nb, dev_n);
     else
@@ -702,8 +720,8 @@ void radix_sort_u64(Context *ctx, uint64_t *keys, uint32_t *values, int64_t n, i
 bool radix_group_u32_u64(Context *ctx, uint32_t *keys, uint64_t *values, uint32_t *keys2,
                          uint64_t *values2, int64_t cap, const unsigned long long *count,
                          int begin_bit, int end_bit, uint32_t *base) {
-  return radix_sort_pingpong<uint32_t, uint64_t, 512>(ctx, keys, values, keys2, values2, cap,
-                                                      begin_bit, end_bit, count, base);
+  return radix_sort_pingpong<uint32_t, uint64_t, 512, false>(ctx, keys, values, keys2, values2, cap,
+                                                             begin_bit, end_bit, count, base);
 }
 
 // Stable LSD radix sort of u32 keys with u32 values in caller-provided
