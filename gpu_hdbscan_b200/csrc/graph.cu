@@ -34,32 +34,13 @@ __device__ __forceinline__ float euclid_ref(const float *__restrict__ a,
   return __fsqrt_rn(soma);
 }
 
-// One warp per row: validate the row (range, self, duplicates) and count
-// in-degrees (countValues, count.cu:10-19).
-// With instances, ids must stay inside the row's instance.
-__global__ void k_degrees(const int32_t *__restrict__ ids, int64_t n, int k, Segments seg,
-                          int32_t *__restrict__ deg, uint32_t *err) {
-  const int lane = lane_id();
-  int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
-  for (; row < n; row += stride) {
-    int32_t v = lane < k ? ids[row * k + lane] : -1 - lane;
-    int64_t lo = 0, hi = n;
-    if (seg.count > 0) {
-      const int32_t t = seg.of_point(row);
-      lo = seg.off[t];
-      hi = seg.off[t + 1];
-    }
-    uint32_t bad = 0;
-    if (lane < k) {
-      if (v < lo || v >= hi) bad |= DEVERR_ID_RANGE;
-      else if (v == row) bad |= DEVERR_SELF_ID;
-    }
-    uint32_t peers = __match_any_sync(0xffffffffu, v);
-    if (lane < k && __popc(peers) > 1) bad |= DEVERR_DUP_ID;
-    if (bad) atomicOr(err, bad);
-    else if (lane < k) atomicAdd(&deg[v], 1);
-  }
+// In-degrees (countValues, count.cu:10-19): the rows that v lists and that list v
+// (mutual), and the rows that list v and that v does not.
+__global__ void k_degrees(const uint32_t *__restrict__ mutual, const int32_t *__restrict__ revcnt,
+                          int64_t n, int32_t *__restrict__ deg) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    deg[i] = __popc(mutual[i]) + revcnt[i];
 }
 
 // Histogram of degrees (clamped to the last bin): the first kDegNear bins,
@@ -264,40 +245,124 @@ __global__ void k_seg_tie_select(const uint32_t *__restrict__ tinst, const uint3
   }
 }
 
-// One warp per row i: which of i's neighbours list i back (findKNNlist,
-// getters.cu:41-49).  Non-mutual edges i->v become reverse entries of v.
-__global__ void k_mutual(const int32_t *__restrict__ ids, int64_t n, int k,
-                         uint32_t *__restrict__ mutual, int32_t *__restrict__ revcnt,
-                         int32_t *__restrict__ nonmutual) {
-  // One warp per row: neighbour t's list is read as one coalesced segment
-  // (lane = position), eight lists in flight at a time, and a vote tells
-  // whether the row is in it.
-  const int lane = lane_id();
-  int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+// One warp per row i: checks the row (range, self, repeats; with instances, ids must
+// stay inside the row's), and which of i's neighbours list i back (findKNNlist,
+// getters.cu:41-49), as bits of mutual[i] (zero before).  Row i reads the lists of
+// its neighbours from i on only, and where i stands in v's list sets both rows'
+// bits: of a pair of rows that list each other, one reads the other.  kV ids a
+// load, so 32 / kV lanes read a list and a warp kV of them; 8 lists ahead.
+// Bound by the random reads: 2M x 32 2.05 ms with every neighbour's list read by 32
+// lanes, eight at a time, 1.61 with half of them, 0.63 with 16-byte loads too (0.69
+// with 16 lists ahead), 0.90 with the checks, which took a kernel of 0.58 with the
+// in-degrees.
+template <int kV>
+__global__ void k_mutual(const int32_t *__restrict__ ids, int64_t n, int k, Segments seg,
+                         uint32_t *__restrict__ mutual, uint32_t *err) {
+  __shared__ uint64_t list[kWarpsPerBlock][32];  // neighbours from i on | their place in i's list
+  constexpr int kLanes = 32 / kV, kAhead = 8 / kV;
+  const int lane = lane_id(), w = threadIdx.x >> 5, g = lane / kLanes, at = kV * (lane % kLanes);
   const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
+  int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + w;
+  int32_t next = row < n && lane < k ? ids[row * k + lane] : -1 - lane;
   for (; row < n; row += stride) {
-    const int32_t v = lane < k ? ids[row * k + lane] : 0;
-    uint32_t m = 0;
-    for (int t0 = 0; t0 < k; t0 += 8) {
-      int32_t x[8];
+    const int32_t v = next;
+    if (row + stride < n && lane < k) next = ids[(row + stride) * k + lane];
+    {
+      // repeats: against the next 16 ids, round the row's end
+      int32_t *ring = reinterpret_cast<int32_t *>(list[w]);
+      ring[lane] = ring[lane + 32] = v;
+      int64_t lo = 0, hi = n;
+      if (seg.count > 0) {
+        const int32_t t = seg.of_point(row);
+        lo = seg.off[t];
+        hi = seg.off[t + 1];
+      }
+      uint32_t bad = 0;
+      if (lane < k) bad = v < lo || v >= hi ? DEVERR_ID_RANGE : v == (int32_t)row ? DEVERR_SELF_ID : 0u;
+      __syncwarp();
 #pragma unroll
-      for (int u = 0; u < 8; u++) {
-        const int t = t0 + u;
-        const int32_t vt = __shfl_sync(0xffffffffu, v, t & 31);
-        x[u] = (t < k && lane < k) ? __ldg(ids + (int64_t)vt * k + lane) : -1;
+      for (int o = 1; o <= 16; o++) bad |= ring[lane + o] == v ? (uint32_t)DEVERR_DUP_ID : 0u;
+      if (bad) atomicOr(err, bad);
+      __syncwarp();  // the ring becomes the list
+    }
+    const bool from = lane < k && v >= (int32_t)row && v < n;
+    const uint32_t todo = __ballot_sync(0xffffffffu, from);
+    if (from) list[w][__popc(todo & lanemask_lt())] = (uint64_t)(uint32_t)v << 32 | lane;
+    __syncwarp();
+    const int c = __popc(todo);
+    uint32_t m = 0;
+    for (int i0 = g; i0 - g < c; i0 += kV * kAhead) {
+      int32_t x[kAhead][kV];
+      uint64_t e[kAhead];
+#pragma unroll
+      for (int u = 0; u < kAhead; u++) {
+        const int i = i0 + u * kV;
+        const bool ok = i < c && at < k;
+        e[u] = list[w][min(i, 31)];
+        const int32_t *src = ids + (int64_t)(e[u] >> 32) * k + at;
+#pragma unroll
+        for (int q = 0; q < kV; q++) x[u][q] = -1;
+        if (ok) {
+          if (kV == 4)
+            *reinterpret_cast<int4 *>(x[u]) = __ldg(reinterpret_cast<const int4 *>(src));
+          else if (kV == 2)
+            *reinterpret_cast<int2 *>(x[u]) = __ldg(reinterpret_cast<const int2 *>(src));
+          else
+            x[u][0] = __ldg(src);
+        }
       }
 #pragma unroll
-      for (int u = 0; u < 8; u++)
-        if (__any_sync(0xffffffffu, x[u] == (int32_t)row)) m |= 1u << (t0 + u);
+      for (int u = 0; u < kAhead; u++) {
+        uint32_t hit = 0;
+#pragma unroll
+        for (int q = 0; q < kV; q++) hit |= x[u][q] == (int32_t)row ? 1u << q : 0u;
+        if (hit) {
+          atomicOr(&mutual[e[u] >> 32], hit << at);
+          m |= 1u << (uint32_t)e[u];
+        }
+      }
     }
-    if (k < 32) m &= (1u << k) - 1u;
-    if (lane < k && !((m >> lane) & 1u)) atomicAdd(&revcnt[v], 1);
-    if (lane == 0) {
-      mutual[row] = m;
-      nonmutual[row] = k - __popc(m);
-    }
+    m = __reduce_or_sync(0xffffffffu, m);
+    if (lane == 0 && m) atomicOr(&mutual[row], m);
+    __syncwarp();  // the list is no longer read
   }
 }
+
+// The non-mutual edges i -> v, which become reverse entries of v: their number per
+// i and per v.  One warp per row.
+__global__ void k_nonmutual(const int32_t *__restrict__ ids, int64_t n, int k,
+                            const uint32_t *__restrict__ mutual, int32_t *__restrict__ revcnt,
+                            int32_t *__restrict__ nonmutual) {
+  const int lane = lane_id();
+  const int64_t stride = (int64_t)gridDim.x * kWarpsPerBlock;
+  for (int64_t row = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); row < n; row += stride) {
+    const uint32_t m = mutual[row];
+    const int32_t v = lane < k && !((m >> lane) & 1u) ? ids[row * k + lane] : -1;
+    if (v >= 0 && v < n) atomicAdd(&revcnt[v], 1);  // a caller's ids, whose check is still queued
+    if (lane == 0) nonmutual[row] = k - __popc(m);
+  }
+}
+
+// The checked rows' mutual flags and the counts of their non-mutual edges, per
+// source and (revcnt) per target.  both: mutual, then revcnt.
+struct Mutual {
+  Buf<uint32_t> both;
+  Buf<int32_t> nonmutual;
+  uint32_t *mutual;
+  int32_t *revcnt;
+  Mutual(Context *ctx, const int32_t *ids, int64_t n, int k, const Segments &seg)
+      : both(ctx, 2 * n), nonmutual(ctx, n), mutual(both), revcnt((int32_t *)(both.get() + n)) {
+    const int grid = grid_for(ctx, n, kWarpsPerBlock);
+    HDB_CUDA(cudaMemsetAsync(both, 0, 2 * n * sizeof(uint32_t), ctx->stream));
+    // ids per load: what the rows' alignment allows
+    const uintptr_t a = reinterpret_cast<uintptr_t>(ids) | 4 * (uintptr_t)k;
+    const auto fn = (a & 15) == 0 ? k_mutual<4> : (a & 7) == 0 ? k_mutual<2> : k_mutual<1>;
+    fn<<<grid, 32 * kWarpsPerBlock, 0, ctx->stream>>>(ids, n, k, seg, mutual, ctx->dev_err);
+    k_nonmutual<<<grid, 32 * kWarpsPerBlock, 0, ctx->stream>>>(ids, n, k, mutual, revcnt, nonmutual);
+    ctx->launches += 2;
+    HDB_CHECK_LAUNCH();
+  }
+};
 
 // Row length: k own ids, the reverse entries, and for an antihub the other
 // antihubs of its instance.
@@ -363,7 +428,7 @@ __global__ void __launch_bounds__(32 * kCoreWarps)
     const int64_t row = r0 + lane;
     const bool active = row < n;
     const uint32_t act = __ballot_sync(0xffffffffu, active);
-    // the ids of a caller's graph are checked later (k_degrees): one outside
+    // the ids of a caller's graph are checked later (k_mutual): one outside
     // [0, n) stands for the row itself here, so that no gather leaves X
     int32_t v = active ? ids[row * k + col] : 0;
     if (active && (v < 0 || v >= n)) v = (int32_t)row;
@@ -669,10 +734,12 @@ void build_enhanced_knng(Context *ctx, const int32_t *ids, const float *core, co
   const int gw = grid_for(ctx, n, kWarpsPerBlock);
   const int ge = grid_for(ctx, n, 256);
 
-  // 1. in-degrees + validation
+  // 1. validation, mutual flags, reverse counts and in-degrees
+  Mutual mu(ctx, ids, n, k, seg);
+  const uint32_t *mutual = mu.mutual;
+  const int32_t *revcnt = mu.revcnt, *nonmutual = mu.nonmutual;
   Buf<int32_t> deg(ctx, n);
-  HDB_CUDA(cudaMemsetAsync(deg, 0, n * sizeof(int32_t), st));
-  k_degrees<<<gw, 32 * kWarpsPerBlock, 0, st>>>(ids, n, k, seg, deg, ctx->dev_err); ctx->launches++;
+  k_degrees<<<ge, 256, 0, st>>>(mutual, revcnt, n, deg); ctx->launches++;
   HDB_CHECK_LAUNCH();
   uint32_t err = ctx->take_dev_err();
   HDB_REQUIRE(!(err & DEVERR_ID_RANGE), HDB_ERR_ARG,
@@ -744,14 +811,7 @@ void build_enhanced_knng(Context *ctx, const int32_t *ids, const float *core, co
   }
   if (times) HDB_CUDA(cudaEventRecord(times->after_antihubs, st));
 
-  // 3. mutual flags and reverse counts
-  Buf<uint32_t> mutual(ctx, n);
-  Buf<int32_t> revcnt(ctx, n), nonmutual(ctx, n);
-  HDB_CUDA(cudaMemsetAsync(revcnt, 0, n * sizeof(int32_t), st));
-  k_mutual<<<gw, 32 * kWarpsPerBlock, 0, st>>>(ids, n, k, mutual, revcnt, nonmutual); ctx->launches++;
-  HDB_CHECK_LAUNCH();
-
-  // 4. row sizes -> nindex
+  // 3. row sizes -> nindex
   ensure_capacity(ctx, (void **)&ctx->g_nindex, &ctx->g_nindex_cap, (n + 1) * sizeof(int64_t));
   {
     Buf<int32_t> sizes(ctx, n);
@@ -759,7 +819,7 @@ void build_enhanced_knng(Context *ctx, const int32_t *ids, const float *core, co
     HDB_CHECK_LAUNCH();
     scan_exclusive_i32_i64(ctx, sizes, ctx->g_nindex, n, ctx->g_nindex + n);
   }
-  // 5. reverse entries (v, i) in i order, stable-sorted by v
+  // 4. reverse entries (v, i) in i order, stable-sorted by v
   Buf<int64_t> roff(ctx, n + 1);
   scan_exclusive_i32_i64(ctx, nonmutual, roff, n, roff.get() + n);
   int64_t hv[2];
@@ -778,7 +838,7 @@ void build_enhanced_knng(Context *ctx, const int32_t *ids, const float *core, co
   Buf<int64_t> rev_off(ctx, n + 1);
   scan_exclusive_i32_i64(ctx, revcnt, rev_off, n, nullptr);
 
-  // 6. fill rows + MRD weights
+  // 5. fill rows + MRD weights
   ensure_capacity(ctx, (void **)&ctx->g_nlist, &ctx->g_nlist_cap, (size_t)E * sizeof(int32_t));
   ensure_capacity(ctx, (void **)&ctx->g_eweight, &ctx->g_eweight_cap, (size_t)E * sizeof(float));
   k_fill<<<gw, 32 * kWarpsPerBlock, 0, st>>>(ids, core, ctx->g_nindex, revcnt, rev_off, rvals, n,
@@ -817,10 +877,10 @@ void build_core_sg(Context *ctx, const int32_t *ids, const float *dist, const fl
   const int ge = grid_for(ctx, n, 256);
   const int64_t m = n - 1;
 
-  Buf<int32_t> deg(ctx, n);
-  HDB_CUDA(cudaMemsetAsync(deg, 0, n * sizeof(int32_t), st));
-  k_degrees<<<gw, 32 * kWarpsPerBlock, 0, st>>>(ids, n, k, Segments{}, deg, ctx->dev_err); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  // mutual flags and reverse counts
+  Mutual mu(ctx, ids, n, k, Segments{});
+  const uint32_t *mutual = mu.mutual;
+  const int32_t *revcnt = mu.revcnt, *nonmutual = mu.nonmutual;
   // MST entries (validated with the ids)
   Buf<int32_t> mdeg(ctx, n);
   Buf<uint32_t> mkeys(ctx, 2 * m), mvals(ctx, 2 * m);
@@ -842,12 +902,7 @@ void build_core_sg(Context *ctx, const int32_t *ids, const float *dist, const fl
   ctx->launches++;
   HDB_CHECK_LAUNCH();
 
-  // mutual flags, reverse entries sorted by target (stable: ascending source)
-  Buf<uint32_t> mutual(ctx, n);
-  Buf<int32_t> revcnt(ctx, n), nonmutual(ctx, n);
-  HDB_CUDA(cudaMemsetAsync(revcnt, 0, n * sizeof(int32_t), st));
-  k_mutual<<<gw, 32 * kWarpsPerBlock, 0, st>>>(ids, n, k, mutual, revcnt, nonmutual); ctx->launches++;
-  HDB_CHECK_LAUNCH();
+  // reverse entries sorted by target (stable: ascending source)
   Buf<int64_t> roff(ctx, n + 1);
   scan_exclusive_i32_i64(ctx, nonmutual, roff, n, roff.get() + n);
   ensure_capacity(ctx, (void **)&ctx->sg_nindex, &ctx->sg_nindex_cap, (n + 1) * sizeof(int64_t));
