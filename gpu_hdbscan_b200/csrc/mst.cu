@@ -90,14 +90,20 @@ __global__ void k_first_rows(const float *__restrict__ first, int64_t stride, Se
 __global__ void k_count_canon(const int64_t *__restrict__ nindex, const int32_t *__restrict__ nlist,
                               int64_t n, int32_t *__restrict__ cnt, uint32_t *err) {
   const int lane = lane_id();
+  const int64_t stride = (int64_t)gridDim.x * kWarps;
   int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
-  for (; row < n; row += (int64_t)gridDim.x * kWarps) {
-    int64_t b = nindex[row], e = nindex[row + 1];
+  int64_t nb = row < n ? nindex[row] : 0, ne = row < n ? nindex[row + 1] : 0;
+  for (; row < n; row += stride) {
+    const int64_t b = nb, e = ne;
+    if (row + stride < n) {  // the next row's bounds, in flight meanwhile
+      nb = nindex[row + stride];
+      ne = nindex[row + stride + 1];
+    }
     int c = 0;
-    for (int64_t j = b + lane; j < e; j += 32) {
-      int32_t v = nlist[j];
-      if (v < 0 || v >= n) { atomicOr(err, DEVERR_ID_RANGE); continue; }
-      c += v > row;
+    for (int64_t j = b + lane; j < e; j += 64) {
+      const int32_t v = nlist[j], u = j + 32 < e ? nlist[j + 32] : 0;
+      if (v < 0 || v >= n || u < 0 || u >= n) { atomicOr(err, DEVERR_ID_RANGE); continue; }
+      c += (v > row) + (u > row);
     }
 #pragma unroll
     for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
@@ -112,24 +118,47 @@ __global__ void k_emit_canon(const int64_t *__restrict__ nindex, const int32_t *
                              int64_t n, const double *__restrict__ quant, Segments seg,
                              CEdge *__restrict__ el) {
   const int lane = lane_id();
+  const int64_t stride = (int64_t)gridDim.x * kWarps;
   int64_t row = (int64_t)blockIdx.x * kWarps + (threadIdx.x >> 5);
-  for (; row < n; row += (int64_t)gridDim.x * kWarps) {
-    int64_t b = nindex[row], e = nindex[row + 1];
-    int64_t p = off[row];
+  int64_t nb = 0, ne = 0, np = 0;
+  if (row < n) {
+    nb = nindex[row];
+    ne = nindex[row + 1];
+    np = off[row];
+  }
+  for (; row < n; row += stride) {
+    const int64_t b = nb, e = ne;
+    int64_t p = np;
+    if (row + stride < n) {  // the next row's bounds, in flight meanwhile
+      nb = nindex[row + stride];
+      ne = nindex[row + stride + 1];
+      np = off[row + stride];
+    }
     const double p10 = quant ? quant[seg.count > 0 ? seg.of_point(row) : 0] : 0.0;
-    for (int64_t j0 = b; j0 < e; j0 += 32) {
-      int64_t j = j0 + lane;
-      bool take = j < e && nlist[j] > row;
-      uint32_t m = __ballot_sync(0xffffffffu, take);
-      if (take) {
-        CEdge c;
-        c.a = (int32_t)row;
-        c.b = nlist[j];
-        c.key = quant ? quant_key(quantise(ew[j], p10), j)
-                      : ((uint64_t)weight_key(ew[j]) << 32) | (uint64_t)(uint32_t)j;
-        el[p + __popc(m & lanemask_lt())] = c;
+    for (int64_t j0 = b; j0 < e; j0 += 64) {
+      int32_t v[2];
+      float wt[2];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int64_t j = j0 + 32 * h + lane;
+        v[h] = j < e ? nlist[j] : -1;
+        wt[h] = j < e ? ew[j] : 0.0f;
       }
-      p += __popc(m);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int64_t j = j0 + 32 * h + lane;
+        const bool take = v[h] > row;
+        const uint32_t m = __ballot_sync(0xffffffffu, take);
+        if (take) {
+          CEdge c;
+          c.a = (int32_t)row;
+          c.b = v[h];
+          c.key = quant ? quant_key(quantise(wt[h], p10), j)
+                        : ((uint64_t)weight_key(wt[h]) << 32) | (uint64_t)(uint32_t)j;
+          el[p + __popc(m & lanemask_lt())] = c;
+        }
+        p += __popc(m);
+      }
     }
   }
 }
