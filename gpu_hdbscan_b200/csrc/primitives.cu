@@ -198,17 +198,34 @@ __global__ void __launch_bounds__(kSortThreads) radix_hist(const K *__restrict__
     counts[count_at<kTileMajor>(i, blockIdx.x, nblocks, kBins)] = hist[i];
 }
 
+// The lanes of the caller's digit d (<= mask, below kBins) among the lanes that are
+// ok: a ballot per bit.  A match_any takes a turn per distinct digit instead, some
+// 58 cycles of a unit that the SM's four partitions share, and bounded the stable
+// scatter (63 % of that unit's rate over the whole kernel): 2M x 32's reverse
+// entries, five passes, 862 -> 627 us; 10M x 12's lists, second passes, 25.7 -> 23.0
+// ms; one block's sort of 5,000 64-bit keys 66 -> 52 us.
+template <int kBins>
+__device__ __forceinline__ uint32_t digit_peers(uint32_t d, bool ok, uint32_t mask) {
+  uint32_t peers = __ballot_sync(0xffffffffu, ok);
+#pragma unroll
+  for (int b = 0; (1 << b) < kBins; b++) {
+    if (!((mask >> b) & 1u)) break;  // for the whole warp: a narrower digit
+    const bool one = (d >> b) & 1u;
+    const uint32_t with = __ballot_sync(0xffffffffu, one);
+    peers &= one ? with : ~with;
+  }
+  return peers;
+}
+
 // Scatter of one tile for one digit.  Keys are ranked, the tile is laid out in
 // digit order in shared memory, and each digit's run is then written by
 // consecutive threads to consecutive addresses.  Values of type V (u32 or u64)
 // move with their keys when kVals.  kStable keeps the input order within a digit:
-// the lanes of a digit find one another with match_any, which takes a turn per
-// distinct digit of the warp and bounds the kernel (63 % of that unit's rate over
-// the whole of it).  Without it the ranks are the arrivals at the digit's count,
-// and one count per digit does for the block, which leaves room for four blocks on
-// an SM: six lists of 100k x 12 in one pass of 9 bits 348 -> 245 us, the first pass
-// of six lists of 1M x 12 2.70 -> 2.36 ms.  (Masks in shared memory instead of
-// match_any are no faster: 2.7 -> 2.9 ms at 6 bits.)
+// the lanes of a digit find one another by ballots (digit_peers).  Without it the
+// ranks are the arrivals at the digit's count, and one count per digit does for the
+// block, which leaves room for four blocks on an SM: six lists of 100k x 12 in one
+// pass of 9 bits 348 -> 245 us, the first pass of six lists of 1M x 12 2.70 -> 2.36
+// ms.  (Masks in shared memory in place of a match are slower: 2.9 ms at 6 bits.)
 template <typename K, typename V, bool kVals, int kBins, int kItems, bool kTileMajor, bool kStable>
 __global__ void __launch_bounds__(kSortThreads, kStable ? 3 : 4) radix_scatter(
     const K *__restrict__ keys_in, const V *__restrict__ vals_in, K *__restrict__ keys_out,
@@ -248,8 +265,7 @@ __global__ void __launch_bounds__(kSortThreads, kStable ? 3 : 4) radix_scatter(
     if (!kStable) {
       if (ok) rank = atomicAdd(&whist[0][d], 1u);
     } else {
-      // past the end: a digit of its own per lane, outside [0, kBins)
-      const uint32_t peers = __match_any_sync(0xffffffffu, ok ? d : d + lane);
+      const uint32_t peers = digit_peers<kBins>(d, ok, mask);
       const int leader = __ffs(peers) - 1;
       if (ok) rank = whist[warp][d];
       __syncwarp();
@@ -474,9 +490,8 @@ void launch_scatter(cudaStream_t st, const K *kin, const V *vin, K *kout, V *vou
 // fewest passes of at most log2(kBins) bits over [begin_bit, end_bit), the bits
 // spread evenly over them (25 bits with 512 bins: 9 + 8 + 8).  Stable with kStable.
 // Without it the first pass leaves a digit's keys in any order and takes as many
-// bits as it can, the later ones, whose match_any is the cheaper the fewer digits
-// there are, the rest (1M x 12, 12 bits: 9 + 3 2.2 ms for the second passes, 6 + 6
-// 2.7).  dev_n: the count
+// bits as it can, the later ones, which take a ballot a bit, the rest (1M x 12, 12
+// bits: 9 + 3 2.2 ms for the second passes, 6 + 6 2.7 with a match).  dev_n: the count
 // on the device, n then being a bound.  base_out (optional): the last pass's
 // base, kBins + 1 values.
 template <typename K, typename V, int kBins, bool kStable = true>
@@ -542,7 +557,7 @@ bool radix_sort_pingpong(Context *ctx, K *keys, V *vals, K *ktmp, V *vtmp, int64
 
 // Up to kBlockSort pairs: every pass in one block and one launch, the pairs in
 // shared memory between passes; a digit that all keys share is skipped.  5,000
-// 64-bit keys: 55 us, where eight passes of three launches took 95 us and their
+// 64-bit keys: 52 us, where eight passes of three launches took 95 us and their
 // gaps.  Up to 1,024 pairs one item a thread.
 constexpr int kBlockSortThreads = 1024;
 constexpr int kBlockSort = 8 * kBlockSortThreads;
@@ -590,15 +605,15 @@ __global__ void __launch_bounds__(kBlockSortThreads)
 #pragma unroll
     for (int j = 0; j < kItems; j++) {
       const bool ok = base + 32 * j < n;
-      const uint32_t d = ok ? ((uint32_t)(k[j] >> shift) & mask) : 256u + lane;
-      const uint32_t peers = __match_any_sync(0xffffffffu, d);
+      const uint32_t d = (uint32_t)(k[j] >> shift) & mask;
+      const uint32_t peers = digit_peers<256>(d, ok, mask);
       const uint32_t below = __popc(peers & ((1u << lane) - 1u));
       uint32_t b = 0;
       if (ok) b = sh.whist[w][d];
       __syncwarp();
       if (ok && below == 0) sh.whist[w][d] = b + __popc(peers);
       __syncwarp();
-      dl[j] = d | ((b + below) << 16);
+      dl[j] = (ok ? d : 256u) | ((b + below) << 16);  // past the end: no digit
     }
     __syncthreads();
     if (tid < 256) {  // the digit's count per warp -> prefix; the digits' starts
