@@ -616,30 +616,25 @@ __global__ void __launch_bounds__(kGroupThreads)
 }
 
 // Start of every bucket in the list grouped by bucket (tgt >> shift), and the
-// end of the last one: bstart[0..buckets].  Four targets per thread.
+// end of the last one: bstart[0..buckets].  A warp searches one bucket's start, 32
+// probes a step.  Six lists of 10M x 12: 0.37 ms, 4.35 with the list read through;
+// 1M x 64: 0.07 and 0.39.
 __global__ void k_bucket_bounds(const uint32_t *__restrict__ tgt,
                                 const unsigned long long *__restrict__ count, int64_t cap, int shift,
                                 int64_t buckets, uint32_t *__restrict__ bstart) {
+  const int lane = lane_id();
   const int64_t c = min((int64_t)*count, cap);
-  const int64_t t0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-  if (c == 0) {
-    for (int64_t b = t0; b <= buckets; b += stride) bstart[b] = 0;
-    return;
-  }
-  for (int64_t i = 4 * t0; i < c; i += 4 * stride) {
-    const uint4 v = *reinterpret_cast<const uint4 *>(tgt + i);  // the buffer has room past its end
-    int64_t prev = i == 0 ? -1 : (int64_t)(tgt[i - 1] >> shift);
-    const uint32_t t[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      if (i + j >= c) break;
-      const int64_t b = min((int64_t)(t[j] >> shift), buckets);
-      for (int64_t q = prev + 1; q <= b; q++) bstart[q] = (uint32_t)(i + j);
-      prev = b > prev ? b : prev;
-      if (i + j == c - 1)
-        for (int64_t q = b + 1; q <= buckets; q++) bstart[q] = (uint32_t)c;
+  const int64_t stride = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t b = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); b <= buckets; b += stride) {
+    int64_t lo = 0, hi = c;  // the start lies in [lo, hi]
+    while (lo < hi) {
+      const int64_t step = (hi - lo + 31) / 32;
+      const int64_t p = lo + (lane + 1) * step - 1;
+      const bool less = p < hi && (int64_t)(tgt[p] >> shift) < b;
+      lo += __popc(__ballot_sync(0xffffffffu, less)) * step;
+      hi = min(hi, lo + step - 1);
     }
+    if (lane == 0) bstart[b] = (uint32_t)min(lo, c);
   }
 }
 
@@ -1765,7 +1760,7 @@ struct NndState {
     uint32_t *tgt = second ? list_tgt2 : list_tgt;
     uint64_t *key = second ? list_key2 : list_key, *out = second ? list_key : list_key2;
     if (bits - shift > 9) {  // several passes: the digit starts of the last one are not the buckets'
-      k_bucket_bounds<<<grid_for(ctx, ceil_div(cl.cap, 4), 256), 256, 0, ctx->stream>>>(
+      k_bucket_bounds<<<grid_for(ctx, buckets + 1, 8), 256, 0, ctx->stream>>>(
           tgt, counters.get() + 3, cl.cap, shift, buckets, bstart);
       ctx->launches++;
       HDB_CHECK_LAUNCH();
