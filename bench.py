@@ -474,8 +474,8 @@ def run_ours(args, w):
         S = w.sample_num
         launches = max(1, last["join_launches"])
         # algorithmic bytes of the local join (per launch): staged sample rows,
-        # the sample lists and counters, and each pushed candidate (inbox entry,
-        # counter atomic, k-th distance read)
+        # the sample lists and counters, and each pushed candidate (list entry
+        # and k-th distance read)
         if prec != g.HDB_PREC_FP32:
             tc = (w.d + 63) // 64 * 64 <= 256  # tensor-core tiles, else the mma.sync join
             jkernel = "k_join_tc" if tc else "k_join_bf16"

@@ -25,9 +25,7 @@
 //   warps 0..3  epilogue: tcgen05.ld of the accumulator (warp w reads TMEM
 //               lanes 32w..32w+31 = tile rows), row minima against the
 //               metadata slot, and the candidates appended to the
-//               target-sorted list of the merge (one reservation per warp and
-//               tile; the per-row inboxes of the SIMT joins would cost a
-//               returning atomic per candidate).
+//               list that is grouped by target before the merge.
 // Three rings, each with full / empty mbarriers: operand stages (one K block
 // of a tile each, held only from the gather to the end of its MMAs), metadata
 // slots (held until the epilogue is done with the tile) and two
@@ -691,9 +689,7 @@ __device__ void epilogue(const JoinArgs &a, Shared &sh, uint32_t tmem, int64_t n
     if (k1 < kNoKey) id1 = M.ids[64 * j + (k1 & 63)];
     __syncwarp();
     if (lane == 0) mbar_arrive(&sh.mempty[m]);
-    // candidates that can enter their target's list, appended to the list
-    // that is sorted by target before the next merge: one reservation per
-    // warp instead of a returning inbox atomic per candidate
+    // candidates that can enter their target's list
     const float d1 = key_dist(k1), d2 = key_dist(k2);
     const bool c1 = vrow && id1 >= 0 && d1 < wst;
     const bool c2 = !isnew && lane < nn && id2 >= 0 && d2 < wst2;

@@ -9,7 +9,7 @@ namespace hdb {
 struct JoinStats {
   double ms = 0.0;
   int64_t launches = 0, rows_gathered = 0, candidates = 0, pairs = 0;
-  int32_t config = 0;  // FP32 join tile slots per lane (1 or 2); 0: a 16-bit join
+  int32_t config = 0;  // FP32 join: the form set on the context, else 1; 0: a 16-bit join
 };
 
 // seg: independent instances in one run (each row's neighbours stay inside
@@ -18,8 +18,8 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
                hdb_nnd_element *G, int64_t *dropped_out, JoinStats *js = nullptr,
                const Segments &seg = Segments{});
 // Device bytes per point that nndescent holds at its peak: X in locality
-// order, the 16-bit rows, lists, samples, inboxes, the candidate list and its
-// sort buffers, the graph before it is mapped back.
+// order, the 16-bit rows, lists, samples, the candidate list and its second
+// buffer, the graph before it is mapped back.
 int64_t nndescent_bytes_per_point(int32_t d, const hdb_knn_params &p);
 // Merge of the kNN graphs of two point sets into the graph of their union
 // (hdb_knn_merge): FP32 join, old samples from the row's own set only.

@@ -109,7 +109,7 @@ typedef struct {
   int32_t num_clusters;
   int64_t condensed_size;
   int32_t mst_rounds;     /* Boruvka rounds */
-  int64_t knn_dropped;    /* NN-Descent candidates lost to a full inbox (normally 0) */
+  int64_t knn_dropped;    /* NN-Descent candidates that found the list full (normally 0) */
   float ms_knn, ms_graph, ms_mst, ms_tree, ms_total; /* device time per stage */
   /* NN-Descent local join, measured with CUDA events around each launch */
   float join_ms;                /* summed over the join launches */
