@@ -785,13 +785,14 @@ __device__ __forceinline__ void tile_sums(float (&acc)[4][kJCols], const float4 
 // new kernel, UpdateGraphForMerge :1582-1640) leaves out the new x new pairs: new
 // neighbours get their closest old one only.
 //
-// Bound by the FMA pipe and the shared-memory pipe together (about 65 % and 70 %
-// busy at 200k x 128, k = 32): a row-join's pairs give a lane some 30 sums, so 11
-// operand loads feed 28 pairs and no more.  Against tiles of 4 x 4, one or two per lane
+// Bound by instruction issue with the FMA and shared-memory pipes close behind (68,
+// 55 and 60 % at 200k x 128, k = 32): a row-join's pairs give a lane some 30 sums, so
+// 11 operand loads feed 28 pairs and no more.  Against tiles of 4 x 4, one or two per lane
 // (the last slot of them mostly empty), six iterations: 200k x 128, k = 16 8.4 ->
 // 6.0 ms, k = 32 12.9 -> 12.3; 1M x 64, k = 32 37.9 -> 37.3; 100k x 784 35.2 ->
 // 33.2.  Chunks of 16 dimensions with the next on its way are 4 % slower than
-// chunks of 32 without, five columns at three blocks per SM 10-20 %.
+// chunks of 32 without, five columns at three blocks per SM 10-20 %, twenty warps
+// per SM at 96 registers (sixteen at 128) 10-14 %.
 __global__ void __launch_bounds__(32 * kJoinWarps, 2)
     k_join(const float *__restrict__ X, int64_t n, int d, int S, const int32_t *__restrict__ newS,
            const int32_t *__restrict__ oldS, const int8_t *__restrict__ nf,
