@@ -988,13 +988,12 @@ __global__ void __launch_bounds__(32 * kJoinWarps, 2)
 // closest new row is a minimum over the warp.  With at most 16 (8) new rows the
 // warp's halves (quarters) take every second (fourth) staged row.  Bound by
 // instruction issue (76 % of the slots at 1M x 12, 1,670 warp instructions a
-// row-join, against 2,040 at 56 % in tiles).
+// row-join).
 //
-// Where the line lies, by the join time of six iterations, rows against the
-// better of the tile forms: 1M points, k = 32: d = 8 9.7 / 14.9 ms, 12 12.2 /
-// 17.4, 16 15.6 / 18.9, 24 19.2 / 22.2, 28 21.4 / 24.1, 32 27.4 / 24.9; 300k,
-// k = 16: d = 31 4.74 / 4.74 ms; 50k x 8, k = 16: 0.40 / 0.58; 1,500 x 8: 0.077 /
-// 0.083.
+// Where the line lies, by the join time of six iterations, rows against tiles: 1M
+// points, k = 32: d = 8 9.7 / 14.7 ms, 12 12.2 / 18.2, 16 15.5 / 20.0, 24 19.2 /
+// 22.6, 28 21.4 / 25.1, 32 27.4 / 24.9; 300k, k = 16: d = 31 4.74 / 4.65 ms; 50k x 8,
+// k = 16: 0.40 / 0.58; 1,500 x 8: 0.076 / 0.080.
 constexpr int kRowJoinMaxDim = 28;
 
 template <int kQ>
