@@ -391,38 +391,54 @@ __device__ __forceinline__ float lambda_of(float w) {
   return w > 0.0f ? __double2float_rn(__drcp_rn((double)w)) : 2147483648.0f;
 }
 
-// Hierarchy input check: children are earlier nodes and sizes add up, so
-// parent pointers always go to larger ids (every upward walk ends at the root).
-__global__ void k_validate_hier(TreeView t, uint32_t *err) {
-  const int64_t m = t.m;
-  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
-       r += (int64_t)gridDim.x * blockDim.x) {
-    hdb_linkage_node h = t.h[r];
-    int64_t lim = t.n + r;
-    bool ok = h.left_node >= 0 && h.left_node < lim && h.right_node >= 0 &&
-              h.right_node < lim && h.left_node != h.right_node;
-    if (ok) ok = (int64_t)t.sz(h.left_node) + t.sz(h.right_node) == h.node_size;
-    if (!ok) atomicOr(err, DEVERR_ID_RANGE);
-  }
-}
-
-// Per internal node: parent pointers, side, kind, visited flag, lambda.
+// Per internal node: parent pointers, side, kind, visited flag, lambda; and the
+// first half of the hierarchy's check: children are earlier nodes and sizes add up,
+// so parent pointers always go to larger ids (every upward walk ends at the root).
+// A node that fails writes nothing.
 __global__ void k_nodes(TreeView t, int32_t *__restrict__ par, int8_t *__restrict__ side,
                         int8_t *__restrict__ kind, int8_t *__restrict__ visited,
-                        float *__restrict__ lam) {
+                        float *__restrict__ lam, uint32_t *err) {
   const int64_t m = t.m;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
        r += (int64_t)gridDim.x * blockDim.x) {
-    hdb_linkage_node h = t.h[r];
-    int64_t x = t.n + r;
+    const hdb_linkage_node h = t.h[r];
+    const int64_t x = t.n + r;
+    bool ok = h.left_node >= 0 && h.left_node < x && h.right_node >= 0 && h.right_node < x &&
+              h.left_node != h.right_node;
+    int64_t ls = 0, rs = 0;
+    if (ok) {
+      ls = t.sz(h.left_node);
+      rs = t.sz(h.right_node);
+      ok = ls + rs == h.node_size;
+    }
+    if (!ok) {
+      atomicOr(err, DEVERR_ID_RANGE);
+      continue;
+    }
     par[h.left_node] = (int32_t)x;
     par[h.right_node] = (int32_t)x;
     side[h.left_node] = 0;
     side[h.right_node] = 1;
-    bool lb = t.sz(h.left_node) >= t.mpts, rb = t.sz(h.right_node) >= t.mpts;
+    const bool lb = ls >= t.mpts, rb = rs >= t.mpts;
     kind[r] = (lb && rb) ? KIND_SPLIT : (!lb && !rb) ? KIND_BOTHSMALL : lb ? KIND_LEFTBIG : KIND_RIGHTBIG;
     visited[r] = t.is_root(r) || h.node_size >= t.mpts;
     lam[r] = lambda_of(h.weight);
+  }
+}
+
+// The other half: no node has two parents (its pointer is one parent's, so it does
+// not point back to the other).  With that, the 2 m children are all the nodes but
+// the roots, which the kernels below rely on: every visited node has its parent's
+// chain or starts one, and every cluster has a node.
+__global__ void k_one_parent(TreeView t, const int32_t *__restrict__ par, uint32_t *err) {
+  const int64_t m = t.m;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const hdb_linkage_node h = t.h[r];
+    const int64_t x = t.n + r;
+    if (h.left_node < 0 || h.left_node >= x || h.right_node < 0 || h.right_node >= x) continue;
+    if (par[h.left_node] != (int32_t)x || par[h.right_node] != (int32_t)x)
+      atomicOr(err, DEVERR_ID_RANGE);
   }
 }
 
@@ -1259,12 +1275,11 @@ void condense_select(Context *ctx, const hdb_linkage_node *h, int64_t n, int32_t
   Buf<int8_t> side(ctx, total), kind(ctx, m), visited(ctx, m);
   Buf<float> lam(ctx, m);
   HDB_CUDA(cudaMemsetAsync(par, 0xff, total * sizeof(int32_t), st));
-  k_validate_hier<<<gm, 256, 0, st>>>(t, ctx->dev_err); ctx->launches++;
+  k_nodes<<<gm, 256, 0, st>>>(t, par, side, kind, visited, lam, ctx->dev_err); ctx->launches++;
+  k_one_parent<<<gm, 256, 0, st>>>(t, par, ctx->dev_err); ctx->launches++;
   HDB_CHECK_LAUNCH();
   HDB_REQUIRE(!(ctx->take_dev_err() & DEVERR_ID_RANGE), HDB_ERR_ARG,
               "condensed tree: hierarchy is not a valid single-linkage tree");
-  k_nodes<<<gm, 256, 0, st>>>(t, par, side, kind, visited, lam); ctx->launches++;
-  HDB_CHECK_LAUNCH();
 
   // chain heads by pointer jumping; the splits and the visited nodes counted
   Buf<int32_t> head(ctx, m), split(ctx, m), vis(ctx, m), changed(ctx, 64);
