@@ -114,7 +114,14 @@ inline int stage_floats(const float *X, int d) {
 __host__ __device__ constexpr int stage_pitch(int d, int kV) {
   return ((d < kStageCols ? d : kStageCols) / kV) | 1;
 }
-inline size_t stage_bytes(int d, int kV) { return (size_t)33 * stage_pitch(d, kV) * kV * 4; }
+__host__ __device__ constexpr size_t stage_bytes(int d, int kV) {
+  return (size_t)33 * stage_pitch(d, kV) * kV * 4;
+}
+// A launch needs no opt-in, which would be an attribute of the whole process.
+static_assert(kStageWarps * stage_bytes(kStageCols, 4) <= 48 * 1024 &&
+                  kStageWarps * stage_bytes(kStageCols, 2) <= 48 * 1024 &&
+                  kStageWarps * stage_bytes(kStageCols, 1) <= 48 * 1024,
+              "staged rows within the default shared memory");
 
 template <int kV>
 __device__ __forceinline__ float diffsum_staged(const float *__restrict__ X, int d, int64_t row,
@@ -1667,7 +1674,6 @@ void launch_staged(Context *ctx, Kernel by4, Kernel by2, Kernel by1, const float
   const Kernel fn = kV == 4 ? by4 : kV == 2 ? by2 : by1;
   const size_t smem = kStageWarps * stage_bytes(d, kV);
   const int resident = (int)std::min<size_t>(8, (size_t(220) << 10) / (smem + 1024));
-  HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   fn<<<grid_for(ctx, n, kStageWarps, 4 * resident), 32 * kStageWarps, smem, ctx->stream>>>(X, n, d, args...);
   ctx->launches++;
 }
@@ -1866,7 +1872,8 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
     smem_bf = JoinSmemBf16::bytes(dpad) * jw16;
     HDB_REQUIRE(smem_bf <= 227 * 1024, HDB_ERR_ARG, "NN-Descent 16-bit form: d too large for the join tile");
     const auto fn = fp16 ? k_join_bf16<true> : k_join_bf16<false>;
-    HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bf));
+    // the most that any call asks for: another thread's call may come between this and the launch
+    HDB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
     int resident = 0;  // a persistent grid, as of the other joins
     HDB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, fn, 32 * jw16, smem_bf));
     grid_bf = grid_for(ctx, n, jw16, std::max(1, resident));
