@@ -44,7 +44,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     _build/), then links libhdb_b200.so."""
     from concurrent.futures import ThreadPoolExecutor
     srcs = _sources()
-    headers = glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + [
+    headers = glob.glob(os.path.join(HERE, "csrc", "*.cuh")) + glob.glob(os.path.join(HERE, "csrc", "*.h")) + [
         os.path.join(ROOT, "include", "hdb", "hdb.h")]
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)

@@ -715,19 +715,22 @@ hdb_status run_batched(hdb_ctx *h, hdb_instance *insts, int32_t count, const hdb
     HDB_CUDA(cudaEventRecord(ctx->ev[0], ctx->stream));
     // consecutive instances of one d, as many points per batch as the free
     // device memory holds (at most 2^25): 70 % of what the driver has free
-    // plus the context's idle cached blocks, over the batch's bytes per point
-    // at its peak (NN-Descent, or the graph / MST stages when the kNN graphs
-    // are given), plus the batch's own arrays
+    // plus the context's idle cached blocks, for the batch's bytes at its
+    // peak (NN-Descent, or the graph / MST stages when the kNN graphs are
+    // given) and the batch's own arrays
     size_t free_b = 0, total_b = 0;
     HDB_CUDA(cudaMemGetInfo(&free_b, &total_b));
     const double avail = 0.7 * ((double)free_b + (double)ctx->cache_bytes);
     for (auto &g : groups) {
       const int64_t d = g.first;
       const int64_t graph_bpp = 40 * (int64_t)k;  // CSR + MST keys, E ~ 1.5 k per point
-      const int64_t nnd_bpp = from_knn ? 0 : nndescent_bytes_per_point(g.first, p.knn);
-      const int64_t bpp = std::max(nnd_bpp, graph_bpp) + 12 * (int64_t)k + 16 + 4 * d;
-      const int64_t cap = std::max<int64_t>(
-          int64_t(1) << 16, std::min<int64_t>(int64_t(1) << 25, (int64_t)(avail / (double)bpp)));
+      auto bytes = [&](int64_t points) {
+        const int64_t nnd = from_knn ? 0 : nndescent_bytes(ctx, points, g.first, p.knn);
+        return (double)(std::max(nnd, graph_bpp * points) + (12 * (int64_t)k + 16 + 4 * d) * points);
+      };
+      int64_t cap = int64_t(1) << 16;
+      for (int64_t step = int64_t(1) << 24; step > 0; step >>= 1)  // the bytes grow with the points
+        if (cap + step <= int64_t(1) << 25 && bytes(cap + step) <= avail) cap += step;
       // batches of about equal size, so that they reuse the same cached blocks
       // (unequal ones would free and allocate multi-GB blocks every call)
       int64_t group_points = 0;

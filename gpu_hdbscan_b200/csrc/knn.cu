@@ -1719,14 +1719,8 @@ struct NndState {
     of = Buf<int8_t>(ctx, n);
     best = Buf<unsigned long long>(ctx, n);
     counters = Buf<unsigned long long>(ctx, 5);
-    // room for an iteration's candidates (about 42 per row where it was
-    // counted; a row's join offers at most 96, so a small list cannot fill up)
-    // and for the tails of the warps' last chunks
-    const uint32_t chunk = list_chunk(40 * n / warps);
-    const int64_t cap =
-        std::min<int64_t>(std::max<int64_t>(64 * n, std::min<int64_t>(96 * n, int64_t(64) << 20)) +
-                              warps * chunk,
-                          (int64_t(1) << 32) - 1);
+    const uint32_t chunk = list_chunk(n, warps);
+    const int64_t cap = list_slots(n, warps);
     list_tgt = Buf<uint32_t>(ctx, cap);
     list_key = Buf<uint64_t>(ctx, cap);
     list_tgt2 = Buf<uint32_t>(ctx, cap);
@@ -1779,14 +1773,6 @@ struct NndState {
   }
 };
 
-// Warps of the joins that append to the list.
-int64_t fp32_join_warps(const Context *ctx, int64_t n) {
-  return (int64_t)kJoinWarps * grid_for(ctx, n, kJoinWarps, 4);
-}
-int64_t tc_join_warps(const Context *ctx, int64_t n) {
-  return 4 * std::min<int64_t>((n + 1) / 2, 2 * (int64_t)ctx->num_sms);
-}
-
 template <int kQ>
 void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
   const size_t smem = (size_t)kJoinWarps * (64 * kQ * 16 + 64 * 4);
@@ -1818,6 +1804,14 @@ void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const NndS
   ctx->launches++;
 }
 
+// Warps of the joins that append to the list.
+int64_t fp32_join_warps(const Context *ctx, int64_t n) {
+  return (int64_t)kJoinWarps * grid_for(ctx, n, kJoinWarps, 4);
+}
+int64_t tc_join_warps(const Context *ctx, int64_t n) {
+  return 4 * std::min<int64_t>((n + 1) / 2, 2 * (int64_t)ctx->num_sms);
+}
+
 struct EventPair {
   cudaEvent_t a = nullptr, b = nullptr;
   EventPair() {
@@ -1832,7 +1826,7 @@ struct EventPair {
 
 }  // namespace
 
-int64_t nndescent_bytes_per_point(int32_t d, const hdb_knn_params &p) {
+int64_t nndescent_bytes(const Context *ctx, int64_t n, int32_t d, const hdb_knn_params &p) {
   const int64_t k = p.k, S = p.sample_num;
   const bool half = p.precision == HDB_PREC_BF16 || p.precision == HDB_PREC_FP16;
   const bool tc = half && tc_dpad(d) <= kTcMaxDpad;
@@ -1840,9 +1834,12 @@ int64_t nndescent_bytes_per_point(int32_t d, const hdb_knn_params &p) {
   int64_t b = 4 * (int64_t)d;                    // X in locality order
   if (half) b += 2 * dpad + 4;                   // 16-bit rows + norms
   b += 8 * k + 4 + 16 * S + 30;                  // lists, worst, samples, counters
-  b += 2 * 12 * 64;                              // candidate list, both buffers
   b += 8 * k;                                    // graph in locality order
-  return b;
+  // the wide 16-bit join's grid depends on what fits on an SM; at most 64 warps do
+  const int64_t warps = tc     ? tc_join_warps(ctx, n)
+                        : half ? std::min<int64_t>((n + 3) & ~int64_t(3), 64 * (int64_t)ctx->num_sms)
+                               : fp32_join_warps(ctx, n);
+  return b * n + list_bytes(list_slots(n, warps));
 }
 
 void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn_params &p,

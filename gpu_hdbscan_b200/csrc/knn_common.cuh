@@ -2,6 +2,7 @@
 // (distance, id) keys and the candidate list that the joins append to.
 #pragma once
 #include "hdb_internal.cuh"
+#include "list_plan.h"
 
 namespace hdb {
 namespace knn {
@@ -36,17 +37,7 @@ struct CandList {
 
 // Space of the candidate list a warp writes into: [pos, end), taken from the
 // list `chunk` slots at a time with one atomic on the list's counter, so that
-// the warps of a join do not all queue on that one counter.  The tail that a
-// warp leaves unused in its last chunk is sorted along as sentinels, so the
-// chunk follows the work: about a quarter of what a warp will append, between
-// kListChunkMin (one append's most) and 768 slots.  (With 1,024 always, the
-// list of 1,500 rows held 1.5 M slots for some 50 k candidates.)
-constexpr uint32_t kListChunkMin = 96, kListChunkMax = 768;
-inline uint32_t list_chunk(int64_t candidates_per_warp) {
-  uint32_t c = kListChunkMin;
-  while (c < kListChunkMax && 8 * (int64_t)c <= candidates_per_warp) c *= 2;
-  return c;
-}
+// the warps of a join do not all queue on that one counter.
 struct ListCursor {
   unsigned long long pos = 0, end = 0;
 };

@@ -1,0 +1,38 @@
+// How large the joins' candidate list is, from the number of rows and of warps that
+// append to it: what is allocated (knn.cu) and what a batch is budgeted for
+// (capi.cu).  Host code without CUDA.
+#pragma once
+#include <algorithm>
+#include <cstdint>
+
+namespace hdb {
+namespace knn {
+
+// Slots that a warp takes from the list at a time.  The tail that it leaves unused in
+// its last chunk is sorted along as sentinels, so the chunk follows the work: about
+// a quarter of what a warp will append, between kListChunkMin (one append's most) and
+// 768 slots.  (With 1,024 always, the list of 1,500 rows held 1.5 M slots for some
+// 50 k candidates.)
+constexpr uint32_t kListChunkMin = 96, kListChunkMax = 768;
+inline uint32_t list_chunk(int64_t n, int64_t warps) {
+  const int64_t candidates_per_warp = 40 * n / warps;
+  uint32_t c = kListChunkMin;
+  while (c < kListChunkMax && 8 * (int64_t)c <= candidates_per_warp) c *= 2;
+  return c;
+}
+
+// Room for an iteration's candidates (about 42 per row where it was counted; a row's
+// join offers at most 96, so a small list cannot fill up) and for the tails of the
+// warps' last chunks.
+inline int64_t list_slots(int64_t n, int64_t warps) {
+  return std::min<int64_t>(std::max<int64_t>(64 * n, std::min<int64_t>(96 * n, int64_t(64) << 20)) +
+                               warps * list_chunk(n, warps),
+                           (int64_t(1) << 32) - 1);
+}
+
+// Bytes of a list: target and candidate, with the second buffer of the grouping, and the
+// grouping's digit counts and offsets (512 of each per 4,096 slots).
+inline int64_t list_bytes(int64_t slots) { return slots * (2 * 12 + 1); }
+
+}  // namespace knn
+}  // namespace hdb
