@@ -23,11 +23,12 @@ inline uint32_t list_chunk(int64_t n, int64_t warps) {
 
 // Room for an iteration's candidates (about 42 per row where it was counted; a row's
 // join offers at most 96, so a small list cannot fill up) and for the tails of the
-// warps' last chunks.
+// warps' last chunks.  Positions are 32-bit, and k_group_rows steps up to a block's
+// 512 threads past a bucket's end: the list stays 4,096 short of 2^32.
 inline int64_t list_slots(int64_t n, int64_t warps) {
   return std::min<int64_t>(std::max<int64_t>(64 * n, std::min<int64_t>(96 * n, int64_t(64) << 20)) +
                                warps * list_chunk(n, warps),
-                           (int64_t(1) << 32) - 1);
+                           (int64_t(1) << 32) - 4096);
 }
 
 // Bytes of a list: target and candidate, with the second buffer of the grouping, and the
