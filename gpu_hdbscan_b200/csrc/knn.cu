@@ -583,7 +583,6 @@ __global__ void k_finalize(int64_t n, int k, const int32_t *__restrict__ gid,
 // rows.  A bucket's part is some 50 KB, so its scattered 8-byte stores meet in
 // L2.  In place of a further pass of the radix sort and of the search for the
 // rows' bounds in the sorted targets.
-constexpr int kBucketRows = 256;    // most rows of a bucket
 constexpr int kGroupThreads = 512;
 __global__ void __launch_bounds__(kGroupThreads)
     k_group_rows(int64_t n, int shift, const uint32_t *__restrict__ tgt,
@@ -1676,17 +1675,6 @@ void launch_staged(Context *ctx, Kernel by4, Kernel by2, Kernel by1, const float
   const int resident = (int)std::min<size_t>(8, (size_t(220) << 10) / (smem + 1024));
   fn<<<grid_for(ctx, n, kStageWarps, 4 * resident), 32 * kStageWarps, smem, ctx->stream>>>(X, n, d, args...);
   ctx->launches++;
-}
-
-// Rows per bucket of the candidate list's grouping, 2^shift: the fewest (from
-// 8) whose buckets, and the one of the unused slots behind them, fit one digit
-// of the radix passes (9 bits), so that one pass and k_group_rows group the list,
-// as long as that is at most kBucketRows; beyond, 128 rows, and two passes up to
-// 2^25 rows.  (Sorting the list by row took two and three passes.)
-int bucket_shift(int64_t n) {
-  int shift = 3;
-  while (ceil_div(n, int64_t(1) << shift) >= 512) shift++;
-  return (1 << shift) <= kBucketRows ? shift : 7;
 }
 
 // Device state of one NN-Descent run over n rows: the graph lists, the

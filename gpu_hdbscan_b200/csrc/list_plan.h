@@ -35,5 +35,21 @@ inline int64_t list_slots(int64_t n, int64_t warps) {
 // grouping's digit counts and offsets (512 of each per 4,096 slots).
 inline int64_t list_bytes(int64_t slots) { return slots * (2 * 12 + 1); }
 
+constexpr int kBucketRows = 256;  // most rows of a bucket
+// Rows per bucket of the candidate list's grouping, 2^shift: the fewest (from
+// 8) whose buckets, and the one of the unused slots behind them, fit one digit
+// of the radix passes (9 bits), so that one pass and k_group_rows group the list,
+// as long as that is at most kBucketRows; beyond, 128 rows and two passes as long as
+// these hold the buckets (2^25 - 128 rows), and past that 256 rows, which two passes
+// hold up to 2^26 - 256 rows.  (NN-Descent of 2^25 x 4, k = 16: 624 ms with 128 rows
+// and a third pass of one bit, 594 with 256; of 200 rows fewer 578.  Sorting the
+// list by row took two and three passes.)
+inline int bucket_shift(int64_t n) {
+  int shift = 3;
+  while ((n - 1) >> shift >= 511) shift++;
+  if ((1 << shift) <= kBucketRows) return shift;
+  return (n - 1) >> 7 >= (1 << 18) - 1 ? 8 : 7;
+}
+
 }  // namespace knn
 }  // namespace hdb
