@@ -100,6 +100,10 @@ def profiled_traffic(kernel):
     return None
 
 
+# hdb_run_stats.join_config of an FP32 run -> the join kernel that ran
+FP32_JOIN = {1: "k_join_rows", 2: "k_join"}
+
+
 def fp32_issue_roofline(stats, d, clk):
     """The FP32 local join against its FP32 issue bound: each computed pair
     (join_pairs, counted live) costs d subtractions and d fused multiply-adds,
@@ -114,7 +118,7 @@ def fp32_issue_roofline(stats, d, clk):
     achieved = pairs * d * 3 / (ms / 1e3) / 1e12
     peak = sms * 128 * 2 * mhz * 1e6 / 1e12
     launches = max(1, stats.get("join_launches", 1))
-    return {"kernel": "k_join (FP32 local join)", "bound": "fp32_issue",
+    return {"kernel": FP32_JOIN[stats["join_config"]] + " (FP32 local join)", "bound": "fp32_issue",
             "achieved": round(achieved, 2), "peak": round(peak, 2), "unit": "TFLOP/s",
             "frac": round(achieved / peak, 4), "pairs_per_launch": round(pairs / launches),
             "sm_mhz": mhz, "form": stats.get("join_config")}
@@ -481,7 +485,7 @@ def run_ours(args, w):
             jkernel = "k_join_tc" if tc else "k_join_bf16"
             row_bytes = ((w.d + 63) // 64 * 64 if tc else (w.d + 15) // 16 * 16) * 2
         else:
-            jkernel, row_bytes = "k_join", w.d * 4
+            jkernel, row_bytes = FP32_JOIN[last["join_config"]], w.d * 4
         join_bytes = (last["join_rows_gathered"] * row_bytes
                       + launches * w.n * (2 * 2 * S * 4 + 2 * 4 + 2 * 1)
                       + last["join_candidates"] * (8 + 4 + 4)) / launches
@@ -526,7 +530,7 @@ def run_ours(args, w):
         if jkernel == "k_join_tc":
             line["tensor_roofline"] = tensor_roofline(w.n, w.d, last, measured_peaks()[1],
                                                       w.iterations)
-        elif jkernel == "k_join":
+        elif prec == g.HDB_PREC_FP32:
             line["issue_roofline"] = fp32_issue_roofline(last, w.d, clk)
         print(json.dumps(line), flush=True)
     ctx.close()
@@ -732,7 +736,7 @@ def run_ours_batch(args, bw):
             jkernel = "k_join_tc"
         else:
             row_bytes = {d: d * 4 for d in per_d}
-            jkernel = "k_join"
+            jkernel = FP32_JOIN[last["join_config"]]
         # gathered rows are not split by d in the stats: weight the row size by points
         mean_row = sum(row_bytes[d] * c for d, c in per_d.items()) / n_total
         join_bytes = (last["join_rows_gathered"] * mean_row

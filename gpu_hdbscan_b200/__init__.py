@@ -75,9 +75,8 @@ class Context:
         _lib.check(self.L.hdb_set_stream(self.h, C.c_void_p(self._stream)))
 
     def set_join_tiles(self, tiles: int):
-        """FP32 local join form: 1 or 2 for distance tiles at any number of
-        dimensions (both the same form), or 0 (the default): by rows up to 28
-        dimensions, in tiles beyond."""
+        """FP32 local join form: 1 by rows (up to 28 dimensions, in tiles beyond), 2 in
+        tiles at any number of dimensions, or 0 (the default): the faster one."""
         _lib.check(self.L.hdb_set_join_tiles(self.h, int(tiles)))
 
     def close(self):

@@ -111,8 +111,8 @@ constexpr size_t kPinnedErrOffset = 3072;
 struct Context {
   int device = 0;
   int num_sms = 148;
-  // FP32 local join: 0 = the form for the number of dimensions, 1 or 2 = in
-  // tiles at any (hdb_set_join_tiles)
+  // FP32 local join: 0 = the form for the number of dimensions, 1 = by rows where
+  // that goes, 2 = in tiles at any (hdb_set_join_tiles)
   int join_tiles = 0;
   cudaStream_t own_stream = nullptr;
   cudaStream_t stream = nullptr;

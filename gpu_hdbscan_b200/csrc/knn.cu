@@ -1771,10 +1771,13 @@ void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndS
   ctx->launches++;
 }
 
-// One FP32 local join over s's samples: by rows up to kRowJoinMaxDim dimensions
-// (unless the context forces tiles), else in tiles.
+// The FP32 join's form: 1 by rows, up to kRowJoinMaxDim dimensions and unless the
+// context forces tiles, else 2, in tiles.
+int fp32_join_form(const Context *ctx, int d) { return d <= kRowJoinMaxDim && ctx->join_tiles != 2 ? 1 : 2; }
+
+// One FP32 local join over s's samples.
 void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
-  if (d <= kRowJoinMaxDim && !ctx->join_tiles) {
+  if (fp32_join_form(ctx, d) == 1) {
     using Join = void (*)(Context *, const float *, int64_t, int, int, const NndState &, int);
     static const Join by_pieces[7] = {join_rows<1>, join_rows<2>, join_rows<3>, join_rows<4>,
                                       join_rows<5>, join_rows<6>, join_rows<7>};
@@ -1942,7 +1945,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
     HDB_CHECK_LAUNCH();
     if (use_tc) tc_join_prepare(ctx, Xb, n, dpad, fp16, dscale, &tj);
   }
-  if (js) js->config = bf16 ? 0 : std::max(1, ctx->join_tiles);
+  if (js) js->config = bf16 ? 0 : fp32_join_form(ctx, d);
   for (int it = 0; it < p.iterations; it++) {
     s.sample(ctx, it > 0, 0);
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it], st));

@@ -9,7 +9,7 @@ namespace hdb {
 struct JoinStats {
   double ms = 0.0;
   int64_t launches = 0, rows_gathered = 0, candidates = 0, pairs = 0;
-  int32_t config = 0;  // FP32 join: the form set on the context, else 1; 0: a 16-bit join
+  int32_t config = 0;  // FP32 join: 1 by rows, 2 in tiles; 0: a 16-bit join
 };
 
 // seg: independent instances in one run (each row's neighbours stay inside

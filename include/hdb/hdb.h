@@ -118,8 +118,8 @@ typedef struct {
   int64_t join_candidates;      /* candidates that passed the k-th distance filter */
   int64_t gpu_launches;         /* kernel launches issued by the call */
   int32_t mst_multiplier;       /* mst_gpu = 1: the weight scale exponent m (single runs) */
-  int32_t join_config;          /* FP32 local join: the form set by hdb_set_join_tiles (1 or
-                                   2), 1 where none is set; 0 for a 16-bit join */
+  int32_t join_config;          /* FP32 local join: the form that ran, 1 by rows, 2 in tiles
+                                   (of a batch the last group's); 0 for a 16-bit join */
   int64_t join_pairs;           /* FP32 local join: distance pairs computed, all launches
                                    (the reference's new x new and new x old pairs); 0 for a
                                    16-bit join */
@@ -136,11 +136,12 @@ HDB_API hdb_status hdb_destroy(hdb_ctx *ctx);
  * context's own stream. */
 HDB_API hdb_status hdb_set_stream(hdb_ctx *ctx, void *stream);
 /* FP32 local join form (no reference counterpart: the reference's join,
- * nndescent.cu:1487-1580, has one form).  0 (the default): up to 28 dimensions
- * a form without tiles, beyond tiles of 4 rows x 1 to 8 columns per lane, as many
- * columns as the row's samples need.  1 or 2: the tiles at any number of
- * dimensions (two numbers from when there were two sizes of tile: the same form).
- * Both forms give the same graph. */
+ * nndescent.cu:1487-1580, has one form).  1: by rows, without tiles, which goes up to
+ * 28 dimensions; tiles beyond.  2: in tiles of 4 rows x 1 to 8 columns per lane, as many
+ * columns as the row's samples need, at any number of dimensions.  0 (the default):
+ * the form that is the faster one at the number of dimensions, which is by rows
+ * wherever that goes.  From the same samples both give the same candidates; two
+ * runs differ in any form by the order in which reverse samples arrive. */
 HDB_API hdb_status hdb_set_join_tiles(hdb_ctx *ctx, int32_t tiles);
 
 /* gpuknn::NNDescent, gpuknn/nndescent.cuh:40-42 (nndescent.cu:2088-2199):
