@@ -787,7 +787,9 @@ struct Addends {
 // neither meets such a tie nor leaves the binade is a sum of integers, in any
 // order: every thread rounds its own addends.  A long chain leaves a binade some
 // twenty times and, once s is large, meets hardly any ties; those stretches
-// are added one by one.
+// are added one by one.  A sum in no such binade (0, infinite, not a number) is
+// kept by addends that leave it as it is: lambdas that equal the birth, or any
+// after an infinite one.
 template <typename T>
 struct Binade {
   double u, inv_u;  // powers of two
@@ -821,14 +823,32 @@ struct Binade {
   __device__ __forceinline__ T after(uint64_t steps) const { return (T)((double)(q + (int64_t)steps) * u); }
 };
 
+// An item's additions leave s as it is.
+template <typename T>
+__device__ __forceinline__ bool keeps(T s, const Addends<T> &ad) {
+  using B = FpBits<T>;
+  return s != s || (B::add(s, ad.y0) == s && B::add(s, ad.y1) == s);
+}
+
 // s after the m items that the warp's first m lanes hold, one by one.
 template <typename T>
-__device__ T add_serially(T s, const ChainItem &mine, float birth, int m) {
+__device__ __noinline__ T add_serially(T s, const ChainItem &mine, float birth, int m) {
   using B = FpBits<T>;
   const Addends<T> ad(mine, birth);
   const int lane = lane_id();
   const uint32_t split_mask = __ballot_sync(0xffffffffu, lane < m && mine.a < 0);
   const uint32_t rep_mask = __ballot_sync(0xffffffffu, lane < m && mine.a > 1);
+  if (rep_mask == 0) {  // unrolled: bound by the chain of additions
+#pragma unroll
+    for (int t = 0; t < 32; t++) {
+      const T y0 = __shfl_sync(0xffffffffu, ad.y0, t), y1 = __shfl_sync(0xffffffffu, ad.y1, t);
+      if (t < m) {
+        s = B::add(s, y0);
+        if ((split_mask >> t) & 1u) s = B::add(s, y1);
+      }
+    }
+    return s;
+  }
   for (int t = 0; t < m; t++) {
     const T y0 = __shfl_sync(0xffffffffu, ad.y0, t), y1 = __shfl_sync(0xffffffffu, ad.y1, t);
     const int32_t m0 = __shfl_sync(0xffffffffu, ad.m0, t);
@@ -846,7 +866,11 @@ __device__ __forceinline__ T add_warp(T s, const ChainItem &mine, float birth, i
   const Addends<T> ad(mine, birth);
   uint64_t steps = 0;
   double about = 0.0;
-  const bool fine = lane_id() >= m || (bin.ok && bin.take(ad.y0, ad.m0, steps, about) &&
+  if (!bin.ok) {  // for the whole warp
+    if (__all_sync(0xffffffffu, lane_id() >= m || keeps<T>(s, ad))) return s;
+    return add_serially<T>(s, mine, birth, m);
+  }
+  const bool fine = lane_id() >= m || (bin.take(ad.y0, ad.m0, steps, about) &&
                                        bin.take(ad.y1, 1, steps, about));
   if (__all_sync(0xffffffffu, fine)) {
 #pragma unroll
@@ -866,7 +890,9 @@ __device__ __forceinline__ T add_warp(T s, const ChainItem &mine, float birth, i
 // Both kernels stream 16 bytes an item and are bound by the latency of a step
 // (load, round, reduce); the sum one by one had a chain of 32 additions and 64
 // shuffles per 32 items instead.  10M x 12, 200 blobs, one chain holding most
-// of the points: 238 -> 6.1 ms; 20M x 128, 200 blobs: 52 ms before.
+// of the points: 238 -> 6.1 ms; 20M x 128, 200 blobs: 52 ms before.  Sums
+// that stay as they are (get_clusters, all of it): two chains of 1M whose lambdas
+// equal the birth 22.4 -> 0.8 ms, one of 2M with infinite ones 41.6 -> 1.0; 12M items, half of them ties, 337 -> 93.
 constexpr int kLongChain = 4096;
 template <bool kBoth>
 __global__ void k_stability(int64_t C, const int64_t *__restrict__ seg_start,
@@ -915,39 +941,49 @@ __device__ T add_block(T s, const ChainItem (&mine)[kLongItems], float birth, in
                        const ChainItem *__restrict__ items, LongStep<T> *sh, T *sh_s) {
   const int lane = lane_id(), w = threadIdx.x >> 5;
   const Binade<T> bin(s);
-  uint64_t steps = 0;
-  double about = 0.0;
-  bool fine = bin.ok;
+  if (bin.ok) {  // for the whole block
+    uint64_t steps = 0;
+    double about = 0.0;
+    bool fine = true;
 #pragma unroll
-  for (int j = 0; j < kLongItems; j++) {
-    if (base + j * kLongThreads + threadIdx.x >= e) continue;
-    const Addends<T> ad(mine[j], birth);
-    fine = fine && bin.take(ad.y0, ad.m0, steps, about) && bin.take(ad.y1, 1, steps, about);
-  }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    steps += __shfl_xor_sync(0xffffffffu, steps, o);
-    about += __shfl_xor_sync(0xffffffffu, about, o);
-  }
-  if (lane == 0) sh[w] = LongStep<T>{steps, about};
-  const bool all = __syncthreads_and(fine);
-  if (all) {
-    steps = sh[lane].steps;
-    about = sh[lane].about;
+    for (int j = 0; j < kLongItems; j++) {
+      if (base + j * kLongThreads + threadIdx.x >= e) continue;
+      const Addends<T> ad(mine[j], birth);
+      fine = fine && bin.take(ad.y0, ad.m0, steps, about) && bin.take(ad.y1, 1, steps, about);
+    }
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
       steps += __shfl_xor_sync(0xffffffffu, steps, o);
       about += __shfl_xor_sync(0xffffffffu, about, o);
     }
-    if (bin.stays(steps, about)) {  // the same in every thread
-      __syncthreads();  // sh is free again
-      return bin.after(steps);
+    if (lane == 0) sh[w] = LongStep<T>{steps, about};
+    const bool all = __syncthreads_and(fine);
+    if (all) {
+      steps = sh[lane].steps;
+      about = sh[lane].about;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) {
+        steps += __shfl_xor_sync(0xffffffffu, steps, o);
+        about += __shfl_xor_sync(0xffffffffu, about, o);
+      }
+      if (bin.stays(steps, about)) {  // the same in every thread
+        __syncthreads();  // sh is free again
+        return bin.after(steps);
+      }
     }
+  } else {
+    bool keep = true;
+#pragma unroll
+    for (int j = 0; j < kLongItems; j++)
+      if (base + j * kLongThreads + threadIdx.x < e) keep = keep && keeps<T>(s, Addends<T>(mine[j], birth));
+    if (__syncthreads_and(keep)) return s;
   }
   if (w == 0) {
     const int64_t end = min(e, base + kLongThreads * kLongItems);
+    ChainItem next = base + lane < end ? items[base + lane] : ChainItem{0.0f, 0, 0, 0};
     for (int64_t i = base; i < end; i += 32) {
-      const ChainItem it = i + lane < end ? items[i + lane] : ChainItem{0.0f, 0, 0, 0};
+      const ChainItem it = next;
+      if (i + 32 + lane < end) next = items[i + 32 + lane];
       s = add_warp<T>(s, it, birth, (int)min((int64_t)32, end - i));
     }
     if (lane == 0) *sh_s = s;
