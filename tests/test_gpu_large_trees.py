@@ -1,6 +1,5 @@
 """Trees above the sizes at which the work leaves one block's shared memory: linkage levels
-outside the blocks on both sides of the number of edges where the block's size changes, and
-more than 8,192 splits and clusters in the condensed tree."""
+outside the blocks of 2,048 ranks, and more than 8,192 splits and clusters in the condensed tree."""
 import numpy as np
 import pytest
 
@@ -20,12 +19,9 @@ def _random_tree(n, oracle, tied, seed):
 
 
 @pytest.mark.parametrize("tied", [False, True])
-@pytest.mark.parametrize("edges", ["most of 2048 a block", "fewest of 512", 700_001, 1 << 20])
+@pytest.mark.parametrize("edges", [2048, 2049, 4097, 303_104, 303_105, 700_001, 1 << 20])
 def test_linkage_tree(ctx, oracle, edges, tied):
     import torch
-    if isinstance(edges, str):
-        sms = torch.cuda.get_device_properties(0).multi_processor_count
-        edges = 2048 * sms + ("512" in edges)
     n = edges + 1
     mst = _random_tree(n, oracle, tied, edges)
     ref = oracle.linkage_tree(mst, n)
