@@ -171,6 +171,22 @@ class Context:
                                                   _ptr(ids), _ptr(counts), tiles, _ptr(out)))
         return out
 
+    def fp32_join_candidates(self, X, newS, oldS, counts, worst, cross_only=False):
+        """Candidates of one FP32 local join for explicit sample lists newS, oldS [m, 2 S] and
+        counts [m, 4]: (start [n + 1], key [start[n]]) (see hdb_fp32_join_candidates)."""
+        torch = self._torch
+        X = self._dev(X, torch.float32)
+        newS, oldS = self._dev(newS, torch.int32), self._dev(oldS, torch.int32)
+        counts = torch.as_tensor(counts).to("cpu", torch.int32).contiguous()
+        worst = self._dev(worst, torch.float32)
+        (n, d), (m, S2) = X.shape, newS.shape
+        start = torch.empty(n + 1, dtype=torch.int32, device=self.device)
+        key = torch.empty(96 * m, dtype=torch.int64, device=self.device)
+        _lib.check(self._call(self.L.hdb_fp32_join_candidates, _ptr(X), n, d, S2 // 2, m, _ptr(newS),
+                              _ptr(oldS), _ptr(counts), _ptr(worst), int(cross_only), _ptr(start),
+                              _ptr(key), len(key)))
+        return start, key[:int(start[n])]
+
     def build_CoreSG(self, ids, dist, X, mst) -> EnhancedGraph:
         """Core-SG (kNN graph + MST, Euclidean weights) of ids/dist [n, k], X and
         the sorted MST (MST_EDGE records, e.g. buildMST's output)."""

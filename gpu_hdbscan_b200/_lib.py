@@ -29,7 +29,7 @@ EXPORTS = ("hdb_version", "hdb_last_error", "hdb_create", "hdb_destroy", "hdb_se
            "hdb_sort_edges", "hdb_linkage_tree", "hdb_condense_select", "hdb_run",
            "hdb_run_with_graph", "hdb_run_knn", "hdb_sort_edges_noalloc", "hdb_bf16_distance_tiles",
            "hdb_core_sg", "hdb_run_batched", "hdb_run_knn_batched", "hdb_mst_quantised",
-           "hdb_knn_merge", "hdb_mst_ordered")
+           "hdb_knn_merge", "hdb_mst_ordered", "hdb_fp32_join_candidates")
 
 
 class HdbError(RuntimeError):
@@ -112,6 +112,8 @@ def load(path: str = LIB_PATH):
                                   C.POINTER(RunStats)]),
         "hdb_sort_edges_noalloc": (C.c_int, [_P, _I64, _P]),
         "hdb_bf16_distance_tiles": (C.c_int, [_P, _P, _I64, _I32, _P, _P, _I64, _P]),
+        "hdb_fp32_join_candidates": (C.c_int, [_P, _P, _I64, _I32, _I32, _I64, _P, _P, _P, _P, _I32, _P,
+                                               _P, _I64]),
         "hdb_core_sg": (C.c_int, [_P, _P, _P, _P, _I64, _I32, _I32, _P, C.POINTER(Graph)]),
         "hdb_run_batched": (C.c_int, [_P, C.POINTER(Instance), _I32, C.POINTER(Params),
                                       C.POINTER(RunStats)]),

@@ -94,6 +94,43 @@ HDB_API hdb_status hdb_fix_distances(hdb_ctx *h, const float *X, int64_t n, int3
   });
 }
 
+HDB_API hdb_status hdb_fp32_join_candidates(hdb_ctx *h, const float *X, int64_t n, int32_t d,
+                                            int32_t S, int64_t m, const int32_t *newS,
+                                            const int32_t *oldS, const int32_t *counts,
+                                            const float *worst, int32_t cross_only,
+                                            uint32_t *start, uint64_t *key, int64_t cap) {
+  return guard([&] {
+    Context *ctx = C(h);
+    require_ptr(X, "X");
+    require_ptr(newS, "newS");
+    require_ptr(oldS, "oldS");
+    require_ptr(counts, "counts");
+    require_ptr(worst, "worst");
+    require_ptr(start, "start");
+    require_ptr(key, "key");
+    HDB_REQUIRE(n >= 1 && n < (int64_t(1) << 31) - 1 && d >= 1 && d <= 4096 && S >= 1 && S <= 16,
+                HDB_ERR_ARG, "bad n, d or S");
+    HDB_REQUIRE(m >= 1 && m <= (int64_t(1) << 24) && cap >= 0 && cap <= (int64_t(1) << 30), HDB_ERR_ARG,
+                "bad list count or capacity");
+    // the lists are small: check them on the host before any device read
+    std::vector<int32_t> ids((size_t)m * 2 * S);
+    for (int old = 0; old < 2; old++) {
+      HDB_CUDA(cudaMemcpy(ids.data(), old ? oldS : newS, ids.size() * sizeof(int32_t),
+                          cudaMemcpyDeviceToHost));
+      for (int64_t j = 0; j < m; j++)
+        for (int rev = 0; rev < 2; rev++) {
+          const int32_t c = counts[4 * j + 2 * rev + old];
+          HDB_REQUIRE(c >= 0 && (rev || c <= S), HDB_ERR_ARG, "sample count outside [0, S]");
+          for (int t = 0; t < std::min(c, S); t++) {
+            const int32_t id = ids[(size_t)j * 2 * S + rev * S + t];
+            HDB_REQUIRE(id >= 0 && id < n, HDB_ERR_ARG, "sample id outside [0, n)");
+          }
+        }
+    }
+    fp32_join_candidates(ctx, X, n, d, S, m, newS, oldS, counts, worst, cross_only != 0, start, key, cap);
+  });
+}
+
 HDB_API hdb_status hdb_bf16_distance_tiles(hdb_ctx *h, const float *X, int64_t n, int32_t d,
                                            const int32_t *ids, const int32_t *counts,
                                            int64_t tiles, float *out) {

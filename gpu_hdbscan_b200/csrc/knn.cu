@@ -1677,68 +1677,31 @@ void launch_staged(Context *ctx, Kernel by4, Kernel by2, Kernel by1, const float
   ctx->launches++;
 }
 
-// Device state of one NN-Descent run over n rows: the graph lists, the
-// samples of an iteration and the join's candidate list (with the second
-// buffer of its grouping).  warps: the most warps that append to the list.
-struct NndState {
+// The candidate list of joins whose targets are n rows, with the second buffer of its
+// grouping.  chunk: what a warp takes of its slots at a time.
+struct Candidates {
   int64_t n;
-  int k, S, shift;
+  int shift;
   int64_t buckets;
-  Buf<int32_t> gid, newS, oldS, nrev, orev;
-  Buf<float> gdist, worst;
-  Buf<int8_t> nf, of;
   Buf<uint64_t> list_key, list_key2;
   Buf<unsigned long long> best, counters;
   Buf<uint32_t> list_tgt, list_tgt2, bstart, rstart;
   CandList cl;
   RowList rl;
 
-  NndState(Context *ctx, int64_t n, int k, int S, int64_t warps)
-      : n(n), k(k), S(S), shift(bucket_shift(n)), buckets(ceil_div(n, int64_t(1) << shift)) {
-    cudaStream_t st = ctx->stream;
-    gid = Buf<int32_t>(ctx, n * k);
-    gdist = Buf<float>(ctx, n * k);
-    worst = Buf<float>(ctx, n);
-    newS = Buf<int32_t>(ctx, n * 2 * S);
-    oldS = Buf<int32_t>(ctx, n * 2 * S);
-    nrev = Buf<int32_t>(ctx, n);
-    orev = Buf<int32_t>(ctx, n);
-    nf = Buf<int8_t>(ctx, n);
-    of = Buf<int8_t>(ctx, n);
+  Candidates(Context *ctx, int64_t n, int64_t slots, uint32_t chunk)
+      : n(n), shift(bucket_shift(n)), buckets(ceil_div(n, int64_t(1) << shift)) {
     best = Buf<unsigned long long>(ctx, n);
     counters = Buf<unsigned long long>(ctx, 5);
-    const uint32_t chunk = list_chunk(n, warps);
-    const int64_t cap = list_slots(n, warps);
-    list_tgt = Buf<uint32_t>(ctx, cap);
-    list_key = Buf<uint64_t>(ctx, cap);
-    list_tgt2 = Buf<uint32_t>(ctx, cap);
-    list_key2 = Buf<uint64_t>(ctx, cap);
+    list_tgt = Buf<uint32_t>(ctx, slots);
+    list_key = Buf<uint64_t>(ctx, slots);
+    list_tgt2 = Buf<uint32_t>(ctx, slots);
+    list_key2 = Buf<uint64_t>(ctx, slots);
     bstart = Buf<uint32_t>(ctx, std::max<int64_t>(513, buckets + 1));
     rstart = Buf<uint32_t>(ctx, n + 1);
-    cl = CandList{best, list_tgt, list_key, counters, cap, chunk, (uint32_t)(buckets << shift)};
-    HDB_CUDA(cudaMemsetAsync(nrev, 0, n * 4, st));
-    HDB_CUDA(cudaMemsetAsync(orev, 0, n * 4, st));
-    HDB_CUDA(cudaMemsetAsync(best, 0xff, n * 8, st));
-    clear_list(ctx);
-  }
-  void clear_list(Context *ctx) {
+    cl = CandList{best, list_tgt, list_key, counters, slots, chunk, (uint32_t)(buckets << shift)};
+    HDB_CUDA(cudaMemsetAsync(best, 0xff, n * 8, ctx->stream));
     HDB_CUDA(cudaMemsetAsync(counters, 0, 5 * sizeof(unsigned long long), ctx->stream));
-  }
-  SampleOut samples() const { return SampleOut{newS, oldS, nf, of, nrev, orev}; }
-
-  // the samples of an iteration; after the first, of the rows merged with the
-  // candidates of the join before
-  void sample(Context *ctx, bool merge, int64_t split) {
-    HDB_CUDA(cudaFuncSetAttribute(k_sample, cudaFuncAttributePreferredSharedMemoryCarveout, kSampleShare));
-    k_sample<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(
-        n, k, S, merge, gid, gdist, worst, rl, counters, samples(), split);
-    ctx->launches++;
-    HDB_CHECK_LAUNCH();
-  }
-  void finalize(Context *ctx, hdb_nnd_element *out) {
-    k_finalize<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(n, k, gid, gdist, rl, out);
-    ctx->launches++;
-    HDB_CHECK_LAUNCH();
   }
   // groups a join's candidates by row
   void group(Context *ctx) {
@@ -1761,13 +1724,58 @@ struct NndState {
   }
 };
 
+// Device state of one NN-Descent run over n rows: the graph lists, the
+// samples of an iteration and the join's candidates.  warps: the most warps that
+// append to their list.
+struct NndState {
+  int64_t n;
+  int k, S;
+  Buf<int32_t> gid, newS, oldS, nrev, orev;
+  Buf<float> gdist, worst;
+  Buf<int8_t> nf, of;
+  Candidates c;
+
+  NndState(Context *ctx, int64_t n, int k, int S, int64_t warps)
+      : n(n), k(k), S(S), c(ctx, n, list_slots(n, warps), list_chunk(n, warps)) {
+    cudaStream_t st = ctx->stream;
+    gid = Buf<int32_t>(ctx, n * k);
+    gdist = Buf<float>(ctx, n * k);
+    worst = Buf<float>(ctx, n);
+    newS = Buf<int32_t>(ctx, n * 2 * S);
+    oldS = Buf<int32_t>(ctx, n * 2 * S);
+    nrev = Buf<int32_t>(ctx, n);
+    orev = Buf<int32_t>(ctx, n);
+    nf = Buf<int8_t>(ctx, n);
+    of = Buf<int8_t>(ctx, n);
+    HDB_CUDA(cudaMemsetAsync(nrev, 0, n * 4, st));
+    HDB_CUDA(cudaMemsetAsync(orev, 0, n * 4, st));
+  }
+  SampleOut samples() const { return SampleOut{newS, oldS, nf, of, nrev, orev}; }
+
+  // the samples of an iteration; after the first, of the rows merged with the
+  // candidates of the join before
+  void sample(Context *ctx, bool merge, int64_t split) {
+    HDB_CUDA(cudaFuncSetAttribute(k_sample, cudaFuncAttributePreferredSharedMemoryCarveout, kSampleShare));
+    k_sample<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(
+        n, k, S, merge, gid, gdist, worst, c.rl, c.counters, samples(), split);
+    ctx->launches++;
+    HDB_CHECK_LAUNCH();
+  }
+  void finalize(Context *ctx, hdb_nnd_element *out) {
+    k_finalize<<<grid_for(ctx, n, 8, 16), 256, 0, ctx->stream>>>(n, k, gid, gdist, c.rl, out);
+    ctx->launches++;
+    HDB_CHECK_LAUNCH();
+  }
+};
+
 template <int kQ>
-void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
+void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const SampleOut &s, const float *worst,
+               const CandList &cl, int cross_only) {
   const size_t smem = (size_t)kJoinWarps * (64 * kQ * 16 + 64 * 4);
   HDB_CUDA(cudaFuncSetAttribute(k_join_rows<kQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = grid_for(ctx, n, kJoinWarps, kQ <= 4 ? 4 : 3);
   k_join_rows<kQ><<<grid, 32 * kJoinWarps, smem, ctx->stream>>>(
-      X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev, s.worst, s.cl, cross_only);
+      X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev, s.orev, worst, cl, cross_only);
   ctx->launches++;
 }
 
@@ -1775,13 +1783,15 @@ void join_rows(Context *ctx, const float *X, int64_t n, int d, int S, const NndS
 // context forces tiles, else 2, in tiles.
 int fp32_join_form(const Context *ctx, int d) { return d <= kRowJoinMaxDim && ctx->join_tiles != 2 ? 1 : 2; }
 
-// One FP32 local join over s's samples.
-void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const NndState &s, int cross_only) {
+// One FP32 local join over n rows' samples s.
+void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const SampleOut &s, const float *worst,
+               const CandList &cl, int cross_only) {
   if (fp32_join_form(ctx, d) == 1) {
-    using Join = void (*)(Context *, const float *, int64_t, int, int, const NndState &, int);
+    using Join = void (*)(Context *, const float *, int64_t, int, int, const SampleOut &, const float *,
+                          const CandList &, int);
     static const Join by_pieces[7] = {join_rows<1>, join_rows<2>, join_rows<3>, join_rows<4>,
                                       join_rows<5>, join_rows<6>, join_rows<7>};
-    by_pieces[(d + 3) / 4 - 1](ctx, X, n, d, S, s, cross_only);
+    by_pieces[(d + 3) / 4 - 1](ctx, X, n, d, S, s, worst, cl, cross_only);
     return;
   }
   // the blocks that fit on the GPU at once (a grid-stride loop over the rows):
@@ -1791,7 +1801,7 @@ void fp32_join(Context *ctx, const float *X, int64_t n, int d, int S, const NndS
   const size_t smem = kJoinWarps * JoinSmem::kBytes;
   HDB_CUDA(cudaFuncSetAttribute(k_join, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   k_join<<<grid, 32 * kJoinWarps, smem, ctx->stream>>>(X, n, d, S, s.newS, s.oldS, s.nf, s.of, s.nrev,
-                                                       s.orev, s.worst, s.cl, cross_only);
+                                                       s.orev, worst, cl, cross_only);
   ctx->launches++;
 }
 
@@ -1871,7 +1881,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
   int32_t *gid = s.gid, *newS = s.newS, *oldS = s.oldS, *nrev = s.nrev, *orev = s.orev;
   float *gdist = s.gdist, *worst = s.worst;
   int8_t *nf = s.nf, *of = s.of;
-  const CandList &cl = s.cl;
+  const CandList &cl = s.c.cl;
   std::vector<cudaEvent_t> jev;
   if (js) {
     jev.resize(2 * (size_t)p.iterations);
@@ -1959,14 +1969,14 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
         k_join_bf16<false><<<grid_bf, 32 * jw16, smem_bf, st>>>(Xb, nrm, n, dpad, S, dscale, newS,
                                                                 oldS, nf, of, nrev, orev, worst, cl);
       else
-        fp32_join(ctx, Xw, n, d, S, s, 0);
+        fp32_join(ctx, Xw, n, d, S, s.samples(), worst, cl, 0);
       if (bf16) ctx->launches++;
     }
     if (js) HDB_CUDA(cudaEventRecord(jev[2 * it + 1], st));
     HDB_CHECK_LAUNCH();
-    s.group(ctx);
+    s.c.group(ctx);
   }
-  if (p.iterations == 0) s.group(ctx);  // an empty list
+  if (p.iterations == 0) s.c.group(ctx);  // an empty list
   s.finalize(ctx, Gp);
   if (bf16) {
     launch_staged(ctx, k_rerank<4>, k_rerank<2>, k_rerank<1>, Xw, n, d, k, Gp.get());
@@ -1974,7 +1984,7 @@ void nndescent(Context *ctx, const float *X, int64_t n, int32_t d, const hdb_knn
   }
   k_loc_restore<<<grid_rows, 32 * wpb, 0, st>>>(Gp, order, n, k, G); ctx->launches++;
   HDB_CHECK_LAUNCH();
-  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.counters, 5 * sizeof(unsigned long long),
+  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.c.counters, 5 * sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
   ctx->sync();
   if (use_tc)
@@ -2033,16 +2043,49 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
   // UpdateGraphForMerge per iteration
   for (int it = 0; it < p.iterations; it++) {
     s.sample(ctx, it > 0, n1);
-    fp32_join(ctx, X, n, d, S, s, 1);
+    fp32_join(ctx, X, n, d, S, s.samples(), s.worst, s.c.cl, 1);
     HDB_CHECK_LAUNCH();
-    s.group(ctx);
+    s.c.group(ctx);
   }
-  if (p.iterations == 0) s.group(ctx);  // an empty list
+  if (p.iterations == 0) s.c.group(ctx);  // an empty list
   s.finalize(ctx, G);
-  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.counters, sizeof(unsigned long long),
+  HDB_CUDA(cudaMemcpyAsync(ctx->pinned, s.c.counters, sizeof(unsigned long long),
                            cudaMemcpyDeviceToHost, st));
   ctx->sync();
   if (dropped_out) *dropped_out = *static_cast<const int64_t *>(ctx->pinned);
+}
+
+void fp32_join_candidates(Context *ctx, const float *X, int64_t n, int32_t d, int32_t S, int64_t m,
+                          const int32_t *newS, const int32_t *oldS, const int32_t *counts,
+                          const float *worst, bool cross_only, uint32_t *start, uint64_t *key,
+                          int64_t cap) {
+  cudaStream_t st = ctx->stream;
+  std::vector<int8_t> hf(2 * (size_t)m);
+  std::vector<int32_t> hr(2 * (size_t)m);
+  for (int64_t j = 0; j < m; j++)
+    for (int old = 0; old < 2; old++) {
+      hf[old * m + j] = (int8_t)counts[4 * j + old];
+      hr[old * m + j] = counts[4 * j + 2 + old];
+    }
+  Buf<int8_t> fwd(ctx, 2 * m);
+  Buf<int32_t> rev(ctx, 2 * m);
+  HDB_CUDA(cudaMemcpyAsync(fwd, hf.data(), hf.size(), cudaMemcpyHostToDevice, st));
+  HDB_CUDA(cudaMemcpyAsync(rev, hr.data(), hr.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
+  // two chunks that follow one another in a warp hold more than one chunk's candidates
+  const int64_t slots = 2 * cap + fp32_join_warps(ctx, m) * kListChunkMin;
+  Candidates c(ctx, n, slots, kListChunkMin);
+  const SampleOut lists{const_cast<int32_t *>(newS), const_cast<int32_t *>(oldS), fwd.get(), fwd.get() + m,
+                        rev.get(), rev.get() + m};
+  fp32_join(ctx, X, m, d, S, lists, worst, c.cl, cross_only);
+  HDB_CHECK_LAUNCH();
+  c.group(ctx);
+  unsigned long long *h = static_cast<unsigned long long *>(ctx->pinned);
+  HDB_CUDA(cudaMemcpyAsync(h, c.counters, 5 * sizeof(*h), cudaMemcpyDeviceToHost, st));
+  ctx->sync();
+  HDB_REQUIRE(h[0] == 0 && (int64_t)h[2] <= cap, HDB_ERR_ARG, "more candidates than key holds");
+  HDB_CUDA(cudaMemcpyAsync(start, c.rstart, (n + 1) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st));
+  HDB_CUDA(cudaMemcpyAsync(key, c.rl.key, h[2] * sizeof(uint64_t), cudaMemcpyDeviceToDevice, st));
+  ctx->sync();
 }
 
 void bf16_distance_tiles(Context *ctx, const float *X, int64_t n, int32_t d, const int32_t *ids,

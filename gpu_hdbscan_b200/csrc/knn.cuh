@@ -29,6 +29,12 @@ void knn_merge(Context *ctx, const float *X1, int64_t n1, const hdb_nnd_element 
 // BF16 tensor-core distances for explicit slot lists (hdb_bf16_distance_tiles).
 void bf16_distance_tiles(Context *ctx, const float *X, int64_t n, int32_t d, const int32_t *ids,
                          const int32_t *counts, int64_t tiles, float *out);
+// The candidates of one FP32 join for given sample lists (counts: host memory),
+// grouped by the row they are offered to (hdb_fp32_join_candidates).
+void fp32_join_candidates(Context *ctx, const float *X, int64_t n, int32_t d, int32_t S, int64_t m,
+                          const int32_t *newS, const int32_t *oldS, const int32_t *counts,
+                          const float *worst, bool cross_only, uint32_t *start, uint64_t *key,
+                          int64_t cap);
 void knn_split(Context *ctx, const hdb_nnd_element *G, int64_t n, int32_t k, int32_t *ids,
                float *dist);
 void fix_distances(Context *ctx, const float *X, int64_t n, int32_t d, const int32_t *ids,

@@ -340,6 +340,25 @@ HDB_API hdb_status hdb_bf16_distance_tiles(hdb_ctx *ctx, const float *X, int64_t
                                            const int32_t *ids, const int32_t *counts,
                                            int64_t tiles, float *out);
 
+/* hdb_fp32_join_candidates -- a diagnostic with no counterpart in the
+ * reference: the candidates that one FP32 local join of hdb_nndescent (in the
+ * form set by hdb_set_join_tiles) offers for given sample lists instead of
+ * NN-Descent's, grouped by the row they are offered to.  List j of the m has its
+ * forward samples in slots 0..S-1 and its reverse ones in S..2S-1 of newS[j*2S..] and
+ * oldS[j*2S..], counts[4 j ..] = {new forward, old forward, new reverse, old reverse}
+ * of them (the forward counts at most S, of the reverse ones the first S count).
+ * Only candidates nearer than worst[row] are offered; cross_only != 0 leaves the new x
+ * new pairs out (the join of hdb_knn_merge).  Row r's candidates are
+ * key[start[r]..start[r+1]), in any order: the bits of the squared distance above
+ * the id.  X [n, d], worst [n], start [n + 1], key [cap] and the lists are device
+ * memory, counts [4 m] is host memory.  Counts and used ids are checked, and that the
+ * candidates fit in cap (HDB_ERR_ARG). */
+HDB_API hdb_status hdb_fp32_join_candidates(hdb_ctx *ctx, const float *X, int64_t n, int32_t d,
+                                            int32_t S, int64_t m, const int32_t *newS,
+                                            const int32_t *oldS, const int32_t *counts,
+                                            const float *worst, int32_t cross_only,
+                                            uint32_t *start, uint64_t *key, int64_t cap);
+
 /* hdb_sort_edges_noalloc -- no counterpart in the reference.  The same
  * stable ascending sort by weight as hdb_sort_edges, for callers that cannot
  * call cudaMalloc (a host framework that owns every device byte, or a device
