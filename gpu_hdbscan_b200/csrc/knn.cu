@@ -1813,18 +1813,6 @@ int64_t tc_join_warps(const Context *ctx, int64_t n) {
   return 4 * std::min<int64_t>((n + 1) / 2, 2 * (int64_t)ctx->num_sms);
 }
 
-struct EventPair {
-  cudaEvent_t a = nullptr, b = nullptr;
-  EventPair() {
-    HDB_CUDA(cudaEventCreate(&a));
-    HDB_CUDA(cudaEventCreate(&b));
-  }
-  ~EventPair() {
-    if (a) cudaEventDestroy(a);
-    if (b) cudaEventDestroy(b);
-  }
-};
-
 }  // namespace
 
 int64_t nndescent_bytes(const Context *ctx, int64_t n, int32_t d, const hdb_knn_params &p) {
