@@ -104,7 +104,7 @@ def profiled_traffic(kernel):
 FP32_JOIN = {1: "k_join_rows", 2: "k_join"}
 
 
-def fp32_issue_roofline(stats, d, clk):
+def fp32_issue_roofline(stats, d, clk, kernel):
     """The FP32 local join against its FP32 issue bound: each computed pair
     (join_pairs, counted live) costs d subtractions and d fused multiply-adds,
     3 FLOP per dimension; the bound is SMs x 128 FP32 lanes x 2 FLOP x the SM
@@ -118,7 +118,7 @@ def fp32_issue_roofline(stats, d, clk):
     achieved = pairs * d * 3 / (ms / 1e3) / 1e12
     peak = sms * 128 * 2 * mhz * 1e6 / 1e12
     launches = max(1, stats.get("join_launches", 1))
-    return {"kernel": FP32_JOIN[stats["join_config"]] + " (FP32 local join)", "bound": "fp32_issue",
+    return {"kernel": kernel + " (FP32 local join)", "bound": "fp32_issue",
             "achieved": round(achieved, 2), "peak": round(peak, 2), "unit": "TFLOP/s",
             "frac": round(achieved / peak, 4), "pairs_per_launch": round(pairs / launches),
             "sm_mhz": mhz, "form": stats.get("join_config")}
@@ -435,7 +435,8 @@ def run_ours(args, w):
                    "stage_ms": {s_: round(ostats[-1][f"ms_{s_}"], 3) for s_ in
                                 ("knn", "graph", "mst", "tree", "total")}}
         if other == g.HDB_PREC_FP32:
-            compare["issue_roofline"] = fp32_issue_roofline(ostats[-1], w.d, clk)
+            compare["issue_roofline"] = fp32_issue_roofline(ostats[-1], w.d, clk,
+                                                            FP32_JOIN[ostats[-1]["join_config"]])
     recall = {}
     if args.recall_queries > 0:
         qidx = torch.randperm(w.n, generator=torch.Generator().manual_seed(7))[:args.recall_queries]
@@ -531,7 +532,7 @@ def run_ours(args, w):
             line["tensor_roofline"] = tensor_roofline(w.n, w.d, last, measured_peaks()[1],
                                                       w.iterations)
         elif prec == g.HDB_PREC_FP32:
-            line["issue_roofline"] = fp32_issue_roofline(last, w.d, clk)
+            line["issue_roofline"] = fp32_issue_roofline(last, w.d, clk, jkernel)
         print(json.dumps(line), flush=True)
     ctx.close()
     if world > 1:
@@ -736,7 +737,8 @@ def run_ours_batch(args, bw):
             jkernel = "k_join_tc"
         else:
             row_bytes = {d: d * 4 for d in per_d}
-            jkernel = FP32_JOIN[last["join_config"]]
+            # the statistics name the form of one width only
+            jkernel = FP32_JOIN[last["join_config"]] if len(per_d) == 1 else " / ".join(FP32_JOIN.values())
         # gathered rows are not split by d in the stats: weight the row size by points
         mean_row = sum(row_bytes[d] * c for d, c in per_d.items()) / n_total
         join_bytes = (last["join_rows_gathered"] * mean_row
@@ -787,7 +789,7 @@ def run_ours_batch(args, bw):
         # tensor-core join when the batch has one d
         if prec == g.HDB_PREC_FP32:
             d_mean = sum(d * c for d, c in per_d.items()) / n_total
-            line["issue_roofline"] = fp32_issue_roofline(last, d_mean, clk)
+            line["issue_roofline"] = fp32_issue_roofline(last, d_mean, clk, jkernel)
         elif len(per_d) == 1:
             line["tensor_roofline"] = tensor_roofline(n_total, next(iter(per_d)), last,
                                                       measured_peaks()[1], bw.iterations)

@@ -993,7 +993,7 @@ __global__ void __launch_bounds__(32 * kJoinWarps, 2)
 // row's closest new and old rows are running minima of the lane, an old row's
 // closest new row is a minimum over the warp.  With at most 16 (8) new rows the
 // warp's halves (quarters) take every second (fourth) staged row.  Bound by
-// instruction issue (76 % of the slots at 1M x 12, 1,670 warp instructions a
+// instruction issue (76 % of the slots at 1M x 12, 1,715 warp instructions a
 // row-join).
 //
 // Where the line lies, by the join time of six iterations, rows against tiles: 1M
