@@ -103,7 +103,11 @@ __device__ __forceinline__ float2 neg_diff2(float2 b, float2 a) {
 // for a short row lets 32 warps run on an SM instead of 24.  64 dimensions, k_init
 // and k_rerank at 20M x 128 and at 200k x 128 in L2: 65.5 + 46.8 ms, 0.44 + 0.38;
 // 128: 67.3 + 48.1, 0.53 + 0.44 (half the warps); 32: 76.4 + 64.8, 0.46 + 0.40 (a row
-// comes from memory in four visits).
+// comes from memory in four visits).  Copies of single floats are bound by the
+// instructions around them: whole groups of 32 go a row after the other without
+// any index arithmetic, only the remainder is numbered through (k_init at 200k x 33, 65, 99, 201,
+// 257: 0.28, 0.41, 0.64, 1.34, 1.73 ms; all numbered through 0.39, 0.69, 0.96, 1.84, 2.31; with
+// loads through registers, 32 dimensions at a time, 0.36, 0.54, 0.89, 2.01, 2.61).
 constexpr int kStageCols = 64;
 constexpr int kStageWarps = 4;  // per block
 
@@ -141,21 +145,35 @@ __device__ __forceinline__ float diffsum_staged(const float *__restrict__ X, int
   float s = 0.0f;
   for (int c0 = 0; c0 < d; c0 += kStageCols) {
     const int w = min(d - c0, kStageCols) / kV;
+    // copies [first, w) of the m rows, numbered through: lane l takes l, l + 32, ...
+    auto numbered = [&](int first) {
+      const int n = w - first, dr = 32 / n, dq = 32 - dr * n;
+      int r = lane / n, q = lane - r * n;
+#pragma unroll 4
+      for (int i = 0; i < m * n; i += 32) {
+        const int32_t rid = __shfl_sync(0xffffffffu, id, r & 31);
+        if (r < m) copy(sm + (r * pitch + first + q) * kV, X + (int64_t)rid * d + c0 + (first + q) * kV);
+        r += dr;
+        q += dq;
+        if (q >= n) {
+          q -= n;
+          r++;
+        }
+      }
+    };
     __syncwarp();  // the rows before are no longer read
     for (int q = lane; q < w; q += 32) copy(own + q * kV, X + row * d + c0 + q * kV);
-    // the m rows' w copies each, numbered through: lane l takes l, l + 32, ...
-    const int dr = 32 / w, dq = 32 - dr * w;
-    int r = lane / w, q = lane - r * w;
-#pragma unroll 4
-    for (int i = 0; i < m * w; i += 32) {
-      const int32_t rid = __shfl_sync(0xffffffffu, id, r & 31);
-      if (r < m) copy(sm + (r * pitch + q) * kV, X + (int64_t)rid * d + c0 + q * kV);
-      r += dr;
-      q += dq;
-      if (q >= w) {
-        q -= w;
-        r++;
+    if (kV == 1 && w >= 32) {  // whole groups of 32 floats a row after the other
+#pragma unroll 8
+      for (int r = 0; r < m; r++) {
+        const float *src = X + (int64_t)__shfl_sync(0xffffffffu, id, r) * d + c0 + lane;
+        float *dst = sm + r * pitch + lane;
+        copy(dst, src);
+        if (w == 64) copy(dst + 32, src + 32);
       }
+      if (w & 31) numbered(32);
+    } else {
+      numbered(0);
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
     __syncwarp();  // every lane's copies have landed
