@@ -104,9 +104,11 @@ struct Buf {
 };
 
 // Pinned host staging area: bytes [0, kPinnedErrOffset) are free for callers,
-// the device error word is read back at kPinnedErrOffset.
+// the device error word is read back at kPinnedErrOffset, and a kernel of a short
+// call raises the flag at kPinnedFlagOffset itself.
 constexpr size_t kPinnedBytes = 4096;
 constexpr size_t kPinnedErrOffset = 3072;
+constexpr size_t kPinnedFlagOffset = 3136;
 
 struct Context {
   int device = 0;
