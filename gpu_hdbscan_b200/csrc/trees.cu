@@ -724,7 +724,8 @@ __device__ T add_repeated(T s, T v, int64_t cnt) {
     const T s1 = B::add(s, v);
     cnt--;
     const int e0 = B::exp_field(s), e1 = B::exp_field(s1);
-    if (!(v < s) || e0 == 0 || e0 != e1) {  // large step, subnormal, or binade change
+    // large step, subnormal ulp (that of a sum below 2^-103, 2^-970 in FP64), or binade change
+    if (!(v < s) || e0 <= B::kMant || e0 != e1) {
       s = s1;
       last_inc = T(-1);
       continue;

@@ -83,6 +83,19 @@ def test_sums_that_stay(ctx, oracle, na, nb, kind):
     _compare(ctx, oracle, mst, n, 5)
 
 
+@pytest.mark.parametrize("scale", [30, 36, -30])
+def test_sums_at_the_ends_of_the_range(ctx, oracle, scale):
+    """Weights near 1e30 make sums whose ulp is subnormal, with many points at once."""
+    rng = np.random.default_rng(scale + 40)
+    n = 20_000
+    e = np.zeros(n - 1, oracle.MST_EDGE)
+    e["to_node"] = np.arange(1, n)
+    e["from_node"] = np.maximum(0, np.arange(n - 1) - rng.integers(0, 3, n - 1))
+    e["weight"] = 10.0 ** (scale + rng.uniform(-2, 2, n - 1))
+    for mpts in (2, 36):
+        _compare(ctx, oracle, oracle.sort_edges(e), n, mpts)
+
+
 def test_sums_that_stay_cost_no_more(ctx, oracle):
     """One by one they took over twenty times as long as sums that move."""
     import torch
